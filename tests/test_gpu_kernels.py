@@ -109,6 +109,26 @@ def test_gemm_f32(M, N, K_):
     assert float(outw[:, :2].abs().max()) == 0.0 and float(outw[:, 2 + N:].abs().max()) == 0.0
 
 
+@pytest.mark.parametrize("N,K_", [(1, 4), (63, 128), (65, 132), (200, 1020), (64, 1024), (130, 2052), (2048, 2048), (72, 8192), (66, 14336), (70, 131)])
+def test_gemm_f32_kernels_agree_to_the_bit(N, K_):
+    """One order of summation everywhere: rows of a batch on the kernel of few rows (every size it is built for, and a K cut
+    over one to eight blocks) and on tiles of 32, 64 and 128 rows (a block or eight to a tile) give the same bits."""
+    g = torch.Generator().manual_seed(N + K_)
+    a, w, bias = torch.randn(300, K_, generator=g).to(DEV), torch.randn(N, K_, generator=g).to(DEV), torch.randn(N, generator=g).to(DEV)
+    full = torch.full((301, N), 7.0, device=DEV)
+    K().gemm_f32(a, w, full[:300], bias)
+    want = a.double() @ w.double().T + bias.double()
+    # chains of 64, their sum, a segment's chunks, eight segments, the bias: one rounding of 2^-24 each, of at most the sum of magnitudes
+    roundings = 64 + 1 + -(-(-(-K_ // 128)) // 8) + 8 + 1
+    bound = roundings * 2.0 ** -24 * 1.01 * (a.double().abs() @ w.double().abs().T + bias.double().abs())
+    assert bool(((full[:300].double() - want).abs() <= bound).all()) and bool((full[300] == 7.0).all())
+    for M in (1, 2, 3, 4, 5, 8, 9, 16, 17, 32, 33, 64, 65, 100, 129, 257):
+        for lo in (0, 300 - M):
+            out = torch.full((M + 1, N), 7.0, device=DEV)
+            K().gemm_f32(a[lo:lo + M], w, out[:M], bias)
+            assert torch.equal(out[:M], full[lo:lo + M]) and bool((out[M] == 7.0).all()), (M, lo)
+
+
 def test_gemm_f32_shape_errors():
     from vllm_oxide_b200.errors import ShapeError
     with pytest.raises(ShapeError):

@@ -1,102 +1,416 @@
-// True 32-bit matrix product: C[M, N] = A[M, K] * W[N, K]^T, float32 in, float32 FMA, float32
-// out. No tensor cores, no TF32, no split over K: each output element is one chain of FMAs over
-// k = 0, 1, 2, ... in order, so its value does not depend on M, on the position of its row in
-// the batch, or on what else runs. This is the matrix product of the 32-bit engine; it exists
-// to show faults that bfloat16 rounding would hide, not to be fast.
+// True 32-bit matrix product: C[M, N] = A[M, K] * W[N, K]^T (+ bias), float32 in, float32 FMA, float32 out. No tensor cores, no
+// TF32. This is the matrix product of the 32-bit engine; it exists to show faults that bfloat16 rounding would hide.
 // Reference op: crates/engine/src/backend/cpu/mod.rs:199-229 (x * W^T with W [out, in]).
-// Launch: 64x64 output tile per block, 256 threads, 4x4 outputs per thread, K in slabs of 16
-// through shared memory. Bound: CUDA-core FMA throughput. Any M, N, K >= 1; edges are guarded.
+//
+// The sum over k is the same in every kernel here, to the bit: K is cut into chunks of 128; a chunk is two chains of FMAs, over
+// its even and its odd k in order, each starting from zero, and their sum; (number of chunks / 8, rounded up) chunks make a
+// segment, whose chunks are added in order; the segments are added in order. An element therefore does not depend on M, on
+// its row's place in the batch, on which kernel computes it or over how many blocks K is shared. (One chain over all of K
+// rounds more often: relative error against 64 bits on normal values 8.1e-7 and 1.6e-6 at K = 2,048 and 8,192, here 1.6e-7 and 1.7e-7.)
+//
+// Two kernels:
+//  * few rows (M <= 16, decode steps): bound by reading W once, 5.9 TB/s at M = 1 and 2.7 TB/s at M = 16 on 128,256 x 2,048, 3.4 and
+//    2.0 TB/s on 16,384 x 2,048 (64 x 64 tiles, which served every M before: 1.06 and 0.6 TB/s; 0.1 TB/s on 2,048 x 8,192, now 2.6). A thread has one or two weight rows and a chunk, all rows of A
+//    in its registers' sums; weights arrive by cp.async into a ring per warp, so that no barrier of the block stands in the stream.
+//  * tiles (everything else): bound by the FMA units. 8 x 8 outputs a thread from shared memory: 42 to 44 TFLOP/s on 16,384 x 2,048
+//    at M = 1,250 and 2,048 (33 and 34 before), 33 TFLOP/s on 2,048 x 8,192 at M = 128 (6).
+// Both multiply and add pairs of k in one instruction (fma.rn.f32x2, each half rounded as fmaf rounds it): single FMAs
+// reach half the rate on this GPU (a tile kernel of 8 x 8 outputs a thread: 37 TFLOP/s with fmaf).
 #include "common.cuh"
+#include <cooperative_groups.h>
 VOB_PDL_SWITCH(gemm_f32)
 
-#define TM 64
-#define TN 64
-#define TK 16
+namespace cg = cooperative_groups;
 
-__global__ void __launch_bounds__(256)
-gemm_f32_kernel(const float* __restrict__ A, long long lda, const float* __restrict__ W, long long ldw,
-                float* __restrict__ C, long long ldc, int M, int N, int K, const float* __restrict__ bias) {
+namespace {
+
+constexpr int CHUNK = 128;
+
+// 16 bytes from global to shared memory, of which `bytes` are read and the rest is zero.
+__device__ __forceinline__ void cp_async16(void* dst, const void* src, int bytes) {
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"((uint32_t)__cvta_generic_to_shared(dst)), "l"(src), "r"(bytes) : "memory");
+}
+__device__ __forceinline__ void cp_async4(void* dst, const void* src, int bytes) {
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;" ::"r"((uint32_t)__cvta_generic_to_shared(dst)), "l"(src), "r"(bytes) : "memory");
+}
+__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
+template <int N> __device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory"); }
+
+// (d0, d1) += (a0, a1) * (b0, b1): two float32 FMAs, each rounded as fmaf rounds it, in one instruction.
+__device__ __forceinline__ void fma2(unsigned long long& d, unsigned long long a, unsigned long long b) {
+    asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(d) : "l"(a), "l"(b));
+}
+__device__ __forceinline__ float sum2(unsigned long long d) {
+    float lo, hi;
+    asm("mov.b64 {%0, %1}, %2;" : "=f"(lo), "=f"(hi) : "l"(d));
+    return lo + hi;
+}
+
+__device__ __forceinline__ void cluster_arrive() { asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory"); }
+__device__ __forceinline__ void cluster_wait() { asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory"); }
+
+// Chunks of a segment.
+__host__ __device__ constexpr int seg_chunks(int nc) { return (nc + 7) / 8; }
+
+// ------------------------------------------------------------------------------------------------ few rows
+// A block takes 64 weight rows and `q` chunks of K, four chunks at a time: a warp has one of the four and 32 of the rows (a lane
+// one row, RN = 1, 8 warps) or all 64 (a lane two, RN = 2, 4 warps: from 5 rows of A on, where reading A from shared memory is
+// what costs). A cluster of `c` blocks shares a row's K; each block leaves the sums of its chunks in its shared memory and the
+// cluster adds them up, each block a part of the outputs. (Clusters that stay and take one set of 64 rows after another, the
+// ring running on over them, are slower: 291 against 214 us at M = 1, 128,256 x 2,048. Their blocks meet twice a set.)
+constexpr int FEW_N = 64, FEW_K = 32;                 // weight rows of a block, k of a ring stage
+
+constexpr int few_rows_a_lane(int mb) { return mb <= 4 ? 1 : 2; }
+// three blocks an SM (two from three rows of A on) for the usual four chunks a block
+__host__ __device__ constexpr int few_blocks(int mb) { return mb <= 2 ? 3 : 2; }
+constexpr int few_stages(int mb) { return mb == 4 ? 3 : 2; }
+
+template <int MB, int RN, int NS>
+__global__ void __launch_bounds__(256 / RN, few_blocks(MB))
+gemm_f32_few_kernel(const float* __restrict__ A, long long lda, const float* __restrict__ W, long long ldw, float* __restrict__ C,
+                    long long ldc, int M, int N, int K, const float* __restrict__ bias, int nc, int q, int c) {
+    constexpr int THREADS = 256 / RN, STAGE = 32 * RN * FEW_K;        // floats of a warp's stage: its rows, 16-byte pieces at (piece ^ row & 7)
+    extern __shared__ __align__(16) float smem[];
+    float* ring = smem;                               // [8 / RN warps][NS][STAGE]
+    float* xs = ring + 8 / RN * NS * STAGE;           // [MB][4 chunks * CHUNK]
+    float* part = xs + 4 * CHUNK * MB;                // [q][MB][FEW_N]
+    pdl_launch_dependents();
+    int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    int rank = blockIdx.x % c, n0 = (blockIdx.x / c) * FEW_N;
+    int half = RN == 1 ? warp & 1 : 0, slot = RN == 1 ? warp >> 1 : warp;
+    int first = rank * q, mine = min(q, nc - first);  // this block's chunks
+    float* wring = ring + warp * NS * STAGE;
+    int lrow = lane >> 3, lpiece = lane & 7;          // loads: 8 lanes take 128 bytes of a row
+    // the next stage to ask for: of the warp's chunk `lchunk` (slot, slot + 4, ...), its `lu`-th
+    int lchunk = slot, lu = 0, lput = 0;
+    auto load = [&]() {
+        if (lchunk < mine) {
+            int k = (first + lchunk) * CHUNK + lu * FEW_K + lpiece * 4;
+            float* dst = wring + lput * STAGE;
+#pragma unroll
+            for (int i = 0; i < 8 * RN; ++i) {
+                int r = i * 4 + lrow, n = n0 + half * 32 + r;
+                bool in = n < N && k < K;             // K is a multiple of 4
+                cp_async16(dst + r * FEW_K + ((lpiece ^ (r & 7)) << 2), in ? W + (size_t)n * ldw + k : W, in ? 16 : 0);
+            }
+            lput = lput + 1 == NS ? 0 : lput + 1;
+            if (++lu == CHUNK / FEW_K) { lu = 0; lchunk += 4; }
+        }
+        cp_async_commit();
+    };
+    // weights are written by no kernel: their first stages are asked for before the wait
+#pragma unroll
+    for (int s = 0; s < NS; ++s) load();
+    pdl_wait(11);
+
+    int get = 0, seg = seg_chunks(nc);
+    for (int t = 0; t * 4 < mine; ++t) {
+        if (t > 0) __syncthreads();                   // everyone has read the chunks in front
+        int kbase = (first + t * 4) * CHUNK;
+        // x of four chunks; what lies beyond K or M is zero
+        for (int i = threadIdx.x; i < CHUNK * MB; i += THREADS) {
+            int m = i / CHUNK, k4 = (i % CHUNK) * 4;  // 4 * CHUNK / 4 pieces of every row
+            float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
+            if (m < M && kbase + k4 < K) v = *reinterpret_cast<const float4*>(A + (size_t)m * lda + kbase + k4);
+            *reinterpret_cast<float4*>(xs + m * 4 * CHUNK + k4) = v;
+        }
+        __syncthreads();
+        if (t * 4 + slot < mine) {
+            unsigned long long acc[RN][MB];
+#pragma unroll
+            for (int r = 0; r < RN; ++r)
+#pragma unroll
+                for (int m = 0; m < MB; ++m) acc[r][m] = 0;
+            const float* xc = xs + slot * CHUNK;
+#pragma unroll 1
+            for (int u = 0; u < CHUNK / FEW_K; ++u) {
+                cp_async_wait<NS - 1>();
+                __syncwarp();
+                const float* row = wring + get * STAGE + lane * FEW_K;
+                const float* xk = xc + u * FEW_K;
+#pragma unroll
+                for (int p = 0; p < FEW_K / 4; ++p) {
+                    ulonglong2 w[RN];
+#pragma unroll
+                    for (int r = 0; r < RN; ++r) w[r] = *reinterpret_cast<const ulonglong2*>(row + r * 32 * FEW_K + ((p ^ (lane & 7)) << 2));
+#pragma unroll
+                    for (int m = 0; m < MB; ++m) {
+                        ulonglong2 x = *reinterpret_cast<const ulonglong2*>(xk + m * 4 * CHUNK + p * 4);
+#pragma unroll
+                        for (int r = 0; r < RN; ++r) { fma2(acc[r][m], w[r].x, x.x); fma2(acc[r][m], w[r].y, x.y); }
+                    }
+                }
+                get = get + 1 == NS ? 0 : get + 1;
+                __syncwarp();                     // the warp has read this stage
+                load();
+            }
+            float* dst = part + (size_t)(t * 4 + slot) * MB * FEW_N + half * 32 + lane;
+#pragma unroll
+            for (int r = 0; r < RN; ++r)
+#pragma unroll
+                for (int m = 0; m < MB; ++m) dst[m * FEW_N + r * 32] = sum2(acc[r][m]);
+        }
+    }
+    if (c > 1) { cluster_arrive(); cluster_wait(); }
+    else __syncthreads();
+    // this block's share of the outputs: the chunks' sums, segment by segment, from the blocks that hold them
+    int total = M * FEW_N, share = (total + c - 1) / c;
+    for (int e = rank * share + threadIdx.x; e < min(total, (rank + 1) * share); e += THREADS) {
+        int m = e / FEW_N, col = e % FEW_N, n = n0 + col;
+        if (n >= N) continue;
+        float sum = 0.f, run = 0.f;
+        int in_seg = 0;
+        bool begun = false;
+        for (int b = 0; b < c; ++b) {
+            const float* p = (c > 1 ? cg::this_cluster().map_shared_rank(part, b) : part) + m * FEW_N + col;
+            int have = min(q, nc - b * q);
+            for (int i0 = 0; i0 < have; i0 += 4) {            // q is a multiple of 4: four reads on their way at once
+                float v[4];
+#pragma unroll
+                for (int i = 0; i < 4; ++i) v[i] = i0 + i < have ? p[(size_t)(i0 + i) * MB * FEW_N] : 0.f;
+#pragma unroll
+                for (int i = 0; i < 4; ++i) {
+                    if (i0 + i >= have) break;
+                    run = in_seg == 0 ? v[i] : run + v[i];
+                    if (++in_seg == seg) { sum = begun ? sum + run : run; begun = true; in_seg = 0; }
+                }
+            }
+        }
+        if (in_seg) sum = begun ? sum + run : run;
+        C[(size_t)m * ldc + n] = bias ? sum + bias[n] : sum;
+    }
+    cp_async_wait<0>();
+    __syncwarp();
+    if (c > 1) { cluster_arrive(); cluster_wait(); }  // peers have read this block's sums
+}
+
+template <int MB>
+int launch_few(const float* A, long long lda, const float* W, long long ldw, float* C, long long ldc, int M, int N, int K,
+               const float* bias, int nc, int q, int c, cudaStream_t stream) {
+    constexpr int RN = few_rows_a_lane(MB), NS = few_stages(MB);
+    size_t smem = sizeof(float) * (size_t)(8 * NS * 32 * FEW_K + 4 * CHUNK * MB + min(q, nc) * MB * FEW_N);
+    if (smem > 200 * 1024) return VOB_ERR_UNSUPPORTED;
+    auto kernel = gemm_f32_few_kernel<MB, RN, NS>;
+    cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (e != cudaSuccess) return (int)e;
+    long long blocks = (long long)((N + FEW_N - 1) / FEW_N) * c;
+    if (blocks > 0x7fffffffLL) return VOB_ERR_UNSUPPORTED;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((unsigned)blocks);
+    cfg.blockDim = dim3(256 / RN);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = stream;
+    cudaLaunchAttribute attr[2];
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = c; attr[0].val.clusterDim.y = 1; attr[0].val.clusterDim.z = 1;
+    attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[1].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = g_vob_pdl ? 2 : 1;
+    e = cudaLaunchKernelEx(&cfg, kernel, A, lda, W, ldw, C, ldc, M, N, K, bias, nc, q, c);
+    return e != cudaSuccess ? (int)e : vob_launch_status();
+}
+
+// ------------------------------------------------------------------------------------------------ tiles
+// A block of 128 threads computes 16 * TR rows by 64 columns, a thread TR x 8 of them (rows tm + 16 i, columns tn + 8 j). K
+// comes in slabs of 16 through a ring of three stages, [row][k] as it lies in memory, rows 20 floats apart: the 16-byte reads
+// of different rows that a warp makes at once fall into different banks. The sums of the chunks so far wait in shared
+// memory: the segment's, and (c == 1) the finished segments'. Or a cluster of c = 8 blocks shares K, a segment each, and
+// adds the segments' sums: eight times the blocks, for few tiles or a last wave that would be nearly empty.
+constexpr int TN = 64, TK = 16, TLD = TK + 4, TSTAGES = 3;
+__host__ __device__ constexpr int tile_blocks(int tr) { return tr == 8 ? 2 : tr == 4 ? 3 : 4; }   // resident on an SM
+
+template <int TR, bool VEC>
+__global__ void __launch_bounds__(128, tile_blocks(TR))
+gemm_f32_tile_kernel(const float* __restrict__ A, long long lda, const float* __restrict__ W, long long ldw, float* __restrict__ C,
+                     long long ldc, int M, int N, int K, const float* __restrict__ bias, int seg, int c, int mtiles) {
+    constexpr int TM = 16 * TR, QUADS = TR * 2;
+    extern __shared__ __align__(16) float smem[];
+    float* stage = smem;                                        // [TSTAGES][(TM + TN)][TLD]
+    float4* sums = reinterpret_cast<float4*>(smem + TSTAGES * (TM + TN) * TLD);    // [c == 1 ? 2 : 1][QUADS][128]
     pdl_launch_dependents();
     pdl_wait(11);
-    __shared__ float As[TK][TM + 4];
-    __shared__ float Ws[TK][TN + 4];
-    int tid = threadIdx.x;
-    int m0 = blockIdx.y * TM, n0 = blockIdx.x * TN;
-    int tx = tid & 15, ty = tid >> 4;          // outputs: rows ty*4.., cols tx*4..
-    int lr = tid >> 2, lk = (tid & 3) * 4;     // loads: row lr of the tile, k offset lk..lk+3
-    float acc[4][4];
+    int tid = threadIdx.x, lane = tid & 31;
+    int tn = (lane & 3) | ((lane >> 4) << 2), tm = ((tid >> 5) << 2) | ((lane >> 2) & 3);
+    int rank = blockIdx.x % c, tile = blockIdx.x / c;
+    int m0 = (tile % mtiles) * TM, n0 = (tile / mtiles) * TN;
+    int kb = min(K, rank * seg * CHUNK), ke = c > 1 ? min(K, kb + seg * CHUNK) : K;
+    int slabs = (ke - kb + TK - 1) / TK;
+    auto load = [&](int s) {
+        if (s < slabs) {
+            float* st = stage + (s % TSTAGES) * (TM + TN) * TLD;
+            int k = kb + s * TK + (tid & 3) * 4;
 #pragma unroll
-    for (int i = 0; i < 4; ++i)
-#pragma unroll
-        for (int j = 0; j < 4; ++j) acc[i][j] = 0.f;
-    bool vecA = ((lda & 3) == 0) && ((((uintptr_t)A) & 15) == 0);
-    bool vecW = ((ldw & 3) == 0) && ((((uintptr_t)W) & 15) == 0);
-    for (int k0 = 0; k0 < K; k0 += TK) {
-        {
-            int gm = m0 + lr, gk = k0 + lk;
-            float v[4] = {0.f, 0.f, 0.f, 0.f};
-            if (gm < M) {
-                const float* p = A + (size_t)gm * lda + gk;
-                if (vecA && gk + 3 < K) {
-                    float4 f = *reinterpret_cast<const float4*>(p);
-                    v[0] = f.x; v[1] = f.y; v[2] = f.z; v[3] = f.w;
+            for (int i = 0; i < (TM + TN) / 32; ++i) {
+                int r = i * 32 + (tid >> 2);
+                bool isA = i < TM / 32;
+                int g = isA ? m0 + r : n0 + r - TM;
+                const float* p = isA ? A + (size_t)g * lda : W + (size_t)g * ldw;
+                bool row = g < (isA ? M : N);
+                float* d = st + r * TLD + (tid & 3) * 4;
+                if constexpr (VEC) {                                      // K is a multiple of 4
+                    bool in = row && k < ke;
+                    cp_async16(d, in ? p + k : A, in ? 16 : 0);
                 } else {
 #pragma unroll
-                    for (int i = 0; i < 4; ++i) if (gk + i < K) v[i] = p[i];
+                    for (int x = 0; x < 4; ++x) {
+                        bool in = row && k + x < ke;
+                        cp_async4(d + x, in ? p + k + x : A, in ? 4 : 0);
+                    }
                 }
             }
-#pragma unroll
-            for (int i = 0; i < 4; ++i) As[lk + i][lr] = v[i];
         }
-        {
-            int gn = n0 + lr, gk = k0 + lk;
-            float v[4] = {0.f, 0.f, 0.f, 0.f};
-            if (gn < N) {
-                const float* p = W + (size_t)gn * ldw + gk;
-                if (vecW && gk + 3 < K) {
-                    float4 f = *reinterpret_cast<const float4*>(p);
-                    v[0] = f.x; v[1] = f.y; v[2] = f.z; v[3] = f.w;
-                } else {
+        cp_async_commit();
+    };
 #pragma unroll
-                    for (int i = 0; i < 4; ++i) if (gk + i < K) v[i] = p[i];
-                }
+    for (int s = 0; s < TSTAGES - 1; ++s) load(s);
+    unsigned long long acc[TR][8];                              // even and odd k
+#pragma unroll
+    for (int i = 0; i < TR; ++i)
+#pragma unroll
+        for (int j = 0; j < 8; ++j) acc[i][j] = 0;
+    int chunk = 0;                                              // of the segment
+    int at = 0;
+    for (int s = 0; s < slabs; ++s) {
+        cp_async_wait<TSTAGES - 2>();
+        __syncthreads();                                        // slab s is here, and slab s - 1 has been read by all
+        load(s + TSTAGES - 1);
+        const float* as = stage + at * (TM + TN) * TLD + tm * TLD;
+        const float* bs = stage + at * (TM + TN) * TLD + (TM + tn) * TLD;
+#pragma unroll
+        for (int k = 0; k < TK; k += 4) {
+            ulonglong2 b[8];
+#pragma unroll
+            for (int j = 0; j < 8; ++j) b[j] = *reinterpret_cast<const ulonglong2*>(bs + j * 8 * TLD + k);
+#pragma unroll
+            for (int i = 0; i < TR; ++i) {
+                ulonglong2 a = *reinterpret_cast<const ulonglong2*>(as + i * 16 * TLD + k);
+#pragma unroll
+                for (int j = 0; j < 8; ++j) fma2(acc[i][j], a.x, b[j].x);
+#pragma unroll
+                for (int j = 0; j < 8; ++j) fma2(acc[i][j], a.y, b[j].y);
             }
-#pragma unroll
-            for (int i = 0; i < 4; ++i) Ws[lk + i][lr] = v[i];
         }
-        __syncthreads();
+        at = at + 1 == TSTAGES ? 0 : at + 1;
+        bool last = s == slabs - 1;
+        if ((s & (CHUNK / TK - 1)) == CHUNK / TK - 1 || last) {                 // the chunk ends
+            bool seg_ends = chunk == seg - 1 || last, first_seg = s < seg * (CHUNK / TK);
+            float4* d = sums + tid;
 #pragma unroll
-        for (int kk = 0; kk < TK; ++kk) {
-            float a[4], b[4];
+            for (int e = 0; e < QUADS; ++e) {
+                const unsigned long long* x = &acc[e >> 1][(e & 1) * 4];
+                float4 v = make_float4(sum2(x[0]), sum2(x[1]), sum2(x[2]), sum2(x[3]));
+                if (chunk > 0) {
+                    float4 o = d[e * 128];
+                    v.x = o.x + v.x; v.y = o.y + v.y; v.z = o.z + v.z; v.w = o.w + v.w;
+                }
+                if (c > 1 || !seg_ends) d[e * 128] = v;
+                else {
+                    if (!first_seg) {
+                        float4 o = d[(QUADS + e) * 128];
+                        v.x = o.x + v.x; v.y = o.y + v.y; v.z = o.z + v.z; v.w = o.w + v.w;
+                    }
+                    d[(QUADS + e) * 128] = v;
+                }
 #pragma unroll
-            for (int i = 0; i < 4; ++i) a[i] = As[kk][ty * 4 + i];
-#pragma unroll
-            for (int j = 0; j < 4; ++j) b[j] = Ws[kk][tx * 4 + j];
-#pragma unroll
-            for (int i = 0; i < 4; ++i)
-#pragma unroll
-                for (int j = 0; j < 4; ++j) acc[i][j] = fmaf(a[i], b[j], acc[i][j]);
+                for (int j = 0; j < 4; ++j) acc[e >> 1][(e & 1) * 4 + j] = 0;
+            }
+            chunk = seg_ends ? 0 : chunk + 1;
         }
-        __syncthreads();
     }
+    cp_async_wait<0>();
+    auto put = [&](int e, float4 v) {                           // quad e of this thread
+        int m = m0 + tm + 16 * (e >> 1), n = n0 + tn + 32 * (e & 1);
+        if (m >= M) return;
+        float o[4] = {v.x, v.y, v.z, v.w};
 #pragma unroll
-    for (int i = 0; i < 4; ++i) {
-        int gm = m0 + ty * 4 + i;
-        if (gm >= M) continue;
+        for (int j = 0; j < 4; ++j)
+            if (n + 8 * j < N) C[(size_t)m * ldc + n + 8 * j] = bias ? o[j] + bias[n + 8 * j] : o[j];
+    };
+    if (c == 1) {                                               // a thread's own sums: no barrier
 #pragma unroll
-        for (int j = 0; j < 4; ++j) {
-            int gn = n0 + tx * 4 + j;
-            if (gn < N) C[(size_t)gm * ldc + gn] = bias ? acc[i][j] + bias[gn] : acc[i][j];
-        }
+        for (int e = 0; e < QUADS; ++e) put(e, sums[(QUADS + e) * 128 + tid]);
+        return;
     }
+    cluster_arrive();
+    cluster_wait();
+    int have = (K + seg * CHUNK - 1) / (seg * CHUNK);           // segments that are not empty
+    for (int e = rank; e < QUADS; e += c) {
+        float4 o[8];
+#pragma unroll
+        for (int b = 0; b < 8; ++b)
+            if (b < have) o[b] = cg::this_cluster().map_shared_rank(sums, b)[e * 128 + tid];
+        float4 v = o[0];
+#pragma unroll
+        for (int b = 1; b < 8; ++b)
+            if (b < have) { v.x += o[b].x; v.y += o[b].y; v.z += o[b].z; v.w += o[b].w; }
+        put(e, v);
+    }
+    cluster_arrive();
+    cluster_wait();                                             // peers have read this block's sums
 }
+
+template <int TR>
+int launch_tile(const float* A, long long lda, const float* W, long long ldw, float* C, long long ldc, int M, int N, int K,
+                const float* bias, int nc, int c, int vec, cudaStream_t stream) {
+    int mtiles = (M + 16 * TR - 1) / (16 * TR);
+    long long blocks = (long long)mtiles * ((N + TN - 1) / TN) * c;
+    if (blocks > 0x7fffffffLL) return VOB_ERR_UNSUPPORTED;
+    auto kernel = vec ? gemm_f32_tile_kernel<TR, true> : gemm_f32_tile_kernel<TR, false>;
+    size_t smem = sizeof(float) * (size_t)(TSTAGES * (16 * TR + TN) * TLD + (c == 1 ? 2 : 1) * TR * 8 * 128);
+    cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (e != cudaSuccess) return (int)e;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((unsigned)blocks);
+    cfg.blockDim = dim3(128);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = stream;
+    cudaLaunchAttribute attr[2];
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = c; attr[0].val.clusterDim.y = 1; attr[0].val.clusterDim.z = 1;
+    attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[1].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = g_vob_pdl ? 2 : 1;
+    e = cudaLaunchKernelEx(&cfg, kernel, A, lda, W, ldw, C, ldc, M, N, K, bias, seg_chunks(nc), c, mtiles);
+    return e != cudaSuccess ? (int)e : vob_launch_status();
+}
+
+}  // namespace
 
 // `bias` (N entries, may be null) is added to every row after the sum over k.
 VOB_EXPORT int vob_gemm_f32(const float* A, long long lda, const float* W, long long ldw, float* C,
                             long long ldc, int M, int N, int K, const float* bias, cudaStream_t stream) {
     if (M <= 0 || N <= 0) return 0;
     if (K <= 0 || lda < K || ldw < K || ldc < N) return VOB_ERR_BAD_ARG;
-    dim3 grid((N + TN - 1) / TN, (M + TM - 1) / TM);
-    if (grid.y > 65535) return VOB_ERR_UNSUPPORTED;
-    return vob_launch(gemm_f32_kernel, grid, dim3(256), 0, stream, A, lda, W, ldw, C, ldc, M, N, K, bias);
+    if ((M + 63) / 64 > 65535) return VOB_ERR_UNSUPPORTED;
+    int nc = (K + CHUNK - 1) / CHUNK;
+    int vec = K % 4 == 0 && lda % 4 == 0 && ldw % 4 == 0 && ((uintptr_t)A & 15) == 0 && ((uintptr_t)W & 15) == 0;
+    // 16 rows: what a lane's registers hold. On 16,384 x 2,048 the kernel of few rows takes 69 us there and the tiles take 96 at 17 (a
+    // tile is 32 rows at least); on 2,048 x 8,192, where a block has its SM to itself, 67 and 58.
+    if (vec && M <= 16) {
+        int q = ((nc + 7) / 8 + 3) / 4 * 4, c = (nc + q - 1) / q;
+        int e = M == 1   ? launch_few<1>(A, lda, W, ldw, C, ldc, M, N, K, bias, nc, q, c, stream)
+                : M == 2 ? launch_few<2>(A, lda, W, ldw, C, ldc, M, N, K, bias, nc, q, c, stream)
+                : M <= 4 ? launch_few<4>(A, lda, W, ldw, C, ldc, M, N, K, bias, nc, q, c, stream)
+                : M <= 8 ? launch_few<8>(A, lda, W, ldw, C, ldc, M, N, K, bias, nc, q, c, stream)
+                         : launch_few<16>(A, lda, W, ldw, C, ldc, M, N, K, bias, nc, q, c, stream);
+        if (e != VOB_ERR_UNSUPPORTED) return e;       // a K whose sums find no room in shared memory: tiles
+    }
+    // Tiles of 128, 64 or 32 rows, a block or eight to a tile: the one whose waves of blocks cost least. A wave's cost is its
+    // rows times its resident blocks; smaller tiles read more from shared memory per FMA (measured at 2,048 x 2,048 and
+    // 16,384 x 2,048: 1.15 and 1.5 times the time per row), a shared K is added up over the cluster.
+    int best_tr = 8, best_c = 1;
+    double best = 1e300;
+    for (int tr = 2; tr <= 8; tr *= 2)
+        for (int c = 1; c <= 8; c += 7) {
+            if (c > 1 && nc < 8) continue;
+            double slots = 148.0 * tile_blocks(tr), blocks = (double)((M + 16 * tr - 1) / (16 * tr)) * ((N + TN - 1) / TN) * c;
+            double waves = (double)(long long)((blocks + slots - 1) / slots);
+            double cost = waves * tile_blocks(tr) * tr * (tr == 8 ? 1.0 : tr == 4 ? 1.15 : 1.5) / c * (c > 1 ? 1.1 : 1.0);
+            if (cost < best) { best = cost; best_tr = tr; best_c = c; }
+        }
+    if (best_tr == 8) return launch_tile<8>(A, lda, W, ldw, C, ldc, M, N, K, bias, nc, best_c, vec, stream);
+    if (best_tr == 4) return launch_tile<4>(A, lda, W, ldw, C, ldc, M, N, K, bias, nc, best_c, vec, stream);
+    return launch_tile<2>(A, lda, W, ldw, C, ldc, M, N, K, bias, nc, best_c, vec, stream);
 }
