@@ -287,6 +287,29 @@ def test_steps_replayed_from_graphs_give_the_same_tokens(tmp_path_factory, dtype
     assert llm.runner.manager.num_free_pages(0) == llm.runner.manager.num_pages(0)
 
 
+@pytest.mark.parametrize("dtype", ["float32", "bfloat16"])
+def test_captured_logits_beside_replayed_and_run_ahead_steps(tmp_path_factory, dtype):
+    """Logits wanted at some generated positions (the first, some in the middle, the last; one request wants none): only the
+    steps that pick those tokens keep their logits, the others are replayed and run ahead, and what comes back is the plain
+    implementation's. Called three times on one engine: launched one by one, recorded, replayed."""
+    name = "B" if dtype == "float32" else "D"
+    cfg, _, page = TINY[name]
+    d = make_model_dir(tmp_path_factory.getbasetemp(), name)
+    pc, pt = plain.load_model(d)
+    prompts = [random_tokens(n, cfg.vocab_size, 80 + n) for n in (21, 5, 33)]
+    wanted = [(0, 11), (), (3, 4, 8)]
+    params = [sp(max_new_tokens=12, stop_token_ids=(), capture_logits=w) for w in wanted]
+    llm = llm_for(d, dtype, page)
+    tol = TOL[torch.float32 if dtype == "float32" else torch.bfloat16]
+    for _ in range(3):
+        for p, o, w in zip(prompts, llm.generate(prompts, params), wanted):
+            assert sorted(o.logits) == list(w) and len(o.token_ids) == 12
+            for i in w:
+                assert max_rel_diff(o.logits[i], plain.forward(pc, pt, p + o.token_ids[:i])[-1]) <= tol
+    assert llm.stats["ahead_steps"] > 0 and llm.runner.step_graph_replays > 0
+    assert {key[3] for key in llm.runner._graphs} == {False, True}
+
+
 def test_tight_pool_and_replayed_steps_change_no_token_in_f32():
     """Forty requests of 5 to 700 tokens, greedy and with temperature, once with room for all and
     steps launched one by one, once with a pool so tight that requests are preempted and

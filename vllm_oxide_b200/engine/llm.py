@@ -74,7 +74,9 @@ class LLM:
         self._logit_buf = None
         self._inflight = None            # a decode step launched but not read yet: (plan, ids, parity, event)
         self._late: List[RequestOutput] = []
-        self._capturing = 0              # live requests that want logits (they are never run ahead of)
+        # live request -> the generated positions whose logits it still wants. Only the step that picks such a
+        # token keeps its logits; every other step of the request runs as if it wanted none.
+        self._wanted: Dict[int, set] = {}
         self.run_ahead = bool(e.run_ahead) and bool(e.cuda_graphs)
         self.stats = {"steps": 0, "preemptions": 0, "decode_steps": 0, "graph_steps": 0, "ahead_steps": 0}
         if isinstance(model, (str, os.PathLike)):
@@ -119,7 +121,7 @@ class LLM:
         self._captured[rid] = {}
         self._generated[rid] = 0
         if params.capture_logits:
-            self._capturing += 1
+            self._wanted[rid] = set(params.capture_logits)
         return rid
 
     def has_unfinished(self) -> bool:
@@ -156,7 +158,11 @@ class LLM:
         return outs + ended
 
     def _may_run_ahead(self) -> bool:
-        return self.run_ahead and self._capturing == 0 and self.scheduler.steady_decode()
+        return self.run_ahead and not self._wants_logits(self._wanted) and self.scheduler.steady_decode()
+
+    def _wants_logits(self, ids) -> bool:
+        """Whether the next token of one of these requests is one whose logits are wanted."""
+        return any(self._generated[i] in self._wanted[i] for i in ids if i in self._wanted)
 
     def _launch_ahead(self, feed: bool, parity: int):
         r, sched = self.runner, self.scheduler
@@ -206,23 +212,24 @@ class LLM:
         if plan.num_entries:
             decode_only = plan.decode_only
             sampling = plan.sampling_ids()
-            want_logits = any(self._params[i].capture_logits for i in sampling)
-            if decode_only and r.graphs_enabled and not want_logits:
-                sampled = r.decode_step_graph(sched, plan)
+            want_logits = self._wants_logits(sampling)
+            buf = None
+            if want_logits:
+                if self._logit_buf is None:
+                    self._logit_buf = torch.empty((r.seqs_cap, r.spec.vocab_size), dtype=torch.float32, device=r.device)
+                buf = self._logit_buf
+            if decode_only and r.graphs_enabled:
+                sampled = r.decode_step_graph(sched, plan, logits_out=buf)
                 self.stats["graph_steps"] += 1
             else:
                 arrays = sched.arrays(plan, r.rows_cap, r.seqs_cap, r.logits_cap, r.max_pages, r.spec.vocab_size)
-                buf = None
-                if want_logits:
-                    if self._logit_buf is None:
-                        self._logit_buf = torch.empty((r.seqs_cap, r.spec.vocab_size), dtype=torch.float32, device=r.device)
-                    buf = self._logit_buf
                 sampled = r.step(arrays, logits_out=buf).tokens()
-                if want_logits:
-                    for row, rid in enumerate(sampling):
-                        g = self._generated[rid]
-                        if g in self._params[rid].capture_logits:
-                            self._captured[rid][g] = buf[row].cpu()
+            if want_logits:
+                for row, rid in enumerate(sampling):
+                    g = self._generated[rid]
+                    if g in self._wanted.get(rid, ()):
+                        self._captured[rid][g] = buf[row].cpu()
+                        self._wanted[rid].discard(g)
             if min(sampled, default=0) < 0:
                 raise NaNError("pick_tokens")        # crates/engine/src/backend/cpu/mod.rs:377-379
             self.stats["steps"] += 1
@@ -246,8 +253,7 @@ class LLM:
         outs = []
         for f in done:
             rid = f.id
-            if self._params[rid].capture_logits:
-                self._capturing -= 1
+            self._wanted.pop(rid, None)
             outs.append(RequestOutput(rid, self._prompts.pop(rid), list(f.output), f.reason,
                                       self.decode(f.output), self._captured.pop(rid), self._preempt.pop(rid, 0)))
             self._params.pop(rid)
@@ -268,9 +274,7 @@ class LLM:
         self._forget(request_id)
 
     def _forget(self, rid: int) -> None:
-        if rid in self._params and self._params[rid].capture_logits:
-            self._capturing -= 1
-        for d in (self._params, self._prompts, self._captured, self._generated, self._preempt):
+        for d in (self._params, self._prompts, self._captured, self._generated, self._preempt, self._wanted):
             d.pop(rid, None)
 
     # ------------------------------------------------------------------ whole jobs

@@ -170,7 +170,8 @@ class ModelRunner:
         self.graphs_enabled = bool(engine.cuda_graphs)
         self.decode_graphs = self.graphs_enabled         # turned off by a decode step that cannot be recorded
         self._graphs = {}
-        self._step_graphs = collections.OrderedDict()    # shape class -> (graph, launches); least recently replayed first
+        # shape class -> (graph, launches, its logits in the workspace); least recently replayed first
+        self._step_graphs = collections.OrderedDict()
         self._step_seen = {}
         self.step_graph_after = int(getattr(engine, "step_graphs", 0))
         self.step_graph_replays = 0
@@ -178,6 +179,8 @@ class ModelRunner:
         self.after_block = None                 # debugging: a function (call number, residual, pending) run behind every block
         self._pending_scale = None
         self._graph_launches = {}
+        self._graph_logits = {}                 # class of a decode step -> its logits in the workspace (None where the head picks without)
+        self._kept_seen = set()                 # classes of decode steps that keep their logits and have come once
         self._graph_pool = None
 
     # ------------------------------------------------------------------ sizes
@@ -354,14 +357,16 @@ class ModelRunner:
         return resid, pending
 
     def _head(self, resid, pending, ctx: StepContext, num_logit_rows: int, logits_out: Optional[torch.Tensor],
-              layout=None, also=()) -> None:
+              layout=None, also=(), keep_logits: bool = False) -> Optional[torch.Tensor]:
         """Final norm and output head on the wanted rows, in chunks; a token is picked from every
         row; logits are copied out only where the caller gave a place for them. `also`: functions
-        (first row, rows) -> a further place the picked tokens of those rows are written to."""
+        (first row, rows) -> a further place the picked tokens of those rows are written to.
+        Returns the logits in the workspace if all rows were one chunk (they stay until the next
+        step); with `keep_logits` a head that could pick without writing them does write them."""
         spec, L = self.spec, layout or self.layout
         d = self._dev
         V = spec.vocab_size
-        if (self.engine.pick_in_head and logits_out is None and self._folded is not None and ctx.decode_only
+        if (self.engine.pick_in_head and logits_out is None and not keep_logits and self._folded is not None and ctx.decode_only
                 and num_logit_rows == ctx.rows <= self.logit_chunk
                 and getattr(spec.lm_head, "can_fold", lambda: False)() and hasattr(spec.lm_head, "pick_folded")):
             # every row is wanted, in order, and only its token: the head reads the folded residual and
@@ -372,7 +377,8 @@ class ModelRunner:
                                      d[L["seeds"]:L["seeds"] + 2 * n], d[L["sample_steps"]:L["sample_steps"] + n],
                                      self.pick_val[:n * tiles].view(n, tiles), self.pick_idx[:n * tiles].view(n, tiles),
                                      self.nan_flags[:n], self.sampled[:n], [f(0, n) for f in also])
-            return
+            return None
+        logits = None
         for c0 in range(0, num_logit_rows, self.logit_chunk):
             n = min(self.logit_chunk, num_logit_rows - c0)
             with ctx.workspace.scope():
@@ -395,6 +401,7 @@ class ModelRunner:
                                     self.pick_idx, temp, seeds, steps, [f(c0, n) for f in also])
                 if logits_out is not None:
                     logits_out[c0:c0 + n].copy_(logits, non_blocking=logits_out.is_cuda)
+        return logits if num_logit_rows <= self.logit_chunk else None
 
     def step(self, arrays, logits_out: Optional[torch.Tensor] = None) -> StepResult:
         """Run one batch. `arrays` comes from `build_arrays` or the scheduler. `logits_out`
@@ -408,17 +415,20 @@ class ModelRunner:
             raise ShapeError("step", f"logits_out must be float32 [>={R}, {self.spec.vocab_size}]")
         self.upload(arrays)
         self._feed_ready = None
-        shape = self._step_shape(arrays) if logits_out is None else None
+        # a step whose wanted rows are one chunk of the head leaves their logits in the workspace, replayed or not
+        shape = self._step_shape(arrays) if logits_out is None or R <= self.logit_chunk else None
         if shape is not None:
             entry = self._step_graphs.get(shape)
             if entry is not None:
                 self._step_graphs.move_to_end(shape)
                 entry[0].replay()
                 kernels.count_launches(entry[1])
+                if logits_out is not None:
+                    logits_out[:R].copy_(entry[2], non_blocking=logits_out.is_cuda)
                 self.steps_run += 1
                 self.step_graph_replays += 1
                 self._mark_read(0)
-                return StepResult(self.sampled, None, R)
+                return StepResult(self.sampled, logits_out, R)
         self.workspace.reset()
         if shape is None:
             ctx = self.context(T, S, arrays)
@@ -474,11 +484,11 @@ class ModelRunner:
             ctx = self.context(rows, S, None)
             ctx.max_new, ctx.lead_single, ctx.long_context = longest, lead, long_context
             resid, pending = self._forward(ctx)
-            self._head(resid, pending, ctx, R, None)
+            logits = self._head(resid, pending, ctx, R, None)
         launches = kernels.launch_count() - n0
         kernels.count_launches(-launches)           # recorded, not run
         self._graph_pool = self._graph_pool or g.pool()
-        self._step_graphs[shape] = (g, launches)
+        self._step_graphs[shape] = (g, launches, logits)
         while len(self._step_graphs) > self.STEP_GRAPHS_KEPT:
             self._step_graphs.popitem(last=False)   # the one replayed longest ago
 
@@ -487,7 +497,7 @@ class ModelRunner:
         return min(decode_bucket(n), self.decode_cap)
 
     def decode_step_graph(self, scheduler, plan, feed_from_device: bool = False, read: bool = True, parity: int = 0,
-                          arrays=None):
+                          arrays=None, logits_out: Optional[torch.Tensor] = None):
         """A step in which every request brings exactly one token. Its kernels are the same as any
         step's, but their launches are replayed from a CUDA graph captured once per batch-size
         class (1, 2, 4, ... requests, the batch padded with rows that attend to nothing) and per
@@ -496,7 +506,9 @@ class ModelRunner:
         (the reference's estimate: docs/decisions/0003-backend-trait-and-memory.md:51).
         The picked tokens land in pinned host buffer `parity`. With `read` the call waits and
         returns them; without, it returns an event to hand to `read_decode` later. `arrays`: the
-        plan's arrays if the caller has built them already (`decode_arrays`)."""
+        plan's arrays if the caller has built them already (`decode_arrays`). `logits_out` (float32
+        [>= requests, vocab] on the device) receives the step's logits: such a step is a class of its own,
+        whose head writes them, and is recorded when it comes the second time (most steps want none)."""
         S = plan.num_entries
         L = self.decode_layout
         if arrays is None:
@@ -515,17 +527,20 @@ class ModelRunner:
             self.upload(arrays, parity)
         long_context = bool(arrays.max_seq_len > TUNING.long_context_keys)
         if not self.decode_graphs:
-            self._decode_eager(S, parity, long_context)      # nothing is recorded: no padding needed
+            logits = self._decode_eager(S, parity, long_context, logits_out is not None)      # nothing is recorded: no padding needed
         else:
             b = self._bucket(S)
-            key = (b, parity, long_context)
+            key = (b, parity, long_context, logits_out is not None)
             graph = self._graphs.get(key)
-            if graph is None:
+            if graph is None and logits_out is not None and key not in self._kept_seen:
+                self._kept_seen.add(key)
+                logits = self._decode_eager(S if self.pools.state else b, parity, long_context, True)
+            elif graph is None:
                 # first step of this class: run it eagerly (that is this step's result), then record
                 # the same launches for the steps to come. Padding requests (no rows, state slot 0)
                 # are something a recorded step's kernels skip on the device; a model with
                 # per-request state is not shown them before it has proved recordable.
-                self._decode_eager(S if self.pools.state else b, parity, long_context)
+                logits = self._decode_eager(S if self.pools.state else b, *key[1:])
                 try:
                     self._record_decode(key)
                 except Exception as e:      # a part that cannot be recorded (it reads device data on the host, say)
@@ -536,6 +551,9 @@ class ModelRunner:
             else:
                 graph.replay()
                 kernels.count_launches(self._graph_launches[key])
+                logits = self._graph_logits[key]
+        if logits_out is not None:
+            logits_out[:S].copy_(logits[:S])
         self.steps_run += 1
         self._mark_read(parity)
         self._feed_ready = 1 - parity
@@ -559,11 +577,12 @@ class ModelRunner:
         n0 = kernels.launch_count()
         try:
             with torch.cuda.graph(g, pool=self._graph_pool):
-                self._decode_eager(*key)
+                logits = self._decode_eager(*key)
         finally:
             launches = kernels.launch_count() - n0
             kernels.count_launches(-launches)                       # recorded, not run
         self._graph_launches[key] = launches
+        self._graph_logits[key] = logits
         self._graphs[key] = g
         self._graph_pool = self._graph_pool or g.pool()
 
@@ -572,7 +591,7 @@ class ModelRunner:
         event.synchronize()
         return self.sampled_host_np[parity, :count].tolist()
 
-    def _decode_eager(self, b: int, parity: int = 0, long_context: bool = False) -> None:
+    def _decode_eager(self, b: int, parity: int = 0, long_context: bool = False, keep_logits: bool = False) -> Optional[torch.Tensor]:
         L = self.decode_layout
         self.workspace.reset()
         self._dev = self._devs[parity]          # this step's metadata (a recorded step keeps reading this buffer)
@@ -587,11 +606,12 @@ class ModelRunner:
             also = [lambda c0, n: other[t0 + c0:t0 + c0 + n]]
             if host is not None:
                 also.append(lambda c0, n: host.at(parity * self.seqs_cap + c0))
-            self._head(resid, pending, ctx, b, None, L, also=also)
+            logits = self._head(resid, pending, ctx, b, None, L, also=also, keep_logits=keep_logits)
         finally:
             self._dev = self.step_dev
         if host is None:
             self.sampled_host[parity, :b].copy_(self.sampled[:b], non_blocking=True)
+        return logits
 
     # ------------------------------------------------------------------ bookkeeping helpers
     def check_kernels(self) -> None:

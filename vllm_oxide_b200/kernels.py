@@ -530,7 +530,9 @@ def glu(gate_up: torch.Tensor, out: torch.Tensor, activation: str = "silu") -> N
 # ------------------------------------------------------------------------------------ matrix products
 @_timed
 def gemm_f32(a: torch.Tensor, w: torch.Tensor, out: torch.Tensor, bias: Optional[torch.Tensor] = None) -> None:
-    """out[M, N] = a[M, K] @ w[N, K]^T (+ bias[N]) in true float32 (FMA chains over k, always added in the same order; no tensor cores)."""
+    """out[M, N] = a[M, K] @ w[N, K]^T (+ bias[N]) in true float32 (FMA chains over k, always added in the same order; no tensor cores).
+    `w` holds weights: with programmatic dependent launch its first rows are read while the kernel in front still runs, so it
+    must not be what such a kernel of this package writes."""
     op = "gemm_f32"
     _cuda(op, a, w, out, bias)
     for name, t in (("a", a), ("w", w), ("out", out)):
