@@ -12,8 +12,8 @@
 //  * few rows (M <= 16, decode steps): bound by reading W once, 5.9 TB/s at M = 1 and 2.7 TB/s at M = 16 on 128,256 x 2,048, 3.4 and
 //    2.0 TB/s on 16,384 x 2,048 (64 x 64 tiles, which served every M before: 1.06 and 0.6 TB/s; 0.1 TB/s on 2,048 x 8,192, now 2.6). A thread has one or two weight rows and a chunk, all rows of A
 //    in its registers' sums; weights arrive by cp.async into a ring per warp, so that no barrier of the block stands in the stream.
-//  * tiles (everything else): bound by the FMA units. 8 x 8 outputs a thread from shared memory: 42 to 44 TFLOP/s on 16,384 x 2,048
-//    at M = 1,250 and 2,048 (33 and 34 before), 33 TFLOP/s on 2,048 x 8,192 at M = 128 (6).
+//  * tiles (everything else): bound by the FMA units. 8 x 8 outputs a thread from shared memory: 40 to 42 TFLOP/s on 16,384 x 2,048
+//    at M = 1,250 and 2,048 (33 and 34 before), 31 TFLOP/s on 2,048 x 8,192 at M = 128 (6).
 // Both multiply and add pairs of k in one instruction (fma.rn.f32x2, each half rounded as fmaf rounds it): single FMAs
 // reach half the rate on this GPU (a tile kernel of 8 x 8 outputs a thread: 37 TFLOP/s with fmaf).
 #include "common.cuh"
@@ -215,31 +215,33 @@ int launch_few(const float* A, long long lda, const float* W, long long ldw, flo
 // A block of 128 threads computes 16 * TR rows by 64 columns, a thread TR x 8 of them (rows tm + 16 i, columns tn + 8 j). K
 // comes in slabs of 16 through a ring of three stages, [row][k] as it lies in memory, rows 20 floats apart: the 16-byte reads
 // of different rows that a warp makes at once fall into different banks. The sums of the chunks so far wait in shared
-// memory: the segment's, and (c == 1) the finished segments'. Or a cluster of c = 8 blocks shares K, a segment each, and
+// memory: the segment's, and (CL == 1) the finished segments'. Or a cluster of CL = 8 blocks shares K, a segment each, and
 // adds the segments' sums: eight times the blocks, for few tiles or a last wave that would be nearly empty.
-constexpr int TN = 64, TK = 16, TLD = TK + 4, TSTAGES = 3;
+constexpr int TN = 64, TK = 16, TLD = TK + 4, TSTAGES = 3, GRID_Y = 32768;
 __host__ __device__ constexpr int tile_blocks(int tr) { return tr == 8 ? 2 : tr == 4 ? 3 : 4; }   // resident on an SM
 
-template <int TR, bool VEC>
+template <int TR, bool VEC, int CL>
 __global__ void __launch_bounds__(128, tile_blocks(TR))
 gemm_f32_tile_kernel(const float* __restrict__ A, long long lda, const float* __restrict__ W, long long ldw, float* __restrict__ C,
-                     long long ldc, int M, int N, int K, const float* __restrict__ bias, int seg, int c, int mtiles) {
+                     long long ldc, int M, int N, int K, const float* __restrict__ bias, int seg) {
     constexpr int TM = 16 * TR, QUADS = TR * 2;
     extern __shared__ __align__(16) float smem[];
     float* stage = smem;                                        // [TSTAGES][(TM + TN)][TLD]
-    float4* sums = reinterpret_cast<float4*>(smem + TSTAGES * (TM + TN) * TLD);    // [c == 1 ? 2 : 1][QUADS][128]
+    float4* sums = reinterpret_cast<float4*>(smem + TSTAGES * (TM + TN) * TLD);    // [CL == 1 ? 2 : 1][QUADS][128]
     pdl_launch_dependents();
     pdl_wait(11);
     int tid = threadIdx.x, lane = tid & 31;
     int tn = (lane & 3) | ((lane >> 4) << 2), tm = ((tid >> 5) << 2) | ((lane >> 2) & 3);
-    int rank = blockIdx.x % c, tile = blockIdx.x / c;
-    int m0 = (tile % mtiles) * TM, n0 = (tile / mtiles) * TN;
-    int kb = min(K, rank * seg * CHUNK), ke = c > 1 ? min(K, kb + seg * CHUNK) : K;
+    int rank = blockIdx.x % CL, m0 = blockIdx.x / CL * TM, n0 = (blockIdx.z * GRID_Y + blockIdx.y) * TN;
+    int kb = min(K, rank * seg * CHUNK), ke = CL > 1 ? min(K, kb + seg * CHUNK) : K;
     int slabs = (ke - kb + TK - 1) / TK;
+    int put_at = 0;
+    const int lk = (tid & 3) * 4;
     auto load = [&](int s) {
         if (s < slabs) {
-            float* st = stage + (s % TSTAGES) * (TM + TN) * TLD;
-            int k = kb + s * TK + (tid & 3) * 4;
+            float* st = stage + put_at * (TM + TN) * TLD;
+            put_at = put_at + 1 == TSTAGES ? 0 : put_at + 1;
+            int k = kb + s * TK + lk;
 #pragma unroll
             for (int i = 0; i < (TM + TN) / 32; ++i) {
                 int r = i * 32 + (tid >> 2);
@@ -304,7 +306,7 @@ gemm_f32_tile_kernel(const float* __restrict__ A, long long lda, const float* __
                     float4 o = d[e * 128];
                     v.x = o.x + v.x; v.y = o.y + v.y; v.z = o.z + v.z; v.w = o.w + v.w;
                 }
-                if (c > 1 || !seg_ends) d[e * 128] = v;
+                if (CL > 1 || !seg_ends) d[e * 128] = v;
                 else {
                     if (!first_seg) {
                         float4 o = d[(QUADS + e) * 128];
@@ -327,7 +329,7 @@ gemm_f32_tile_kernel(const float* __restrict__ A, long long lda, const float* __
         for (int j = 0; j < 4; ++j)
             if (n + 8 * j < N) C[(size_t)m * ldc + n + 8 * j] = bias ? o[j] + bias[n + 8 * j] : o[j];
     };
-    if (c == 1) {                                               // a thread's own sums: no barrier
+    if constexpr (CL == 1) {                                               // a thread's own sums: no barrier
 #pragma unroll
         for (int e = 0; e < QUADS; ++e) put(e, sums[(QUADS + e) * 128 + tid]);
         return;
@@ -335,7 +337,7 @@ gemm_f32_tile_kernel(const float* __restrict__ A, long long lda, const float* __
     cluster_arrive();
     cluster_wait();
     int have = (K + seg * CHUNK - 1) / (seg * CHUNK);           // segments that are not empty
-    for (int e = rank; e < QUADS; e += c) {
+    for (int e = rank; e < QUADS; e += CL) {
         float4 o[8];
 #pragma unroll
         for (int b = 0; b < 8; ++b)
@@ -353,15 +355,14 @@ gemm_f32_tile_kernel(const float* __restrict__ A, long long lda, const float* __
 template <int TR>
 int launch_tile(const float* A, long long lda, const float* W, long long ldw, float* C, long long ldc, int M, int N, int K,
                 const float* bias, int nc, int c, int vec, cudaStream_t stream) {
-    int mtiles = (M + 16 * TR - 1) / (16 * TR);
-    long long blocks = (long long)mtiles * ((N + TN - 1) / TN) * c;
-    if (blocks > 0x7fffffffLL) return VOB_ERR_UNSUPPORTED;
-    auto kernel = vec ? gemm_f32_tile_kernel<TR, true> : gemm_f32_tile_kernel<TR, false>;
+    int mtiles = (M + 16 * TR - 1) / (16 * TR), ntiles = (N + TN - 1) / TN;
+    auto kernel = c == 1 ? (vec ? gemm_f32_tile_kernel<TR, true, 1> : gemm_f32_tile_kernel<TR, false, 1>)
+                         : (vec ? gemm_f32_tile_kernel<TR, true, 8> : gemm_f32_tile_kernel<TR, false, 8>);
     size_t smem = sizeof(float) * (size_t)(TSTAGES * (16 * TR + TN) * TLD + (c == 1 ? 2 : 1) * TR * 8 * 128);
     cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return (int)e;
     cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3((unsigned)blocks);
+    cfg.gridDim = dim3((unsigned)(mtiles * c), (unsigned)min(ntiles, GRID_Y), (unsigned)((ntiles + GRID_Y - 1) / GRID_Y));
     cfg.blockDim = dim3(128);
     cfg.dynamicSmemBytes = smem;
     cfg.stream = stream;
@@ -372,7 +373,7 @@ int launch_tile(const float* A, long long lda, const float* W, long long ldw, fl
     attr[1].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attr;
     cfg.numAttrs = g_vob_pdl ? 2 : 1;
-    e = cudaLaunchKernelEx(&cfg, kernel, A, lda, W, ldw, C, ldc, M, N, K, bias, seg_chunks(nc), c, mtiles);
+    e = cudaLaunchKernelEx(&cfg, kernel, A, lda, W, ldw, C, ldc, M, N, K, bias, seg_chunks(nc));
     return e != cudaSuccess ? (int)e : vob_launch_status();
 }
 
