@@ -241,6 +241,41 @@ def test_paged_attention_window_edge(dt, window):
         r += n
 
 
+@pytest.mark.parametrize("H,KV,hd,page,window", [(4, 4, 64, 16, 0), (8, 2, 64, 8, 33), (6, 2, 128, 16, 0), (16, 2, 128, 24, 40), (32, 8, 64, 16, 0),
+                                                 (5, 1, 64, 16, 100), (2, 1, 128, 8, 0), (8, 1, 64, 16, 1)])
+def test_f32_attention_of_portions_and_of_single_tokens_agree_to_the_bit(H, KV, hd, page, window):
+    """The 32-bit engine's two kernels (single tokens over one to eight blocks, rows of portions) give a row the same bits, whatever
+    shares its block; a padding row gives zeros; an infinity among a later token's values reaches no earlier row."""
+    # 349 rows: the rows' kernel takes what lies behind the single tokens while it is more than 256 rows
+    seqs = [(0, 70), (131, 1), (30, 5), (0, 1), (31, 2), (63, 66), (700, 1), (255, 200)]
+    qrows, kc, vc, bt, row_seq, pos, qs, ks, vs = _paged_case(torch.float32, H, KV, hd, page, seqs, seed=H + hd + window, poison=True,
+                                                             scale_key=lambda L: L // 2)
+    # the last token of the first request: values that are infinite
+    vc[int(bt[0, 69 // page]), :, 69 % page, :] = float("inf")
+    pad = 3
+    T = len(pos) + pad
+    qrows, row_seq, pos = torch.cat([qrows, qrows[:pad]]).to(DEV), torch.cat([row_seq, row_seq[:pad]]).to(DEV), torch.cat([pos, pos[:pad] * 0 - 1]).to(DEV)
+    kc, vc, bt = kc.to(DEV), vc.to(DEV), bt.to(DEV)
+
+    def go(singles, rows=slice(0, T)):
+        out = torch.full_like(qrows[rows], 7.0)
+        K().paged_attention(qrows[rows], out, kc, vc, bt, row_seq[rows].contiguous(), pos[rows].contiguous(), H, KV, hd, 1.0 / math.sqrt(hd), window, singles)
+        return out
+    full = go(0)
+    assert bool((full[-pad:] == 0).all())
+    same = lambda a, b: torch.equal(torch.nan_to_num(a, 9e9), torch.nan_to_num(b, 9e9))  # noqa: E731
+    for singles in (1, 2, 50, T - 1, T):
+        assert same(go(singles), full), singles
+    for lo, n in ((0, 1), (3, 40), (69, 3), (13, 300), (T - 9, 9)):
+        assert same(go(0, slice(lo, lo + n)), full[lo:lo + n]) and same(go(n, slice(lo, lo + n)), full[lo:lo + n]), (lo, n)
+    r = 0
+    for s, (c, n) in enumerate(seqs):
+        want = plain.causal_attention(qs[s].double(), ks[s].double(), vs[s].double(), H, KV, hd, window=window or None)[c:]
+        m = n - 1 if s == 0 else n
+        assert rel(full[r:r + m], want[:m]) <= ATOL[torch.float32], s
+        r += n
+
+
 def test_paged_attention_refuses_bad_sizes():
     from vllm_oxide_b200.errors import ShapeError
     q = torch.zeros(1, 4 * 20, device=DEV)

@@ -191,8 +191,9 @@ class Attention(Mixer):
                 kernels.attn_prefill_mma(q, out, cache.k, cache.v, bt[lead:], ctx.seq_starts[lead:], ctx.context_lens[lead:],
                                          ctx.seqs - lead, ctx.max_new, self.H, self.KV, self.hd, self.scale, self.window)
                 return
+        singles = ctx.rows if ctx.decode_only else ctx.lead_single
         kernels.paged_attention(q, out, cache.k, cache.v, bt, ctx.row_seq, ctx.positions, self.H, self.KV, self.hd,
-                                self.scale, self.window)
+                                self.scale, self.window, singles)
 
     def _attend_single(self, q, out, ctx: StepContext, cache: LayerCache, bt, count: int) -> None:
         """The decode kernel on the first `count` rows, row i belonging to request i."""
