@@ -567,6 +567,44 @@ def test_attn_decode_mma_merge_through_global_memory(H, KV, hd, page, window, sp
         k.attn_decode_mma(qrows.to(DEV), out, *args[:10], partials[:100], arrived)
 
 
+@pytest.mark.parametrize("H,KV,hd,page,S,balance,most", [(8, 2, 64, 16, 1, 2, 400), (8, 2, 64, 16, 1, 64, 9000), (6, 2, 128, 32, 12, 37, 3000),
+                                                         (32, 8, 64, 16, 33, 55, 1500), (4, 4, 64, 8, 70, 3, 300), (3, 1, 128, 64, 128, 64, 700),
+                                                         (16, 1, 64, 16, 128, 5, 64), (8, 2, 64, 64, 20, 2, 5000)])
+def test_attn_decode_mma_balanced(H, KV, hd, page, S, balance, most):
+    """Blocks dealt out by length: one long request among short ones, all alike, single keys, padding rows in between, tile edges,
+    as many requests as a launch takes and few blocks for them; what one block per request computes, up to rounding, and
+    counters left at zero."""
+    g = torch.Generator().manual_seed(S + most)
+    k = K()
+    pages = -(-most // page)
+    spread = torch.exp(torch.rand(S, generator=g) * math.log(most)).long().clamp(1, most)
+    one = torch.ones(S, dtype=torch.long)
+    one[S // 2] = most
+    edges = torch.tensor([[1, 63, 64, 65, 128, 0][i % 6] for i in range(S)]).clamp(max=most)
+    bt = torch.arange(S * pages, dtype=torch.int32).view(S, pages)[:, torch.randperm(pages, generator=g)].contiguous().to(DEV)
+    kc = torch.randn(S * pages, KV, page, hd, generator=g).to(torch.bfloat16).to(DEV)
+    vc = torch.randn(S * pages, KV, page, hd, generator=g).to(torch.bfloat16).to(DEV)
+    q = (2 * torch.randn(S, H * hd, generator=g)).to(torch.bfloat16).to(DEV)
+    partials = torch.full((k.attn_decode_partial_floats(1, KV, hd, 2 * balance),), float("nan"), device=DEV)
+    arrived = torch.zeros(S * KV, dtype=torch.int32, device=DEV)
+    for lens in (spread, one, torch.full((S,), most), edges, one * 0):
+        pos = (lens - 1).to(torch.int32).to(DEV)
+        want, got = torch.full_like(q, 7.0), torch.full_like(q, 7.0)
+        args = (kc, vc, bt, pos, H, KV, hd, 1.0 / math.sqrt(hd))
+        k.attn_decode_mma(q, want, *args)
+        k.attn_decode_mma(q, got, *args, 0, 1, partials, arrived, balance=balance)
+        # P is rounded to bfloat16 relative to another maximum, and so is the result: two roundings of 2^-9 of either
+        assert rel(got, want.double().cpu()) <= 2 ** -7 if int(lens.max()) else bool((got == 0).all())
+        assert bool((got[pos < 0] == 0).all()) and int(arrived.abs().max()) == 0
+    from vllm_oxide_b200.errors import ShapeError
+    with pytest.raises(ShapeError, match="balance must be"):
+        k.attn_decode_mma(q, got, *args, 0, 1, partials, arrived, balance=65)
+    with pytest.raises(ShapeError, match="balance must be"):
+        k.attn_decode_mma(q, got, *args, 0, 1, balance=balance)
+    with pytest.raises(ShapeError, match="partials must be"):
+        k.attn_decode_mma(q, got, *args, 0, 1, partials[:100], arrived, balance=balance)
+
+
 def test_attn_mma_refusals():
     from vllm_oxide_b200.errors import ShapeError
     k = K()

@@ -23,6 +23,7 @@
 // softmax's denominator once, a key with no value), a gate (the result times sigmoid(gate[row,
 // head * hd + d]), or sigmoid(gate[row, head]) with one number per head) and a constant factor.
 #include "common.cuh"
+#include <algorithm>
 VOB_PDL_SWITCH(attention_mma)
 
 namespace {
@@ -700,7 +701,70 @@ __device__ __noinline__ void merge_partials(const float* __restrict__ all, int s
 // blocks as it has tiles for (at least DEC_MIN_TILES each; the others leave at once), every
 // block writes its partial to global memory and counts itself in, and the block that arrives
 // last adds the partials up in rank order and puts the counter back to zero. Nobody waits.
+//
+// Requests of very different lengths (`balance` blocks per kv head): with the same number of blocks for every request the longest
+// one's blocks work long after the others have left. The grid is then one row of blocks per kv head, and a request gets blocks by its
+// length: `share` tiles each, the smallest share (at least DEC_MIN_TILES) at which the blocks suffice. Every block works that out for
+// itself from the positions, before its wait; the merge is the one through global memory.
+// 16 requests of 17 to 8,000 keys, 8 kv heads of 64 / 128: 39 / 64 us with three blocks each in clusters, 17 / 28 us so (7.5 / 15 us of
+// bytes); 12 requests of 130 to 3,000 keys, kv heads of 128: 22 -> 16.5 us.
 // ---------------------------------------------------------------------------------------------
+
+constexpr int DEC_BALANCE_SEQS = 128;      // most requests of a balanced launch: four a lane
+
+// Tiles a block takes at first, with `want` blocks for `total` tiles; the search below ends at twice this.
+__host__ __device__ constexpr int balance_share(long long total, int want) {
+    return (int)((total + want - 1) / want) > DEC_MIN_TILES ? (int)((total + want - 1) / want) : DEC_MIN_TILES;
+}
+
+// Which request and which of its blocks block `b` of a kv head is. Returns false if it is none's. `want`: the blocks that are to be
+// filled evenly, `blocks` those there are. Partials are kept for requests of more than one block: at most 2 want of them. (At twice the first share the requests need at most want / 2 blocks
+// for whole shares and one each for the rest: they fit, as `blocks` is at least want / 2 + requests.)
+__device__ __forceinline__ bool balance_place(const int* __restrict__ positions, int S, int want, int blocks, int b, int lane, int& seq,
+                                              int& split, int& splits, int& share, int& first_part) {
+    int n[DEC_BALANCE_SEQS / 32], total = 0;
+#pragma unroll
+    for (int i = 0; i < DEC_BALANCE_SEQS / 32; ++i) {
+        const int r = i * 32 + lane;
+        n[i] = r < S ? max(positions[r] + BN, 0) / BN : 0;            // tiles of keys 0 .. position (0 for a padding row's -1)
+        total += n[i];
+    }
+    total = __reduce_add_sync(0xffffffffu, total);
+    const int share0 = balance_share(total, want);
+    share = share0;
+    while (true) {
+        int need = 0;
+#pragma unroll
+        for (int i = 0; i < DEC_BALANCE_SEQS / 32; ++i) need += i * 32 + lane < S ? max(1, (n[i] + share - 1) / share) : 0;
+        if (share >= 2 * share0 || (int)__reduce_add_sync(0xffffffffu, need) <= blocks) break;
+        share = min(2 * share0, share + (share + 7) / 8);
+    }
+    int before = 0;                                   // blocks of the requests in front
+    first_part = 0;                                   // and of those that have more than one
+#pragma unroll
+    for (int i = 0; i < DEC_BALANCE_SEQS / 32; ++i) {
+        if (i * 32 >= S) break;
+        const int mine = i * 32 + lane < S ? max(1, (n[i] + share - 1) / share) : 0;
+        int upto = mine, parts = mine > 1 ? mine : 0;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const int v = __shfl_up_sync(0xffffffffu, upto, o), u = __shfl_up_sync(0xffffffffu, parts, o);
+            if (lane >= o) { upto += v; parts += u; }
+        }
+        const unsigned at = __ballot_sync(0xffffffffu, b < before + upto);
+        if (at) {
+            const int l = __ffs(at) - 1;
+            seq = i * 32 + l;
+            splits = __shfl_sync(0xffffffffu, mine, l);
+            split = b - (before + __shfl_sync(0xffffffffu, upto, l) - splits);
+            first_part += __shfl_sync(0xffffffffu, parts, l) - (splits > 1 ? splits : 0);
+            return true;
+        }
+        before += __shfl_sync(0xffffffffu, upto, 31);
+        first_part += __shfl_sync(0xffffffffu, parts, 31);
+    }
+    return false;
+}
 
 // Shared memory of a decode block: the K/V ring (used again for the combine of the four warps),
 // then what the cluster's peers send, then the block's page list.
@@ -719,7 +783,7 @@ attn_decode_mma_kernel(const __nv_bfloat16* __restrict__ q, long long q_stride, 
                        long long out_stride, const __nv_bfloat16* __restrict__ kc, const __nv_bfloat16* __restrict__ vc,
                        const int* __restrict__ block_tables, int max_pages, const int* __restrict__ positions,
                        int H, int KV, int page_shift, int window, float scale_log2, float* __restrict__ partials,
-                       int* __restrict__ arrived, AttnTail tail, ScoreShape shape) {
+                       int* __restrict__ arrived, AttnTail tail, ScoreShape shape, int balance, int S) {
     constexpr int LD = HD + 8;
     constexpr int PART = 16 * HD + 32;                                          // floats of one block's partial
     pdl_launch_dependents();
@@ -740,8 +804,13 @@ attn_decode_mma_kernel(const __nv_bfloat16* __restrict__ q, long long q_stride, 
     // every key but the newest was written by earlier steps: all of that may be read before the
     // wait, while the kernel in front (which writes the newest key and this step's q) still runs.
     const int G = H / KV;
-    const int seq = blockIdx.x, kvh = blockIdx.y, split = blockIdx.z;
+    int seq = blockIdx.x, kvh = blockIdx.y, split = blockIdx.z;
     int splits = gridDim.z;
+    int first_part = (seq * KV + kvh) * gridDim.z, share = 0;       // the request's first partial; tiles of a block (balanced)
+    if (!SHAPED && balance) {
+        if (!balance_place(positions, S, balance, gridDim.x, blockIdx.x, threadIdx.x & 31, seq, split, splits, share, first_part)) return;
+        first_part += kvh * 2 * balance;
+    }
     // every block of the cluster has started (and owns its shared memory) before anyone is sent
     // anything: arrive now, wait just before the first store to a peer
     if (!partials && splits > 1) asm volatile("barrier.cluster.arrive.relaxed.aligned;" ::: "memory");
@@ -756,13 +825,13 @@ attn_decode_mma_kernel(const __nv_bfloat16* __restrict__ q, long long q_stride, 
     const int n_tiles = p >= 0 ? (hi + BN - 1) / BN - t_first + kt : 0;
     // the request's tile number n (0 .. n_tiles - 1) holds the keys from BN * tile_of(n) on
     auto tile_of = [&](int n) { return KV1 && n < kt ? n : t_first + n - kt; };
-    if (partials) {
+    if (partials && (SHAPED || !balance)) {
         splits = max(1, min(splits, n_tiles / DEC_MIN_TILES));
-        const int share = max(1, (n_tiles + splits - 1) / splits);
+        share = max(1, (n_tiles + splits - 1) / splits);
         splits = max(1, (n_tiles + share - 1) / share);      // no block without a tile
         if (split >= splits) return;                  // the whole block: this request has no tiles for it
     }
-    const int per = (n_tiles + splits - 1) / splits;
+    const int per = !SHAPED && balance ? share : (n_tiles + splits - 1) / splits;
     const int n_begin = split * per;
     const int n_end = min(n_tiles, n_begin + per);
     // this block's pages: those of its tiles, BN / page_size of them each, one coalesced read of the block table
@@ -912,7 +981,7 @@ attn_decode_mma_kernel(const __nv_bfloat16* __restrict__ q, long long q_stride, 
         }
     }
     if (splits > 1 && partials) {
-        float* mine = partials + ((size_t)(seq * KV + kvh) * gridDim.z + split) * PART;
+        float* mine = partials + (size_t)(first_part + split) * PART;
         __syncthreads();
         for (int e = threadIdx.x; e < G * HD; e += NTHREADS) mine[e] = fin[e];
         if (threadIdx.x < 32) mine[16 * HD + threadIdx.x] = fin[16 * HD + threadIdx.x];
@@ -922,7 +991,7 @@ attn_decode_mma_kernel(const __nv_bfloat16* __restrict__ q, long long q_stride, 
         __syncthreads();
         if (!s_last) return;
         __threadfence();
-        merge_partials<HD>(partials + (size_t)(seq * KV + kvh) * gridDim.z * PART, splits, G, reinterpret_cast<float*>(sK0),
+        merge_partials<HD>(partials + (size_t)first_part * PART, splits, G, reinterpret_cast<float*>(sK0),
                            out + (size_t)seq * out_stride + (size_t)kvh * G * HD, tail, seq, kvh * G);
         if (threadIdx.x == 0) arrived[seq * KV + kvh] = 0;      // ready for the next launch
     } else if (splits > 1) {
@@ -1001,19 +1070,21 @@ int launch_prefill(const void* q, long long q_stride, void* out, long long out_s
 template <int HD, int ST, bool SHAPED, bool KV1>
 int launch_decode_st(const void* q, long long q_stride, void* out, long long out_stride, const void* kc, const void* vc,
                      const int* bt, int max_pages, const int* positions, int S, int H, int KV, int page_size, int window,
-                     float scale, int splits, float* partials, int* arrived, AttnTail tail, ScoreShape shape, cudaStream_t stream) {
+                     float scale, int splits, float* partials, int* arrived, AttnTail tail, ScoreShape shape, int balance, int grid_blocks,
+                     cudaStream_t stream) {
     static size_t configured = 0;
     // a block's page list: its share of the tiles of the longest request the block table can hold
     // (a request with few tiles uses fewer blocks, but then the tiles are few)
     long long tiles_max = ((long long)max_pages * page_size + BN - 1) / BN;
     long long per_max = (tiles_max + splits - 1) / splits;
     if (partials && per_max < 2 * DEC_MIN_TILES) per_max = 2 * DEC_MIN_TILES;
+    if (balance) per_max = std::max<long long>(1, std::min<long long>(tiles_max, 2 * balance_share(S * tiles_max, balance)));
     long long pages_cta = per_max * (BN / page_size) + 1;
     size_t smem = decode_smem<HD, ST, KV1>(H / KV, splits > 1 && !partials) + (size_t)pages_cta * sizeof(int);
     int e = ensure_smem(attn_decode_mma_kernel<HD, ST, SHAPED, KV1>, smem, &configured);
     if (e) return e;
     cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3(S, KV, splits);
+    cfg.gridDim = balance ? dim3(grid_blocks, KV) : dim3(S, KV, splits);
     cfg.blockDim = dim3(NTHREADS);
     cfg.dynamicSmemBytes = smem;
     cfg.stream = stream;
@@ -1028,14 +1099,16 @@ int launch_decode_st(const void* q, long long q_stride, void* out, long long out
     cfg.numAttrs = g_vob_pdl ? 2 : 1;
     cudaError_t ce = cudaLaunchKernelEx(&cfg, attn_decode_mma_kernel<HD, ST, SHAPED, KV1>, (const __nv_bfloat16*)q, q_stride, (__nv_bfloat16*)out,
                                         out_stride, (const __nv_bfloat16*)kc, (const __nv_bfloat16*)vc, bt, max_pages, positions,
-                                        H, KV, log2_exact(page_size), window, scale * 1.4426950408889634f, partials, arrived, tail, shape);
+                                        H, KV, log2_exact(page_size), window, scale * 1.4426950408889634f, partials, arrived, tail, shape,
+                                        balance, S);
     return ce != cudaSuccess ? (int)ce : vob_launch_status();
 }
 
 template <int HD, bool SHAPED, bool KV1 = false>
 int launch_decode(const void* q, long long q_stride, void* out, long long out_stride, const void* kc, const void* vc,
                   const int* bt, int max_pages, const int* positions, int S, int H, int KV, int page_size, int window,
-                  float scale, int splits, float* partials, int* arrived, AttnTail tail, ScoreShape shape, cudaStream_t stream) {
+                  float scale, int splits, float* partials, int* arrived, AttnTail tail, ScoreShape shape, int balance, int grid_blocks,
+                  cudaStream_t stream) {
     static int num_sms = 0;
     if (!num_sms) {
         int dev = 0;
@@ -1044,13 +1117,13 @@ int launch_decode(const void* q, long long q_stride, void* out, long long out_st
         if (num_sms <= 0) num_sms = 148;
     }
     // three stages while every block of the grid can be resident at once with them; else two
-    long long blocks = (long long)S * KV * splits;
+    long long blocks = balance ? (long long)balance * KV : (long long)S * KV * splits;
     long long fit3 = (long long)num_sms * ((227 * 1024) / (long long)(decode_smem<HD, 3, KV1>(H / KV, splits > 1 && !partials) + 2048));
     if (blocks <= fit3)
         return launch_decode_st<HD, 3, SHAPED, KV1>(q, q_stride, out, out_stride, kc, vc, bt, max_pages, positions, S, H, KV, page_size,
-                                               window, scale, splits, partials, arrived, tail, shape, stream);
+                                               window, scale, splits, partials, arrived, tail, shape, balance, grid_blocks, stream);
     return launch_decode_st<HD, 2, SHAPED, KV1>(q, q_stride, out, out_stride, kc, vc, bt, max_pages, positions, S, H, KV, page_size,
-                                           window, scale, splits, partials, arrived, tail, shape, stream);
+                                           window, scale, splits, partials, arrived, tail, shape, balance, grid_blocks, stream);
 }
 
 template <int HD, int HDV, bool SHAPED, bool KV1>
@@ -1187,21 +1260,25 @@ VOB_EXPORT int vob_attn_prefill_shaped(const void* q, long long q_stride, void* 
 // `splits` (1..8) blocks share each (request, kv head) as one cluster. With `partials` (float32
 // [S * KV * splits * (16 * hd + 32)]) and `arrived` (int32 [S * KV], zero; left zero) up to 64 blocks
 // share it without a cluster and merge through global memory.
+// `balance`: see "Requests of very different lengths"; no window, at most DEC_BALANCE_SEQS requests.
 VOB_EXPORT int vob_attn_decode_mma(const void* q, long long q_stride, void* out, long long out_stride, const void* kcache,
                                    const void* vcache, const int* block_tables, int max_pages, const int* positions, int S,
                                    int H, int KV, int hd, int page_size, int window, float scale, int splits,
                                    void* partials, int* arrived, const float* sink, const void* gate, long long gate_stride,
-                                   float out_scale, cudaStream_t stream) {
+                                   float out_scale, int balance, cudaStream_t stream) {
     const AttnTail tail{sink, (const __nv_bfloat16*)gate, gate_stride, out_scale, 0};
     const ScoreShape none = make_shape(0, 0.f, nullptr, nullptr, scale);
     if (S <= 0) return 0;
     if (!sizes_ok(H, KV, hd, page_size) || H / KV > 16) return VOB_ERR_UNSUPPORTED;
     if ((partials == nullptr) != (arrived == nullptr)) return VOB_ERR_BAD_ARG;
     if (q_stride % 8 != 0 || splits < 1 || splits > (partials ? DEC_MAX_SPLITS_WIDE : 8) || KV > 65535) return VOB_ERR_BAD_ARG;
+    // blocks a kv head: as many as are to be filled, and enough for a rest of every request
+    int grid_blocks = std::max(balance, balance / 2 + S);
+    if (balance < 0 || (balance && (!partials || balance < 2 || balance > DEC_MAX_SPLITS_WIDE || window || S > DEC_BALANCE_SEQS))) return VOB_ERR_BAD_ARG;
     if (hd == 64) return launch_decode<64, false>(q, q_stride, out, out_stride, kcache, vcache, block_tables, max_pages, positions, S,
-                                                 H, KV, page_size, window, scale, splits, (float*)partials, arrived, tail, none, stream);
+                                                 H, KV, page_size, window, scale, splits, (float*)partials, arrived, tail, none, balance, grid_blocks, stream);
     return launch_decode<128, false>(q, q_stride, out, out_stride, kcache, vcache, block_tables, max_pages, positions, S, H, KV,
-                                     page_size, window, scale, splits, (float*)partials, arrived, tail, none, stream);
+                                     page_size, window, scale, splits, (float*)partials, arrived, tail, none, balance, grid_blocks, stream);
 }
 
 // vob_attn_decode_mma with shaped scores (see vob_attn_prefill_shaped).
@@ -1220,12 +1297,12 @@ VOB_EXPORT int vob_attn_decode_shaped(const void* q, long long q_stride, void* o
     if (q_stride % 8 != 0 || splits < 1 || splits > (partials ? DEC_MAX_SPLITS_WIDE : 8) || KV > 65535) return VOB_ERR_BAD_ARG;
     if (kcache == vcache) {                    // the values are the cached keys
         if (hd == 64) return launch_decode<64, true, true>(q, q_stride, out, out_stride, kcache, vcache, block_tables, max_pages, positions, S,
-                                                          H, KV, page_size, window, scale, splits, (float*)partials, arrived, tail, shape, stream);
+                                                          H, KV, page_size, window, scale, splits, (float*)partials, arrived, tail, shape, 0, 0, stream);
         return launch_decode<128, true, true>(q, q_stride, out, out_stride, kcache, vcache, block_tables, max_pages, positions, S, H, KV,
-                                              page_size, window, scale, splits, (float*)partials, arrived, tail, shape, stream);
+                                              page_size, window, scale, splits, (float*)partials, arrived, tail, shape, 0, 0, stream);
     }
     if (hd == 64) return launch_decode<64, true>(q, q_stride, out, out_stride, kcache, vcache, block_tables, max_pages, positions, S,
-                                                H, KV, page_size, window, scale, splits, (float*)partials, arrived, tail, shape, stream);
+                                                H, KV, page_size, window, scale, splits, (float*)partials, arrived, tail, shape, 0, 0, stream);
     return launch_decode<128, true>(q, q_stride, out, out_stride, kcache, vcache, block_tables, max_pages, positions, S, H, KV,
-                                    page_size, window, scale, splits, (float*)partials, arrived, tail, shape, stream);
+                                    page_size, window, scale, splits, (float*)partials, arrived, tail, shape, 0, 0, stream);
 }

@@ -65,6 +65,7 @@ struct StepArrays {
     int max_new = 0;                // longest portion in the batch
     int lead_single = 0;            // leading requests that bring exactly one token (rows 0 .. lead_single - 1)
     int64_t max_seq_len = 0;        // longest context after this step
+    int64_t total_len = 0;          // all contexts after this step, summed
     bool any_sampling = false;      // some row has temperature > 0
     std::vector<int64_t> ids;       // request of each sequence, in batch order
     std::vector<int32_t> new_counts;
@@ -146,6 +147,7 @@ inline StepArrays build_step(const CacheManager& cache, const std::vector<StepEn
         A.max_new = std::max(A.max_new, n);
         if (n == 1 && A.lead_single == (int)A.ids.size()) ++A.lead_single;
         A.max_seq_len = std::max<int64_t>(A.max_seq_len, ctx + n);
+        A.total_len += ctx + n;
         A.ids.push_back(e.id);
         A.new_counts.push_back(n);
     }

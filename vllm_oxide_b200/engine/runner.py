@@ -27,6 +27,7 @@ from ..config import EngineConfig, architecture_for, read_config_json
 from ..csrc.build import runtime_module
 from ..errors import CapacityError, KernelError, ShapeError
 from ..tuning import TUNING
+from ..parts.attention import decode_balance_rule
 from ..parts.base import ModelSpec, StepContext, Workspace, aligned
 from ..weights import load_safetensors_weights, weights_from_tensors
 
@@ -179,6 +180,7 @@ class ModelRunner:
         self.after_block = None                 # debugging: a function (call number, residual, pending) run behind every block
         self._pending_scale = None
         self._graph_launches = {}
+        self._balance_rule = None               # (kv heads, head size, SMs) of `_balance`, () for none; read off the parts at first use
         self._graph_logits = {}                 # class of a decode step -> its logits in the workspace (None where the head picks without)
         self._kept_seen = set()                 # classes of decode steps that keep their logits and have come once
         self._graph_pool = None
@@ -527,14 +529,14 @@ class ModelRunner:
             self.upload(arrays, parity)
         long_context = bool(arrays.max_seq_len > TUNING.long_context_keys)
         if not self.decode_graphs:
-            logits = self._decode_eager(S, parity, long_context, logits_out is not None)      # nothing is recorded: no padding needed
+            logits = self._decode_eager(S, parity, long_context, logits_out is not None, self._balance(arrays, S))      # nothing is recorded: no padding needed
         else:
             b = self._bucket(S)
-            key = (b, parity, long_context, logits_out is not None)
+            key = (b, parity, long_context, logits_out is not None, self._balance(arrays, b))
             graph = self._graphs.get(key)
             if graph is None and logits_out is not None and key not in self._kept_seen:
                 self._kept_seen.add(key)
-                logits = self._decode_eager(S if self.pools.state else b, parity, long_context, True)
+                logits = self._decode_eager(S if self.pools.state else b, *key[1:])
             elif graph is None:
                 # first step of this class: run it eagerly (that is this step's result), then record
                 # the same launches for the steps to come. Padding requests (no rows, state slot 0)
@@ -565,6 +567,16 @@ class ModelRunner:
         torch.cuda.current_stream().synchronize()
         return self.sampled_host_np[parity, :S].tolist()
 
+    def _balance(self, arrays, seqs: int) -> int:
+        """`StepContext.balance` of a decode step of `seqs` requests: what the first of the model's attention mixers that can
+        deal its blocks out by length is best given (they are alike in the models there are; a model without one gets 0)."""
+        if self._balance_rule is None:
+            rules = (getattr(b.mixer, "balance_rule", lambda: None)() for b in self.spec.blocks if getattr(b, "mixer", None) is not None)
+            self._balance_rule = next((r for r in rules if r is not None), ())
+        if not self._balance_rule:
+            return 0
+        return decode_balance_rule(seqs, *self._balance_rule, int(arrays.max_seq_len), int(arrays.total_len))
+
     def decode_arrays(self, scheduler, plan):
         """The device arrays of a decode step's plan, in the decode steps' layout."""
         L = self.decode_layout
@@ -591,13 +603,14 @@ class ModelRunner:
         event.synchronize()
         return self.sampled_host_np[parity, :count].tolist()
 
-    def _decode_eager(self, b: int, parity: int = 0, long_context: bool = False, keep_logits: bool = False) -> Optional[torch.Tensor]:
+    def _decode_eager(self, b: int, parity: int = 0, long_context: bool = False, keep_logits: bool = False,
+                      balance: int = 0) -> Optional[torch.Tensor]:
         L = self.decode_layout
         self.workspace.reset()
         self._dev = self._devs[parity]          # this step's metadata (a recorded step keeps reading this buffer)
         try:
             ctx = self.context(b, b, None, L)
-            ctx.decode_only, ctx.max_new, ctx.long_context = True, 1, long_context
+            ctx.decode_only, ctx.max_new, ctx.long_context, ctx.balance = True, 1, long_context, balance
             resid, pending = self._forward(ctx)
             # the picks also go to the host buffer of this parity and, as the next decode step's
             # tokens should it be fed from the device, to the token rows of the other metadata buffer:

@@ -2131,7 +2131,7 @@ def attn_prefill_sm100(q, out, kcache, vcache, block_tables, seq_starts, context
 def attn_decode_mma(q, out, kcache, vcache, block_tables, positions, num_heads: int, num_kv_heads: int, head_dim: int,
                     scale: float, window: int = 0, splits: int = 1, partials=None, arrived=None, sink=None, gate=None,
                     out_scale: float = 1.0, chunk: int = 0, softcap: float = 0.0, dist_bias=None, keep_first: int = 0,
-                    dist_slopes=None, key_scale=None) -> None:
+                    dist_slopes=None, key_scale=None, balance: int = 0) -> None:
     """`sink`, `gate`, `out_scale`: see `_attn_tail`; `chunk`, `softcap`, `dist_bias`, `keep_first`, `dist_slopes`, `key_scale` and
     `vcache is kcache`: see `_score_shape` (`gate` may have one column per head there).
     Tensor-core attention for a step of single tokens, row i belonging to request i (bfloat16).
@@ -2139,7 +2139,9 @@ def attn_decode_mma(q, out, kcache, vcache, block_tables, positions, num_heads: 
     which merge their partial results through distributed shared memory. With `partials` (float32,
     `attn_decode_partial_floats` elements) and `arrived` (int32 zeros, one per request and kv head;
     the kernel leaves them zero) up to 64 blocks share a request without a cluster and merge
-    through global memory: for few requests with long contexts."""
+    through global memory: for few requests with long contexts. With `balance` (2 to 64; no window, no shaped scores, at most
+    `DECODE_BALANCE_SEQS` requests) some `balance` blocks per kv head are dealt out to the requests by their lengths, merging the
+    same way (`splits` is not used): for requests of very different lengths."""
     op = "attn_decode_mma"
     shape = _score_shape(op, q, num_heads, chunk, softcap, dist_bias, window, keep_first, dist_slopes, key_scale, kcache, vcache, gate)
     if shape is None and not scale > 0:
@@ -2154,12 +2156,15 @@ def attn_decode_mma(q, out, kcache, vcache, block_tables, positions, num_heads: 
         raise ShapeError(op, f"{num_heads // num_kv_heads} heads per kv head: the decode kernel takes at most 16")
     if (partials is None) != (arrived is None):
         raise ShapeError(op, "partials and arrived go together")
+    if balance and (partials is None or not 2 <= balance <= 64 or window or shape is not None or S > DECODE_BALANCE_SEQS):
+        raise ShapeError(op, f"balance must be 2..64, with partials, no window, no shaped scores and at most {DECODE_BALANCE_SEQS} requests")
     most = 8 if partials is None else 64
     if not 1 <= splits <= most:
         raise ShapeError(op, f"splits must be 1..{most}, got {splits}")
     if partials is not None:
         _cuda(op, partials, arrived)
-        need = attn_decode_partial_floats(S, num_kv_heads, head_dim, splits)
+        need = attn_decode_partial_floats(1, num_kv_heads, head_dim, 2 * balance) if balance else \
+            attn_decode_partial_floats(S, num_kv_heads, head_dim, splits)
         if partials.dtype != torch.float32 or not partials.is_contiguous() or partials.numel() < need or partials.data_ptr() % 16:
             raise ShapeError(op, f"partials must be contiguous float32, 16-byte aligned, with at least {need} elements")
         if arrived.dtype != torch.int32 or not arrived.is_contiguous() or arrived.numel() < S * num_kv_heads:
@@ -2171,9 +2176,12 @@ def attn_decode_mma(q, out, kcache, vcache, block_tables, positions, num_heads: 
             block_tables.shape[1], _ptr(positions), S, num_heads, num_kv_heads, head_dim, kcache.shape[2], int(window),
             float(scale), int(splits), _ptr(partials), _ptr(arrived), *tail)
     if shape is None:
-        _check(_fn("attention_mma", "vob_attn_decode_mma", sig + [_P])(*args, _stream()), op)
+        _check(_fn("attention_mma", "vob_attn_decode_mma", sig + [_I, _P])(*args, int(balance), _stream()), op)
     else:
         _check(_fn("attention_mma", "vob_attn_decode_shaped", sig + [_I, _F, _P, _P, _I, _P, _I, _P])(*args, *shape[0], *shape[1], gate_heads, _stream()), op)
+
+
+DECODE_BALANCE_SEQS = 128        # most requests of a balanced decode launch
 
 
 def attn_decode_partial_floats(num_seqs: int, num_kv_heads: int, head_dim: int, splits: int) -> int:

@@ -49,6 +49,24 @@ def decode_split_rule(num_seqs: int, kv_heads: int, num_sms: int, long_context: 
     return max(1, min(8, hi if lo < hi <= 6 else lo)), False
 
 
+def decode_balance_rule(num_seqs: int, kv_heads: int, head_dim: int, num_sms: int, max_len: int, total_len: int) -> int:
+    """Blocks per kv head to deal out by length (0: every request gets the same number, `decode_split_rule`). Worth it where a
+    block of the longest request would walk so many more tiles of 64 keys than its share of all of them that this takes longer
+    than the merge through global memory costs over the merge in a cluster. Measured with 8 kv heads of 64, in clusters / balanced, and
+    how many tiles more: 8 requests of 100 to 2,000 keys 8.8 / 9.9 us (3), two of 4,000 and 200 keys 9.0 / 10.4 (5), 16 of 100 to 2,000
+    13.2 / 10.9 (7), 16 of 100 to 4,000 22.0 / 14.4 (15), 64 of 17 to 1,000 19.6 / 18.3 (10); heads of 128, where a tile takes twice as
+    long: 8 of 100 to 2,000 13.3 / 12.5 (3), 16 of 17 to 1,000 12.5 / 11.0 (3), 16 of 100 to 4,000 38 / 22 (13)."""
+    # three blocks an SM with three stages at head size 64, two at 128
+    want = min(64, num_sms * (3 if head_dim <= 64 else 2) // kv_heads)
+    if want < 2 or num_seqs > kernels.DECODE_BALANCE_SEQS:
+        return 0
+    splits, wide = decode_split_rule(num_seqs, kv_heads, num_sms, max_len > TUNING.long_context_keys)
+    longest = -(-max_len // 64)
+    walks = -(-longest // min(splits, max(1, longest // 3)) if wide else -longest // splits)
+    share = max(3, -(-(total_len // 64 + num_seqs) // want))
+    return want if (walks - share) * head_dim >= TUNING.balance_tiles * 64 else 0
+
+
 class Attention(Mixer):
     def __init__(self, wq: torch.Tensor, wk: Optional[torch.Tensor], wv: Optional[torch.Tensor], wo: torch.Tensor,
                  num_heads: int, num_kv_heads: int, head_dim: int, position=None, window: Optional[int] = None,
@@ -198,12 +216,25 @@ class Attention(Mixer):
     def _attend_single(self, q, out, ctx: StepContext, cache: LayerCache, bt, count: int) -> None:
         """The decode kernel on the first `count` rows, row i belonging to request i."""
         splits, wide = self.decode_splits(count, ctx.long_context)
-        if wide and self._partials is None:
-            floats = kernels.attn_decode_partial_floats(1, 1, self.hd, 3 * self.num_sms)    # requests x kv heads x splits <= 3 SMs
+        balance = ctx.balance if ctx.decode_only and self.window == 0 else 0
+        if (wide or balance) and self._partials is None:
+            # requests x kv heads x splits <= 3 SMs; of a balanced launch at most 2 x 64 per kv head and 2 x 3 SMs in all
+            blocks = max(3 * self.num_sms, min(6 * self.num_sms, 128 * self.KV))
+            floats = kernels.attn_decode_partial_floats(1, 1, self.hd, blocks)
             self._partials = torch.empty(floats, dtype=torch.float32, device=q.device)
-            self._arrived = torch.zeros(self.num_sms, dtype=torch.int32, device=q.device)
+            self._arrived = torch.zeros(max(self.num_sms, kernels.DECODE_BALANCE_SEQS * self.KV), dtype=torch.int32, device=q.device)
+        if balance:
+            kernels.attn_decode_mma(q[:count], out[:count], cache.k, cache.v, bt, ctx.positions[:count], self.H, self.KV, self.hd,
+                                    self.scale, 0, 1, self._partials, self._arrived, balance=balance)
+            return
         kernels.attn_decode_mma(q[:count], out[:count], cache.k, cache.v, bt, ctx.positions[:count], self.H, self.KV, self.hd,
                                 self.scale, self.window, splits, self._partials if wide else None, self._arrived if wide else None)
+
+    def balance_rule(self):
+        """(kv heads, head size, SMs) for `decode_balance_rule`, or None where this mixer's single tokens never run balanced."""
+        if self.dtype != torch.bfloat16 or self.window or self.hd not in kernels.TENSOR_CORE_HEAD_DIMS or self.H // self.KV > 16:
+            return None
+        return self.KV, self.hd, self.num_sms
 
     def decode_splits(self, num_seqs: int, long_context: bool = False):
         return decode_split_rule(num_seqs, self.KV, self.num_sms, long_context)

@@ -158,7 +158,7 @@ class StepContext:
 
     Steps are recorded as CUDA graphs and replayed for later steps of the same shape class, so
     what a part launches may depend only on the host facts below that make up the class (`rows`,
-    `seqs`, `max_new` as an upper bound, `decode_only`, `lead_single`, `long_context`) and on its
+    `seqs`, `max_new` as an upper bound, `decode_only`, `lead_single`, `long_context`, `balance`) and on its
     own constants; everything else must be read on the device, from the tensors. `max_seq_len`
     and `host` are there for checks and debugging only (a recording is made with neither)."""
     rows: int                       # rows the kernels run over (real rows, or the padded count)
@@ -182,6 +182,8 @@ class StepContext:
                                     # rows 0 .. lead_single - 1 are theirs, row i belonging to request i
     long_context: bool = False      # some request is longer than TUNING.long_context_keys (host fact; a replayed
                                     # step was recorded with the same value)
+    balance: int = 0                # in a step of single tokens: blocks per kv head that attention deals out to the requests by
+                                    # length (host fact; 0: the same number for every request)
     host: Optional[object] = None   # the host-side StepArrays (ids, counts) for parts that want them
     shared: Dict[str, torch.Tensor] = field(default_factory=dict)   # what one layer of this step leaves for later layers of
                                     # the same step, by name: the buffers `ModelSpec.step_buffers` names, one row per row
