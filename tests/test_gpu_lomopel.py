@@ -588,3 +588,41 @@ def test_command_line_generates_from_a_lomopel_folder(tmp_path):
     assert len(got) == 6
     logits = _plain_logits(d, toks + got)
     assert got[0] == int(logits[3].argmax())
+
+
+@pytest.mark.parametrize("K,V,H,G,dt", [(128, 128, 4, 2, torch.bfloat16), (64, 64, 2, 2, torch.float32), (32, 32, 3, 1, torch.bfloat16), (20, 8, 2, 1, torch.float32),
+                                        (256, 40, 2, 2, torch.bfloat16), (100, 24, 2, 1, torch.float32), (512, 4, 1, 1, torch.bfloat16), (8, 2, 1, 1, torch.float32)])
+def test_gated_delta_scan_of_aligned_rows_gives_the_same_bits(K, V, H, G, dt):
+    """Operands that 16-byte copies can take go to a kernel of their own; shifted by one element they go to the general one. Same sums
+    in the same order: outputs, states and the convolution's inputs are the same to the bit, for portions around its stage of four
+    tokens, requests without rows, and a second portion behind the first."""
+    from vllm_oxide_b200 import kernels
+    g = torch.Generator().manual_seed(K + V)
+    lens = [5, 1, 0, 4, 33, 16, 3]
+    T, S, C, taps = sum(lens), len(lens), 24, 4
+    starts = torch.tensor([0] + lens).cumsum(0).to(torch.int32).to(DEV)
+    slots = torch.tensor([3, 0, 1, 2, 7, 5, 6], dtype=torch.int32, device=DEV)
+
+    def off(t, n):          # the same values, n elements behind an aligned address
+        buf = torch.zeros(t.shape[0], t.shape[1] + 16, dtype=t.dtype, device=DEV)
+        buf[:, n:n + t.shape[1]] = t.to(DEV)
+        return buf[:, n:n + t.shape[1]]
+    r, k = (torch.randn(T, G * K, generator=g) / K ** 0.5 for _ in range(2))
+    v = torch.randn(T, H * V, generator=g).to(dt)
+    w = torch.rand(T, H * K, generator=g).to(DEV)
+    b = torch.rand(T, H, generator=g).to(DEV)
+    cx = torch.randn(T, C, generator=g).to(dt).to(DEV)
+    state0 = torch.randn(8, H, K, V, generator=g).to(DEV)
+    conv0 = torch.randn(8, taps - 1, C, generator=g).to(DEV)
+    got = []
+    for shift in (0, 1):
+        state, conv, outs = state0.clone(), conv0.clone(), []
+        for _ in range(2):
+            out = torch.full((T, H * V), 7.0, device=DEV)
+            kernels.recurrence_scan(2, off(r, shift), off(k, shift), off(v, shift), w, b, None, state, starts, slots, S, H, out, rk_heads=G,
+                                    conv_x=cx, conv_state=conv)
+            outs.append(out)
+        got.append((state, conv, *outs))
+    for x, y in zip(*got):
+        assert torch.equal(x, y)
+    assert torch.equal(got[0][0][4], state0[4]) and torch.equal(got[0][0][1], state0[1]) and not torch.equal(got[0][0][7], state0[7])

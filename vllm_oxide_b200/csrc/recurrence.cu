@@ -739,6 +739,247 @@ recurrence_scan_kernel(const TRK* __restrict__ r, long ld_r, const TRK* __restri
     }
 }
 
+// ---------------------------------------------------------------------------------------------
+// Mode 2 for float32 r and k in rows that 16-byte copies can take: the same sums in the same order (the same bits) as the kernel
+// above. What bounds a long portion is the chain from token to token, and of its 730 clocks a token (one request, K = V = 128)
+// little was arithmetic: tokens went through registers into shared memory (some 80 instructions a token and thread), four warps
+// each read the whole of r, k and w, and single FMAs run at half rate. Here tokens arrive by cp.async in a ring of stages, whose
+// addresses a thread works out once; a thread may have two columns (NC), so that what it reads of r, k and w serves twice, in
+// blocks of two warps; and products are formed in pairs of channels (mul and fma .f32x2, each half rounded as the single operation).
+// 16 heads of 128: one request of 1,500 tokens 726 -> 466 us, four of 200 to 766 tokens 588 -> 341, 16 of 128 tokens 462 -> 219. What is
+// left is the chain itself: 206 instructions a token and warp, most of whose clocks wait for the result in front. (A third warp that
+// does all the copying was no faster, 441 and 336 us, and slower at single tokens.)
+// Grid (ceil(V / VT), H, requests), VT = NC * 64 / KS columns a block.
+// ---------------------------------------------------------------------------------------------
+__device__ __forceinline__ void fma2(unsigned long long& d, unsigned long long a, unsigned long long b) {
+    asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(d) : "l"(a), "l"(b));
+}
+__device__ __forceinline__ unsigned long long pack2(float lo, float hi) {
+    unsigned long long x;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(x) : "f"(lo), "f"(hi));
+    return x;
+}
+__device__ __forceinline__ float sum2(unsigned long long d) {
+    float lo, hi;
+    asm("mov.b64 {%0, %1}, %2;" : "=f"(lo), "=f"(hi) : "l"(d));
+    return lo + hi;
+}
+template <int BYTES> __device__ __forceinline__ void cp_async(void* dst, const void* src) {
+    const unsigned d = (unsigned)__cvta_generic_to_shared(dst);
+    if constexpr (BYTES == 16) asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(d), "l"(src) : "memory");
+    else asm volatile("cp.async.ca.shared.global [%0], [%1], %2;" ::"r"(d), "l"(src), "n"(BYTES) : "memory");
+}
+
+// One or two neighbouring columns.
+template <int NC> __device__ __forceinline__ void load_cols(float* x, const float* p, bool in) {
+    if constexpr (NC == 2) {
+        const float2 f = in ? *reinterpret_cast<const float2*>(p) : make_float2(0.f, 0.f);
+        x[0] = f.x; x[1] = f.y;
+    } else x[0] = in ? *p : 0.f;
+}
+template <int NC> __device__ __forceinline__ void store_cols(float* p, const float* x) {
+    if constexpr (NC == 2) *reinterpret_cast<float2*>(p) = make_float2(x[0], x[1]);
+    else *p = x[0];
+}
+
+constexpr int DELTA_CT = 4, DELTA_STAGES = 4;        // tokens of a stage, stages of the ring
+
+// One token in shared memory, in floats: r, k, w as in the kernel above, the columns of v in their own type, the strength.
+template <int KPT, int KS, int NC, typename TV> struct DeltaToken {
+    static constexpr int KPADP = KS * (KPT + 4), VT = NC * 64 / KS;
+    static constexpr int V_PIECE = VT * (int)sizeof(TV) < 16 ? VT * (int)sizeof(TV) : 16;      // bytes of a copy of v
+    static constexpr int V_AT = 3 * KPADP, B_AT = V_AT + (VT * (int)sizeof(TV) + 15) / 16 * 4, FLOATS = B_AT + 4;
+};
+
+template <int KPT, int KS, int NC, typename TV>
+__global__ void __launch_bounds__(64, KPT * KS <= 256 ? 6 : 1)
+delta_scan_kernel(const float* __restrict__ r, long ld_r, const float* __restrict__ k, long ld_k, const TV* __restrict__ v, long ld_v,
+                  const float* __restrict__ w, const float* __restrict__ b, float* __restrict__ state, const int* __restrict__ seq_starts,
+                  const int* __restrict__ state_slots, float* __restrict__ o, int H, int K, int V, int rk_div,
+                  const TV* __restrict__ conv_x, long ld_cx, int conv_c, int conv_taps, float* __restrict__ conv_state) {
+    using Tok = DeltaToken<KPT, KS, NC, TV>;
+    constexpr int KPAD = KS * KPT, VT = Tok::VT, CT = DELTA_CT, ST = DELTA_STAGES;
+    constexpr int NV = VT * (int)sizeof(TV) / Tok::V_PIECE, PIECES = 3 * KPAD / 4 + NV + 1, NPT = (PIECES + 63) / 64;
+    pdl_launch_dependents();
+    extern __shared__ __align__(16) float sm[];      // [ST][CT][Tok::FLOATS]
+    const int tid = threadIdx.x;
+    for (int i = tid; i < ST * CT * Tok::FLOATS; i += 64) sm[i] = 0.f;       // channels beyond K stay zero
+    pdl_wait(43);
+    const int s = blockIdx.z, h = blockIdx.y, hk = h / rk_div;
+    const int r0 = seq_starts[s], r1 = seq_starts[s + 1];
+    if (r1 <= r0) return;
+    const int slot = state_slots[s];
+    if (conv_x) {
+        float* st = conv_state + (size_t)slot * (conv_taps - 1) * conv_c;
+        const int blocks = gridDim.x * gridDim.y;
+        for (int c = (blockIdx.y * gridDim.x + blockIdx.x) * 64 + tid; c < conv_c; c += blocks * 64)
+            conv_state_shift(conv_x, ld_cx, conv_c, conv_taps, st, r0, r1 - r0, c);
+    }
+    const int q = tid % KS, jj = tid / KS * NC;
+    const int j0 = blockIdx.x * VT, j = j0 + jj;
+    const bool col = j < V;                          // with two columns V is even: both or none
+    // this thread's pieces of a token: where they come from (row 0), how far apart rows are, where they go
+    const char* src[NPT];
+    long step[NPT];
+    int dst[NPT];                                    // float index; -1: none
+    const int k4 = K / 4;
+#pragma unroll
+    for (int i = 0; i < NPT; ++i) {
+        const int x = tid + i * 64;
+        src[i] = nullptr; step[i] = 0; dst[i] = -1;
+        if (x < 3 * k4) {
+            const int a = x / k4, c = x % k4 * 4;
+            const float* p = a == 0 ? r + (size_t)hk * K + c : a == 1 ? k + (size_t)hk * K + c : w + (size_t)h * K + c;
+            src[i] = reinterpret_cast<const char*>(p);
+            step[i] = 4 * (a == 0 ? ld_r : a == 1 ? ld_k : (long)H * K);
+            dst[i] = a * Tok::KPADP + (c / KPT) * (KPT + 4) + c % KPT;
+        } else if (x < 3 * k4 + NV) {
+            const int e = (x - 3 * k4) * (Tok::V_PIECE / (int)sizeof(TV));
+            if (j0 + e < V) {
+                src[i] = reinterpret_cast<const char*>(v + (size_t)h * V + j0 + e);
+                step[i] = (long)sizeof(TV) * ld_v;
+                dst[i] = Tok::V_AT + e * (int)sizeof(TV) / 4;
+            }
+        } else if (x == 3 * k4 + NV) {
+            src[i] = reinterpret_cast<const char*>(b + h);
+            step[i] = 4 * (long)H;
+            dst[i] = Tok::B_AT;
+        }
+    }
+    __syncthreads();                                 // the zeros are there before anything is copied over them
+    auto fetch = [&](int c0, int stage) {
+#pragma unroll
+        for (int tt = 0; tt < CT; ++tt) {
+            if (c0 + tt < r1) {
+#pragma unroll
+                for (int i = 0; i < NPT; ++i) {
+                    if (dst[i] < 0) continue;
+                    float* d = sm + (stage * CT + tt) * Tok::FLOATS + dst[i];
+                    const char* p = src[i] + (size_t)(c0 + tt) * step[i];
+                    if (dst[i] < Tok::V_AT) cp_async<16>(d, p);
+                    else if (dst[i] < Tok::B_AT) cp_async<Tok::V_PIECE>(d, p);
+                    else cp_async<4>(d, p);
+                }
+            }
+        }
+        asm volatile("cp.async.commit_group;" ::: "memory");
+    };
+#pragma unroll
+    for (int g = 0; g < ST - 1; ++g) fetch(r0 + g * CT, g);
+    float* S_glob = state + ((size_t)slot * H + h) * K * V;
+    unsigned long long S[NC][KPT / 2];               // channels 2 i and 2 i + 1 of column j (and j + 1)
+#pragma unroll
+    for (int i = 0; i < KPT / 2; ++i) {
+        float x[2][NC];
+#pragma unroll
+        for (int e = 0; e < 2; ++e) {
+            const int c = q * KPT + 2 * i + e;
+            load_cols<NC>(x[e], S_glob + (size_t)c * V + j, col && c < K);
+        }
+#pragma unroll
+        for (int m = 0; m < NC; ++m) S[m][i] = pack2(x[0][m], x[1][m]);
+    }
+    auto token = [&](const float* t, int row) {
+        const ulonglong2* pr = reinterpret_cast<const ulonglong2*>(t + q * (KPT + 4));
+        const ulonglong2* pk = reinterpret_cast<const ulonglong2*>(t + Tok::KPADP + q * (KPT + 4));
+        const ulonglong2* pw = reinterpret_cast<const ulonglong2*>(t + 2 * Tok::KPADP + q * (KPT + 4));
+        const TV* pv = reinterpret_cast<const TV*>(t + Tok::V_AT) + jj;
+        const float strength = t[Tok::B_AT];
+        unsigned long long kk[KPT / 2], d[NC][2] = {}, e[NC][2] = {}, f[2] = {0, 0};
+#pragma unroll
+        for (int i = 0; i < KPT / 4; ++i) {
+            const ulonglong2 rr = pr[i], k2 = pk[i], ww = pw[i];
+            kk[2 * i] = k2.x; kk[2 * i + 1] = k2.y;
+#pragma unroll
+            for (int m = 0; m < NC; ++m) {
+                asm("mul.rn.f32x2 %0, %0, %1;" : "+l"(S[m][2 * i]) : "l"(ww.x));
+                asm("mul.rn.f32x2 %0, %0, %1;" : "+l"(S[m][2 * i + 1]) : "l"(ww.y));
+                fma2(d[m][0], k2.x, S[m][2 * i]); fma2(d[m][1], k2.y, S[m][2 * i + 1]);
+                fma2(e[m][0], rr.x, S[m][2 * i]); fma2(e[m][1], rr.y, S[m][2 * i + 1]);
+            }
+            fma2(f[0], rr.x, k2.x); fma2(f[1], rr.y, k2.y);
+        }
+        float dot[NC], read[NC], rk = sum2(f[0]) + sum2(f[1]);
+#pragma unroll
+        for (int m = 0; m < NC; ++m) { dot[m] = sum2(d[m][0]) + sum2(d[m][1]); read[m] = sum2(e[m][0]) + sum2(e[m][1]); }
+#pragma unroll
+        for (int off = 1; off < KS; off <<= 1) {
+#pragma unroll
+            for (int m = 0; m < NC; ++m) {
+                dot[m] += __shfl_xor_sync(0xffffffffu, dot[m], off);
+                read[m] += __shfl_xor_sync(0xffffffffu, read[m], off);
+            }
+            rk += __shfl_xor_sync(0xffffffffu, rk, off);
+        }
+        float uu[NC], out[NC];
+#pragma unroll
+        for (int m = 0; m < NC; ++m) {
+            uu[m] = strength * (ld_f(pv + m) - dot[m]);
+            const unsigned long long u2 = pack2(uu[m], uu[m]);
+#pragma unroll
+            for (int i = 0; i < KPT / 2; ++i) fma2(S[m][i], kk[i], u2);
+        }
+#pragma unroll
+        for (int m = 0; m < NC; ++m) out[m] = fmaf(rk, uu[m], read[m]);
+        if (q == 0 && col) store_cols<NC>(o + (size_t)row * H * V + (size_t)h * V + j, out);
+    };
+    int stage = 0;
+    for (int c0 = r0; c0 < r1; c0 += CT) {
+        asm volatile("cp.async.wait_group %0;" ::"n"(ST - 2) : "memory");
+        __syncthreads();                             // this stage is here for everyone, and everyone is through with the one in front
+        fetch(c0 + (ST - 1) * CT, stage == 0 ? ST - 1 : stage - 1);
+        const float* t = sm + stage * CT * Tok::FLOATS;
+        if (c0 + CT <= r1) {
+#pragma unroll
+            for (int tt = 0; tt < CT; ++tt) token(t + tt * Tok::FLOATS, c0 + tt);
+        } else {
+            for (int tt = 0; c0 + tt < r1; ++tt) token(t + tt * Tok::FLOATS, c0 + tt);
+        }
+        stage = stage + 1 == ST ? 0 : stage + 1;
+    }
+    asm volatile("cp.async.wait_group 0;" ::: "memory");
+#pragma unroll
+    for (int i = 0; i < KPT / 2; ++i) {
+        float x[2][NC];
+#pragma unroll
+        for (int m = 0; m < NC; ++m) asm("mov.b64 {%0, %1}, %2;" : "=f"(x[0][m]), "=f"(x[1][m]) : "l"(S[m][i]));
+#pragma unroll
+        for (int e = 0; e < 2; ++e) {
+            const int c = q * KPT + 2 * i + e;
+            if (col && c < K) store_cols<NC>(S_glob + (size_t)c * V + j, x[e]);
+        }
+    }
+}
+
+// One column a thread where its warps find no second one on their scheduler anyway (at most 512 warps of one column on 592
+// schedulers, as one request of 16 heads of 128): the chain of a token is shorter. 16 heads of 128, one / two columns: one request of
+// 1,500 tokens 466 / 522 us, two of 500 tokens 219 / 196 us, four of 200 to 766 tokens 419 / 341 us.
+static bool delta_scan_one_column(int seqs, int H, int V, int ks) { return (long)seqs * H * V * ks <= 512L * 32; }
+
+// Whether the kernel above takes these operands: 16-byte pieces of r, k and w, pieces of v, pairs of columns.
+template <int KS, int NC, typename TV>
+static bool delta_scan_takes(const void* r, long ld_r, const void* k, long ld_k, const void* v, long ld_v, const void* w, const void* state,
+                             const void* o, int K, int V) {
+    using Tok = DeltaToken<16, KS, NC, TV>;
+    const long v_elems = Tok::V_PIECE / (long)sizeof(TV);
+    return K % 4 == 0 && V % NC == 0 && V % v_elems == 0 && ld_r % 4 == 0 && ld_k % 4 == 0 && ld_v % v_elems == 0 &&
+           (((uintptr_t)r | (uintptr_t)k | (uintptr_t)w) & 15) == 0 && ((uintptr_t)v & (Tok::V_PIECE - 1)) == 0 &&
+           (((uintptr_t)state | (uintptr_t)o) & 7) == 0;
+}
+
+template <int KPT, int KS, int NC, typename TV>
+static int delta_scan(const void* r, long ld_r, const void* k, long ld_k, const void* v, long ld_v, const float* w, const float* b,
+                      float* state, const int* seq_starts, const int* state_slots, float* o, int seqs, int H, int K, int V, int rk_div,
+                      const void* conv_x, long ld_cx, int conv_c, int conv_taps, float* conv_state, cudaStream_t stream) {
+    using Tok = DeltaToken<KPT, KS, NC, TV>;
+    const size_t smem = sizeof(float) * DELTA_STAGES * DELTA_CT * Tok::FLOATS;
+    const cudaError_t e = cudaFuncSetAttribute(delta_scan_kernel<KPT, KS, NC, TV>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (e != cudaSuccess) return (int)e;
+    return vob_launch(delta_scan_kernel<KPT, KS, NC, TV>, dim3((V + Tok::VT - 1) / Tok::VT, H, seqs), dim3(64), smem, stream, (const float*)r, ld_r,
+                      (const float*)k, ld_k, (const TV*)v, ld_v, w, b, state, seq_starts, state_slots, o, H, K, V, rk_div, (const TV*)conv_x,
+                      ld_cx, conv_c, conv_taps, conv_state);
+}
+
 // How the key channels are shared out: KS lanes per column (a power of two) with KPT state registers each:
 // K <= 32: 4 x 8; <= 64: 4 x 16; <= 128: 8 x 16; <= 256: 16 x 16; <= 512: 32 x 16.
 template <int MODE, typename TRK, typename TV>
@@ -746,13 +987,21 @@ static int scan_launch(const void* r, long ld_r, const void* k, long ld_k, const
                        const float* u, float* state, const int* seq_starts, const int* state_slots, float* o, int seqs, int H, int K,
                        int V, int rk_div, const void* conv_x, long ld_cx, int conv_c, int conv_taps, float* conv_state, cudaStream_t stream) {
 #define VOB_SCAN(P, KS_)                                                                                                        \
+    if constexpr (MODE == 2) {                                                                                                  \
+        if (delta_scan_one_column(seqs, H, V, KS_) && delta_scan_takes<KS_, 1, TV>(r, ld_r, k, ld_k, v, ld_v, w, state, o, K, V)) \
+            return delta_scan<P, KS_, 1, TV>(r, ld_r, k, ld_k, v, ld_v, w, b, state, seq_starts, state_slots, o, seqs, H, K, V, rk_div, \
+                                             conv_x, ld_cx, conv_c, conv_taps, conv_state, stream);                             \
+        if (delta_scan_takes<KS_, 2, TV>(r, ld_r, k, ld_k, v, ld_v, w, state, o, K, V))                                         \
+            return delta_scan<P, KS_, 2, TV>(r, ld_r, k, ld_k, v, ld_v, w, b, state, seq_starts, state_slots, o, seqs, H, K, V, rk_div, \
+                                             conv_x, ld_cx, conv_c, conv_taps, conv_state, stream);                             \
+    }                                                                                                                           \
     return vob_launch(recurrence_scan_kernel<MODE, P, KS_, TRK, TV>, dim3((V + 128 / KS_ - 1) / (128 / KS_), H, seqs), dim3(128), 0,  \
                       stream, (const TRK*)r, ld_r, (const TRK*)k, ld_k, (const TV*)v, ld_v, w, b, u, state, seq_starts, state_slots, o, \
                       H, K, V, rk_div, (const TV*)conv_x, ld_cx, conv_c, conv_taps, conv_state)
-    if (K <= 32) VOB_SCAN(8, 4);
-    if (K <= 64) VOB_SCAN(16, 4);
-    if (K <= 128) VOB_SCAN(16, 8);
-    if (K <= 256) VOB_SCAN(16, 16);
+    if (K <= 32) { VOB_SCAN(8, 4); }
+    if (K <= 64) { VOB_SCAN(16, 4); }
+    if (K <= 128) { VOB_SCAN(16, 8); }
+    if (K <= 256) { VOB_SCAN(16, 16); }
     VOB_SCAN(16, 32);
 #undef VOB_SCAN
 }
