@@ -593,7 +593,7 @@ def test_attn_decode_mma_balanced(H, KV, hd, page, S, balance, most):
         args = (kc, vc, bt, pos, H, KV, hd, 1.0 / math.sqrt(hd))
         k.attn_decode_mma(q, want, *args)
         k.attn_decode_mma(q, got, *args, 0, 1, partials, arrived, balance=balance)
-        # P is rounded to bfloat16 relative to another maximum, and so is the result: two roundings of 2^-9 of either
+        # P is rounded to bfloat16 relative to another maximum, and so is the result: two roundings of 2^-8 at most
         assert rel(got, want.double().cpu()) <= 2 ** -7 if int(lens.max()) else bool((got == 0).all())
         assert bool((got[pos < 0] == 0).all()) and int(arrived.abs().max()) == 0
     from vllm_oxide_b200.errors import ShapeError
@@ -621,6 +621,21 @@ def test_attn_mma_refusals():
 
 
 # ----------------------------------------------------------------------------- tcgen05 matrix product (bfloat16)
+@pytest.mark.parametrize("T,N,Kd", [(1, 128, 64), (3, 200, 136), (8, 3072, 2048), (16, 130, 2048), (17, 2048, 2048), (32, 77, 200), (33, 256, 512)])
+def test_linear_bf16_with_a_bias(T, N, Kd):
+    """A bias is added to the float32 sum before the result is rounded, once under a split of K too: one rounding to bfloat16 away
+    from float64, on this package's product (up to `TUNING.few_rows` rows) and on the library's behind it."""
+    g = torch.Generator().manual_seed(T + N)
+    a, w = (torch.randn(n, Kd, generator=g).to(torch.bfloat16).to(DEV) for n in (T, N))
+    bias = (30 * torch.randn(N, generator=g)).to(torch.bfloat16).to(DEV)
+    out = torch.full((T + 1, N), 7.0, dtype=torch.bfloat16, device=DEV)
+    K().linear(a, w, out[:T], bias)
+    want = a.double() @ w.double().T + bias.double()
+    # half a unit in the last of bfloat16's 8 bits (2^-8 of the value at most), and float32 sums of Kd products
+    bound = 2.0 ** -8 * 1.01 * want.abs() + Kd * 2.0 ** -24 * (a.double().abs() @ w.double().abs().T)
+    assert bool(((out[:T].double() - want).abs() <= bound).all()) and bool((out[T] == 7.0).all())
+
+
 @pytest.mark.parametrize("odt", [torch.bfloat16, torch.float32], ids=["bf16out", "f32out"])
 @pytest.mark.parametrize("T,N,Kd,splits", [
     (1, 128, 64, 1), (8, 128, 256, None), (5, 640, 8192, 8), (8, 2048, 2048, 3), (16, 256, 512, 2), (17, 200, 136, None),

@@ -130,6 +130,8 @@ struct EpiArgs {
     int* part_idx;                     // [T][ld_part] its vocabulary index
     int* nan_flags;                    // [T] raised for a row that holds a NaN
     long long ld_part;
+    // EPI_STORE
+    const __nv_bfloat16* bias;         // [N] or null: added to the float32 sum
 };
 typedef EpiArgs QkvArgs;
 
@@ -343,6 +345,8 @@ gemm_sm100_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_consta
         if (!MS) finish_scales();
         float next_w = 0.f;
         if (EPI == EPI_RESID) next_w = f < N ? qa.next_w[f] : 0.f;      // the next norm's weight of this feature
+        const bool biased = EPI == EPI_STORE && qa.bias;
+        const float bias = biased && f < N ? __bfloat162float(qa.bias[f]) : 0.f;
         asm volatile("bar.sync 1, 128;" ::: "memory");
         // Shared memory over the operand stages (every product that read them has completed by the time
         // it is written): `tile` [BT][128] is this block's tile (a partial one under a split, which
@@ -430,7 +434,7 @@ gemm_sm100_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_consta
                 if (f < N) {
 #pragma unroll
                     for (int j = 0; j < 16; ++j)
-                        if (t0 + c + j < T) store_out<OutT>(C + (size_t)(t0 + c + j) * ldc + f, r[j]);
+                        if (t0 + c + j < T) store_out<OutT>(C + (size_t)(t0 + c + j) * ldc + f, biased ? r[j] + bias : r[j]);
                 }
             }
         } else if (ok && EPI == EPI_PICK) {
@@ -539,7 +543,7 @@ gemm_sm100_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_consta
 #pragma unroll
                     for (int p = 0; p < 8; ++p) acc += part[p];       // rank order, zeros beyond the last rank
                     if (EPI == EPI_STORE) {
-                        if (f < N) store_out<OutT>(C + (size_t)(t0 + j) * ldc + f, acc);
+                        if (f < N) store_out<OutT>(C + (size_t)(t0 + j) * ldc + f, biased ? acc + bias : acc);
                     } else {
                         fin[k * BM + col] = old + acc;
                     }

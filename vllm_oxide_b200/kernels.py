@@ -736,7 +736,7 @@ class _EpiArgs(ctypes.Structure):
                 ("q_dim", _I), ("kv_dim", _I), ("hd", _I), ("KV", _I), ("page_size", _I),
                 ("ssq_tiles", _I), ("ld_ssq", _I), ("inv_h", _F), ("eps", _F), ("act", _I),
                 ("temperature", _P), ("seeds", _P), ("steps", _P), ("part_val", _P), ("part_idx", _P), ("nan_flags", _P),
-                ("ld_part", _L)]
+                ("ld_part", _L), ("bias", _P)]
 
 
 def _dp(t: Optional[torch.Tensor]) -> int:
@@ -769,11 +769,11 @@ def embed_fold(table: torch.Tensor, tokens: torch.Tensor, resid: torch.Tensor, n
 @_timed
 def gemm_fused(a: torch.Tensor, w: torch.Tensor, out: Optional[torch.Tensor], mode: int, n_features: int, *,
                ssq_in: Optional[torch.Tensor] = None, eps: float = 0.0, qkv=None, resid=None, pick=None,
-               splits: Optional[int] = None) -> None:
+               splits: Optional[int] = None, bias: Optional[torch.Tensor] = None) -> None:
     """The tcgen05 product for at most 64 rows with a fused epilogue and, optionally, the RMSNorm of
     its input folded in: `a` holds bf16(x * norm weight), `ssq_in` [tiles, ld] the per-tile sums of
     squares of x, and each token's accumulator is multiplied by 1 / sqrt(mean(x^2) + eps).
-      EPI_STORE  out[T, n] (bfloat16 or float32) = result
+      EPI_STORE  out[T, n] (bfloat16 or float32) = result (+ `bias`, contiguous bfloat16 [n], added in float32)
       EPI_SWIGLU out[T, n] = silu(gate) * up, w = [Wg; Wu] of shape [2n, K]
       EPI_QKV    qkv = (positions, slots, inv_freq, kcache, vcache, H, KV, hd): out[T, H*hd] = rotated q,
                  rotated k and v go to their cache slots
@@ -798,6 +798,11 @@ def gemm_fused(a: torch.Tensor, w: torch.Tensor, out: Optional[torch.Tensor], mo
         if ssq_in.dtype != torch.float32 or ssq_in.dim() != 2 or ssq_in.shape[0] != -(-K // 128) or ssq_in.shape[1] < T or not ssq_in.is_contiguous():
             raise ShapeError(op, f"ssq_in must be contiguous float32 [{-(-K // 128)}, >={T}], got {list(ssq_in.shape)}")
         ea.ssq_in, ea.ssq_tiles, ea.ld_ssq, ea.inv_h, ea.eps = _dp(ssq_in), ssq_in.shape[0], ssq_in.shape[1], 1.0 / K, float(eps)
+    if bias is not None:
+        _cuda(op, bias)
+        if mode != EPI_STORE or bias.dtype != torch.bfloat16 or bias.shape != (n_features,) or not bias.is_contiguous():
+            raise ShapeError(op, f"a bias goes with EPI_STORE and must be contiguous bfloat16 [{n_features}]")
+        ea.bias = _dp(bias)
     out_code, ldc, out_ptr = 1, n_features, 0
     if mode in (EPI_STORE, EPI_SWIGLU):
         if out is None or out.shape != (T, n_features) or out.stride(1) != 1 or out.dtype not in (torch.bfloat16, torch.float32):
@@ -892,7 +897,7 @@ def gemm_sm100_check() -> None:
 
 def linear(a: torch.Tensor, w: torch.Tensor, out: torch.Tensor, bias: Optional[torch.Tensor] = None) -> None:
     """out = a @ w^T (+ bias, a vector of the operands' type: added to the float32 sum before the result is
-    rounded; with a bias the bfloat16 product is the library's, whose epilogue adds it). float32 operands: the true 32-bit kernel. bfloat16 operands: this package's
+    rounded). float32 operands: the true 32-bit kernel. bfloat16 operands: this package's
     tcgen05 kernel (TMA operands, float32 accumulation in tensor memory); for many rows, or
     operands TMA cannot address (K not a multiple of 8, unaligned rows), the library product
     (cuBLAS through torch, float32 accumulation; above `TUNING.few_rows` rows), as the reference plans for its own matrix
@@ -911,7 +916,12 @@ def linear(a: torch.Tensor, w: torch.Tensor, out: torch.Tensor, bias: Optional[t
     if bias is not None:
         if bias.dtype != torch.bfloat16 or bias.shape != (w.shape[0],) or out.dtype != torch.bfloat16:
             raise ShapeError(op, f"a bias must be bfloat16 [{w.shape[0]}] with a bfloat16 result, got {bias.dtype} {list(bias.shape)}")
-        _library_gemm_bf16(a, w, out, bias)
+        # Four rows at 3,072 and 2,048 x 2,048 in a decode step: 8.6 and 7.0 us with the library, beside which no other kernel starts
+        # early; 5.6 here, and the kernels around them 0.3 to 0.5 us less each.
+        if a.shape[0] <= min(TUNING.few_rows, FUSED_GEMM_MAX_ROWS) and gemm_sm100_supported(a, w) and out.stride(1) == 1 and bias.is_contiguous():
+            gemm_fused(a, w, out, EPI_STORE, w.shape[0], bias=bias)
+        else:
+            _library_gemm_bf16(a, w, out, bias)
     elif a.shape[0] <= TUNING.few_rows and gemm_sm100_supported(a, w):
         gemm_sm100(a, w, out)
     else:
