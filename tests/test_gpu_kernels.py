@@ -276,6 +276,32 @@ def test_f32_attention_of_portions_and_of_single_tokens_agree_to_the_bit(H, KV, 
         r += n
 
 
+@pytest.mark.parametrize("hd,H,KV,window", [(64, 8, 2, 0), (128, 4, 4, 0), (64, 5, 1, 150)])
+def test_f32_attention_keys_of_minus_infinite_score_weigh_nothing(hd, H, KV, window):
+    """Keys whose score is minus infinity, for whole tiles of 32 and 64 at the front, in the middle and at the end of a row's keys:
+    the row is what its other keys give, in both of the 32-bit engine's kernels."""
+    # (context, rows): the infinite tiles lie at keys 0-31, 64-127 and 160-191 of each request
+    seqs = [(150, 1), (32, 260), (191, 1), (0, 400), (223, 1)]
+    qrows, kc, vc, bt, row_seq, pos, qs, ks, vs = _paged_case(torch.float32, H, KV, hd, 16, seqs, seed=hd + window)
+    qrows[:, ::hd] = 1.0
+    for s, (c, n) in enumerate(seqs):
+        qs[s][:, ::hd] = 1.0
+        for j in (*range(32), *range(64, 128), *range(160, 192)):
+            if j < c + n:
+                kc[int(bt[s, j // 16]), :, j % 16, 0] = float("-inf")
+                ks[s][j].view(KV, hd)[:, 0] = float("-inf")
+    T = len(pos)
+    for singles in (0, T):
+        out = torch.full((T, H * hd), 7.0, device=DEV)
+        K().paged_attention(qrows.to(DEV), out, kc.to(DEV), vc.to(DEV), bt.to(DEV), row_seq.to(DEV), pos.to(DEV), H, KV, hd, 1.0 / math.sqrt(hd), window, singles)
+        r = 0
+        for s, (c, n) in enumerate(seqs):
+            # (rows 0-31 have no other key: not asked)
+            want = plain.causal_attention(qs[s].double(), ks[s].double(), vs[s].double(), H, KV, hd, window=window or None)[max(c, 32):]
+            assert rel(out[r + max(c, 32) - c:r + n], want) <= ATOL[torch.float32], (s, singles)
+            r += n
+
+
 def test_paged_attention_refuses_bad_sizes():
     from vllm_oxide_b200.errors import ShapeError
     q = torch.zeros(1, 4 * 20, device=DEV)

@@ -11,6 +11,7 @@
 // Cache layout per layer: K and V are [num_pages][KV][page_size][hd]; key j of a request lives
 // in page block_table[seq][j / page_size] at offset j % page_size.
 #include "common.cuh"
+#include <cfloat>
 #include <cooperative_groups.h>
 #include <type_traits>
 VOB_PDL_SWITCH(attention)
@@ -139,9 +140,10 @@ paged_attention_warp_kernel(const T* __restrict__ q, long long q_stride, T* __re
 // for single tokens. Both form a row's result in the same steps, so that a row's bits depend neither on the batch nor on which
 // of the two computed it. Keys are taken in tiles of 32 (key 32 t .. 32 t + 31 of the request, t ascending); of a tile
 //   s_j = scale * (q . k_j)      two chains of FMAs, over even and odd d, and their sum
-//   m_t = max s_j,  p_j = expf(s_j - m_t),  l_t = sum p_j,  o_t[d] = sum p_j v_j[d]     chains over the keys in order
+//   m_t = max(max s_j, -FLT_MAX),  p_j = expf(s_j - m_t),  l_t = sum p_j,  o_t[d] = sum p_j v_j[d]     chains over the keys in order
 // and the tile joins what is behind it: M' = max(M, m_t), acc = acc expf(M - M') + o_t expf(m_t - M'), l likewise. Keys that a
-// row may not see take no part (what they hold, infinities too, does not reach the row).
+// row may not see take no part (what they hold, infinities too, does not reach the row). A tile whose scores are all minus infinity
+// weighs nothing: with -FLT_MAX for its maximum expf gives zeros, and not the NaN of minus infinity less itself.
 // (The general kernel above sums over all keys in one chain: relative error against 64 bits at 4,000 keys 1.2e-6, here 3.4e-7.)
 // ---------------------------------------------------------------------------------------------
 namespace cg = cooperative_groups;
@@ -280,6 +282,7 @@ attn_f32_rows_kernel(const float* __restrict__ q, long long q_stride, float* __r
                         m[0] = fmaxf(m[0], __shfl_xor_sync(0xffffffffu, m[0], o));
                         m[1] = fmaxf(m[1], __shfl_xor_sync(0xffffffffu, m[1], o));
                     }
+                    m[0] = fmaxf(m[0], -FLT_MAX); m[1] = fmaxf(m[1], -FLT_MAX);
 #pragma unroll
                     for (int j = 0; j < 4; ++j) {
                         int key = k0 + sk + 16 * j;
@@ -435,7 +438,7 @@ attn_f32_single_kernel(const float* __restrict__ q, long long q_stride, float* _
             float mt[G];
 #pragma unroll
             for (int g = 0; g < G; ++g) {
-                mt[g] = warp_max(s[g]);
+                mt[g] = fmaxf(warp_max(s[g]), -FLT_MAX);
                 ps[warp][g][lane] = valid ? expf(s[g] - mt[g]) : 0.f;
             }
             __syncwarp();
