@@ -123,6 +123,23 @@ def test_how_decode_attention_shares_a_request_over_blocks():
     assert decode_split_rule(8, 8, 148, True) == (6, True)
 
 
+def test_every_kind_of_attention_mixer_gets_blocks_and_scratch_of_its_own():
+    """Blocks dealt out by length: whatever the kv heads, the number is one that the kernel takes and whose partial results fit the
+    scratch a mixer of these sizes keeps; layers of different kv heads or head sizes in one model get a number each."""
+    from vllm_oxide_b200.parts.attention import decode_balance, decode_balance_rule, decode_scratch_blocks, decode_split_rule
+    for sms in (7, 108, 132, 148):
+        for kv in range(1, 33):
+            for seqs in (1, 2, 16, 128, 129):
+                splits, wide = decode_split_rule(seqs, kv, sms, True)
+                assert not wide or seqs * kv * splits <= decode_scratch_blocks(kv, sms)
+                for hd in (64, 128):
+                    blocks = decode_balance_rule(seqs, kv, hd, sms, 100000, 100000 + seqs)
+                    assert blocks == 0 or 2 <= blocks <= 64
+                    assert 2 * blocks * kv <= decode_scratch_blocks(kv, sms)
+    assert decode_balance(((8, 64, 148), (16, 64, 148), (8, 128, 148)), 16, 5000, 9000) == (((8, 64), 55), ((16, 64), 27), ((8, 128), 37))
+    assert decode_balance(((8, 64, 148), (16, 64, 148)), 16, 100, 1600) == decode_balance((), 16, 5000, 9000) == ()
+
+
 def test_batch_size_classes_of_decode_steps():
     from vllm_oxide_b200.engine.runner import decode_bucket
     assert [decode_bucket(n) for n in range(1, 18)] == [1, 2, 3, 4, 6, 6, 8, 8, 12, 12, 12, 12, 16, 16, 16, 16, 24]

@@ -27,7 +27,7 @@ from ..config import EngineConfig, architecture_for, read_config_json
 from ..csrc.build import runtime_module
 from ..errors import CapacityError, KernelError, ShapeError
 from ..tuning import TUNING
-from ..parts.attention import decode_balance_rule
+from ..parts.attention import decode_balance
 from ..parts.base import ModelSpec, StepContext, Workspace, aligned
 from ..weights import load_safetensors_weights, weights_from_tensors
 
@@ -180,7 +180,7 @@ class ModelRunner:
         self.after_block = None                 # debugging: a function (call number, residual, pending) run behind every block
         self._pending_scale = None
         self._graph_launches = {}
-        self._balance_rule = None               # (kv heads, head size, SMs) of `_balance`, () for none; read off the parts at first use
+        self._balance_rules = None              # (kv heads, head size, SMs) of the mixers `_balance` asks for; read off the parts at first use
         self._graph_logits = {}                 # class of a decode step -> its logits in the workspace (None where the head picks without)
         self._kept_seen = set()                 # classes of decode steps that keep their logits and have come once
         self._graph_pool = None
@@ -567,15 +567,14 @@ class ModelRunner:
         torch.cuda.current_stream().synchronize()
         return self.sampled_host_np[parity, :S].tolist()
 
-    def _balance(self, arrays, seqs: int) -> int:
-        """`StepContext.balance` of a decode step of `seqs` requests: what the first of the model's attention mixers that can
-        deal its blocks out by length is best given (they are alike in the models there are; a model without one gets 0)."""
-        if self._balance_rule is None:
-            rules = (getattr(b.mixer, "balance_rule", lambda: None)() for b in self.spec.blocks if getattr(b, "mixer", None) is not None)
-            self._balance_rule = next((r for r in rules if r is not None), ())
-        if not self._balance_rule:
-            return 0
-        return decode_balance_rule(seqs, *self._balance_rule, int(arrays.max_seq_len), int(arrays.total_len))
+    def _balance(self, arrays, seqs: int) -> tuple:
+        """`StepContext.balance` of a decode step of `seqs` requests, for every kind of attention mixer in the model that can deal
+        its blocks out by length."""
+        if self._balance_rules is None:
+            mixers = (getattr(b, "mixer", None) for b in self.spec.blocks)
+            rules = (getattr(m, "balance_rule", lambda page: None)(self.engine.block_size) for m in mixers if m is not None)
+            self._balance_rules = tuple(dict.fromkeys(r for r in rules if r is not None))
+        return decode_balance(self._balance_rules, seqs, int(arrays.max_seq_len), int(arrays.total_len))
 
     def decode_arrays(self, scheduler, plan):
         """The device arrays of a decode step's plan, in the decode steps' layout."""
@@ -604,7 +603,7 @@ class ModelRunner:
         return self.sampled_host_np[parity, :count].tolist()
 
     def _decode_eager(self, b: int, parity: int = 0, long_context: bool = False, keep_logits: bool = False,
-                      balance: int = 0) -> Optional[torch.Tensor]:
+                      balance: tuple = ()) -> Optional[torch.Tensor]:
         L = self.decode_layout
         self.workspace.reset()
         self._dev = self._devs[parity]          # this step's metadata (a recorded step keeps reading this buffer)

@@ -67,6 +67,18 @@ def decode_balance_rule(num_seqs: int, kv_heads: int, head_dim: int, num_sms: in
     return want if (walks - share) * head_dim >= TUNING.balance_tiles * 64 else 0
 
 
+def decode_balance(rules, num_seqs: int, max_len: int, total_len: int) -> tuple:
+    """`StepContext.balance` for mixers of these (kv heads, head size, SMs): what the rule above gives each, where it gives any."""
+    got = (((kv, hd), decode_balance_rule(num_seqs, kv, hd, sms, max_len, total_len)) for kv, hd, sms in rules)
+    return tuple((sizes, blocks) for sizes, blocks in got if blocks)
+
+
+def decode_scratch_blocks(kv_heads: int, num_sms: int) -> int:
+    """Blocks whose partial results the decode kernel's merge through global memory may have to hold: requests x kv heads x splits
+    are at most 3 SMs; of a balanced launch twice what `decode_balance_rule` gives each kv head (at most 64, and 3 SMs over all)."""
+    return max(3 * num_sms, min(6 * num_sms, 128 * kv_heads))
+
+
 class Attention(Mixer):
     def __init__(self, wq: torch.Tensor, wk: Optional[torch.Tensor], wv: Optional[torch.Tensor], wo: torch.Tensor,
                  num_heads: int, num_kv_heads: int, head_dim: int, position=None, window: Optional[int] = None,
@@ -216,11 +228,9 @@ class Attention(Mixer):
     def _attend_single(self, q, out, ctx: StepContext, cache: LayerCache, bt, count: int) -> None:
         """The decode kernel on the first `count` rows, row i belonging to request i."""
         splits, wide = self.decode_splits(count, ctx.long_context)
-        balance = ctx.balance if ctx.decode_only and self.window == 0 else 0
+        balance = dict(ctx.balance).get((self.KV, self.hd), 0) if ctx.decode_only and self.window == 0 else 0
         if (wide or balance) and self._partials is None:
-            # requests x kv heads x splits <= 3 SMs; of a balanced launch at most 2 x 64 per kv head and 2 x 3 SMs in all
-            blocks = max(3 * self.num_sms, min(6 * self.num_sms, 128 * self.KV))
-            floats = kernels.attn_decode_partial_floats(1, 1, self.hd, blocks)
+            floats = kernels.attn_decode_partial_floats(1, 1, self.hd, decode_scratch_blocks(self.KV, self.num_sms))
             self._partials = torch.empty(floats, dtype=torch.float32, device=q.device)
             self._arrived = torch.zeros(max(self.num_sms, kernels.DECODE_BALANCE_SEQS * self.KV), dtype=torch.int32, device=q.device)
         if balance:
@@ -230,9 +240,10 @@ class Attention(Mixer):
         kernels.attn_decode_mma(q[:count], out[:count], cache.k, cache.v, bt, ctx.positions[:count], self.H, self.KV, self.hd,
                                 self.scale, self.window, splits, self._partials if wide else None, self._arrived if wide else None)
 
-    def balance_rule(self):
+    def balance_rule(self, page_size: int):
         """(kv heads, head size, SMs) for `decode_balance_rule`, or None where this mixer's single tokens never run balanced."""
-        if self.dtype != torch.bfloat16 or self.window or self.hd not in kernels.TENSOR_CORE_HEAD_DIMS or self.H // self.KV > 16:
+        if (self.dtype != torch.bfloat16 or self.impl == "general" or not self.scale > 0 or self.window
+                or not kernels.attn_mma_supported(self.H, self.KV, self.hd, page_size, True)):
             return None
         return self.KV, self.hd, self.num_sms
 

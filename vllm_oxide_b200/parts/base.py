@@ -182,8 +182,9 @@ class StepContext:
                                     # rows 0 .. lead_single - 1 are theirs, row i belonging to request i
     long_context: bool = False      # some request is longer than TUNING.long_context_keys (host fact; a replayed
                                     # step was recorded with the same value)
-    balance: int = 0                # in a step of single tokens: blocks per kv head that attention deals out to the requests by
-                                    # length (host fact; 0: the same number for every request)
+    balance: tuple = ()             # in a step of single tokens: ((kv heads, head size), blocks) of the attention mixers that
+                                    # deal so many blocks per kv head out to the requests by length (host fact; a mixer of sizes
+                                    # that are not named gives every request the same number)
     host: Optional[object] = None   # the host-side StepArrays (ids, counts) for parts that want them
     shared: Dict[str, torch.Tensor] = field(default_factory=dict)   # what one layer of this step leaves for later layers of
                                     # the same step, by name: the buffers `ModelSpec.step_buffers` names, one row per row
