@@ -115,3 +115,25 @@ def test_layers_of_different_kv_heads_are_balanced_each_by_its_own(monkeypatch):
         assert (((8, HD), min(64, 3 * sms // 8)), ((16, HD), min(64, 3 * sms // 16))) in {key[4] for key in llm.runner._graphs}
     finally:
         unregister_architecture(NAME)
+
+
+def test_batches_that_become_even_and_uneven_again(monkeypatch):
+    """The long request ends first: its steps are balanced, those behind are not, and the next call begins balanced again. Launched
+    one by one, recorded and replayed at other lengths; a call whose steps are all replayed gives the bits of the one before."""
+    from vllm_oxide_b200.config import unregister_architecture
+    from vllm_oxide_b200.tuning import TUNING
+    monkeypatch.setattr(TUNING, "balance_tiles", 2)
+    try:
+        llm, cfg, tensors = _engine((8, 8))
+        prompts = [random_tokens(n, VOCAB, 40 + n) for n in LENGTHS]
+        new = [9 if n > 2000 else 20 for n in LENGTHS]
+        wanted = [(3, n - 1) for n in new]
+        got = [_generate(llm, cfg, tensors, prompts, new, wanted) for _ in range(4)]
+        balances = {key[4] for key in llm.runner._graphs}
+        assert () in balances and len(balances) == 2 and llm.stats["ahead_steps"] > 0
+        for a, b in zip(got[2], got[3]):
+            assert a.token_ids == b.token_ids and all(torch.equal(a.logits[i], b.logits[i]) for i in a.logits)
+        # other lengths on the same recordings
+        _generate(llm, cfg, tensors, [random_tokens(n, VOCAB, 90 + n) for n in (3000, 70, 20, 90, 33, 45, 28, 61)], [9, 20, 20, 20, 20, 20, 20, 20], [(8,)] + [(19,)] * 7)
+    finally:
+        unregister_architecture(NAME)

@@ -123,6 +123,18 @@ def test_how_decode_attention_shares_a_request_over_blocks():
     assert decode_split_rule(8, 8, 148, True) == (6, True)
 
 
+def _decode_arrays(lens):
+    """A step in which every request brings one token behind so many cached ones that it then has these lengths."""
+    pages = sum(-(-n // 64) for n in lens)
+    c = rt.CacheManager(64, [rt.GroupSpec(rt.FULL, 0, pages)], len(lens))
+    for i, n in enumerate(lens):
+        c.admit(i)
+        if n > 1:
+            c.reserve(i, n - 1), c.commit(i, n - 1)
+        c.reserve(i, 1)
+    return rt.build_step(c, [rt.StepEntry(i, [1], [0]) for i in range(len(lens))], len(lens), len(lens), len(lens), -(-max(lens) // 64), 10)
+
+
 def test_every_kind_of_attention_mixer_gets_blocks_and_scratch_of_its_own():
     """Blocks dealt out by length: whatever the kv heads, the number is one that the kernel takes and whose partial results fit the
     scratch a mixer of these sizes keeps; layers of different kv heads or head sizes in one model get a number each."""
@@ -133,11 +145,57 @@ def test_every_kind_of_attention_mixer_gets_blocks_and_scratch_of_its_own():
                 splits, wide = decode_split_rule(seqs, kv, sms, True)
                 assert not wide or seqs * kv * splits <= decode_scratch_blocks(kv, sms)
                 for hd in (64, 128):
-                    blocks = decode_balance_rule(seqs, kv, hd, sms, 100000, 100000 + seqs)
+                    blocks = decode_balance_rule(seqs, kv, hd, sms, 100000, lambda want, requests: 3)
                     assert blocks == 0 or 2 <= blocks <= 64
                     assert 2 * blocks * kv <= decode_scratch_blocks(kv, sms)
-    assert decode_balance(((8, 64, 148), (16, 64, 148), (8, 128, 148)), 16, 5000, 9000) == (((8, 64), 55), ((16, 64), 27), ((8, 128), 37))
-    assert decode_balance(((8, 64, 148), (16, 64, 148)), 16, 100, 1600) == decode_balance((), 16, 5000, 9000) == ()
+    share = _decode_arrays([5000] + [100] * 15).balanced_share
+    assert decode_balance(((8, 64, 148), (16, 64, 148), (8, 128, 148)), 16, 5000, share) == (((8, 64), 55), ((16, 64), 27), ((8, 128), 37))
+    assert decode_balance(((8, 64, 148), (16, 64, 148)), 16, 100, _decode_arrays([100] * 16).balanced_share) == ()
+    assert decode_balance((), 16, 5000, share) == ()
+
+
+def _walks(seqs, kv, sms, longest):
+    """Tiles that a block of the longest request walks when every request gets the same number of blocks."""
+    from vllm_oxide_b200.parts.attention import decode_split_rule
+    from vllm_oxide_b200.tuning import TUNING
+    splits, wide = decode_split_rule(seqs, kv, sms, longest > TUNING.long_context_keys)
+    tiles = -(-longest // 64)
+    return -(-tiles // (min(splits, max(1, tiles // 3)) if wide else splits))
+
+
+def test_blocks_dealt_out_by_length_shorten_the_longest_walk():
+    """The share that host and kernel find is the smallest one that the blocks suffice for, padding requests included; a step is
+    balanced only where that share is shorter than the longest request's walk by the tiles the merge costs, so requests of equal
+    length never are for nothing; the measured cases keep their choices."""
+    from vllm_oxide_b200.parts.attention import decode_balance_rule
+    from vllm_oxide_b200.tuning import TUNING
+
+    def spread(n, lo, hi):
+        return [int(round(lo * (hi / lo) ** (i / (n - 1)))) for i in range(n)]
+
+    def smallest(lens, want, requests):
+        tiles = [-(-x // 64) for x in lens]
+        blocks = max(want, want // 2 + requests)
+        share = max(3, -(-sum(tiles) // want))
+        while requests - len(lens) + sum(max(1, -(-t // share)) for t in tiles) > blocks:
+            share += 1
+        assert share <= 2 * max(3, -(-sum(tiles) // want))
+        return share
+    cases = [spread(8, 100, 2000), [4000, 200], spread(16, 100, 2000), spread(16, 17, 8000), spread(64, 17, 1000), [1], [1] * 128, [9000] + [1] * 90,
+             [64, 65, 128, 129], spread(12, 130, 3000), *([n] * s for n in (60, 700, 8192, 16384, 32768) for s in (1, 2, 8, 12, 16, 24, 64, 128))]
+    for lens in cases:
+        a = _decode_arrays(lens)
+        for want in (2, 3, 18, 37, 55, 64):
+            for requests in (len(lens), len(lens) + 3):
+                assert a.balanced_share(want, requests) == smallest(lens, want, requests)
+        for kv, hd in ((8, 64), (8, 128), (2, 64), (16, 128)):
+            want = decode_balance_rule(len(lens), kv, hd, 148, max(lens), a.balanced_share)
+            if want:
+                assert (_walks(len(lens), kv, 148, max(lens)) - smallest(lens, want, len(lens))) * hd >= 64 * TUNING.balance_tiles
+    for kv, hd, lens, want in [(8, 64, spread(8, 100, 2000), 0), (8, 64, [4000, 200], 0), (8, 64, spread(16, 100, 2000), 55), (8, 64, spread(16, 100, 4000), 55),
+                               (8, 64, spread(64, 17, 1000), 55), (8, 128, spread(8, 100, 2000), 37), (8, 128, spread(16, 17, 1000), 37),
+                               (8, 128, spread(16, 100, 4000), 37), (8, 64, [32768] * 8, 0), (8, 64, [16384] * 12, 0), (8, 64, [16384] * 16, 0), (8, 64, [8192] * 24, 0)]:
+        assert decode_balance_rule(len(lens), kv, hd, 148, max(lens), _decode_arrays(lens).balanced_share) == want, (kv, hd, lens)
 
 
 def test_batch_size_classes_of_decode_steps():

@@ -23,6 +23,7 @@
 // softmax's denominator once, a key with no value), a gate (the result times sigmoid(gate[row,
 // head * hd + d]), or sigmoid(gate[row, head]) with one number per head) and a constant factor.
 #include "common.cuh"
+#include "decode_share.h"
 #include <algorithm>
 VOB_PDL_SWITCH(attention_mma)
 
@@ -628,7 +629,6 @@ attn_prefill_mma_any_kernel(const __nv_bfloat16* __restrict__ q, long long q_str
     }
 }
 
-constexpr int DEC_MIN_TILES = 3;            // measured on whole decode steps at batch 1: 8,192 keys 0.808 ms with 3, 0.838 with 2, 0.812 with 4
 constexpr int DEC_MAX_SPLITS_WIDE = 64;
 
 // The block of a request and kv head that arrives last adds the partials of all `splits` blocks
@@ -712,14 +712,11 @@ __device__ __noinline__ void merge_partials(const float* __restrict__ all, int s
 
 constexpr int DEC_BALANCE_SEQS = 128;      // most requests of a balanced launch: four a lane
 
-// Tiles a block takes at first, with `want` blocks for `total` tiles; the search below ends at twice this.
-__host__ __device__ constexpr int balance_share(long long total, int want) {
-    return (int)((total + want - 1) / want) > DEC_MIN_TILES ? (int)((total + want - 1) / want) : DEC_MIN_TILES;
-}
+static_assert(BN == DEC_TILE_KEYS, "a tile is what the shares are counted in");
 
 // Which request and which of its blocks block `b` of a kv head is. Returns false if it is none's. `want`: the blocks that are to be
-// filled evenly, `blocks` those there are. Partials are kept for requests of more than one block: at most 2 want of them. (At twice the first share the requests need at most want / 2 blocks
-// for whole shares and one each for the rest: they fit, as `blocks` is at least want / 2 + requests.)
+// filled evenly, `blocks` those there are. Partials are kept for requests of more than one block: at most 2 want of them (a request
+// of more than one share needs fewer than twice its tiles over the share).
 __device__ __forceinline__ bool balance_place(const int* __restrict__ positions, int S, int want, int blocks, int b, int lane, int& seq,
                                               int& split, int& splits, int& share, int& first_part) {
     int n[DEC_BALANCE_SEQS / 32], total = 0;
@@ -730,15 +727,12 @@ __device__ __forceinline__ bool balance_place(const int* __restrict__ positions,
         total += n[i];
     }
     total = __reduce_add_sync(0xffffffffu, total);
-    const int share0 = balance_share(total, want);
-    share = share0;
-    while (true) {
+    share = balance_share(total, want, blocks, [&](int x) {
         int need = 0;
 #pragma unroll
-        for (int i = 0; i < DEC_BALANCE_SEQS / 32; ++i) need += i * 32 + lane < S ? max(1, (n[i] + share - 1) / share) : 0;
-        if (share >= 2 * share0 || (int)__reduce_add_sync(0xffffffffu, need) <= blocks) break;
-        share = min(2 * share0, share + (share + 7) / 8);
-    }
+        for (int i = 0; i < DEC_BALANCE_SEQS / 32; ++i) need += i * 32 + lane < S ? max(1, (n[i] + x - 1) / x) : 0;
+        return (int)__reduce_add_sync(0xffffffffu, need);
+    });
     int before = 0;                                   // blocks of the requests in front
     first_part = 0;                                   // and of those that have more than one
 #pragma unroll
@@ -1078,7 +1072,7 @@ int launch_decode_st(const void* q, long long q_stride, void* out, long long out
     long long tiles_max = ((long long)max_pages * page_size + BN - 1) / BN;
     long long per_max = (tiles_max + splits - 1) / splits;
     if (partials && per_max < 2 * DEC_MIN_TILES) per_max = 2 * DEC_MIN_TILES;
-    if (balance) per_max = std::max<long long>(1, std::min<long long>(tiles_max, 2 * balance_share(S * tiles_max, balance)));
+    if (balance) per_max = std::max<long long>(1, std::min<long long>(tiles_max, 2 * std::max<long long>(DEC_MIN_TILES, (S * tiles_max + balance - 1) / balance)));
     long long pages_cta = per_max * (BN / page_size) + 1;
     size_t smem = decode_smem<HD, ST, KV1>(H / KV, splits > 1 && !partials) + (size_t)pages_cta * sizeof(int);
     int e = ensure_smem(attn_decode_mma_kernel<HD, ST, SHAPED, KV1>, smem, &configured);
@@ -1272,8 +1266,7 @@ VOB_EXPORT int vob_attn_decode_mma(const void* q, long long q_stride, void* out,
     if (!sizes_ok(H, KV, hd, page_size) || H / KV > 16) return VOB_ERR_UNSUPPORTED;
     if ((partials == nullptr) != (arrived == nullptr)) return VOB_ERR_BAD_ARG;
     if (q_stride % 8 != 0 || splits < 1 || splits > (partials ? DEC_MAX_SPLITS_WIDE : 8) || KV > 65535) return VOB_ERR_BAD_ARG;
-    // blocks a kv head: as many as are to be filled, and enough for a rest of every request
-    int grid_blocks = std::max(balance, balance / 2 + S);
+    const int grid_blocks = balance_blocks(balance, S);
     if (balance < 0 || (balance && (!partials || balance < 2 || balance > DEC_MAX_SPLITS_WIDE || window || S > DEC_BALANCE_SEQS))) return VOB_ERR_BAD_ARG;
     if (hd == 64) return launch_decode<64, false>(q, q_stride, out, out_stride, kcache, vcache, block_tables, max_pages, positions, S,
                                                  H, KV, page_size, window, scale, splits, (float*)partials, arrived, tail, none, balance, grid_blocks, stream);

@@ -148,6 +148,7 @@ def runtime_module():
         rdir = os.path.join(_HERE, "runtime")
         srcs = sorted(os.path.join(rdir, f) for f in os.listdir(rdir) if f.endswith(".cpp"))
         hdrs = sorted(os.path.join(rdir, f) for f in os.listdir(rdir) if f.endswith((".h", ".hpp")))
+        hdrs += [f for f in _headers() if f.endswith(".h")]        # what host and kernels share
         tag = _digest(srcs + hdrs, _CXX_FLAGS + [sys.version])
         bdir = _build_dir()
         so = os.path.join(bdir, f"vob200_runtime_{tag}.so")
@@ -164,7 +165,7 @@ def runtime_module():
             print("[vllm_oxide_b200] compiling the host runtime (C++) ...", file=sys.stderr, flush=True)
             tmp = so + f".{os.getpid()}.tmp"
             _run([cxx] + _CXX_FLAGS + [f"-DVOB_MODULE_NAME=vob200_runtime_{tag}",
-                  "-I", pybind11.get_include(), "-I", sysconfig.get_paths()["include"], "-I", rdir,
+                  "-I", pybind11.get_include(), "-I", sysconfig.get_paths()["include"], "-I", rdir, "-I", _HERE,
                   "-o", tmp] + srcs, "runtime")
             os.replace(tmp, so)
         spec = importlib.util.spec_from_file_location(f"vob200_runtime_{tag}", so)

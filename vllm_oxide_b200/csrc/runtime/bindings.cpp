@@ -77,7 +77,7 @@ PYBIND11_MODULE(VOB_MODULE_NAME, m) {
         .def_readonly("max_new", &StepArrays::max_new)
         .def_readonly("lead_single", &StepArrays::lead_single)
         .def_readonly("max_seq_len", &StepArrays::max_seq_len)
-        .def_readonly("total_len", &StepArrays::total_len)
+        .def("balanced_share", &StepArrays::balanced_share, py::arg("want"), py::arg("requests"))
         .def_readonly("any_sampling", &StepArrays::any_sampling)
         .def_readonly("ids", &StepArrays::ids)
         .def_readonly("new_counts", &StepArrays::new_counts)

@@ -10,6 +10,7 @@
 #pragma once
 #include <cstring>
 #include "cache_manager.h"
+#include "decode_share.h"
 
 namespace vob {
 
@@ -65,11 +66,25 @@ struct StepArrays {
     int max_new = 0;                // longest portion in the batch
     int lead_single = 0;            // leading requests that bring exactly one token (rows 0 .. lead_single - 1)
     int64_t max_seq_len = 0;        // longest context after this step
-    int64_t total_len = 0;          // all contexts after this step, summed
     bool any_sampling = false;      // some row has temperature > 0
     std::vector<int64_t> ids;       // request of each sequence, in batch order
     std::vector<int32_t> new_counts;
     int used = 0;                   // ints from the start of `data` that this batch actually fills
+
+    // Tiles that a block of a balanced decode launch with `want` blocks a kv head to fill takes in this step, the batch padded to
+    // `requests` (padding requests have no keys and a block each).
+    int balanced_share(int want, int requests) const {
+        if (want < 1 || requests < seqs) throw CacheError("balanced_share: bad sizes");
+        const int32_t* lens = data.data() + layout.seq_lens;
+        auto tiles = [&](int s) { return (lens[s] + DEC_TILE_KEYS - 1) / DEC_TILE_KEYS; };
+        int64_t total = 0;
+        for (int s = 0; s < seqs; ++s) total += tiles(s);
+        return balance_share(total, want, balance_blocks(want, requests), [&](int share) {
+            int64_t n = requests - seqs;
+            for (int s = 0; s < seqs; ++s) n += std::max(1, (tiles(s) + share - 1) / share);
+            return n;
+        });
+    }
 };
 
 // Lay the entries out. Every request must be admitted and must already hold pages for its new
@@ -147,7 +162,6 @@ inline StepArrays build_step(const CacheManager& cache, const std::vector<StepEn
         A.max_new = std::max(A.max_new, n);
         if (n == 1 && A.lead_single == (int)A.ids.size()) ++A.lead_single;
         A.max_seq_len = std::max<int64_t>(A.max_seq_len, ctx + n);
-        A.total_len += ctx + n;
         A.ids.push_back(e.id);
         A.new_counts.push_back(n);
     }

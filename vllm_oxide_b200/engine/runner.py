@@ -574,7 +574,7 @@ class ModelRunner:
             mixers = (getattr(b, "mixer", None) for b in self.spec.blocks)
             rules = (getattr(m, "balance_rule", lambda page: None)(self.engine.block_size) for m in mixers if m is not None)
             self._balance_rules = tuple(dict.fromkeys(r for r in rules if r is not None))
-        return decode_balance(self._balance_rules, seqs, int(arrays.max_seq_len), int(arrays.total_len))
+        return decode_balance(self._balance_rules, seqs, int(arrays.max_seq_len), arrays.balanced_share)
 
     def decode_arrays(self, scheduler, plan):
         """The device arrays of a decode step's plan, in the decode steps' layout."""

@@ -49,10 +49,11 @@ def decode_split_rule(num_seqs: int, kv_heads: int, num_sms: int, long_context: 
     return max(1, min(8, hi if lo < hi <= 6 else lo)), False
 
 
-def decode_balance_rule(num_seqs: int, kv_heads: int, head_dim: int, num_sms: int, max_len: int, total_len: int) -> int:
+def decode_balance_rule(num_seqs: int, kv_heads: int, head_dim: int, num_sms: int, max_len: int, share_of) -> int:
     """Blocks per kv head to deal out by length (0: every request gets the same number, `decode_split_rule`). Worth it where a
-    block of the longest request would walk so many more tiles of 64 keys than its share of all of them that this takes longer
-    than the merge through global memory costs over the merge in a cluster. Measured with 8 kv heads of 64, in clusters / balanced, and
+    block of the longest request would walk so many more tiles of 64 keys than a block does when they are dealt out
+    (`share_of(blocks, requests)`, `StepArrays.balanced_share`: the share that the kernel will find) that this takes longer than the
+    merge through global memory costs over the merge in a cluster. Measured with 8 kv heads of 64, in clusters / balanced, and
     how many tiles more: 8 requests of 100 to 2,000 keys 8.8 / 9.9 us (3), two of 4,000 and 200 keys 9.0 / 10.4 (5), 16 of 100 to 2,000
     13.2 / 10.9 (7), 16 of 100 to 4,000 22.0 / 14.4 (15), 64 of 17 to 1,000 19.6 / 18.3 (10); heads of 128, where a tile takes twice as
     long: 8 of 100 to 2,000 13.3 / 12.5 (3), 16 of 17 to 1,000 12.5 / 11.0 (3), 16 of 100 to 4,000 38 / 22 (13)."""
@@ -63,13 +64,14 @@ def decode_balance_rule(num_seqs: int, kv_heads: int, head_dim: int, num_sms: in
     splits, wide = decode_split_rule(num_seqs, kv_heads, num_sms, max_len > TUNING.long_context_keys)
     longest = -(-max_len // 64)
     walks = -(-longest // min(splits, max(1, longest // 3)) if wide else -longest // splits)
-    share = max(3, -(-(total_len // 64 + num_seqs) // want))
-    return want if (walks - share) * head_dim >= TUNING.balance_tiles * 64 else 0
+    if walks * head_dim < TUNING.balance_tiles * 64:         # most steps: no share is small enough
+        return 0
+    return want if (walks - share_of(want, num_seqs)) * head_dim >= TUNING.balance_tiles * 64 else 0
 
 
-def decode_balance(rules, num_seqs: int, max_len: int, total_len: int) -> tuple:
+def decode_balance(rules, num_seqs: int, max_len: int, share_of) -> tuple:
     """`StepContext.balance` for mixers of these (kv heads, head size, SMs): what the rule above gives each, where it gives any."""
-    got = (((kv, hd), decode_balance_rule(num_seqs, kv, hd, sms, max_len, total_len)) for kv, hd, sms in rules)
+    got = (((kv, hd), decode_balance_rule(num_seqs, kv, hd, sms, max_len, share_of)) for kv, hd, sms in rules)
     return tuple((sizes, blocks) for sizes, blocks in got if blocks)
 
 
