@@ -186,6 +186,14 @@ def _paged_case(dt, H, KV, hd, page, seqs, seed, scale_key=None, poison=False):
             qs, ks, vs)
 
 
+def _last_row(q, k, v, H, KV, hd, window=0):
+    """Attention of a request's last row in float64: q [H * hd], k and v [L, KV * hd]."""
+    L = len(k)
+    k, v = (x.double().view(L, KV, 1, hd)[-(window or L):].expand(-1, -1, H // KV, -1).reshape(-1, H, hd) for x in (k, v))
+    p = torch.softmax(torch.einsum("hd,lhd->hl", q.double().view(H, hd), k) / math.sqrt(hd), -1)
+    return torch.einsum("hl,lhd->hd", p, v).reshape(1, H * hd)
+
+
 ATOL = {torch.float32: 1e-5, torch.bfloat16: 2 ** -7}      # reference: 1e-5 relative for paged attention (cpu/tests.rs:161-334)
 
 
@@ -629,6 +637,54 @@ def test_attn_decode_mma_balanced(H, KV, hd, page, S, balance, most):
         k.attn_decode_mma(q, got, *args, 0, 1, balance=balance)
     with pytest.raises(ShapeError, match="partials must be"):
         k.attn_decode_mma(q, got, *args, 0, 1, partials[:100], arrived, balance=balance)
+
+
+@pytest.mark.parametrize("H,KV,hd,page,window,splits", [(8, 2, 64, 1, 0, 1), (8, 2, 64, 4, 0, 1), (6, 2, 128, 2, 0, 2), (4, 4, 64, 1, 1500, 1), (8, 2, 64, 16, 0, 1),
+                                                        (4, 1, 128, 8, 0, 1)])
+def test_attn_decode_mma_page_list_is_refilled(H, KV, hd, page, window, splits):
+    """A block's page list holds 512 pages and is filled again, half by half, as the block walks on: requests of more pages than that
+    and of lengths around its halves, in clusters, with the merge through global memory and balanced."""
+    half = 256 * page
+    seqs = [(n - 1, 1) for n in (2 * half - 1, 2 * half + 1, 3 * half, 5 * half + 70, 64, 3 * half + 65)]
+    dt = torch.bfloat16
+    qrows, kc, vc, bt, row_seq, pos, qs, ks, vs = _paged_case(dt, H, KV, hd, page, seqs, seed=hd + page, scale_key=lambda L: max(L - 3 - page, 0))
+    want = torch.cat([_last_row(qs[s][-1], ks[s], vs[s], H, KV, hd, window) for s in range(len(seqs))])
+    k = K()
+    args = (kc.to(DEV), vc.to(DEV), bt.to(DEV), pos.to(DEV), H, KV, hd, 1.0 / math.sqrt(hd))
+    arrived = torch.zeros(len(seqs) * KV, dtype=torch.int32, device=DEV)
+
+    def go(*more, **kw):
+        out = torch.full_like(qrows, 7.0).to(DEV)
+        k.attn_decode_mma(qrows.to(DEV), out, *args, *more, **kw)
+        assert rel(out, want) <= 2 ** -6
+    go(window, splits)
+    go(window, 2, torch.empty(k.attn_decode_partial_floats(len(seqs), KV, hd, 2), device=DEV), arrived)
+    if not window:
+        go(0, 1, torch.empty(k.attn_decode_partial_floats(1, KV, hd, 4), device=DEV), arrived, balance=2)
+
+
+@pytest.mark.parametrize("page,balance", [(16, 37), (1, 37), (16, 0)])
+def test_attn_decode_mma_takes_block_tables_of_any_width(page, balance):
+    """What a block needs in shared memory does not grow with the longest request that the block table could hold: 32 short requests
+    beside a table of 524,288 tokens, head size 128, with the bits of the same launch on a table just wide enough."""
+    H, KV, hd, S = 16, 8, 128, 32
+    g = torch.Generator().manual_seed(page)
+    lens = torch.randint(1, 200, (S,), generator=g)
+    pages = 200 // page + 1
+    narrow = torch.randperm(S * pages, generator=g).to(torch.int32).view(S, pages).to(DEV)
+    wide = torch.full((S, 524288 // page), -1, dtype=torch.int32, device=DEV)
+    wide[:, :pages] = narrow
+    kc, vc = (torch.randn(S * pages, KV, page, hd, generator=g).to(torch.bfloat16).to(DEV) for _ in range(2))
+    q = torch.randn(S, H * hd, generator=g).to(torch.bfloat16).to(DEV)
+    k = K()
+    partials = torch.empty(k.attn_decode_partial_floats(1, KV, hd, max(2 * balance, 2)), device=DEV) if balance else None
+    arrived = torch.zeros(S * KV, dtype=torch.int32, device=DEV) if balance else None
+    got = []
+    for bt in (narrow, wide):
+        out = torch.full_like(q, 7.0)
+        k.attn_decode_mma(q, out, kc, vc, bt, (lens - 1).to(torch.int32).to(DEV), H, KV, hd, 1.0 / math.sqrt(hd), 0, 1, partials, arrived, balance=balance)
+        got.append(out)
+    assert torch.equal(*got) and bool(torch.isfinite(got[0]).all())
 
 
 def test_attn_mma_refusals():

@@ -761,7 +761,11 @@ __device__ __forceinline__ bool balance_place(const int* __restrict__ positions,
 }
 
 // Shared memory of a decode block: the K/V ring (used again for the combine of the four warps),
-// then what the cluster's peers send, then the block's page list.
+// then what the cluster's peers send, then the block's page list: a ring of two halves, so that its size follows neither from the
+// longest request that the block tables can hold nor from how many tiles fall to a block. (Sized for the longest request it took 28 KB
+// at 131,072 tokens of pages of 16, one block an SM instead of two at head size 128, and did not fit at 524,288.) A half holds
+// at least four tiles' pages (pages of one token), 64 tiles' at pages of 16.
+constexpr int DEC_PAGE_LIST = 512;
 template <int HD, int DEC_STAGES, bool KV1> __host__ __device__ constexpr size_t decode_ring_bytes() {
     size_t ring = (size_t)(16 + (KV1 ? 1 : 2) * DEC_STAGES * BN) * (HD + 8) * sizeof(__nv_bfloat16) + (KV1 ? DEC_STAGES * BN * sizeof(float) : 0);
     size_t combine = 16 * (HD + 8) * sizeof(__nv_bfloat16) + (size_t)(128 + 4 * 16 * HD + 16 * HD + 32) * sizeof(float);
@@ -828,16 +832,20 @@ attn_decode_mma_kernel(const __nv_bfloat16* __restrict__ q, long long q_stride, 
     const int per = !SHAPED && balance ? share : (n_tiles + splits - 1) / splits;
     const int n_begin = split * per;
     const int n_end = min(n_tiles, n_begin + per);
-    // this block's pages: those of its tiles, BN / page_size of them each, one coalesced read of the block table
+    // this block's pages: those of its tiles, BN / page_size of them each, coalesced reads of the block table
     const int ppt_shift = 6 - page_shift;
-    for (int i = threadIdx.x; i < (max(n_end - n_begin, 0) << ppt_shift); i += NTHREADS) {
-        const int lp = (tile_of(n_begin + (i >> ppt_shift)) << ppt_shift) + (i & ((1 << ppt_shift) - 1));
-        s_pages[i] = lp <= (hi - 1) >> page_shift ? bt[lp] : 0;
-    }
+    const int entries = max(n_end - n_begin, 0) << ppt_shift;
+    auto list_pages = [&](int from, int to) {
+        for (int i = from + threadIdx.x; i < min(to, entries); i += NTHREADS) {
+            const int lp = (tile_of(n_begin + (i >> ppt_shift)) << ppt_shift) + (i & ((1 << ppt_shift) - 1));
+            s_pages[i & (DEC_PAGE_LIST - 1)] = lp <= (hi - 1) >> page_shift ? bt[lp] : 0;
+        }
+    };
+    list_pages(0, DEC_PAGE_LIST);
     __syncthreads();
     auto load_tile = [&](int n, int buf) {
         const int t = tile_of(n);
-        const int* pages = s_pages + ((n - n_begin) << ppt_shift);
+        const int* pages = s_pages + (((n - n_begin) << ppt_shift) & (DEC_PAGE_LIST - 1));
         load_kv_tile<HD, !KV1>(sK0 + buf * BN * LD, sV0 + buf * BN * LD, kc, vc, pages, t << ppt_shift, kvh, KV, page_shift, t * BN, lo_key, hi, keep);
         if (KV1) load_key_scales(sR0 + buf * BN, shape.kscale, pages, t << ppt_shift, page_shift, t * BN, lo_key, hi, keep);
     };
@@ -897,6 +905,10 @@ attn_decode_mma_kernel(const __nv_bfloat16* __restrict__ q, long long q_stride, 
         int buf = (n - n_begin) % DEC_STAGES;
         __nv_bfloat16* sK = sK0 + buf * BN * LD;
         __nv_bfloat16* sV = sV0 + buf * BN * LD;
+        // the tile asked for behind the barrier begins a half of the page list: the half's last entries served a tile that was
+        // asked for four tiles ago or more, so nobody reads them any more, and the barrier shows everyone the new ones
+        const int entry = (n + DEC_STAGES - 1 - n_begin) << ppt_shift;
+        if (entry >= DEC_PAGE_LIST && (entry & (DEC_PAGE_LIST / 2 - 1)) == 0) list_pages(entry, entry + DEC_PAGE_LIST / 2);
         cp_async_wait<DEC_STAGES - 2>();        // tile n has landed (one newer group may be in flight)
         __syncthreads();                        // ... for every thread; and everyone is done with tile n-1
         {
@@ -1067,14 +1079,7 @@ int launch_decode_st(const void* q, long long q_stride, void* out, long long out
                      float scale, int splits, float* partials, int* arrived, AttnTail tail, ScoreShape shape, int balance, int grid_blocks,
                      cudaStream_t stream) {
     static size_t configured = 0;
-    // a block's page list: its share of the tiles of the longest request the block table can hold
-    // (a request with few tiles uses fewer blocks, but then the tiles are few)
-    long long tiles_max = ((long long)max_pages * page_size + BN - 1) / BN;
-    long long per_max = (tiles_max + splits - 1) / splits;
-    if (partials && per_max < 2 * DEC_MIN_TILES) per_max = 2 * DEC_MIN_TILES;
-    if (balance) per_max = std::max<long long>(1, std::min<long long>(tiles_max, 2 * std::max<long long>(DEC_MIN_TILES, (S * tiles_max + balance - 1) / balance)));
-    long long pages_cta = per_max * (BN / page_size) + 1;
-    size_t smem = decode_smem<HD, ST, KV1>(H / KV, splits > 1 && !partials) + (size_t)pages_cta * sizeof(int);
+    const size_t smem = decode_smem<HD, ST, KV1>(H / KV, splits > 1 && !partials) + DEC_PAGE_LIST * sizeof(int);
     int e = ensure_smem(attn_decode_mma_kernel<HD, ST, SHAPED, KV1>, smem, &configured);
     if (e) return e;
     cudaLaunchConfig_t cfg = {};
@@ -1110,7 +1115,7 @@ int launch_decode(const void* q, long long q_stride, void* out, long long out_st
         cudaDeviceGetAttribute(&num_sms, cudaDevAttrMultiProcessorCount, dev);
         if (num_sms <= 0) num_sms = 148;
     }
-    // three stages while every block of the grid can be resident at once with them; else two
+    // three stages while every block of the grid can be resident at once with them (2 KB beside the ring: the page list); else two
     long long blocks = balance ? (long long)balance * KV : (long long)S * KV * splits;
     long long fit3 = (long long)num_sms * ((227 * 1024) / (long long)(decode_smem<HD, 3, KV1>(H / KV, splits > 1 && !partials) + 2048));
     if (blocks <= fit3)
