@@ -642,21 +642,27 @@ def test_attn_decode_mma_balanced(H, KV, hd, page, S, balance, most):
 @pytest.mark.parametrize("H,KV,hd,page,window,splits", [(8, 2, 64, 1, 0, 1), (8, 2, 64, 4, 0, 1), (6, 2, 128, 2, 0, 2), (4, 4, 64, 1, 1500, 1), (8, 2, 64, 16, 0, 1),
                                                         (4, 1, 128, 8, 0, 1)])
 def test_attn_decode_mma_page_list_is_refilled(H, KV, hd, page, window, splits):
-    """A block's page list holds 512 pages and is filled again, half by half, as the block walks on: requests of more pages than that
-    and of lengths around its halves, in clusters, with the merge through global memory and balanced."""
-    half = 256 * page
+    """Beside a table whose pages no block could hold, its list of 1,024 is filled again, half by half, as the block walks on: requests
+    of lengths around its halves, in clusters, with the merge through global memory and balanced. The bits are those of a table just
+    wide enough."""
+    half = 512 * page
     seqs = [(n - 1, 1) for n in (2 * half - 1, 2 * half + 1, 3 * half, 5 * half + 70, 64, 3 * half + 65)]
     dt = torch.bfloat16
     qrows, kc, vc, bt, row_seq, pos, qs, ks, vs = _paged_case(dt, H, KV, hd, page, seqs, seed=hd + page, scale_key=lambda L: max(L - 3 - page, 0))
     want = torch.cat([_last_row(qs[s][-1], ks[s], vs[s], H, KV, hd, window) for s in range(len(seqs))])
     k = K()
-    args = (kc.to(DEV), vc.to(DEV), bt.to(DEV), pos.to(DEV), H, KV, hd, 1.0 / math.sqrt(hd))
+    wide = torch.full((len(seqs), 131072), -1, dtype=torch.int32)
+    wide[:, :bt.shape[1]] = bt
+    caches, tables = (kc.to(DEV), vc.to(DEV)), (bt.to(DEV), wide.to(DEV))
     arrived = torch.zeros(len(seqs) * KV, dtype=torch.int32, device=DEV)
 
     def go(*more, **kw):
-        out = torch.full_like(qrows, 7.0).to(DEV)
-        k.attn_decode_mma(qrows.to(DEV), out, *args, *more, **kw)
-        assert rel(out, want) <= 2 ** -6
+        outs = []
+        for table in tables:
+            outs.append(torch.full_like(qrows, 7.0).to(DEV))
+            k.attn_decode_mma(qrows.to(DEV), outs[-1], *caches, table, pos.to(DEV), H, KV, hd, 1.0 / math.sqrt(hd), *more, **kw)
+            assert rel(outs[-1], want) <= 2 ** -6
+        assert torch.equal(*outs)
     go(window, splits)
     go(window, 2, torch.empty(k.attn_decode_partial_floats(len(seqs), KV, hd, 2), device=DEV), arrived)
     if not window:

@@ -730,7 +730,10 @@ __device__ __forceinline__ bool balance_place(const int* __restrict__ positions,
     share = balance_share(total, want, blocks, [&](int x) {
         int need = 0;
 #pragma unroll
-        for (int i = 0; i < DEC_BALANCE_SEQS / 32; ++i) need += i * 32 + lane < S ? max(1, (n[i] + x - 1) / x) : 0;
+        for (int i = 0; i < DEC_BALANCE_SEQS / 32; ++i) {
+            if (i * 32 >= S) break;
+            need += i * 32 + lane < S ? max(1, (n[i] + x - 1) / x) : 0;
+        }
         return (int)__reduce_add_sync(0xffffffffu, need);
     });
     int before = 0;                                   // blocks of the requests in front
@@ -761,11 +764,14 @@ __device__ __forceinline__ bool balance_place(const int* __restrict__ positions,
 }
 
 // Shared memory of a decode block: the K/V ring (used again for the combine of the four warps),
-// then what the cluster's peers send, then the block's page list: a ring of two halves, so that its size follows neither from the
-// longest request that the block tables can hold nor from how many tiles fall to a block. (Sized for the longest request it took 28 KB
-// at 131,072 tokens of pages of 16, one block an SM instead of two at head size 128, and did not fit at 524,288.) A half holds
-// at least four tiles' pages (pages of one token), 64 tiles' at pages of 16.
-constexpr int DEC_PAGE_LIST = 512;
+// then what the cluster's peers send, then the block's page list. A list for the longest request that the block tables can hold takes
+// 28 KB at 131,072 tokens of pages of 16 in a balanced launch, one block an SM instead of two at head size 128, and finds no room at
+// 524,288. Where it would cost a block its place on the SM, the kernel is another build (REFILL), whose list is a ring of two halves of
+// DEC_PAGE_LIST / 2 that a block fills as it walks on; a half holds at least eight tiles' pages (pages of one token), 128 tiles' at pages
+// of 16. 16 requests of 17 to 8,000 keys beside a table of 131,072 tokens, head size 128, balanced: 46.8 -> 32.5 us; the same in
+// clusters, where the whole list costs no block: 67.8 us with it, 70.9 with the ring. (The ring in every launch: 0.25 us of 5.9 at one
+// request of 517 keys, 3 % at eight of 32,768.)
+constexpr int DEC_PAGE_LIST = 1024;
 template <int HD, int DEC_STAGES, bool KV1> __host__ __device__ constexpr size_t decode_ring_bytes() {
     size_t ring = (size_t)(16 + (KV1 ? 1 : 2) * DEC_STAGES * BN) * (HD + 8) * sizeof(__nv_bfloat16) + (KV1 ? DEC_STAGES * BN * sizeof(float) : 0);
     size_t combine = 16 * (HD + 8) * sizeof(__nv_bfloat16) + (size_t)(128 + 4 * 16 * HD + 16 * HD + 32) * sizeof(float);
@@ -775,7 +781,7 @@ __host__ __device__ constexpr size_t decode_recv_bytes(int G, int HD) { return (
 
 // KV1: the values are the cached keys; the ring holds one tile a stage, which serves both products, and a number per key.
 // Kept first tokens (ScoreShape::keep): their tiles come first in a request's list of tiles, in front of the window's.
-template <int HD, int DEC_STAGES, bool SHAPED, bool KV1>
+template <int HD, int DEC_STAGES, bool SHAPED, bool KV1, bool REFILL>
 __global__ void __launch_bounds__(NTHREADS)
 attn_decode_mma_kernel(const __nv_bfloat16* __restrict__ q, long long q_stride, __nv_bfloat16* __restrict__ out,
                        long long out_stride, const __nv_bfloat16* __restrict__ kc, const __nv_bfloat16* __restrict__ vc,
@@ -838,14 +844,14 @@ attn_decode_mma_kernel(const __nv_bfloat16* __restrict__ q, long long q_stride, 
     auto list_pages = [&](int from, int to) {
         for (int i = from + threadIdx.x; i < min(to, entries); i += NTHREADS) {
             const int lp = (tile_of(n_begin + (i >> ppt_shift)) << ppt_shift) + (i & ((1 << ppt_shift) - 1));
-            s_pages[i & (DEC_PAGE_LIST - 1)] = lp <= (hi - 1) >> page_shift ? bt[lp] : 0;
+            s_pages[REFILL ? i & (DEC_PAGE_LIST - 1) : i] = lp <= (hi - 1) >> page_shift ? bt[lp] : 0;
         }
     };
-    list_pages(0, DEC_PAGE_LIST);
+    list_pages(0, REFILL ? DEC_PAGE_LIST : entries);
     __syncthreads();
     auto load_tile = [&](int n, int buf) {
         const int t = tile_of(n);
-        const int* pages = s_pages + (((n - n_begin) << ppt_shift) & (DEC_PAGE_LIST - 1));
+        const int* pages = s_pages + (REFILL ? ((n - n_begin) << ppt_shift) & (DEC_PAGE_LIST - 1) : (n - n_begin) << ppt_shift);
         load_kv_tile<HD, !KV1>(sK0 + buf * BN * LD, sV0 + buf * BN * LD, kc, vc, pages, t << ppt_shift, kvh, KV, page_shift, t * BN, lo_key, hi, keep);
         if (KV1) load_key_scales(sR0 + buf * BN, shape.kscale, pages, t << ppt_shift, page_shift, t * BN, lo_key, hi, keep);
     };
@@ -900,15 +906,19 @@ attn_decode_mma_kernel(const __nv_bfloat16* __restrict__ q, long long q_stride, 
         for (int i = 0; i < 4; ++i) o[n][i] = 0.f;
     uint32_t qf[HD / 16][4];
 
+    const int half = (DEC_PAGE_LIST / 2) >> ppt_shift;          // tiles of a half of the page list
+    int listed = n_begin + 2 * half;                            // the first tile whose pages are not in the list
     for (int n = n_begin; n < n_end; ++n) {
+        // The half is filled in front of the barrier behind which its first tile is asked for. Its old entries served a tile asked
+        // for two barriers ago at least: nobody reads them any more.
+        if (REFILL && n + DEC_STAGES - 1 == listed) {
+            list_pages((listed - n_begin) << ppt_shift, (listed + half - n_begin) << ppt_shift);
+            listed += half;
+        }
         const int t = tile_of(n);
         int buf = (n - n_begin) % DEC_STAGES;
         __nv_bfloat16* sK = sK0 + buf * BN * LD;
         __nv_bfloat16* sV = sV0 + buf * BN * LD;
-        // the tile asked for behind the barrier begins a half of the page list: the half's last entries served a tile that was
-        // asked for four tiles ago or more, so nobody reads them any more, and the barrier shows everyone the new ones
-        const int entry = (n + DEC_STAGES - 1 - n_begin) << ppt_shift;
-        if (entry >= DEC_PAGE_LIST && (entry & (DEC_PAGE_LIST / 2 - 1)) == 0) list_pages(entry, entry + DEC_PAGE_LIST / 2);
         cp_async_wait<DEC_STAGES - 2>();        // tile n has landed (one newer group may be in flight)
         __syncthreads();                        // ... for every thread; and everyone is done with tile n-1
         {
@@ -1073,14 +1083,14 @@ int launch_prefill(const void* q, long long q_stride, void* out, long long out_s
         scale * 1.4426950408889634f, tail);
 }
 
-template <int HD, int ST, bool SHAPED, bool KV1>
-int launch_decode_st(const void* q, long long q_stride, void* out, long long out_stride, const void* kc, const void* vc,
+template <int HD, int ST, bool SHAPED, bool KV1, bool REFILL>
+int launch_decode_build(const void* q, long long q_stride, void* out, long long out_stride, const void* kc, const void* vc,
                      const int* bt, int max_pages, const int* positions, int S, int H, int KV, int page_size, int window,
                      float scale, int splits, float* partials, int* arrived, AttnTail tail, ScoreShape shape, int balance, int grid_blocks,
-                     cudaStream_t stream) {
+                     long long list, cudaStream_t stream) {
     static size_t configured = 0;
-    const size_t smem = decode_smem<HD, ST, KV1>(H / KV, splits > 1 && !partials) + DEC_PAGE_LIST * sizeof(int);
-    int e = ensure_smem(attn_decode_mma_kernel<HD, ST, SHAPED, KV1>, smem, &configured);
+    const size_t smem = decode_smem<HD, ST, KV1>(H / KV, splits > 1 && !partials) + (size_t)list * sizeof(int);
+    int e = ensure_smem(attn_decode_mma_kernel<HD, ST, SHAPED, KV1, REFILL>, smem, &configured);
     if (e) return e;
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = balance ? dim3(grid_blocks, KV) : dim3(S, KV, splits);
@@ -1096,11 +1106,32 @@ int launch_decode_st(const void* q, long long q_stride, void* out, long long out
     attr[1].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attr;
     cfg.numAttrs = g_vob_pdl ? 2 : 1;
-    cudaError_t ce = cudaLaunchKernelEx(&cfg, attn_decode_mma_kernel<HD, ST, SHAPED, KV1>, (const __nv_bfloat16*)q, q_stride, (__nv_bfloat16*)out,
+    cudaError_t ce = cudaLaunchKernelEx(&cfg, attn_decode_mma_kernel<HD, ST, SHAPED, KV1, REFILL>, (const __nv_bfloat16*)q, q_stride, (__nv_bfloat16*)out,
                                         out_stride, (const __nv_bfloat16*)kc, (const __nv_bfloat16*)vc, bt, max_pages, positions,
                                         H, KV, log2_exact(page_size), window, scale * 1.4426950408889634f, partials, arrived, tail, shape,
                                         balance, S);
     return ce != cudaSuccess ? (int)ce : vob_launch_status();
+}
+
+template <int HD, int ST, bool SHAPED, bool KV1>
+int launch_decode_st(const void* q, long long q_stride, void* out, long long out_stride, const void* kc, const void* vc,
+                     const int* bt, int max_pages, const int* positions, int S, int H, int KV, int page_size, int window,
+                     float scale, int splits, float* partials, int* arrived, AttnTail tail, ScoreShape shape, int balance, int grid_blocks,
+                     cudaStream_t stream) {
+    // a block's page list: its share of the tiles of the longest request the block table can hold
+    // (a request with few tiles uses fewer blocks, but then the tiles are few)
+    const long long tiles_max = ((long long)max_pages * page_size + BN - 1) / BN;
+    long long tiles = (tiles_max + splits - 1) / splits;
+    if (balance) tiles = std::min(tiles_max, 2 * ((S * tiles_max + balance - 1) / balance));
+    if (partials) tiles = std::max<long long>(tiles, 2 * DEC_MIN_TILES);
+    const long long list = tiles * (BN / page_size);
+    // blocks of so much shared memory that an SM holds (1 KB of each is the system's)
+    auto resident = [&](long long ints) { return 228 * 1024 / (long long)(decode_smem<HD, ST, KV1>(H / KV, splits > 1 && !partials) + ints * sizeof(int) + 1024); };
+    if (list > DEC_PAGE_LIST && resident(list) < resident(DEC_PAGE_LIST))
+        return launch_decode_build<HD, ST, SHAPED, KV1, true>(q, q_stride, out, out_stride, kc, vc, bt, max_pages, positions, S, H, KV, page_size, window,
+                                                              scale, splits, partials, arrived, tail, shape, balance, grid_blocks, DEC_PAGE_LIST, stream);
+    return launch_decode_build<HD, ST, SHAPED, KV1, false>(q, q_stride, out, out_stride, kc, vc, bt, max_pages, positions, S, H, KV, page_size, window,
+                                                           scale, splits, partials, arrived, tail, shape, balance, grid_blocks, list, stream);
 }
 
 template <int HD, bool SHAPED, bool KV1 = false>
@@ -1115,7 +1146,7 @@ int launch_decode(const void* q, long long q_stride, void* out, long long out_st
         cudaDeviceGetAttribute(&num_sms, cudaDevAttrMultiProcessorCount, dev);
         if (num_sms <= 0) num_sms = 148;
     }
-    // three stages while every block of the grid can be resident at once with them (2 KB beside the ring: the page list); else two
+    // three stages while every block of the grid can be resident at once with them; else two
     long long blocks = balance ? (long long)balance * KV : (long long)S * KV * splits;
     long long fit3 = (long long)num_sms * ((227 * 1024) / (long long)(decode_smem<HD, 3, KV1>(H / KV, splits > 1 && !partials) + 2048));
     if (blocks <= fit3)

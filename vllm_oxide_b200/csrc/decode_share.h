@@ -14,16 +14,25 @@ constexpr int DEC_MIN_TILES = 3;           // fewest tiles a block is started fo
 // The smallest number of tiles a block (at least DEC_MIN_TILES, and an even share of `total` tiles over `want` blocks) at which
 // the requests need no more than `blocks` blocks. need(share): the sum over the requests of max(1, ceil(tiles / share)). Twice the
 // even share always suffices where blocks >= want / 2 + requests: want / 2 blocks hold the whole shares, every request has one rest.
-template <typename Need> VOB_BOTH int balance_share(long long total, int want, int blocks, Need need) {
-    int lo = (int)((total + want - 1) / want);
+template <typename Need> VOB_BOTH int balance_share(int total, int want, int blocks, Need need) {
+    int lo = (total + want - 1) / want;
     if (lo < DEC_MIN_TILES) lo = DEC_MIN_TILES;
-    int hi = 2 * lo;
-    if (need(lo) <= blocks) return lo;
-    ++lo;
+    // upwards in steps that double until a share suffices (mostly the first or the second does), then by halving. `need` stands here
+    // once: the kernel comes by with cold instruction caches.
+    int hi = 2 * lo, at = lo, step = 1;
+    bool found = false;
     while (lo < hi) {
-        const int mid = (lo + hi) / 2;
-        if (need(mid) <= blocks) hi = mid;
-        else lo = mid + 1;
+        if (need(at) <= blocks) {
+            hi = at;
+            found = true;
+        } else {
+            lo = at + 1;
+        }
+        at = (lo + hi) / 2;
+        if (!found) {
+            at = lo + step - 1 < hi ? lo + step - 1 : hi - 1;
+            step *= 2;
+        }
     }
     return lo;
 }

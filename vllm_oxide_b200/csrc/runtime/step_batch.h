@@ -77,10 +77,10 @@ struct StepArrays {
         if (want < 1 || requests < seqs) throw CacheError("balanced_share: bad sizes");
         const int32_t* lens = data.data() + layout.seq_lens;
         auto tiles = [&](int s) { return (lens[s] + DEC_TILE_KEYS - 1) / DEC_TILE_KEYS; };
-        int64_t total = 0;
+        int total = 0;
         for (int s = 0; s < seqs; ++s) total += tiles(s);
         return balance_share(total, want, balance_blocks(want, requests), [&](int share) {
-            int64_t n = requests - seqs;
+            int n = requests - seqs;
             for (int s = 0; s < seqs; ++s) n += std::max(1, (tiles(s) + share - 1) / share);
             return n;
         });
