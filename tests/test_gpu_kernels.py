@@ -129,6 +129,35 @@ def test_gemm_f32_kernels_agree_to_the_bit(N, K_):
             assert torch.equal(out[:M], full[lo:lo + M]) and bool((out[M] == 7.0).all()), (M, lo)
 
 
+@pytest.mark.parametrize("dt", DT, ids=IDS)
+def test_a_matrix_written_by_the_kernel_in_front(dt):
+    """`w` of a product may be what the kernel in front writes, with a bias and without: nothing of it is read before that kernel is
+    done unless the caller says that no kernel writes it. (bfloat16 without a bias always takes `w` for weights.)"""
+    g = torch.Generator().manual_seed(5)
+    N, Kd, inner = 512 if dt == torch.float32 else 32, 1024, 2048         # (few rows of `w`: written by this package's kernel)
+    x = torch.randn(16, Kd, generator=g).to(dt).to(DEV)
+    w_t = torch.randn(Kd, inner, generator=g).to(dt).to(DEV)
+    bias = torch.randn(N, generator=g).to(dt).to(DEV)
+    k = K()
+    makers = [torch.randn(N, inner, generator=g).to(dt).to(DEV) for _ in range(12)]
+    w = torch.zeros(N, Kd, dtype=dt, device=DEV)
+    for M in (1, 3, 16):
+        outs = [torch.empty(M, N, dtype=dt, device=DEV) for _ in makers]
+        torch.cuda.synchronize()
+        for a, out in zip(makers, outs):
+            k.linear(a, w_t, w)                    # w = a @ w_t^T
+            k.linear(x[:M], w, out, bias)
+        for a, out in zip(makers, outs):
+            k.linear(a, w_t, w)
+            torch.cuda.synchronize()
+            again = torch.empty_like(out)
+            k.linear(x[:M], w, again, bias)
+            assert torch.equal(out, again), M
+            if dt == torch.float32:                # read early or not: the same bits
+                k.linear(x[:M], w, again, bias, fixed_w=True)
+                assert torch.equal(out, again), M
+
+
 def test_gemm_f32_shape_errors():
     from vllm_oxide_b200.errors import ShapeError
     with pytest.raises(ShapeError):
@@ -716,12 +745,13 @@ def test_linear_bf16_with_a_bias(T, N, Kd):
     g = torch.Generator().manual_seed(T + N)
     a, w = (torch.randn(n, Kd, generator=g).to(torch.bfloat16).to(DEV) for n in (T, N))
     bias = (30 * torch.randn(N, generator=g)).to(torch.bfloat16).to(DEV)
-    out = torch.full((T + 1, N), 7.0, dtype=torch.bfloat16, device=DEV)
-    K().linear(a, w, out[:T], bias)
     want = a.double() @ w.double().T + bias.double()
     # half a unit in the last of bfloat16's 8 bits (2^-8 of the value at most), and float32 sums of Kd products
     bound = 2.0 ** -8 * 1.01 * want.abs() + Kd * 2.0 ** -24 * (a.double().abs() @ w.double().abs().T)
-    assert bool(((out[:T].double() - want).abs() <= bound).all()) and bool((out[T] == 7.0).all())
+    for fixed_w in (False, True):                  # read before the kernels in front are done, or not
+        out = torch.full((T + 1, N), 7.0, dtype=torch.bfloat16, device=DEV)
+        K().linear(a, w, out[:T], bias, fixed_w)
+        assert bool(((out[:T].double() - want).abs() <= bound).all()) and bool((out[T] == 7.0).all())
 
 
 @pytest.mark.parametrize("odt", [torch.bfloat16, torch.float32], ids=["bf16out", "f32out"])

@@ -68,7 +68,7 @@ constexpr int few_stages(int mb) { return mb == 4 ? 3 : 2; }
 template <int MB, int RN, int NS>
 __global__ void __launch_bounds__(256 / RN, few_blocks(MB))
 gemm_f32_few_kernel(const float* __restrict__ A, long long lda, const float* __restrict__ W, long long ldw, float* __restrict__ C,
-                    long long ldc, int M, int N, int K, const float* __restrict__ bias, int nc, int q, int c) {
+                    long long ldc, int M, int N, int K, const float* __restrict__ bias, int nc, int q, int c, int early) {
     constexpr int THREADS = 256 / RN, STAGE = 32 * RN * FEW_K;        // floats of a warp's stage: its rows, 16-byte pieces at (piece ^ row & 7)
     extern __shared__ __align__(16) float smem[];
     float* ring = smem;                               // [8 / RN warps][NS][STAGE]
@@ -98,10 +98,11 @@ gemm_f32_few_kernel(const float* __restrict__ A, long long lda, const float* __r
         }
         cp_async_commit();
     };
-    // weights are written by no kernel: their first stages are asked for before the wait
+    // `early`: no kernel writes W, so its first stages are asked for before the wait
+    if (!early) pdl_wait(11);
 #pragma unroll
     for (int s = 0; s < NS; ++s) load();
-    pdl_wait(11);
+    if (early) pdl_wait(11);
 
     int get = 0, seg = seg_chunks(nc);
     for (int t = 0; t * 4 < mine; ++t) {
@@ -186,7 +187,7 @@ gemm_f32_few_kernel(const float* __restrict__ A, long long lda, const float* __r
 
 template <int MB>
 int launch_few(const float* A, long long lda, const float* W, long long ldw, float* C, long long ldc, int M, int N, int K,
-               const float* bias, int nc, int q, int c, cudaStream_t stream) {
+               const float* bias, int nc, int q, int c, int early, cudaStream_t stream) {
     constexpr int RN = few_rows_a_lane(MB), NS = few_stages(MB);
     size_t smem = sizeof(float) * (size_t)(8 * NS * 32 * FEW_K + 4 * CHUNK * MB + min(q, nc) * MB * FEW_N);
     if (smem > 200 * 1024) return VOB_ERR_UNSUPPORTED;
@@ -207,7 +208,7 @@ int launch_few(const float* A, long long lda, const float* W, long long ldw, flo
     attr[1].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attr;
     cfg.numAttrs = g_vob_pdl ? 2 : 1;
-    e = cudaLaunchKernelEx(&cfg, kernel, A, lda, W, ldw, C, ldc, M, N, K, bias, nc, q, c);
+    e = cudaLaunchKernelEx(&cfg, kernel, A, lda, W, ldw, C, ldc, M, N, K, bias, nc, q, c, early);
     return e != cudaSuccess ? (int)e : vob_launch_status();
 }
 
@@ -379,9 +380,10 @@ int launch_tile(const float* A, long long lda, const float* W, long long ldw, fl
 
 }  // namespace
 
-// `bias` (N entries, may be null) is added to every row after the sum over k.
+// `bias` (N entries, may be null) is added to every row after the sum over k. `early`: W holds weights, which no kernel writes, and
+// may be read while the kernels in front still run.
 VOB_EXPORT int vob_gemm_f32(const float* A, long long lda, const float* W, long long ldw, float* C,
-                            long long ldc, int M, int N, int K, const float* bias, cudaStream_t stream) {
+                            long long ldc, int M, int N, int K, const float* bias, int early, cudaStream_t stream) {
     if (M <= 0 || N <= 0) return 0;
     if (K <= 0 || lda < K || ldw < K || ldc < N) return VOB_ERR_BAD_ARG;
     if ((M + 63) / 64 > 65535) return VOB_ERR_UNSUPPORTED;
@@ -391,11 +393,11 @@ VOB_EXPORT int vob_gemm_f32(const float* A, long long lda, const float* W, long 
     // tile is 32 rows at least); on 2,048 x 8,192, where a block has its SM to itself, 67 and 58.
     if (vec && M <= 16) {
         int q = ((nc + 7) / 8 + 3) / 4 * 4, c = (nc + q - 1) / q;
-        int e = M == 1   ? launch_few<1>(A, lda, W, ldw, C, ldc, M, N, K, bias, nc, q, c, stream)
-                : M == 2 ? launch_few<2>(A, lda, W, ldw, C, ldc, M, N, K, bias, nc, q, c, stream)
-                : M <= 4 ? launch_few<4>(A, lda, W, ldw, C, ldc, M, N, K, bias, nc, q, c, stream)
-                : M <= 8 ? launch_few<8>(A, lda, W, ldw, C, ldc, M, N, K, bias, nc, q, c, stream)
-                         : launch_few<16>(A, lda, W, ldw, C, ldc, M, N, K, bias, nc, q, c, stream);
+        int e = M == 1   ? launch_few<1>(A, lda, W, ldw, C, ldc, M, N, K, bias, nc, q, c, early, stream)
+                : M == 2 ? launch_few<2>(A, lda, W, ldw, C, ldc, M, N, K, bias, nc, q, c, early, stream)
+                : M <= 4 ? launch_few<4>(A, lda, W, ldw, C, ldc, M, N, K, bias, nc, q, c, early, stream)
+                : M <= 8 ? launch_few<8>(A, lda, W, ldw, C, ldc, M, N, K, bias, nc, q, c, early, stream)
+                         : launch_few<16>(A, lda, W, ldw, C, ldc, M, N, K, bias, nc, q, c, early, stream);
         if (e != VOB_ERR_UNSUPPORTED) return e;       // a K whose sums find no room in shared memory: tiles
     }
     // Tiles of 128, 64 or 32 rows, a block or eight to a tile: the one whose waves of blocks cost least. A wave's cost is its

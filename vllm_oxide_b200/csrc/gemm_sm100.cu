@@ -132,6 +132,7 @@ struct EpiArgs {
     long long ld_part;
     // EPI_STORE
     const __nv_bfloat16* bias;         // [N] or null: added to the float32 sum
+    int late_w;                        // W may be what a kernel in front writes: not read before those are done
 };
 typedef EpiArgs QkvArgs;
 
@@ -210,8 +211,9 @@ gemm_sm100_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_consta
 
     if (warp == 0) {
         if (lane == 0) {
-            // Weights are written by no kernel, so their loads start at once and overlap whatever
+            // Weights are written by no kernel (unless the caller says so), so their loads start at once and overlap whatever
             // still runs before this kernel; the activations are loaded only after the wait.
+            if (qa.late_w) pdl_wait();
             const int pre = nkb < STAGES ? nkb : STAGES;
             for (int i = 0; i < pre; ++i) {
                 unsigned char* a = tiles + i * SB;

@@ -529,10 +529,10 @@ def glu(gate_up: torch.Tensor, out: torch.Tensor, activation: str = "silu") -> N
 
 # ------------------------------------------------------------------------------------ matrix products
 @_timed
-def gemm_f32(a: torch.Tensor, w: torch.Tensor, out: torch.Tensor, bias: Optional[torch.Tensor] = None) -> None:
+def gemm_f32(a: torch.Tensor, w: torch.Tensor, out: torch.Tensor, bias: Optional[torch.Tensor] = None, fixed_w: bool = False) -> None:
     """out[M, N] = a[M, K] @ w[N, K]^T (+ bias[N]) in true float32 (FMA chains over k, always added in the same order; no tensor cores).
-    `w` holds weights: with programmatic dependent launch its first rows are read while the kernel in front still runs, so it
-    must not be what such a kernel of this package writes."""
+    `fixed_w`: no kernel writes `w` (a model's weights): with programmatic dependent launch its first rows are then read while the
+    kernels in front still run."""
     op = "gemm_f32"
     _cuda(op, a, w, out, bias)
     for name, t in (("a", a), ("w", w), ("out", out)):
@@ -547,8 +547,8 @@ def gemm_f32(a: torch.Tensor, w: torch.Tensor, out: torch.Tensor, bias: Optional
         raise ShapeError(op, f"out must be [{M}, {N}], got {list(out.shape)}")
     if bias is not None and (bias.dtype != torch.float32 or bias.shape != (N,) or not bias.is_contiguous()):
         raise ShapeError(op, f"bias must be contiguous float32 [{N}], got {bias.dtype} {list(bias.shape)}")
-    f = _fn("gemm_f32", "vob_gemm_f32", [_P, _L, _P, _L, _P, _L, _I, _I, _I, _P, _P])
-    _check(f(_ptr(a), a.stride(0), _ptr(w), w.stride(0), _ptr(out), out.stride(0), M, N, K, _ptr(bias), _stream()), op)
+    f = _fn("gemm_f32", "vob_gemm_f32", [_P, _L, _P, _L, _P, _L, _I, _I, _I, _P, _I, _P])
+    _check(f(_ptr(a), a.stride(0), _ptr(w), w.stride(0), _ptr(out), out.stride(0), M, N, K, _ptr(bias), int(fixed_w), _stream()), op)
 
 
 class _GemmScratch:
@@ -736,7 +736,7 @@ class _EpiArgs(ctypes.Structure):
                 ("q_dim", _I), ("kv_dim", _I), ("hd", _I), ("KV", _I), ("page_size", _I),
                 ("ssq_tiles", _I), ("ld_ssq", _I), ("inv_h", _F), ("eps", _F), ("act", _I),
                 ("temperature", _P), ("seeds", _P), ("steps", _P), ("part_val", _P), ("part_idx", _P), ("nan_flags", _P),
-                ("ld_part", _L), ("bias", _P)]
+                ("ld_part", _L), ("bias", _P), ("late_w", _I)]
 
 
 def _dp(t: Optional[torch.Tensor]) -> int:
@@ -769,10 +769,11 @@ def embed_fold(table: torch.Tensor, tokens: torch.Tensor, resid: torch.Tensor, n
 @_timed
 def gemm_fused(a: torch.Tensor, w: torch.Tensor, out: Optional[torch.Tensor], mode: int, n_features: int, *,
                ssq_in: Optional[torch.Tensor] = None, eps: float = 0.0, qkv=None, resid=None, pick=None,
-               splits: Optional[int] = None, bias: Optional[torch.Tensor] = None) -> None:
+               splits: Optional[int] = None, bias: Optional[torch.Tensor] = None, late_w: bool = False) -> None:
     """The tcgen05 product for at most 64 rows with a fused epilogue and, optionally, the RMSNorm of
     its input folded in: `a` holds bf16(x * norm weight), `ssq_in` [tiles, ld] the per-tile sums of
-    squares of x, and each token's accumulator is multiplied by 1 / sqrt(mean(x^2) + eps).
+    squares of x, and each token's accumulator is multiplied by 1 / sqrt(mean(x^2) + eps). `w` is taken for weights, which
+    no kernel writes, and read while the kernels in front still run; with `late_w` it is not read before they are done.
       EPI_STORE  out[T, n] (bfloat16 or float32) = result (+ `bias`, contiguous bfloat16 [n], added in float32)
       EPI_SWIGLU out[T, n] = silu(gate) * up, w = [Wg; Wu] of shape [2n, K]
       EPI_QKV    qkv = (positions, slots, inv_freq, kcache, vcache, H, KV, hd): out[T, H*hd] = rotated q,
@@ -794,6 +795,7 @@ def gemm_fused(a: torch.Tensor, w: torch.Tensor, out: Optional[torch.Tensor], mo
     if w.shape != (w_rows, K):
         raise ShapeError(op, f"w must be [{w_rows}, {K}], got {list(w.shape)}")
     ea = _EpiArgs()
+    ea.late_w = int(late_w)
     if ssq_in is not None:
         if ssq_in.dtype != torch.float32 or ssq_in.dim() != 2 or ssq_in.shape[0] != -(-K // 128) or ssq_in.shape[1] < T or not ssq_in.is_contiguous():
             raise ShapeError(op, f"ssq_in must be contiguous float32 [{-(-K // 128)}, >={T}], got {list(ssq_in.shape)}")
@@ -895,16 +897,18 @@ def gemm_sm100_check() -> None:
                               "18-21 softmax rows); its result is not valid")
 
 
-def linear(a: torch.Tensor, w: torch.Tensor, out: torch.Tensor, bias: Optional[torch.Tensor] = None) -> None:
+def linear(a: torch.Tensor, w: torch.Tensor, out: torch.Tensor, bias: Optional[torch.Tensor] = None, fixed_w: bool = False) -> None:
     """out = a @ w^T (+ bias, a vector of the operands' type: added to the float32 sum before the result is
     rounded). float32 operands: the true 32-bit kernel. bfloat16 operands: this package's
     tcgen05 kernel (TMA operands, float32 accumulation in tensor memory); for many rows, or
     operands TMA cannot address (K not a multiple of 8, unaligned rows), the library product
     (cuBLAS through torch, float32 accumulation; above `TUNING.few_rows` rows), as the reference plans for its own matrix
-    products (CLAUDE.md:107). `out` may be bfloat16 or float32."""
+    products (CLAUDE.md:107). `out` may be bfloat16 or float32. `fixed_w`: no kernel writes `w` (a model's weights), so that the 32-bit
+    kernel and the tcgen05 kernel with a bias may read it while the kernels in front still run, as the tcgen05 kernel without a
+    bias always does."""
     op = "linear"
     if a.dtype == torch.float32:
-        gemm_f32(a, w, out, bias)
+        gemm_f32(a, w, out, bias, fixed_w)
         return
     _cuda(op, a, w, out, bias)
     if a.dtype != torch.bfloat16 or w.dtype != torch.bfloat16:
@@ -919,7 +923,7 @@ def linear(a: torch.Tensor, w: torch.Tensor, out: torch.Tensor, bias: Optional[t
         # Four rows at 3,072 and 2,048 x 2,048 in a decode step: 8.6 and 7.0 us with the library, beside which no other kernel starts
         # early; 5.6 here, and the kernels around them 0.3 to 0.5 us less each.
         if a.shape[0] <= min(TUNING.few_rows, FUSED_GEMM_MAX_ROWS) and gemm_sm100_supported(a, w) and out.stride(1) == 1 and bias.is_contiguous():
-            gemm_fused(a, w, out, EPI_STORE, w.shape[0], bias=bias)
+            gemm_fused(a, w, out, EPI_STORE, w.shape[0], bias=bias, late_w=not fixed_w)
         else:
             _library_gemm_bf16(a, w, out, bias)
     elif a.shape[0] <= TUNING.few_rows and gemm_sm100_supported(a, w):

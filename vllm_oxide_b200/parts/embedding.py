@@ -88,7 +88,7 @@ class LMHead:
         return ("gemm_f32",) if dtype == torch.float32 else ("gemm_sm100",)
 
     def forward(self, normed: torch.Tensor, out: torch.Tensor) -> torch.Tensor:
-        kernels.linear(normed, self.weight, out)
+        kernels.linear(normed, self.weight, out, fixed_w=True)
         return out
 
     def can_fold(self) -> bool:

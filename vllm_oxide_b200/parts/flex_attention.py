@@ -382,9 +382,9 @@ class SoftmaxAttention(Mixer):
     def forward(self, x: torch.Tensor, ctx: StepContext, cache: Optional[LayerCache], state=None, out=None) -> torch.Tensor:
         T = x.shape[0]
         proj = ctx.alloc((T, self.w_in.shape[0]))
-        kernels.linear(x, self.w_in, proj, self.b_in)
+        kernels.linear(x, self.w_in, proj, self.b_in, fixed_w=True)
         pre = ctx.alloc((T, self.n_pre))
         self.core(proj, ctx, cache, state, pre)
         out = out if out is not None else ctx.alloc((T, self.hidden))
-        kernels.linear(pre, self.w_o, out, self.b_o)
+        kernels.linear(pre, self.w_o, out, self.b_o, fixed_w=True)
         return out

@@ -182,12 +182,12 @@ class LatentAttention(Mixer):
         else:
             q_lat = ctx.alloc((T, H, L), torch.float32)
             for h in range(H):
-                kernels.linear(q_heads[:, h], self.w_qlat[h], q_lat[:, h])
+                kernels.linear(q_heads[:, h], self.w_qlat[h], q_lat[:, h], fixed_w=True)
             out_lat = ctx.alloc((T, H, L))
             kernels.latent_attend(q_lat, q_rot, lat, kr, bt, ctx.row_seq, ctx.positions, self.scale, out_lat, splits, partials, self.window)
             attn = ctx.alloc((T, H * V))
             for h in range(H):
-                kernels.linear(out_lat[:, h], self.w_val[h], attn[:, h * V:(h + 1) * V])
+                kernels.linear(out_lat[:, h], self.w_val[h], attn[:, h * V:(h + 1) * V], fixed_w=True)
             if gate is not None:
                 kernels.latent_gate(attn.view(T, H, V), gate, attn)
         return matmul(attn, self.w_o, out if out is not None else ctx.alloc((T, self.hidden)))

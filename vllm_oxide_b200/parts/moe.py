@@ -124,14 +124,14 @@ class RoutedExperts(FeedForward):
         if (self.activation == "silu" and not gated and self.dtype == torch.bfloat16 and x.shape[0] <= TUNING.few_rows
                 and kernels.gemm_sm100_supported(x, w_gu)):
             kernels.gemm_swiglu(x, w_gu, hs)             # few rows: the gate in the product's epilogue
-            kernels.linear(hs, w_down, sh)
+            kernels.linear(hs, w_down, sh, fixed_w=True)
             return
-        kernels.linear(x, w_gu, gu)
+        kernels.linear(x, w_gu, gu, fixed_w=True)
         if self.activation == "clamped_swish":
             kernels.glu_clamped(gu[:, :2 * fs], hs, slimit)
         else:
             kernels.glu(gu[:, :2 * fs], hs, "silu")
-        kernels.linear(hs, w_down, sh)
+        kernels.linear(hs, w_down, sh, fixed_w=True)
 
     def forward(self, x: torch.Tensor, ctx: StepContext, out=None) -> torch.Tensor:
         T = x.shape[0]

@@ -84,7 +84,7 @@ class ParallelMixer(Mixer):
     def forward(self, x: torch.Tensor, ctx: StepContext, cache: Optional[LayerCache], state, out=None) -> torch.Tensor:
         T = x.shape[0]
         proj = ctx.alloc((T, self.w_in.shape[0]))
-        kernels.linear(x, self.w_in, proj, self.b_in)
+        kernels.linear(x, self.w_in, proj, self.b_in, fixed_w=True)
         pre = ctx.alloc((T, self.w_o.shape[1]))
         st = () if state is None else (tuple(state) if isinstance(state, (tuple, list)) else (state,))
         ls, rs = st[:self.n_left_state], st[self.n_left_state:]
@@ -96,5 +96,5 @@ class ParallelMixer(Mixer):
             self.right.core(proj[:, self.n_left_in:], ctx, cache if self.right.cache_spec() is not None else None, rs or None,
                             pre[:, nl:], self.right_scale)
         out = out if out is not None else ctx.alloc((T, self.hidden))
-        kernels.linear(pre, self.w_o, out, self.b_o)
+        kernels.linear(pre, self.w_o, out, self.b_o, fixed_w=True)
         return out

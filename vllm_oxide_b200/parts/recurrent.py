@@ -245,7 +245,7 @@ class GatedDelta(Mixer):
         T, gk, hk, hv = proj.shape[0], self.G * self.K, self.H * self.K, self.H * self.V
         if self.w_low is not None:
             low = ctx.alloc((T, hk + hv))
-            kernels.linear(proj[:, self.low_off:self.low_off + self.ra + self.rg], self.w_low, low)
+            kernels.linear(proj[:, self.low_off:self.low_off + self.ra + self.rg], self.w_low, low, fixed_w=True)
             a_src, a_off, g_src = low, 0, low[:, hk:]
         else:       # [.. | W_a h (heads) | W_g h (heads * vdim) | ..] are columns of the first product
             a_src, a_off = proj, self.low_off
