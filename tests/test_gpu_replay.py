@@ -328,6 +328,30 @@ def test_f32_cuts_agree_closely(tmp_path_factory):
             assert max_rel_diff(c[k], a[k]) <= 1e-5
 
 
+def test_a_function_behind_every_block_is_called_in_every_step(tmp_path_factory):
+    """`ModelRunner.after_block` on an engine that records its steps: steps of one shape class again and again, and decode steps whose
+    logits are wanted, come by it each time."""
+    from vllm_oxide_b200.engine import LLM
+    from vllm_oxide_b200.replay.trace import TraceSession
+    from vllm_oxide_b200.sampling import SamplingParams
+    cfg, _, page = TINY["B"]
+    llm = LLM(make_model_dir(tmp_path_factory.getbasetemp(), "B"), dtype="float32", max_batch_tokens=64, max_seqs=4, max_model_len=64,
+              block_size=page, num_pages=64)
+    s, calls = TraceSession(llm.runner), len(llm.runner.spec.schedule)
+    seen = []
+    for hooked in (True, False, True):
+        llm.runner.after_block = (lambda i, resid, pending: seen.append((i, resid.clone()))) if hooked else None
+        for n in range(4):
+            seen.clear()
+            toks = random_tokens(20, cfg.vocab_size, 70 + n)
+            s.run_step({"step": n, "entries": [{"id": "a", "tokens": toks, "want": [19]}], "end": ["a"]})
+            assert [i for i, _ in seen] == (list(range(calls)) if hooked else [])
+        seen.clear()
+        llm.generate([toks], SamplingParams(max_new_tokens=3, stop_token_ids=(), capture_logits=(0, 1, 2)))
+        assert [i for i, _ in seen] == (3 * list(range(calls)) if hooked else [])
+    assert llm.runner.step_graph_replays > 0
+
+
 def test_trace_run_program(tmp_path):
     """bin/trace_run as a user runs it: JSON lines in, `done <step>` lines and .f32 files out."""
     cfg, _, page = TINY["A"]

@@ -177,7 +177,9 @@ class ModelRunner:
         self.step_graph_after = int(getattr(engine, "step_graphs", 0))
         self.step_graph_replays = 0
         self._folded = None
-        self.after_block = None                 # debugging: a function (call number, residual, pending) run behind every block
+        # debugging: a function (call number, residual, pending) run behind every block; while there is one, steps are launched one
+        # by one (a replayed step would not come by it)
+        self.after_block = None
         self._pending_scale = None
         self._graph_launches = {}
         self._balance_rules = None              # (kv heads, head size, SMs) of the mixers `_balance` asks for; read off the parts at first use
@@ -469,7 +471,7 @@ class ModelRunner:
         padding: position -1, they attend to nothing and write nothing, as in a decode step's
         graph) and so is the longest portion (kernels take it as an upper bound). None: this step
         is not replayed (graphs off, a decode step, no logits wanted)."""
-        if not (self.graphs_enabled and self.step_graph_after > 0):
+        if not (self.graphs_enabled and self.step_graph_after > 0) or self.after_block is not None:
             return None
         return step_shape_class(arrays.rows, arrays.seqs, arrays.logit_count, arrays.max_new, arrays.lead_single,
                                 arrays.max_seq_len, self.rows_cap)
@@ -528,7 +530,7 @@ class ModelRunner:
         else:
             self.upload(arrays, parity)
         long_context = bool(arrays.max_seq_len > TUNING.long_context_keys)
-        if not self.decode_graphs:
+        if not self.decode_graphs or self.after_block is not None:
             logits = self._decode_eager(S, parity, long_context, logits_out is not None, self._balance(arrays, S))      # nothing is recorded: no padding needed
         else:
             b = self._bucket(S)
