@@ -389,10 +389,12 @@ VOB_EXPORT int vob_gemm_f32(const float* A, long long lda, const float* W, long 
     if ((M + 63) / 64 > 65535) return VOB_ERR_UNSUPPORTED;
     int nc = (K + CHUNK - 1) / CHUNK;
     int vec = K % 4 == 0 && lda % 4 == 0 && ldw % 4 == 0 && ((uintptr_t)A & 15) == 0 && ((uintptr_t)W & 15) == 0;
-    // 16 rows: what a lane's registers hold. On 16,384 x 2,048 the kernel of few rows takes 69 us there and the tiles take 96 at 17 (a
-    // tile is 32 rows at least); on 2,048 x 8,192, where a block has its SM to itself, 67 and 58.
-    if (vec && M <= 16) {
-        int q = ((nc + 7) / 8 + 3) / 4 * 4, c = (nc + q - 1) / q;
+    // 16 rows: what a lane's registers hold. Cold, 9 to 16 rows, us here / in tiles (32 rows at least): 2,048 x 512 16 / 23, 2,048 x 2,048
+    // 19 / 21, 4,096 x 4,096 41 / 55, 16,384 x 2,048 68 / 94, 128,256 x 2,048 391 / 644; where K has more than 32 chunks a block of 16
+    // rows has its SM to itself, and the tiles win: 2,048 x 8,192 66 / 57, 4,096 x 14,336 209 / 170. Up to 8 rows the tiles never do: there
+    // 29 / 57 and 83 / 169 at 8 rows, 25 / 57 and 70 / 170 at one.
+    int q = ((nc + 7) / 8 + 3) / 4 * 4, c = (nc + q - 1) / q;
+    if (vec && (M <= 8 || (M <= 16 && q == 4))) {
         int e = M == 1   ? launch_few<1>(A, lda, W, ldw, C, ldc, M, N, K, bias, nc, q, c, early, stream)
                 : M == 2 ? launch_few<2>(A, lda, W, ldw, C, ldc, M, N, K, bias, nc, q, c, early, stream)
                 : M <= 4 ? launch_few<4>(A, lda, W, ldw, C, ldc, M, N, K, bias, nc, q, c, early, stream)
