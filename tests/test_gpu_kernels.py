@@ -283,7 +283,7 @@ def test_paged_attention_window_edge(dt, window):
 def test_f32_attention_of_portions_and_of_single_tokens_agree_to_the_bit(H, KV, hd, page, window):
     """The 32-bit engine's two kernels (single tokens over one to eight blocks, rows of portions) give a row the same bits, whatever
     shares its block; a padding row gives zeros; an infinity among a later token's values reaches no earlier row."""
-    # 349 rows: the rows' kernel takes what lies behind the single tokens while it is more than 256 rows
+    # 349 rows: the rows' kernel takes what lies behind the single tokens while it is more than 128 rows
     seqs = [(0, 70), (131, 1), (30, 5), (0, 1), (31, 2), (63, 66), (700, 1), (255, 200)]
     qrows, kc, vc, bt, row_seq, pos, qs, ks, vs = _paged_case(torch.float32, H, KV, hd, page, seqs, seed=H + hd + window, poison=True,
                                                              scale_key=lambda L: L // 2)

@@ -552,9 +552,13 @@ template <int HD>
 static int attn_f32(const float* q, long long q_stride, float* out, long long out_stride, const float* kcache, const float* vcache,
                     const int* block_tables, int max_pages, const int* row_seq, const int* positions, int T, int G, int KV,
                     int page_size, int window, float scale, int singles, cudaStream_t stream) {
-    // A few rows of portions make too few blocks for the rows' kernel. 32 heads of 64 on 8: 24 / 100 / 200 / 400 rows without a context
-    // take 12 / 27 / 49 / 129 us here and 35 / 43 / 55 / 107 us there, 24 and 100 rows behind 1,000 keys 48 and 143 against 170 and 182.
-    if (T - singles <= 256) singles = T;
+    // A few rows of portions make too few blocks for the rows' kernel. us here / there for 64, 128, 256 rows of one request, without a
+    // context, behind 1,000 and behind 8,000 keys:
+    //   32 heads of 64 on 8     14 / 25, 27 / 33, 59 / 49    89 / 158, 174 / 166, 330 / 183     612 / 1,067, 1,203 / 1,077, 2,192 / 1,092
+    //   32 heads of 128 on 8    19 / 39, 39 / 51, 94 / 76    150 / 235, 299 / 248, 573 / 274    1,067 / 1,584, 1,944 / 1,591, 3,857 / 1,608
+    //   8 heads of 64 on 8      11 / 31, 21 / 39, 45 / 58    69 / 164, 133 / 174, 248 / 191     462 / 1,069, 925 / 1,078, 1,649 / 1,099
+    // The lines cross between 95 rows (heads of 128, long contexts) and 200 (no context); what context a step has is not known here.
+    if (T - singles <= 128) singles = T;
     if (singles > 0) {
         auto f = G == 1 ? attn_f32_single<1, HD> : G == 2 ? attn_f32_single<2, HD> : G <= 4 ? attn_f32_single<4, HD> : attn_f32_single<8, HD>;
         int e = f(q, q_stride, out, out_stride, kcache, vcache, block_tables, max_pages, row_seq, positions, singles, G, KV, page_size,
