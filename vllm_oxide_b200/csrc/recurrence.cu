@@ -952,8 +952,10 @@ delta_scan_kernel(const float* __restrict__ r, long ld_r, const float* __restric
 }
 
 // One column a thread where its warps find no second one on their scheduler anyway (at most 512 warps of one column on 592
-// schedulers, as one request of 16 heads of 128): the chain of a token is shorter. 16 heads of 128, one / two columns: one request of
-// 1,500 tokens 466 / 522 us, two of 500 tokens 219 / 196 us, four of 200 to 766 tokens 419 / 341 us.
+// schedulers, as one request of 16 heads of 128): the chain of a token is shorter. 400 tokens a request, one / two columns, us at 256,
+// 512, 1,024 and 2,048 warps: K = V = 64 107 / 126, 114 / 126, 145 / 129, 318 / 171; 128 117 / 138, 123 / 138, 164 / 142, 317 / 187; 256
+// - / -, 159 / 173, 305 / 181, 484 / 348; K = 32 and V = 64 93 / 101, 95 / 101, 111 / 103, 150 / 123. The same however the warps come
+// together (4 to 64 heads, one to eight requests).
 static bool delta_scan_one_column(int seqs, int H, int V, int ks) { return (long)seqs * H * V * ks <= 512L * 32; }
 
 // Whether the kernel above takes these operands: 16-byte pieces of r, k and w, pieces of v, pairs of columns.
