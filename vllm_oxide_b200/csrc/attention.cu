@@ -174,8 +174,9 @@ constexpr int KT = 32;            // keys of a tile
 
 // Portions of prompts. A block takes 64 / G rows (64 queries) of one kv head, and two tiles of keys at a time. Rows of several
 // requests may meet in a block: it goes through the requests one after another, the rows of the others sitting out.
-// Bound: FMA units and shared-memory reads, about half and half. 32 heads of 64 on 8, 700 / 2,048 rows: 175 / 837 us (general kernel
-// 1,009 / 7,738).
+// Bound: at 700 rows the walk of the longest block (352 blocks are one wave; while they run the FMA units are busy 39 % of the cycles
+// and waits for the result in front lead), with more rows the FMA units and shared-memory reads. 32 heads of 64 on 8, 700 / 2,048
+// rows: 175 / 837 us (general kernel 1,009 / 7,738).
 template <int HD>
 __global__ void __launch_bounds__(128)
 attn_f32_rows_kernel(const float* __restrict__ q, long long q_stride, float* __restrict__ out, long long out_stride,
@@ -378,7 +379,7 @@ attn_f32_rows_kernel(const float* __restrict__ q, long long q_stride, float* __r
 
 // Single tokens. A cluster of `c` blocks takes one row of one kv head, 8 c tiles at a time, a tile to a warp; the tiles' sums
 // are joined in order, each block a part of the (head, feature) pairs. Bound: the latency of a tile (its keys and values are
-// asked for at once), so the blocks are as many as the GPU holds. 32 heads of 64 on 8, one row with 100 / 700 / 4,000 keys: 16 / 19 /
+// asked for at once) and of the cluster's barriers around the joining, so the blocks are as many as the GPU holds. 32 heads of 64 on 8, one row with 100 / 700 / 4,000 keys: 16 / 19 /
 // 35 us (general kernel 66 / 392 / 2,205), 16 rows with 1,000 keys 37 us (571).
 template <int G, int HD>
 __global__ void __launch_bounds__(256, 2)
