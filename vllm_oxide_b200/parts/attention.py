@@ -56,7 +56,7 @@ def decode_balance_rule(num_seqs: int, kv_heads: int, head_dim: int, num_sms: in
     merge through global memory costs over the merge in a cluster. Measured with 8 kv heads of 64, in clusters / balanced, and
     how many tiles more: 8 requests of 100 to 2,000 keys 8.8 / 9.9 us (3), two of 4,000 and 200 keys 9.0 / 10.4 (5), 16 of 100 to 2,000
     13.2 / 10.9 (7), 16 of 100 to 4,000 22.0 / 14.4 (15), 64 of 17 to 1,000 19.6 / 18.3 (10); heads of 128, where a tile takes twice as
-    long: 8 of 100 to 2,000 13.3 / 12.5 (3), 16 of 17 to 1,000 12.5 / 11.0 (3), 16 of 100 to 4,000 38 / 22 (13)."""
+    long: 8 of 100 to 2,000 13.3 / 12.5 (3), 16 of 17 to 1,000 12.5 / 11.0 (3), 16 of 100 to 4,000 38 / 22 (11)."""
     # three blocks an SM with three stages at head size 64, two at 128
     want = min(64, num_sms * (3 if head_dim <= 64 else 2) // kv_heads)
     if want < 2 or num_seqs > kernels.DECODE_BALANCE_SEQS:

@@ -28,7 +28,7 @@ class Tuning:
     # ties at batch 4.
     long_context_keys: int = 5120
     # A decode step deals attention's blocks out by the requests' lengths where a block of the longest request would otherwise walk
-    # so many tiles of 64 keys of 64 features more than an even share (`parts.attention.decode_balance_rule`).
+    # so many tiles of 64 keys of 64 features more than a block does when they are dealt out (`parts.attention.decode_balance_rule`).
     balance_tiles: int = 6
     # In a block with a norm on both sides of its sub-layers the norm behind a sub-layer can do two more things on its way:
     # move on the state of the convolution that ran in front of the sub-layer, and file the block's result and hand on the
