@@ -393,9 +393,10 @@ VOB_EXPORT int vob_gemm_f32(const float* A, long long lda, const float* W, long 
     // 16 rows: what a lane's registers hold. Cold, 9 to 16 rows, us here / in tiles (32 rows at least): 2,048 x 512 16 / 23, 2,048 x 2,048
     // 19 / 21, 4,096 x 4,096 41 / 55, 16,384 x 2,048 68 / 94, 128,256 x 2,048 391 / 644; where K has more than 32 chunks a block of 16
     // rows has its SM to itself, and the tiles win: 2,048 x 8,192 66 / 57, 4,096 x 14,336 209 / 170. Up to 8 rows the tiles never do: there
-    // 29 / 57 and 83 / 169 at 8 rows, 25 / 57 and 70 / 170 at one.
+    // 29 / 57 and 83 / 169 at 8 rows, 25 / 57 and 70 / 170 at one. A single chunk is too short for what a block of 5 rows and more sets
+    // up (back to back, 16 rows: 64 x 64 7.3 / 2.9, 2,048 x 64 7.7 / 3.1, 128 x 128 7.5 / 4.7; 8 rows 4.4 / 2.9, 4.6 / 3.1, 4.5 / 4.7).
     int q = ((nc + 7) / 8 + 3) / 4 * 4, c = (nc + q - 1) / q;
-    if (vec && (M <= 8 || (M <= 16 && q == 4))) {
+    if (vec && (M <= (K <= 64 ? 4 : 8) || (M <= 16 && q == 4 && nc > 1))) {
         int e = M == 1   ? launch_few<1>(A, lda, W, ldw, C, ldc, M, N, K, bias, nc, q, c, early, stream)
                 : M == 2 ? launch_few<2>(A, lda, W, ldw, C, ldc, M, N, K, bias, nc, q, c, early, stream)
                 : M <= 4 ? launch_few<4>(A, lda, W, ldw, C, ldc, M, N, K, bias, nc, q, c, early, stream)
@@ -405,7 +406,9 @@ VOB_EXPORT int vob_gemm_f32(const float* A, long long lda, const float* W, long 
     }
     // Tiles of 128, 64 or 32 rows, a block or eight to a tile: the one whose waves of blocks cost least. A wave's cost is its
     // rows times its resident blocks; smaller tiles read more from shared memory per FMA (measured at 2,048 x 2,048 and
-    // 16,384 x 2,048: 1.15 and 1.5 times the time per row), a shared K is added up over the cluster.
+    // 16,384 x 2,048: 1.15 and 1.5 times the time per row), a shared K is added up over the cluster (dearer where operands come by 4
+    // bytes: 8,192 x 2,050 at 300 rows 579 us shared, 429 not). A grid that finds an SM of its own for every block beside the
+    // neighbouring kernel's costs half: 512 x 2,048 at 48 rows 13.7 us in 64 blocks of 64 rows, 21.6 in 128 of 32; 4,096 x 130 10.5 and 17.0.
     int best_tr = 8, best_c = 1;
     double best = 1e300;
     for (int tr = 2; tr <= 8; tr *= 2)
@@ -413,7 +416,8 @@ VOB_EXPORT int vob_gemm_f32(const float* A, long long lda, const float* W, long 
             if (c > 1 && nc < 8) continue;
             double slots = 148.0 * tile_blocks(tr), blocks = (double)((M + 16 * tr - 1) / (16 * tr)) * ((N + TN - 1) / TN) * c;
             double waves = (double)(long long)((blocks + slots - 1) / slots);
-            double cost = waves * tile_blocks(tr) * tr * (tr == 8 ? 1.0 : tr == 4 ? 1.15 : 1.5) / c * (c > 1 ? 1.1 : 1.0);
+            if (tr < 8 && blocks <= 74) waves = 0.5;
+            double cost = waves * tile_blocks(tr) * tr * (tr == 8 ? 1.0 : tr == 4 ? 1.15 : 1.5) / c * (c == 1 ? 1.0 : vec ? 1.1 : 1.4);
             if (cost < best) { best = cost; best_tr = tr; best_c = c; }
         }
     if (best_tr == 8) return launch_tile<8>(A, lda, W, ldw, C, ldc, M, N, K, bias, nc, best_c, vec, stream);
