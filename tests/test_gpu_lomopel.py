@@ -593,7 +593,7 @@ def test_command_line_generates_from_a_lomopel_folder(tmp_path):
 @pytest.mark.parametrize("K,V,H,G,dt", [(128, 128, 4, 2, torch.bfloat16), (64, 64, 2, 2, torch.float32), (32, 32, 3, 1, torch.bfloat16), (20, 8, 2, 1, torch.float32),
                                         (256, 40, 2, 2, torch.bfloat16), (100, 24, 2, 1, torch.float32), (512, 4, 1, 1, torch.bfloat16), (8, 2, 1, 1, torch.float32),
                                         (8, 4, 1, 1, torch.float32),
-                                        # two columns a thread (seven requests x H x V x lanes a column above 512 warps), for every number of lanes
+                                        # two columns a thread (seven requests x H x V x lanes a column above 512 warps), for 4, 8 and 16 lanes; K above 256: the general kernel
                                         (32, 64, 16, 8, torch.float32), (64, 64, 16, 8, torch.bfloat16), (20, 130, 14, 7, torch.bfloat16), (128, 64, 8, 4, torch.float32),
                                         (256, 64, 4, 2, torch.float32), (200, 48, 8, 4, torch.bfloat16), (512, 64, 2, 2, torch.bfloat16)])
 def test_gated_delta_scan_of_aligned_rows_gives_the_same_bits(K, V, H, G, dt):

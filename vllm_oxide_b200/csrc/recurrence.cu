@@ -958,6 +958,16 @@ delta_scan_kernel(const float* __restrict__ r, long ld_r, const float* __restric
 // together (4 to 64 heads, one to eight requests).
 static bool delta_scan_one_column(int seqs, int H, int V, int ks) { return (long)seqs * H * V * ks <= 512L * 32; }
 
+// Where the general kernel is faster, us there / here. Its 32 lanes a column, K above 256, always: 512 x 128, 4 heads, one token of 16
+// requests 44 / 83, 200 tokens 893 / 1,514 (a block of the kernel above sets up and zeroes 124 KB there). 16 lanes a column with fewer than
+// four rows a request and more than one column's warps: 256 x 256, 4 heads, 16 requests of 1, 2, 4 and 200 tokens 24 / 31, 29 / 33, 39 / 37,
+// 787 / 490. Channels up to 32 with few rows and few warps: 32 x 64, 8 heads, 4 and 16 requests of one token 2.26 / 2.38, 3.42 / 3.21.
+static bool delta_scan_pays(int seqs, long rows, int H, int V, int kpt, int ks) {
+    if (rows >= 4L * seqs) return true;
+    if (ks == 16) return delta_scan_one_column(seqs, H, V, ks);
+    return kpt > 8 || (long)seqs * H * V * ks > 384L * 32;
+}
+
 // Whether the kernel above takes these operands: 16-byte pieces of r, k and w, pieces of v, pairs of columns.
 template <int KS, int NC, typename TV>
 static bool delta_scan_takes(const void* r, long ld_r, const void* k, long ld_k, const void* v, long ld_v, const void* w, const void* state,
@@ -986,17 +996,19 @@ static int delta_scan(const void* r, long ld_r, const void* k, long ld_k, const 
 // K <= 32: 4 x 8; <= 64: 4 x 16; <= 128: 8 x 16; <= 256: 16 x 16; <= 512: 32 x 16.
 template <int MODE, typename TRK, typename TV>
 static int scan_launch(const void* r, long ld_r, const void* k, long ld_k, const void* v, long ld_v, const float* w, const float* b,
-                       const float* u, float* state, const int* seq_starts, const int* state_slots, float* o, int seqs, int H, int K,
+                       const float* u, float* state, const int* seq_starts, const int* state_slots, float* o, int seqs, int rows, int H, int K,
                        int V, int rk_div, const void* conv_x, long ld_cx, int conv_c, int conv_taps, float* conv_state, cudaStream_t stream) {
-#define VOB_SCAN(P, KS_)                                                                                                        \
-    if constexpr (MODE == 2) {                                                                                                  \
-        if (delta_scan_one_column(seqs, H, V, KS_) && delta_scan_takes<KS_, 1, TV>(r, ld_r, k, ld_k, v, ld_v, w, state, o, K, V)) \
-            return delta_scan<P, KS_, 1, TV>(r, ld_r, k, ld_k, v, ld_v, w, b, state, seq_starts, state_slots, o, seqs, H, K, V, rk_div, \
-                                             conv_x, ld_cx, conv_c, conv_taps, conv_state, stream);                             \
-        if (delta_scan_takes<KS_, 2, TV>(r, ld_r, k, ld_k, v, ld_v, w, state, o, K, V))                                         \
-            return delta_scan<P, KS_, 2, TV>(r, ld_r, k, ld_k, v, ld_v, w, b, state, seq_starts, state_slots, o, seqs, H, K, V, rk_div, \
-                                             conv_x, ld_cx, conv_c, conv_taps, conv_state, stream);                             \
-    }                                                                                                                           \
+#define VOB_SCAN(P, KS_)                                                                                                    \
+    if constexpr (MODE == 2 && KS_ <= 16) {                                                                                 \
+        if (delta_scan_pays(seqs, rows, H, V, P, KS_)) {                                                                    \
+            if (delta_scan_one_column(seqs, H, V, KS_) && delta_scan_takes<KS_, 1, TV>(r, ld_r, k, ld_k, v, ld_v, w, state, o, K, V)) \
+                return delta_scan<P, KS_, 1, TV>(r, ld_r, k, ld_k, v, ld_v, w, b, state, seq_starts, state_slots, o, seqs, H, K, V, \
+                                                 rk_div, conv_x, ld_cx, conv_c, conv_taps, conv_state, stream);             \
+            if (delta_scan_takes<KS_, 2, TV>(r, ld_r, k, ld_k, v, ld_v, w, state, o, K, V))                                 \
+                return delta_scan<P, KS_, 2, TV>(r, ld_r, k, ld_k, v, ld_v, w, b, state, seq_starts, state_slots, o, seqs, H, K, V, \
+                                                 rk_div, conv_x, ld_cx, conv_c, conv_taps, conv_state, stream);             \
+        }                                                                                                                   \
+    }                                                                                                                       \
     return vob_launch(recurrence_scan_kernel<MODE, P, KS_, TRK, TV>, dim3((V + 128 / KS_ - 1) / (128 / KS_), H, seqs), dim3(128), 0,  \
                       stream, (const TRK*)r, ld_r, (const TRK*)k, ld_k, (const TV*)v, ld_v, w, b, u, state, seq_starts, state_slots, o, \
                       H, K, V, rk_div, (const TV*)conv_x, ld_cx, conv_c, conv_taps, conv_state)
@@ -1010,7 +1022,7 @@ static int scan_launch(const void* r, long ld_r, const void* k, long ld_k, const
 
 VOB_EXPORT int vob_recurrence_scan(int mode, const void* r, long ld_r, const void* k, long ld_k, int rk_code, const void* v, long ld_v,
                                    int v_code, const float* w, const float* b, const float* u, float* state, const int* seq_starts,
-                                   const int* state_slots, float* o, int seqs, int H, int K, int V, int rk_div, const void* conv_x,
+                                   const int* state_slots, float* o, int seqs, int rows, int H, int K, int V, int rk_div, const void* conv_x,
                                    long ld_cx, int conv_c, int conv_taps, float* conv_state, cudaStream_t stream) {
     if (seqs <= 0) return 0;
     if (H <= 0 || K <= 0 || V <= 0 || H > 65535 || seqs > 65535) return VOB_ERR_BAD_ARG;
@@ -1023,7 +1035,7 @@ VOB_EXPORT int vob_recurrence_scan(int mode, const void* r, long ld_r, const voi
     // conv_x (mode 2, optional): columns of the activations' type (v's) whose last conv_taps - 1 rows per request are
     // left in conv_state [slots, conv_taps - 1, conv_c]
     if (conv_x && (mode != 2 || conv_c <= 0 || conv_taps < 2 || !conv_state)) return VOB_ERR_BAD_ARG;
-#define VOB_ARGS r, ld_r, k, ld_k, v, ld_v, w, b, u, state, seq_starts, state_slots, o, seqs, H, K, V, rk_div, conv_x, ld_cx, conv_c, conv_taps, conv_state, stream
+#define VOB_ARGS r, ld_r, k, ld_k, v, ld_v, w, b, u, state, seq_starts, state_slots, o, seqs, rows, H, K, V, rk_div, conv_x, ld_cx, conv_c, conv_taps, conv_state, stream
     if (mode == 0 && rk_code == VOB_F32 && v_code == VOB_F32) return scan_launch<0, float, float>(VOB_ARGS);
     if (mode == 0 && rk_code == VOB_BF16 && v_code == VOB_BF16) return scan_launch<0, __nv_bfloat16, __nv_bfloat16>(VOB_ARGS);
     if (mode == 1 && rk_code == VOB_F32 && v_code == VOB_F32) return scan_launch<1, float, float>(VOB_ARGS);

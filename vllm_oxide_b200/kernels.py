@@ -1100,10 +1100,10 @@ def recurrence_scan(mode: int, r: torch.Tensor, k: torch.Tensor, v: torch.Tensor
                 or conv_state.shape[1] < 1 or conv_x.shape != (T, conv_state.shape[2]) or conv_x.dtype != v.dtype):
             raise ShapeError(op, "conv_x [T, C] of v's type goes with mode 2 and a contiguous float32 conv_state [slots, taps - 1, C]")
         conv_c, conv_taps = conv_state.shape[2], conv_state.shape[1] + 1
-    f = _fn("recurrence", "vob_recurrence_scan", [_I, _P, _L, _P, _L, _I, _P, _L, _I, _P, _P, _P, _P, _P, _P, _P, _I, _I, _I, _I, _I,
+    f = _fn("recurrence", "vob_recurrence_scan", [_I, _P, _L, _P, _L, _I, _P, _L, _I, _P, _P, _P, _P, _P, _P, _P, _I, _I, _I, _I, _I, _I,
                                                   _P, _L, _I, _I, _P, _P])
     _check(f(mode, _ptr(r), r.stride(0), _ptr(k), k.stride(0), _code(r, op), _ptr(v), v.stride(0), _code(v, op), _ptr(w), _ptr(b), _ptr(u),
-             _ptr(state), _ptr(seq_starts), _ptr(state_slots), _ptr(out), num_seqs, heads, K, V, heads // rk_heads,
+             _ptr(state), _ptr(seq_starts), _ptr(state_slots), _ptr(out), num_seqs, T, heads, K, V, heads // rk_heads,
              _ptr(conv_x), conv_x.stride(0) if conv_x is not None else 0, conv_c, conv_taps,
              _ptr(conv_state) if conv_x is not None else _P(0), _stream()), op)
 
