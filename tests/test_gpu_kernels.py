@@ -283,7 +283,6 @@ def test_paged_attention_window_edge(dt, window):
 def test_f32_attention_of_portions_and_of_single_tokens_agree_to_the_bit(H, KV, hd, page, window):
     """The 32-bit engine's two kernels (single tokens over one to eight blocks, rows of portions) give a row the same bits, whatever
     shares its block; a padding row gives zeros; an infinity among a later token's values reaches no earlier row."""
-    # 349 rows: the rows' kernel takes what lies behind the single tokens while it is more than 128 rows
     seqs = [(0, 70), (131, 1), (30, 5), (0, 1), (31, 2), (63, 66), (700, 1), (255, 200)]
     qrows, kc, vc, bt, row_seq, pos, qs, ks, vs = _paged_case(torch.float32, H, KV, hd, page, seqs, seed=H + hd + window, poison=True,
                                                              scale_key=lambda L: L // 2)
@@ -294,15 +293,21 @@ def test_f32_attention_of_portions_and_of_single_tokens_agree_to_the_bit(H, KV, 
     qrows, row_seq, pos = torch.cat([qrows, qrows[:pad]]).to(DEV), torch.cat([row_seq, row_seq[:pad]]).to(DEV), torch.cat([pos, pos[:pad] * 0 - 1]).to(DEV)
     kc, vc, bt = kc.to(DEV), vc.to(DEV), bt.to(DEV)
 
-    def go(singles, rows=slice(0, T)):
+    def go(singles, rows=slice(0, T), portions=0):
         out = torch.full_like(qrows[rows], 7.0)
-        K().paged_attention(qrows[rows], out, kc, vc, bt, row_seq[rows].contiguous(), pos[rows].contiguous(), H, KV, hd, 1.0 / math.sqrt(hd), window, singles)
+        K().paged_attention(qrows[rows], out, kc, vc, bt, row_seq[rows].contiguous(), pos[rows].contiguous(), H, KV, hd, 1.0 / math.sqrt(hd), window, singles,
+                            portions)
         return out
-    full = go(0)
+    full = go(0, portions=-1)
     assert bool((full[-pad:] == 0).all())
     same = lambda a, b: torch.equal(torch.nan_to_num(a, 9e9), torch.nan_to_num(b, 9e9))  # noqa: E731
     for singles in (1, 2, 50, T - 1, T):
-        assert same(go(singles), full), singles
+        assert same(go(singles), full) and same(go(singles, portions=-1), full), singles
+    for portions in (0, 1, 8, 100):
+        assert same(go(0, portions=portions), full), portions
+    # several rows a block: row counts around its choices, with padding rows among them
+    for n in (75, 149, 296, 297, 340, T):
+        assert same(go(n, slice(T - n, T)), full[T - n:]), n
     for lo, n in ((0, 1), (3, 40), (69, 3), (13, 300), (T - 9, 9)):
         assert same(go(0, slice(lo, lo + n)), full[lo:lo + n]) and same(go(n, slice(lo, lo + n)), full[lo:lo + n]), (lo, n)
     r = 0
@@ -330,7 +335,8 @@ def test_f32_attention_keys_of_minus_infinite_score_weigh_nothing(hd, H, KV, win
     T = len(pos)
     for singles in (0, T):
         out = torch.full((T, H * hd), 7.0, device=DEV)
-        K().paged_attention(qrows.to(DEV), out, kc.to(DEV), vc.to(DEV), bt.to(DEV), row_seq.to(DEV), pos.to(DEV), H, KV, hd, 1.0 / math.sqrt(hd), window, singles)
+        K().paged_attention(qrows.to(DEV), out, kc.to(DEV), vc.to(DEV), bt.to(DEV), row_seq.to(DEV), pos.to(DEV), H, KV, hd, 1.0 / math.sqrt(hd), window, singles,
+                            -1)
         r = 0
         for s, (c, n) in enumerate(seqs):
             # (rows 0-31 have no other key: not asked)

@@ -192,16 +192,16 @@ attn_f32_rows_kernel(const float* __restrict__ q, long long q_stride, float* __r
     float2* ab = reinterpret_cast<float2*>(ps + 64 * 68);      // [2 tiles][64]: the factors of a tile's joining
     __shared__ float run_max[64];
     __shared__ int last[64], first[64];              // the keys a query sees in the current request: first .. last (-1: none)
+    __shared__ int slot[2][64];
     pdl_launch_dependents();
     pdl_wait(6);
     int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     int rows = 64 / G, kvh = blockIdx.y;
     int r0 = (gridDim.x - 1 - blockIdx.x) * rows;    // late rows have the most keys: they go first
     int rn = min(rows, T - r0), nq = rn * G;
-    for (int i = tid; i < 64 * HD; i += 128) {
-        int x = i / HD, d = i % HD;
-        qs[x * LD + d] = x < nq ? q[(size_t)(r0 + x / G) * q_stride + (size_t)(kvh * G + x % G) * HD + d] : 0.f;
-    }
+#pragma unroll 8
+    for (int x = tid / HD; x < 64; x += 128 / HD)
+        qs[x * LD + tid % HD] = x < nq ? q[(size_t)(r0 + x / G) * q_stride + (size_t)(kvh * G + x % G) * HD + tid % HD] : 0.f;
     if (tid < 64) run_max[tid] = -INFINITY;
     // first product: queries sq + 8 i, keys sk + 16 j (j / 2 = tile); second: queries 8 og + i, features 4 od .. (+ 64)
     int sq = warp * 2 + (lane >> 4), sk = lane & 15;
@@ -237,14 +237,20 @@ attn_f32_rows_kernel(const float* __restrict__ q, long long q_stride, float* __r
             lo_last = min(lo_last, last[x]); hi_first = max(hi_first, first[x]);
         }
         const int* bt = block_tables + (size_t)seq * max_pages;
+        // where the keys of two tiles lie (-1: no key of this request's), looked up one step ahead
+        auto find = [&](int k0) {
+            int j = k0 + tid;
+            if (tid < 64) slot[k0 >> 6 & 1][tid] = j >= lo && j <= hi ? (bt[j / page_size] * KV + kvh) * page_size + j % page_size : -1;
+        };
+        find(lo / 64 * 64);
+        __syncthreads();
         for (int k0 = lo / 64 * 64; k0 <= hi; k0 += 64) {
             for (int i = tid; i < 64 * (HD / 4); i += 128) {
-                int r = i / (HD / 4), d = i % (HD / 4) * 4, j = k0 + r;
-                bool in = j >= lo && j <= hi;
-                size_t row = in ? ((size_t)bt[j / page_size] * KV + kvh) * page_size + j % page_size : 0;
-                cp_async16(ks + r * LD + d, kcache + row * HD + d, in);
-                cp_async16(vs + r * HD + d, vcache + row * HD + d, in);
+                int r = i / (HD / 4), d = i % (HD / 4) * 4, at = slot[k0 >> 6 & 1][r];
+                cp_async16(ks + r * LD + d, kcache + (size_t)max(at, 0) * HD + d, at >= 0);
+                cp_async16(vs + r * HD + d, vcache + (size_t)max(at, 0) * HD + d, at >= 0);
             }
+            find(k0 + 64);
             asm volatile("cp.async.wait_all;" ::: "memory");
             __syncthreads();
             // every query of the block sees every key
@@ -378,45 +384,69 @@ attn_f32_rows_kernel(const float* __restrict__ q, long long q_stride, float* __r
 }
 
 // Single tokens. A cluster of `c` blocks takes one row of one kv head, 8 c tiles at a time, a tile to a warp; the tiles' sums
-// are joined in order, each block a part of the (head, feature) pairs. Bound: the latency of a tile (its keys and values are
-// asked for at once) and of the cluster's barriers around the joining, so the blocks are as many as the GPU holds. 32 heads of 64 on 8, one row with 100 / 700 / 4,000 keys: 16 / 19 /
-// 35 us (general kernel 66 / 392 / 2,205), 16 rows with 1,000 keys 37 us (571).
+// are joined in order, each block a part of the (head, feature) pairs. With more rows than blocks fit at once a block takes
+// `rows` of them (c = 1), whose tiles its warps take one after another. Bound: the latency of a tile (its keys and values are
+// asked for at once) and of the barriers around the joining, so the blocks are as many as the GPU holds.
 template <int G, int HD>
 __global__ void __launch_bounds__(256, 2)
 attn_f32_single_kernel(const float* __restrict__ q, long long q_stride, float* __restrict__ out, long long out_stride,
                        const float* __restrict__ kcache, const float* __restrict__ vcache, const int* __restrict__ block_tables,
-                       int max_pages, const int* __restrict__ row_seq, const int* __restrict__ positions, int heads, int KV,
-                       int page_size, int window, float scale, int c) {
+                       int max_pages, const int* __restrict__ row_seq, const int* __restrict__ positions, int T, int heads, int KV,
+                       int page_size, int window, float scale, int rows, int c) {
     constexpr int DL = HD / 32;                      // features of a lane
     constexpr int PER = HD + 4;                      // floats of a tile's sums for a head: o, m, l
-    __shared__ __align__(16) float qs[G * HD];
-    __shared__ __align__(16) float ps[8][G][KT];
-    __shared__ __align__(16) float part[8][G][PER];
+    extern __shared__ __align__(16) float smem[];
+    float (*ps)[G][KT] = reinterpret_cast<float (*)[G][KT]>(smem);                              // [8]
+    float (*part)[G][PER] = reinterpret_cast<float (*)[G][PER]>(smem + 8 * G * KT);             // [8]
+    float* qs = smem + 8 * G * (KT + PER);           // [rows][G * HD]
+    // the block's rows; tiles first_of[r] .. first_of[r + 1] - 1 of the block are row r's
+    __shared__ int pos_of[8], key_of[8], tile_of[8], seq_of[8], first_of[9];
     pdl_launch_dependents();
     pdl_wait(6);
     int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    int rank = blockIdx.x % c, row = blockIdx.x / c, kvh = blockIdx.y;
-    int pos = positions[row];
-    if (pos < 0) {                                   // a padding row: no keys, zero output (the whole cluster leaves)
-        for (int i = tid; i < heads * HD && rank == 0; i += 256) out[(size_t)row * out_stride + (size_t)kvh * heads * HD + i] = 0.f;
-        return;
+    int rank = blockIdx.x % c, row0 = blockIdx.x / c, apart = gridDim.x / c, kvh = blockIdx.y;
+    if (warp == 0) {
+        int row = row0 + lane * apart, pos = lane < rows && row < T ? positions[row] : -1;
+        int first = window > 0 ? max(0, pos + 1 - window) : 0, upto = pos < 0 ? 0 : pos / KT + 1 - first / KT;
+        if (lane < 8) { pos_of[lane] = pos; key_of[lane] = first; tile_of[lane] = first / KT; seq_of[lane] = pos < 0 ? 0 : row_seq[row]; }
+#pragma unroll
+        for (int o = 1; o < 8; o <<= 1) {
+            int v = __shfl_up_sync(0xffffffffu, upto, o);
+            if (lane >= o) upto += v;
+        }
+        if (lane < 8) first_of[lane + 1] = upto;
+        if (lane == 0) first_of[0] = 0;
     }
-    for (int i = tid; i < G * HD; i += 256) qs[i] = i < heads * HD ? q[(size_t)row * q_stride + (size_t)kvh * heads * HD + i] : 0.f;
+    for (int i = tid; i < rows * G * HD; i += 256) {
+        int row = row0 + i / (G * HD) * apart, e = i % (G * HD);
+        qs[i] = row < T && e < heads * HD ? q[(size_t)row * q_stride + (size_t)kvh * heads * HD + e] : 0.f;
+    }
     __syncthreads();
-    const int* bt = block_tables + (size_t)row_seq[row] * max_pages;
-    int first = window > 0 ? max(0, pos + 1 - window) : 0;
-    int t0 = first / KT, t1 = pos / KT + 1;
+    const int tiles = first_of[rows];
+    auto out_of = [&](int r) { return out + (size_t)(row0 + r * apart) * out_stride + (size_t)kvh * heads * HD; };
+    for (int r = 0; r < rows && rank == 0; ++r)      // a padding row: no keys, zero output
+        if (pos_of[r] < 0 && row0 + r * apart < T)
+            for (int i = tid; i < heads * HD; i += 256) out_of(r)[i] = 0.f;
+    if (c > 1 && tiles <= 8) {                       // a block's worth of tiles: the others leave (and no block of the cluster waits)
+        if (rank) return;
+        c = 1;
+    }
     // this block's (head, feature) pairs of the joining: at most four a thread
     constexpr int MOST = (G * HD + 255) / 256;
     int total = heads * HD, share = (total + c - 1) / c;
     float acc[MOST], l[MOST], m[MOST];
 #pragma unroll
     for (int i = 0; i < MOST; ++i) { acc[i] = 0.f; l[i] = 0.f; m[i] = -INFINITY; }
-    for (int tr = t0; tr < t1; tr += 8 * c) {
-        int t = tr + rank * 8 + warp;
-        if (t < t1) {
-            int j = t * KT + lane;
-            bool valid = j >= first && j <= pos;
+    for (int tr = 0; tr < tiles; tr += 8 * c) {
+        int p = tr + rank * 8 + warp;
+        if (p < tiles) {
+            int r = 0;
+            while (p >= first_of[r + 1]) ++r;
+            int k0 = (tile_of[r] + p - first_of[r]) * KT, k_lo = max(key_of[r] - k0, 0), k_hi = min(pos_of[r] - k0, KT - 1);    // the tile's keys
+            const int* bt = block_tables + (size_t)seq_of[r] * max_pages;
+            const float* qr = qs + r * G * HD;
+            int j = k0 + lane;
+            bool valid = lane >= k_lo && lane <= k_hi;
             int slot = valid ? (bt[j / page_size] * KV + kvh) * page_size + j % page_size : 0;
             float s[G];
             {
@@ -424,12 +454,12 @@ attn_f32_single_kernel(const float* __restrict__ q, long long q_stride, float* _
 #pragma unroll
                 for (int g = 0; g < G; ++g) s2[g] = 0;
                 const ulonglong2* kp = reinterpret_cast<const ulonglong2*>(kcache + (size_t)slot * HD);
-#pragma unroll 8
+#pragma unroll(G == 8 ? 4 : 8)
                 for (int d = 0; d < HD / 4; ++d) {
                     ulonglong2 kf = valid ? kp[d] : make_ulonglong2(0, 0);
 #pragma unroll
                     for (int g = 0; g < G; ++g) {
-                        ulonglong2 qf = *reinterpret_cast<const ulonglong2*>(qs + g * HD + d * 4);
+                        ulonglong2 qf = *reinterpret_cast<const ulonglong2*>(qr + g * HD + d * 4);
                         fma2(s2[g], qf.x, kf.x); fma2(s2[g], qf.y, kf.y);
                     }
                 }
@@ -451,9 +481,8 @@ attn_f32_single_kernel(const float* __restrict__ q, long long q_stride, float* _
 #pragma unroll
                 for (int d = 0; d < DL / 2; ++d) o[g][d] = 0;
             }
-            int k_lo = max(first - t * KT, 0), k_hi = min(pos - t * KT, KT - 1);
 #pragma unroll 1
-            for (int kb = 0; kb < KT; kb += 8) {     // eight values' rows on their way at once
+            for (int kb = k_lo & ~7; kb <= k_hi; kb += 8) {     // eight values' rows on their way at once
                 unsigned long long vf[8][DL / 2];
 #pragma unroll
                 for (int k = 0; k < 8; ++k) {
@@ -488,7 +517,27 @@ attn_f32_single_kernel(const float* __restrict__ q, long long q_stride, float* _
         else __syncthreads();
         for (int b = 0; b < c; ++b) {
             const float* pb = c > 1 ? cg::this_cluster().map_shared_rank(&part[0][0][0], b) : &part[0][0][0];
-            int n = min(8, t1 - tr - b * 8);
+            int n = min(8, tiles - tr - b * 8);
+            if (rows > 1) {                          // tiles of several rows: a row begins, goes on or ends with each
+                for (int w = 0; w < n; ++w) {
+                    int p = tr + w, r = 0;
+                    while (p >= first_of[r + 1]) ++r;
+                    bool begins = p == first_of[r], ends = p + 1 == first_of[r + 1];
+#pragma unroll
+                    for (int i = 0; i < MOST; ++i) {
+                        int e = tid + i * 256;
+                        if (e >= total) continue;
+                        if (begins) { acc[i] = 0.f; l[i] = 0.f; m[i] = -INFINITY; }
+                        const float* pw = pb + (w * G + e / HD) * PER;
+                        float mt = pw[HD], to = fmaxf(m[i], mt), fa = expf(m[i] - to), fb = expf(mt - to);
+                        l[i] = fmaf(l[i], fa, __fmul_rn(pw[HD + 1], fb));
+                        acc[i] = fmaf(acc[i], fa, __fmul_rn(pw[e % HD], fb));
+                        m[i] = to;
+                        if (ends) out_of(r)[e] = __fmul_rn(acc[i], 1.0f / l[i]);
+                    }
+                }
+                continue;
+            }
 #pragma unroll
             for (int i = 0; i < MOST; ++i) {
                 int e = rank * share + tid + i * 256;
@@ -507,10 +556,11 @@ attn_f32_single_kernel(const float* __restrict__ q, long long q_stride, float* _
         if (c > 1) cg::this_cluster().sync();        // the sums have been read
         else __syncthreads();
     }
+    if (rows > 1 || tiles == 0) return;
 #pragma unroll
     for (int i = 0; i < MOST; ++i) {
         int e = rank * share + tid + i * 256;
-        if (e < min(total, (rank + 1) * share)) out[(size_t)row * out_stride + (size_t)kvh * heads * HD + e] = __fmul_rn(acc[i], 1.0f / l[i]);
+        if (e < min(total, (rank + 1) * share)) out_of(0)[e] = __fmul_rn(acc[i], 1.0f / l[i]);
     }
 }
 
@@ -533,9 +583,21 @@ static int attn_f32_single(const float* q, long long q_stride, float* out, long 
     // a cluster as wide as the GPU has room for with two blocks an SM
     int c = 8;
     while (c > 1 && (long long)T * KV * c > 296) c /= 2;
+    // Rows that do not fit at once share blocks: the number whose waves of blocks cost least, a block's start counted as one row. Rows
+    // of a block are far apart, so that neighbours with long contexts meet in none.
+    int rows = 1;
+    long long best = 1LL << 60;
+    for (int r = 1; r <= 8 && (long long)T * KV > 296; ++r) {
+        long long cost = ((long long)((T + r - 1) / r) * KV + 295) / 296 * (r + 1);
+        if (cost <= best) { best = cost; rows = r; }
+    }
+    const size_t smem = sizeof(float) * (size_t)(8 * G * (KT + HD + 4) + rows * G * HD);
+    cudaError_t e = cudaFuncSetAttribute(attn_f32_single_kernel<G, HD>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (e != cudaSuccess) return (int)e;
     cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3((unsigned)(T * c), (unsigned)KV);
+    cfg.gridDim = dim3((unsigned)((T + rows - 1) / rows * c), (unsigned)KV);
     cfg.blockDim = dim3(256);
+    cfg.dynamicSmemBytes = smem;
     cfg.stream = stream;
     cudaLaunchAttribute attr[2];
     attr[0].id = cudaLaunchAttributeClusterDimension;
@@ -544,22 +606,23 @@ static int attn_f32_single(const float* q, long long q_stride, float* out, long 
     attr[1].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attr;
     cfg.numAttrs = g_vob_pdl ? 2 : 1;
-    cudaError_t e = cudaLaunchKernelEx(&cfg, attn_f32_single_kernel<G, HD>, q, q_stride, out, out_stride, kcache, vcache, block_tables, max_pages,
-                                       row_seq, positions, heads, KV, page_size, window, scale, c);
+    e = cudaLaunchKernelEx(&cfg, attn_f32_single_kernel<G, HD>, q, q_stride, out, out_stride, kcache, vcache, block_tables, max_pages, row_seq,
+                           positions, T, heads, KV, page_size, window, scale, rows, c);
     return e != cudaSuccess ? (int)e : vob_launch_status();
 }
 
 template <int HD>
 static int attn_f32(const float* q, long long q_stride, float* out, long long out_stride, const float* kcache, const float* vcache,
                     const int* block_tables, int max_pages, const int* row_seq, const int* positions, int T, int G, int KV,
-                    int page_size, int window, float scale, int singles, cudaStream_t stream) {
-    // A few rows of portions make too few blocks for the rows' kernel. us here / there for 64, 128, 256 rows of one request, without a
-    // context, behind 1,000 and behind 8,000 keys:
-    //   32 heads of 64 on 8     14 / 25, 27 / 33, 59 / 49    89 / 158, 174 / 166, 330 / 183     612 / 1,067, 1,203 / 1,077, 2,192 / 1,092
-    //   32 heads of 128 on 8    19 / 39, 39 / 51, 94 / 76    150 / 235, 299 / 248, 573 / 274    1,067 / 1,584, 1,944 / 1,591, 3,857 / 1,608
-    //   8 heads of 64 on 8      11 / 31, 21 / 39, 45 / 58    69 / 164, 133 / 174, 248 / 191     462 / 1,069, 925 / 1,078, 1,649 / 1,099
-    // The lines cross between 95 rows (heads of 128, long contexts) and 200 (no context); what context a step has is not known here.
-    if (T - singles <= 128) singles = T;
+                    int page_size, int window, float scale, int singles, int portions, cudaStream_t stream) {
+    // Few rows make too few blocks for the rows' kernel, and a block of it goes through its requests one after another. What a row costs
+    // here grows with the kv heads and, half as fast, with their group; there a step's time hardly depends on either while the blocks
+    // fit at once. us here / there, no context and behind 500 to 1,500 keys: 32 heads of 64 on 8, 128 rows of one request 27 / 33 and
+    // 174 / 166 (1,000 keys), three requests of 128 rows 58 / 45 and 836 / 334, six of 64 39 / 32 and 821 / 307, ten of 32 19 / 31 and 671 / 317,
+    // 64 of 4 9 / 76 and 172 / 440; 4 heads of 64 on 2, one of 300 27 / 53, two of 300 134 / 201 (500 keys); 8 of 64 on one 30 / 50, 130 / 190;
+    // 8 heads of 128 on 8, one of 300 106 / 90, two 706 / 328. Short prompts are the usual case of many portions.
+    const int rest = T - singles;
+    if (portions >= 0 && ((long long)rest * KV * (4 + G) <= 10800 || rest < portions * 64LL)) singles = T;
     if (singles > 0) {
         auto f = G == 1 ? attn_f32_single<1, HD> : G == 2 ? attn_f32_single<2, HD> : G <= 4 ? attn_f32_single<4, HD> : attn_f32_single<8, HD>;
         int e = f(q, q_stride, out, out_stride, kcache, vcache, block_tables, max_pages, row_seq, positions, singles, G, KV, page_size,
@@ -570,24 +633,25 @@ static int attn_f32(const float* q, long long q_stride, float* out, long long ou
                              row_seq + singles, positions + singles, T - singles, G, KV, page_size, window, scale, stream);
 }
 
-// `singles`: so many of the leading rows are single tokens of requests of their own (which kernel computes a row of the 32-bit
-// engine changes its speed, not its bits).
+// `singles`: so many of the leading rows are single tokens of requests of their own; `portions`: so many requests bring the rows behind
+// them (0: not known; -1: they all go to the portions' kernel). Which kernel computes a row of the 32-bit engine changes its speed,
+// not its bits.
 VOB_EXPORT int vob_paged_attention(const void* q, long long q_stride, void* out, long long out_stride,
                                    const void* kcache, const void* vcache, int code,
                                    const int* block_tables, int max_pages, const int* row_seq,
                                    const int* positions, int T_rows, int H, int KV, int hd, int page_size,
-                                   int window, float scale, int singles, cudaStream_t stream) {
+                                   int window, float scale, int singles, int portions, cudaStream_t stream) {
     if (T_rows <= 0) return 0;
     if (H <= 0 || KV <= 0 || H % KV != 0 || page_size <= 0 || max_pages <= 0) return VOB_ERR_BAD_ARG;
     if (hd <= 0 || hd % 8 != 0 || hd > 256) return VOB_ERR_UNSUPPORTED;
-    if (singles < 0 || singles > T_rows) return VOB_ERR_BAD_ARG;
+    if (singles < 0 || singles > T_rows || portions < -1) return VOB_ERR_BAD_ARG;
     int G = H / KV;
     // wider groups would not leave a lane of the single-token kernel its registers; KV and T bound the grids
     if (code == VOB_F32 && (hd == 64 || hd == 128) && G <= 8 && KV <= 65535 && T_rows <= (1 << 27) &&
         (((uintptr_t)kcache | (uintptr_t)vcache) & 15) == 0) {
         auto f = hd == 64 ? attn_f32<64> : attn_f32<128>;
         return f((const float*)q, q_stride, (float*)out, out_stride, (const float*)kcache, (const float*)vcache, block_tables, max_pages, row_seq,
-                 positions, T_rows, G, KV, page_size, window, scale, singles, stream);
+                 positions, T_rows, G, KV, page_size, window, scale, singles, portions, stream);
     }
     long long warps = (long long)T_rows * H;
     long long blocks = (warps + 3) / 4;

@@ -1889,10 +1889,11 @@ def flex_attention(q: torch.Tensor, out: torch.Tensor, kcache: torch.Tensor, vca
 def paged_attention(q: torch.Tensor, out: torch.Tensor, kcache: torch.Tensor, vcache: torch.Tensor,
                     block_tables: torch.Tensor, row_seq: torch.Tensor, positions: torch.Tensor,
                     num_heads: int, num_kv_heads: int, head_dim: int, scale: float, window: int = 0,
-                    singles: int = 0) -> None:
+                    singles: int = 0, portions: int = 0) -> None:
     """Causal GQA attention of every row of q [T, H*hd] over its request's pages.
     block_tables int32 [S, max_pages]; row_seq, positions int32 [T]; window 0 = all keys. `singles`: so many leading rows
-    are single tokens, each of a request of its own (changes speed, never results)."""
+    are single tokens, each of a request of its own; `portions`: so many requests bring the rows behind them, 0 if that is not
+    known, -1 to send them all to the 32-bit engine's kernel for portions (tests). Both change speed, never results."""
     op = "paged_attention"
     _cuda(op, q, out, kcache, vcache, block_tables, row_seq, positions)
     _rows_2d(q, op, "q")
@@ -1918,10 +1919,10 @@ def paged_attention(q: torch.Tensor, out: torch.Tensor, kcache: torch.Tensor, vc
     _int32_vec(row_seq, T, op, "row_seq")
     _int32_vec(positions, T, op, "positions")
     f = _fn("attention", "vob_paged_attention",
-            [_P, _L, _P, _L, _P, _P, _I, _P, _I, _P, _P, _I, _I, _I, _I, _I, _I, _F, _I, _P])
+            [_P, _L, _P, _L, _P, _P, _I, _P, _I, _P, _P, _I, _I, _I, _I, _I, _I, _F, _I, _I, _P])
     _check(f(_ptr(q), q.stride(0), _ptr(out), out.stride(0), _ptr(kcache), _ptr(vcache), _code(q, op),
              _ptr(block_tables), block_tables.shape[1], _ptr(row_seq), _ptr(positions), T, num_heads,
-             num_kv_heads, head_dim, kcache.shape[2], int(window), float(scale), int(singles), _stream()), op)
+             num_kv_heads, head_dim, kcache.shape[2], int(window), float(scale), int(singles), int(portions), _stream()), op)
 
 
 def attn_mma_supported(num_heads: int, num_kv_heads: int, head_dim: int, page_size: int, decode: bool) -> bool:

@@ -225,7 +225,7 @@ class Attention(Mixer):
                 return
         singles = ctx.rows if ctx.decode_only else ctx.lead_single
         kernels.paged_attention(q, out, cache.k, cache.v, bt, ctx.row_seq, ctx.positions, self.H, self.KV, self.hd,
-                                self.scale, self.window, singles)
+                                self.scale, self.window, singles, max(0, ctx.seqs - singles))
 
     def _attend_single(self, q, out, ctx: StepContext, cache: LayerCache, bt, count: int) -> None:
         """The decode kernel on the first `count` rows, row i belonging to request i."""
