@@ -210,7 +210,7 @@ gemm_sm100_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_consta
     const uint32_t tmem_base = MS ? 0u : *tmem_holder;
 
     if (warp == 0) {
-        if (lane == 0) {
+        if (elect_one()) {
             // Weights are written by no kernel (unless the caller says so), so their loads start at once and overlap whatever
             // still runs before this kernel; the activations are loaded only after the wait.
             if (qa.late_w) pdl_wait();
@@ -245,13 +245,13 @@ gemm_sm100_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_consta
             }
         }
     } else if (!MS && (warp == 1 || warp >= 6)) {
-        // ISSUERS issuing threads. One thread gets a tcgen05.mma through about every 125 clocks
-        // whatever its size, and an instruction of 128 x 16 x 16 consumes only 4 KB of weights: a
+        // ISSUERS issuing threads. One thread gets a small tcgen05.mma through about every 42 clocks
+        // (and a commit more per stage), and an instruction of 128 x 16 x 16 consumes only 4 KB of weights: a
         // single issuer just about keeps pace with HBM, and its chain is what a block with few
         // k-blocks waits for. Each thread takes its share of every stage's K steps into an
         // accumulator of its own; the epilogue adds them in a fixed order. (Measured on a decode
         // step of 8 rows: two issuers +2.5 %, four +2.7 %.)
-        if (lane == 0) {
+        if (elect_one()) {
             constexpr uint32_t idesc = umma_idesc(BT);
             constexpr int KSTEPS = BK / UMMA_K / ISSUERS;
             const int w = warp >= 6 ? warp - 5 : 0;
@@ -702,7 +702,7 @@ gemm_sm100_persistent_kernel(const __grid_constant__ CUtensorMap map_w, const __
     pdl_wait(13);
 
     if (warp == 0) {
-        if (lane == 0) {
+        if (elect_one()) {
             uint32_t it = 0;
             bool ok = true;
             for (int tile = blockIdx.x; tile < num_tiles && ok; tile += gridDim.x) {
@@ -719,7 +719,7 @@ gemm_sm100_persistent_kernel(const __grid_constant__ CUtensorMap map_w, const __
             }
         }
     } else if (warp == 1) {
-        if (lane == 0) {
+        if (elect_one()) {
             constexpr uint32_t idesc = umma_idesc(BT);
             uint32_t it = 0, local = 0;
             bool ok = true;

@@ -6,9 +6,8 @@
 // holding its 128 weight rows (the A operand) and its 128 of the 256 tokens (half of the B
 // operand) in its own shared memory, and each block's tensor memory receives its 128 weight rows
 // of the result for all 256 tokens. Per byte of operand fetched from shared memory an SM does
-// twice the work of a one-SM instruction, and one issued instruction (an issuing thread gets one
-// through in about 125-170 clocks whatever its size) is worth 256 clocks of tensor-core time on
-// each SM: that is what lifts this kernel over the one-SM persistent product.
+// twice the work of a one-SM instruction, and one issued instruction is worth 128 clocks of tensor-core
+// time on both SMs: that is what lifts this kernel over the one-SM persistent product.
 //
 // Roles in each block of 320 threads: warp 0 (one lane) issues its block's TMA loads, whose bytes
 // are counted on the leader block's barrier (cp.async.bulk.tensor with .cta_group::2; no
@@ -123,7 +122,7 @@ gemm_sm100_pair_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_c
     pdl_wait(15);
 
     if (warp == 0) {
-        if (lane == 0) {
+        if (elect_one()) {
             uint32_t it = 0;
             bool ok = true;
             for (int tile = pair; tile < num_tiles && ok; tile += num_pairs) {
@@ -146,7 +145,7 @@ gemm_sm100_pair_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_c
             }
         }
     } else if (warp == 1) {
-        if (lane == 0 && rank == 0) {
+        if (rank == 0 && elect_one()) {
             constexpr uint32_t idesc = umma_idesc_bf16(2 * BMH, 2 * BTH, false);
             uint32_t it = 0, local = 0;
             bool ok = true;
