@@ -998,6 +998,26 @@ def test_gemm_pair_swiglu(T, I, Kd):
     assert torch.equal(out, out2)
 
 
+@pytest.mark.parametrize("T,I,Kd,early", [(33, 8192, 64, True), (64, 128, 832, True), (100, 64, 704, False), (300, 8192, 72, True), (517, 4224, 128, False),
+                                          (600, 8192, 64, True), (1201, 640, 200, True)])
+def test_gemm_pair_swiglu_token_tiles(T, I, Kd, early):
+    """Token tiles of every width the launcher picks (32 to 256), more K blocks than a ring of ten stages holds, several tiles a
+    pair of SMs; weights asked for before the kernels in front are done or behind them: the same bits."""
+    g = torch.Generator().manual_seed(T * 3 + I)
+    a = torch.randn(T, Kd, generator=g).to(torch.bfloat16).to(DEV)
+    w = (torch.randn(2 * I, Kd, generator=g) / math.sqrt(Kd) * 2).to(torch.bfloat16).to(DEV)
+    out, other = (torch.full((T, I), 7.0, dtype=torch.bfloat16, device=DEV) for _ in range(2))
+    k = K()
+    torch.cuda.synchronize()
+    k.gemm_pair_swiglu(a, w, out, fixed_w=early)
+    k.gemm_pair_swiglu(a, w, other, fixed_w=not early)
+    torch.cuda.synchronize()
+    k.gemm_sm100_check()
+    want = plain.swiglu(plain.linear(a.double(), w[:I].double()), plain.linear(a.double(), w[I:].double()))
+    assert rel(out, want.cpu()) <= 2 ** -8                       # one rounding to bfloat16, as above
+    assert torch.equal(out, other)
+
+
 def test_a_wait_that_runs_out_raises_the_error_word_and_harms_nothing():
     """The give-up path of the tensor-core kernels: a one-block launch of the few-token product is
     told to expect 16 bytes more than its loads bring, with the wait limit lowered to 10 ms. The

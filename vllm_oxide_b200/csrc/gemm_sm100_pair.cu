@@ -15,27 +15,30 @@
 // commits them to both blocks' barriers (tcgen05.commit ... multicast::cluster); warps 2-9, two
 // groups of four taking alternate rounds of 16 tokens, read their block's accumulator and write C
 // (through shared memory, so that C is written in 16-byte pieces). The kernel is persistent: a pair walks over output tiles
-// (256 weight rows x 256 tokens), the accumulator is double buffered (2 x 256 columns), the TMA
-// ring runs ahead across tile boundaries.
+// (256 weight rows x 256 tokens, or fewer tokens where that makes fewer or cheaper waves: pick_tokens), the accumulator is double
+// buffered (2 x 256 columns), the TMA ring runs ahead across tile boundaries. `early`: no kernel writes W, and a block asks for its
+// first ring of weights before it waits for the kernels in front.
 //
 // Every mbarrier wait is bounded (sm100.cuh); a block that gives up still meets its partner at the
 // cluster barriers at the start and the end, so neither is left waiting.
 #include "common.cuh"
 VOB_PDL_SWITCH(gemm_sm100_pair)
 #include "sm100.cuh"
+#include <algorithm>
+#include <cmath>
 #include <unordered_map>
 
 namespace {
 using namespace vob_sm100;
 
 constexpr int BMH = 128;          // weight rows per block (256 per pair)
-constexpr int BTH = 128;          // tokens per block (256 per pair)
+constexpr int BN_MAX = 256;       // tokens of an instruction at most (half of them in each block), in steps of 32
 constexpr int BK = 64;            // K elements per stage: 128 bytes, one swizzle span
 constexpr int UMMA_K = 16;
 constexpr int NTHREADS = 320;          // TMA warp, MMA warp, two epilogue groups of four warps
 constexpr int EPI_GROUP_BYTES = 12288;  // per epilogue group: exchange and staging buffers
-constexpr int STAGES = 6;
-constexpr int STAGE_BYTES = (BMH + BTH) * BK * 2;            // 32 KB per block and stage
+constexpr int STAGES_MAX = 10;
+constexpr int RING_BYTES = 6 * 32768;    // per block: six stages of 256 tokens, more of fewer
 constexpr uint32_t PEER_MASK = 0xFEFFFFFFu;                  // a shared::cluster address with this mask is the pair's even block's
 
 template <typename OutT> __device__ __forceinline__ void store_out(OutT* p, float v);
@@ -82,14 +85,18 @@ enum { PAIR_STORE = 0, PAIR_SWIGLU = 1 };
 template <typename OutT, int EPI, int ACT>
 __global__ void __launch_bounds__(NTHREADS, 1)
 gemm_sm100_pair_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUtensorMap map_x,
-                       OutT* __restrict__ C, long long ldc, int T, int N, int K, int wide, int* __restrict__ err_flag) {
+                       OutT* __restrict__ C, long long ldc, int T, int N, int K, int wide, int* __restrict__ err_flag, int bn, int early) {
     constexpr int FEATS = EPI == PAIR_SWIGLU ? BMH / 2 : BMH;        // output features per block and tile
+    constexpr int A_BYTES = BMH * BK * 2;
+    const int half = bn >> 1;                                        // a block's tokens of a tile
+    const int stage_bytes = A_BYTES + half * (BK * 2);
+    const int stages = min(STAGES_MAX, RING_BYTES / stage_bytes);
     pdl_launch_dependents();
     extern __shared__ unsigned char smem_raw[];
     unsigned char* tiles = reinterpret_cast<unsigned char*>(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
-    uint64_t* full_bar = reinterpret_cast<uint64_t*>(tiles + STAGES * STAGE_BYTES);      // [STAGES] used in the even block
-    uint64_t* empty_bar = full_bar + STAGES;                                             // [STAGES] in both blocks
-    uint64_t* acc_full = empty_bar + STAGES;                                             // [2] in both blocks
+    uint64_t* full_bar = reinterpret_cast<uint64_t*>(tiles + RING_BYTES);                // [STAGES_MAX] used in the even block
+    uint64_t* empty_bar = full_bar + STAGES_MAX;                                         // [STAGES_MAX] in both blocks
+    uint64_t* acc_full = empty_bar + STAGES_MAX;                                             // [2] in both blocks
     uint64_t* acc_empty = acc_full + 2;                                                  // [2] used in the even block
     uint32_t* tmem_holder = reinterpret_cast<uint32_t*>(acc_empty + 2);
     volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_holder + 1);
@@ -100,12 +107,12 @@ gemm_sm100_pair_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_c
     const uint32_t rank = cluster_ctarank();              // 0: the even block (issues the products), 1: its partner
     const int pair = blockIdx.x >> 1, num_pairs = gridDim.x >> 1;
     const int total_kb = (K + BK - 1) / BK;
-    const int m_tiles = (N + 2 * FEATS - 1) / (2 * FEATS), n_tiles = (T + 2 * BTH - 1) / (2 * BTH);
+    const int m_tiles = (N + 2 * FEATS - 1) / (2 * FEATS), n_tiles = (T + bn - 1) / bn;
     const int num_tiles = m_tiles * n_tiles;
-    constexpr int ACC_COLS = 512;                         // two accumulators of 256 token columns
+    constexpr int ACC_COLS = 512;                         // two accumulators of up to 256 token columns
 
     if (threadIdx.x == 0) {
-        for (int s = 0; s < STAGES; ++s) { mbar_init(full_bar + s, 1); mbar_init(empty_bar + s, 1); }
+        for (int s = 0; s < STAGES_MAX; ++s) { mbar_init(full_bar + s, 1); mbar_init(empty_bar + s, 1); }
         for (int b = 0; b < 2; ++b) { mbar_init(acc_full + b, 1); mbar_init(acc_empty + b, 512); }
         *abort_flag = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
@@ -119,53 +126,65 @@ gemm_sm100_pair_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_c
     cluster_sync_all();                                   // both blocks' barriers exist before either signals the other's
     tcgen05_fence_after();
     const uint32_t tmem_base = *tmem_holder;
-    pdl_wait(15);
+    if (warp != 0) pdl_wait(15);
 
     if (warp == 0) {
         if (elect_one()) {
-            uint32_t it = 0;
+            auto load_w = [&](int m_tile, int kb, int s) {
+                unsigned char* a = tiles + s * stage_bytes;
+                if (rank == 0) mbar_expect_tx(full_bar + s, 2 * stage_bytes);        // both blocks' bytes
+                if (EPI == PAIR_SWIGLU) {
+                    const int f0 = (m_tile * 2 + (int)rank) * FEATS;
+                    tma_load_2d_pair(a, &map_w, kb * BK, f0, full_bar + s);                             // 64 gate rows
+                    tma_load_2d_pair(a + FEATS * BK * 2, &map_w, kb * BK, N + f0, full_bar + s);        // their up rows
+                } else {
+                    tma_load_2d_pair(a, &map_w, kb * BK, m_tile * 2 * BMH + (int)rank * BMH, full_bar + s);
+                }
+            };
+            auto load_x = [&](int n_tile, int kb, int s) {
+                tma_load_2d_pair(tiles + s * stage_bytes + A_BYTES, &map_x, kb * BK, n_tile * bn + (int)rank * half, full_bar + s);
+            };
+            // weights that no kernel writes are asked for before the kernels in front are done
+            const int pre = early ? min(stages, total_kb) : 0;
+            for (int kb = 0; kb < pre; ++kb) load_w(pair / n_tiles, kb, kb);
+            pdl_wait(15);
+            int s = 0;
+            uint32_t ph = 0;
             bool ok = true;
             for (int tile = pair; tile < num_tiles && ok; tile += num_pairs) {
                 const int m_tile = tile / n_tiles, n_tile = tile % n_tiles;
-                for (int kb = 0; kb < total_kb; ++kb, ++it) {
-                    const int s = it % STAGES;
-                    const uint32_t ph = (it / STAGES) & 1;
-                    if (!mbar_wait(empty_bar + s, ph ^ 1, abort_flag, err_flag, 31)) { ok = false; break; }
-                    unsigned char* a = tiles + s * STAGE_BYTES;
-                    if (rank == 0) mbar_expect_tx(full_bar + s, 2 * STAGE_BYTES);        // both blocks' bytes
-                    if (EPI == PAIR_SWIGLU) {
-                        const int f0 = (m_tile * 2 + (int)rank) * FEATS;
-                        tma_load_2d_pair(a, &map_w, kb * BK, f0, full_bar + s);                             // 64 gate rows
-                        tma_load_2d_pair(a + FEATS * BK * 2, &map_w, kb * BK, N + f0, full_bar + s);        // their up rows
-                    } else {
-                        tma_load_2d_pair(a, &map_w, kb * BK, m_tile * 2 * BMH + (int)rank * BMH, full_bar + s);
+                for (int kb = 0; kb < total_kb; ++kb) {
+                    if (tile != pair || kb >= pre) {
+                        if (!mbar_wait(empty_bar + s, ph ^ 1, abort_flag, err_flag, 31)) { ok = false; break; }
+                        load_w(m_tile, kb, s);
                     }
-                    tma_load_2d_pair(a + BMH * BK * 2, &map_x, kb * BK, n_tile * 2 * BTH + (int)rank * BTH, full_bar + s);
+                    load_x(n_tile, kb, s);
+                    if (++s == stages) { s = 0; ph ^= 1; }
                 }
             }
         }
     } else if (warp == 1) {
         if (rank == 0 && elect_one()) {
-            constexpr uint32_t idesc = umma_idesc_bf16(2 * BMH, 2 * BTH, false);
-            uint32_t it = 0, local = 0;
+            const uint32_t idesc = umma_idesc_bf16(2 * BMH, bn, false);
+            uint32_t local = 0, ph = 0;
+            int s = 0;
             bool ok = true;
             for (int tile = pair; tile < num_tiles && ok; tile += num_pairs, ++local) {
                 const uint32_t buf = local & 1, aph = (local >> 1) & 1;
                 if (!mbar_wait(acc_empty + buf, aph ^ 1, abort_flag, err_flag, 32)) break;      // drained by both blocks' epilogues
                 tcgen05_fence_after();
-                const uint32_t tmem_d = tmem_base + buf * (2 * BTH);
-                for (int kb = 0; kb < total_kb; ++kb, ++it) {
-                    const int s = it % STAGES;
-                    const uint32_t ph = (it / STAGES) & 1;
+                const uint32_t tmem_d = tmem_base + buf * 256;
+                for (int kb = 0; kb < total_kb; ++kb) {
                     if (!mbar_wait(full_bar + s, ph, abort_flag, err_flag, 32)) { ok = false; break; }
                     tcgen05_fence_after();
-                    unsigned char* a = tiles + s * STAGE_BYTES;
+                    unsigned char* a = tiles + s * stage_bytes;
                     const uint64_t adesc = umma_desc_sw128(a);
-                    const uint64_t bdesc = umma_desc_sw128(a + BMH * BK * 2);
+                    const uint64_t bdesc = umma_desc_sw128(a + A_BYTES);
 #pragma unroll
                     for (int k = 0; k < BK / UMMA_K; ++k)
                         umma_bf16_pair(tmem_d, adesc + 2 * k, bdesc + 2 * k, idesc, (kb > 0 || k > 0) ? 1u : 0u);
                     umma_commit_pair(empty_bar + s);                  // the stage is free in both blocks
+                    if (++s == stages) { s = 0; ph ^= 1; }
                 }
                 if (ok) umma_commit_pair(acc_full + buf);             // the accumulator is complete in both blocks
             }
@@ -193,15 +212,16 @@ gemm_sm100_pair_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_c
             }
             if (!ok) break;
             tcgen05_fence_after();
-            const uint32_t taddr = tmem_base + buf * (2 * BTH) + ((uint32_t)(quad * 32) << 16);
-            const int t0 = n_tile * 2 * BTH;
+            const uint32_t taddr = tmem_base + buf * 256 + ((uint32_t)(quad * 32) << 16);
+            const int t0 = n_tile * bn;
+            const int rounds = (min(bn, T - t0) + 15) / 16;            // of 16 tokens, none of them beyond the last
             if (EPI == PAIR_STORE && sizeof(OutT) == 2 && wide) {
                 // 16 tokens at a time through shared memory, so that C is written in 16-byte pieces
                 // along the features (a thread of the accumulator holds one feature of 16 tokens:
                 // stored directly that would be 2-byte writes). Two buffers, one barrier per round.
                 __nv_bfloat16* stg = reinterpret_cast<__nv_bfloat16*>(xg);
                 const int fbase = m_tile * 2 * BMH + (int)rank * BMH;
-                for (int round = grp, n = 0; round < 2 * BTH / 16; round += 2, ++n) {
+                for (int round = grp, n = 0; round < rounds; round += 2, ++n) {
                     const int c = round * 16;
                     uint32_t r[16];
                     tmem_ld16(taddr + c, r);
@@ -222,7 +242,7 @@ gemm_sm100_pair_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_c
                 group_sync();                                      // the buffers are free for the next tile
             } else if (EPI == PAIR_STORE) {
                 const int f = m_tile * 2 * BMH + (int)rank * BMH + row;
-                for (int round = grp; round < 2 * BTH / 16; round += 2) {
+                for (int round = grp; round < rounds; round += 2) {
                     const int c = round * 16;
                     uint32_t r[16];
                     tmem_ld16(taddr + c, r);
@@ -246,7 +266,7 @@ gemm_sm100_pair_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_c
                 const int fbase = (m_tile * 2 + (int)rank) * FEATS;
                 float* xbuf = reinterpret_cast<float*>(xg);                                   // 2 x [8][2][64] float32
                 __nv_bfloat16* stg = reinterpret_cast<__nv_bfloat16*>(xg + 2 * 8 * 2 * FEATS * 4);   // 2 x [16][64] bfloat16
-                for (int round = grp, n = 0; round < 2 * BTH / 16; round += 2, ++n) {
+                for (int round = grp, n = 0; round < rounds; round += 2, ++n) {
                     const int c = round * 16;
                     uint32_t r[16];
                     tmem_ld16(taddr + c, r);
@@ -344,10 +364,28 @@ int make_map(CUtensorMap* out, const void* ptr, long long rows, long long cols, 
     return 0;
 }
 
-constexpr size_t SMEM_BYTES = (size_t)STAGES * STAGE_BYTES + 1024 + 256 + 2 * EPI_GROUP_BYTES;     // tiles, alignment slack, barriers, epilogue buffers
+constexpr size_t SMEM_BYTES = (size_t)RING_BYTES + 1024 + 256 + 2 * EPI_GROUP_BYTES;     // tiles, alignment slack, barriers, epilogue buffers
+
+// Tokens of a tile: 32 to 256 in steps of 32, the count whose waves of tiles cost least. A wave costs its tokens and some 120 more
+// (both blocks' weights, and what a tile begins and ends with); a last wave that is nearly empty costs less than a whole one.
+// Gate/up with SwiGLU at 8,192 x 2,048, us, tiles of 256 tokens / these: 517 rows 43.6 / 32.9 (three of 192), 600 rows 43 / 35.7 (three of
+// 224), 800 rows 51 / 45.2 (four of 224); library product and activation kernel 36.3, 39.3 and 51.4. 1,000, 1,280, 1,536 and 2,048 rows keep 256
+// (50.9, 61.9, 72.4, 90.0; the next best 55.0, 65.3, 74.5, 97.8). Two instructions side by side on one set of weights (up to 512
+// tokens in one accumulator) were never ahead by more than 2 us and lost where the epilogue had nothing to hide behind: 350 rows 27.7 / 25.2.
+int pick_tokens(int T, long long m_tiles, long long pairs) {
+    int best = BN_MAX;
+    double least = 1e300;
+    for (int bn = BN_MAX; bn >= 32; bn -= 32) {
+        const double per_pair = (double)(m_tiles * ((T + bn - 1) / bn)) / (double)pairs;
+        const double cost = (0.7 * std::ceil(per_pair) + 0.3 * std::max(1.0, per_pair)) * (bn + 120);
+        if (cost < least) { least = cost; best = bn; }
+    }
+    return best;
+}
 
 template <typename OutT, int EPI, int ACT = 0>
-int launch(const CUtensorMap& mw, const CUtensorMap& mx, void* C, long long ldc, int T, int N, int K, int* err_flag, cudaStream_t stream) {
+int launch(const CUtensorMap& mw, const void* X, long long ldx, void* C, long long ldc, int T, int N, int K, int early, int* err_flag,
+           cudaStream_t stream) {
     // 16-byte stores of C need aligned rows and a feature count that no piece of 8 straddles
     const int wide = (ldc % 8 == 0 && ((uintptr_t)C & 15) == 0 && N % 8 == 0) ? 1 : 0;
     static bool configured = false;
@@ -362,8 +400,13 @@ int launch(const CUtensorMap& mw, const CUtensorMap& mx, void* C, long long ldc,
         configured = true;
     }
     constexpr int FEATS = EPI == PAIR_SWIGLU ? BMH / 2 : BMH;
-    const long long tiles = (long long)((N + 2 * FEATS - 1) / (2 * FEATS)) * ((T + 2 * BTH - 1) / (2 * BTH));
+    const long long m_tiles = (N + 2 * FEATS - 1) / (2 * FEATS);
     long long pairs = num_sms / 2;
+    const int bn = pick_tokens(T, m_tiles, pairs);
+    const long long tiles = m_tiles * ((T + bn - 1) / bn);
+    CUtensorMap mx;
+    int me = make_map(&mx, X, T, K, ldx, bn / 2);
+    if (me) return me;
     if (tiles < pairs) pairs = tiles;
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3((unsigned)(2 * pairs));
@@ -379,7 +422,7 @@ int launch(const CUtensorMap& mw, const CUtensorMap& mx, void* C, long long ldc,
     attr[1].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attr;
     cfg.numAttrs = g_vob_pdl ? 2 : 1;
-    cudaError_t e = cudaLaunchKernelEx(&cfg, gemm_sm100_pair_kernel<OutT, EPI, ACT>, mw, mx, (OutT*)C, ldc, T, N, K, wide, err_flag);
+    cudaError_t e = cudaLaunchKernelEx(&cfg, gemm_sm100_pair_kernel<OutT, EPI, ACT>, mw, mx, (OutT*)C, ldc, T, N, K, wide, err_flag, bn, early);
     return e != cudaSuccess ? (int)e : vob_launch_status();
 }
 
@@ -392,41 +435,35 @@ VOB_EXPORT int vob_gemm_sm100_pair(const void* X, long long ldx, const void* W, 
     if (K <= 0 || ldx < K || ldw < K || ldc < N) return VOB_ERR_BAD_ARG;
     if (K % 8 != 0 || ldx % 8 != 0 || ldw % 8 != 0 || ((uintptr_t)X % 16) != 0 || ((uintptr_t)W % 16) != 0) return VOB_ERR_UNSUPPORTED;
     if (out_code != VOB_F32 && out_code != VOB_BF16) return VOB_ERR_BAD_ARG;
-    CUtensorMap mw, mx;
+    CUtensorMap mw;
     int e = make_map(&mw, W, N, K, ldw, BMH);
     if (e) return e;
-    e = make_map(&mx, X, T, K, ldx, BTH);
-    if (e) return e;
-    return out_code == VOB_F32 ? launch<float, PAIR_STORE>(mw, mx, C, ldc, T, N, K, err_flag, stream)
-                               : launch<__nv_bfloat16, PAIR_STORE>(mw, mx, C, ldc, T, N, K, err_flag, stream);
+    return out_code == VOB_F32 ? launch<float, PAIR_STORE>(mw, X, ldx, C, ldc, T, N, K, 0, err_flag, stream)
+                               : launch<__nv_bfloat16, PAIR_STORE>(mw, X, ldx, C, ldc, T, N, K, 0, err_flag, stream);
 }
 
 // C[T, I] (bfloat16) = silu(X Wg^T) * (X Wu^T), W = [Wg; Wu] of shape [2I, K].
 VOB_EXPORT int vob_gemm_sm100_pair_swiglu(const void* X, long long ldx, const void* W, long long ldw, void* C, long long ldc,
-                                          int T, int I, int K, int* err_flag, cudaStream_t stream) {
+                                          int T, int I, int K, int early, int* err_flag, cudaStream_t stream) {
     if (T <= 0 || I <= 0) return 0;
     if (K <= 0 || ldx < K || ldw < K || ldc < I) return VOB_ERR_BAD_ARG;
     if (K % 8 != 0 || ldx % 8 != 0 || ldw % 8 != 0 || ((uintptr_t)X % 16) != 0 || ((uintptr_t)W % 16) != 0) return VOB_ERR_UNSUPPORTED;
-    CUtensorMap mw, mx;
+    CUtensorMap mw;
     int e = make_map(&mw, W, 2LL * I, K, ldw, BMH / 2);         // boxes of 64 rows: half a block's operand from each half of W
     if (e) return e;
-    e = make_map(&mx, X, T, K, ldx, BTH);
-    if (e) return e;
-    return launch<__nv_bfloat16, PAIR_SWIGLU>(mw, mx, C, ldc, T, I, K, err_flag, stream);
+    return launch<__nv_bfloat16, PAIR_SWIGLU>(mw, X, ldx, C, ldc, T, I, K, early, err_flag, stream);
 }
 
 // The same with the gate's activation chosen: act 0 silu, 1 the tanh form of gelu.
 VOB_EXPORT int vob_gemm_sm100_pair_glu(const void* X, long long ldx, const void* W, long long ldw, void* C, long long ldc,
-                                       int T, int I, int K, int act, int* err_flag, cudaStream_t stream) {
-    if (act == 0) return vob_gemm_sm100_pair_swiglu(X, ldx, W, ldw, C, ldc, T, I, K, err_flag, stream);
+                                       int T, int I, int K, int act, int early, int* err_flag, cudaStream_t stream) {
+    if (act == 0) return vob_gemm_sm100_pair_swiglu(X, ldx, W, ldw, C, ldc, T, I, K, early, err_flag, stream);
     if (act != 1) return VOB_ERR_BAD_ARG;
     if (T <= 0 || I <= 0) return 0;
     if (K <= 0 || ldx < K || ldw < K || ldc < I) return VOB_ERR_BAD_ARG;
     if (K % 8 != 0 || ldx % 8 != 0 || ldw % 8 != 0 || ((uintptr_t)X % 16) != 0 || ((uintptr_t)W % 16) != 0) return VOB_ERR_UNSUPPORTED;
-    CUtensorMap mw, mx;
+    CUtensorMap mw;
     int e = make_map(&mw, W, 2LL * I, K, ldw, BMH / 2);
     if (e) return e;
-    e = make_map(&mx, X, T, K, ldx, BTH);
-    if (e) return e;
-    return launch<__nv_bfloat16, PAIR_SWIGLU, 1>(mw, mx, C, ldc, T, I, K, err_flag, stream);
+    return launch<__nv_bfloat16, PAIR_SWIGLU, 1>(mw, X, ldx, C, ldc, T, I, K, early, err_flag, stream);
 }

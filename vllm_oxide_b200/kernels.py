@@ -625,10 +625,12 @@ def gemm_sm100_pair(a: torch.Tensor, w: torch.Tensor, out: torch.Tensor) -> None
 
 
 @_timed
-def gemm_pair_swiglu(a: torch.Tensor, w_gate_up: torch.Tensor, out: torch.Tensor, activation: str = "silu") -> None:
+def gemm_pair_swiglu(a: torch.Tensor, w_gate_up: torch.Tensor, out: torch.Tensor, activation: str = "silu",
+                     fixed_w: bool = False) -> None:
     """out[T, I] = act(a @ Wg^T) * (a @ Wu^T) with w_gate_up = [Wg; Wu] ([2I, K], bfloat16) for many rows:
     the two-SM tcgen05 product whose epilogue applies the activation (gate and up never go to memory);
-    act is "silu" or "gelu_tanh"."""
+    act is "silu" or "gelu_tanh". `fixed_w`: no kernel writes `w_gate_up` (a model's weights), so that its first
+    tiles may be read while the kernels in front still run."""
     op = "gemm_pair_swiglu"
     if activation not in GLU_ACTIVATIONS:
         raise ShapeError(op, f"activation {activation!r} is not known ({', '.join(GLU_ACTIVATIONS)})")
@@ -641,9 +643,9 @@ def gemm_pair_swiglu(a: torch.Tensor, w_gate_up: torch.Tensor, out: torch.Tensor
     I = w_gate_up.shape[0] // 2
     if out.shape != (T, I) or out.dtype != torch.bfloat16 or out.stride(1) != 1:
         raise ShapeError(op, f"out must be bfloat16 [{T}, {I}], got {out.dtype} {list(out.shape)}")
-    f = _fn("gemm_sm100_pair", "vob_gemm_sm100_pair_glu", [_P, _L, _P, _L, _P, _L, _I, _I, _I, _I, _P, _P])
+    f = _fn("gemm_sm100_pair", "vob_gemm_sm100_pair_glu", [_P, _L, _P, _L, _P, _L, _I, _I, _I, _I, _I, _P, _P])
     _check(f(_ptr(a), a.stride(0), _ptr(w_gate_up), w_gate_up.stride(0), _ptr(out), out.stride(0), T, I, K,
-             GLU_ACTIVATIONS[activation], _ptr(_scratch_for(a.device).err), _stream()), op)
+             GLU_ACTIVATIONS[activation], int(fixed_w), _ptr(_scratch_for(a.device).err), _stream()), op)
 
 
 def _pick_splits(T: int, N: int, K: int, device) -> int:

@@ -88,7 +88,7 @@ class SwiGLU(FeedForward):
         elif path == "pair":
             # many rows: the two-SM product with the activation in its epilogue (gate and up never
             # go to memory)
-            kernels.gemm_pair_swiglu(x, self.w_gate_up, act, self.activation)
+            kernels.gemm_pair_swiglu(x, self.w_gate_up, act, self.activation, fixed_w=True)
         else:
             gate_up = matmul(x, self.w_gate_up, ctx.alloc((T, 2 * self.inter)))
             kernels.glu(gate_up, act, self.activation)
