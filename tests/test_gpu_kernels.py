@@ -941,6 +941,32 @@ def test_gemm_fused_residual_and_folded_norm(T, N, Kd, splits):
     assert rel(out, want_delta) <= max(2e-6, 2.0 ** -22 * math.sqrt(Kd)) * 4
 
 
+@pytest.mark.parametrize("I,Kd", [(1, 4), (33, 64), (40, 516), (96, 1152), (160, 4100), (64, 8192)])
+@pytest.mark.parametrize("M", [1, 2, 3, 8, 9, 16])
+def test_gemm_f32_swiglu(M, I, Kd):
+    """Gate/up and activation in the few-row product's epilogue: the bits of the product and the activation kernel one behind the
+    other, for features that are no multiple of a block's 32, K of one chunk to many; other sizes are refused."""
+    from vllm_oxide_b200.errors import ShapeError
+    g = torch.Generator().manual_seed(M * 1000 + I + Kd)
+    a = torch.randn(M, Kd + 4, generator=g).to(DEV)[:, :Kd]
+    w = (torch.randn(2 * I, Kd, generator=g) / math.sqrt(Kd) * 2).to(DEV)
+    k = K()
+    out = torch.full((M, I + 3), 7.0, device=DEV)
+    assert not k.gemm_f32_swiglu_supported(a[:, :Kd - 1], w[:, :Kd - 1]) and not k.gemm_f32_swiglu_supported(a.repeat(17, 1), w)
+    if not k.gemm_f32_swiglu_supported(a, w):
+        assert M > (4 if Kd <= 64 else 8) and (Kd > 4096 or Kd <= 128)
+        with pytest.raises(ShapeError):
+            k.gemm_f32_swiglu(a, w, out[:, :I])
+        return
+    torch.cuda.synchronize()
+    k.gemm_f32_swiglu(a, w, out[:, :I], fixed_w=True)
+    gu, want = torch.empty(M, 2 * I, device=DEV), torch.empty(M, I, device=DEV)
+    k.gemm_f32(a, w, gu)
+    k.glu(gu, want)
+    assert torch.equal(out[:, :I], want)
+    assert float((out[:, I:] - 7.0).abs().max()) == 0.0
+
+
 # ----------------------------------------------------------------------------- tcgen05 product on pairs of SMs
 @pytest.mark.parametrize("odt", [torch.bfloat16, torch.float32], ids=["bf16out", "f32out"])
 @pytest.mark.parametrize("T,N,Kd", [(1, 8, 64), (256, 256, 64), (300, 520, 264), (129, 1000, 1032), (700, 384, 96), (1030, 2048, 512)])

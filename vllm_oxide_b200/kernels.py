@@ -551,6 +551,31 @@ def gemm_f32(a: torch.Tensor, w: torch.Tensor, out: torch.Tensor, bias: Optional
     _check(f(_ptr(a), a.stride(0), _ptr(w), w.stride(0), _ptr(out), out.stride(0), M, N, K, _ptr(bias), int(fixed_w), _stream()), op)
 
 
+def gemm_f32_swiglu_supported(a: torch.Tensor, w_gate_up: torch.Tensor) -> bool:
+    """Whether `gemm_f32_swiglu` takes these operands: float32, few rows, K a multiple of 4, 16-byte aligned rows."""
+    if a.dtype != torch.float32 or w_gate_up.dtype != torch.float32 or a.dim() != 2 or w_gate_up.dim() != 2 or w_gate_up.shape[0] % 2:
+        return False
+    if any(t.stride(1) != 1 or t.stride(0) % 4 or t.data_ptr() % 16 for t in (a, w_gate_up)):
+        return False
+    return bool(_fn("gemm_f32", "vob_gemm_f32_swiglu_supported", [_I, _I, _I])(a.shape[0], w_gate_up.shape[0] // 2, a.shape[1]))
+
+
+@_timed
+def gemm_f32_swiglu(a: torch.Tensor, w_gate_up: torch.Tensor, out: torch.Tensor, fixed_w: bool = False) -> None:
+    """out[M, I] = silu(a @ Wg^T) * (a @ Wu^T) with w_gate_up = [Wg; Wu] ([2I, K]) in true float32, for the few rows that
+    `gemm_f32_swiglu_supported` names: the bits that `gemm_f32` and `glu` give one behind the other, in one kernel."""
+    op = "gemm_f32_swiglu"
+    _cuda(op, a, w_gate_up, out)
+    if not gemm_f32_swiglu_supported(a, w_gate_up):
+        raise ShapeError(op, f"not for a {a.dtype} {list(a.shape)} and w {w_gate_up.dtype} {list(w_gate_up.shape)}")
+    M, K = a.shape
+    I = w_gate_up.shape[0] // 2
+    if w_gate_up.shape[1] != K or out.shape != (M, I) or out.dtype != torch.float32 or out.stride(1) != 1:
+        raise ShapeError(op, f"w must be [2I, {K}] and out float32 [{M}, I], got {list(w_gate_up.shape)} and {out.dtype} {list(out.shape)}")
+    f = _fn("gemm_f32", "vob_gemm_f32_swiglu", [_P, _L, _P, _L, _P, _L, _I, _I, _I, _I, _P])
+    _check(f(_ptr(a), a.stride(0), _ptr(w_gate_up), w_gate_up.stride(0), _ptr(out), out.stride(0), M, I, K, int(fixed_w), _stream()), op)
+
+
 class _GemmScratch:
     """Per device: the error word that a timed-out wait inside the tensor-core product raises."""
 

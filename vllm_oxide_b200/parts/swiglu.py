@@ -81,6 +81,9 @@ class SwiGLU(FeedForward):
     def forward(self, x: torch.Tensor, ctx: StepContext, out=None) -> torch.Tensor:
         T = x.shape[0]
         act = ctx.alloc((T, self.inter))
+        if self.dtype == torch.float32 and self.fused and self.activation == "silu" and kernels.gemm_f32_swiglu_supported(x, self.w_gate_up):
+            kernels.gemm_f32_swiglu(x, self.w_gate_up, act, fixed_w=True)        # few rows: the activation in the product's epilogue
+            return matmul(act, self.w_down, out if out is not None else ctx.alloc((T, self.hidden)))
         path = self._path(T, kernels.gemm_sm100_supported(x, self.w_gate_up))
         if path == "few":
             # few rows: one kernel, the activation applied in the product's epilogue
