@@ -941,7 +941,24 @@ def test_gemm_fused_residual_and_folded_norm(T, N, Kd, splits):
     assert rel(out, want_delta) <= max(2e-6, 2.0 ** -22 * math.sqrt(Kd)) * 4
 
 
-@pytest.mark.parametrize("I,Kd", [(1, 4), (33, 64), (40, 516), (96, 1152), (160, 4100), (64, 8192)])
+@pytest.mark.parametrize("N,Kd", [(16390, 2000), (16384, 1024), (8200, 4096), (4100, 8192), (32777, 1536)])
+def test_gemm_f32_few_rows_chunks_of_a_block(N, Kd):
+    """A block of the few-row kernel that has all, half or a quarter of K's chunks; every count of rows
+    gives the bits that the same rows have in a product of 40, which the tiles compute."""
+    g = torch.Generator().manual_seed(N + Kd)
+    a = torch.randn(40, Kd, generator=g).to(DEV)
+    w = torch.randn(N, Kd, generator=g).to(DEV)
+    k = K()
+    want = torch.empty(40, N, device=DEV)
+    k.gemm_f32(a, w, want)
+    assert rel(want[:2], (a[:2].double() @ w.double().t()).cpu()) <= 2.0 ** -22 * math.sqrt(Kd)
+    for M in (1, 2, 3, 4, 5, 8, 16):
+        out = torch.full((M, N), 7.0, device=DEV)
+        k.gemm_f32(a[:M], w, out)
+        assert torch.equal(out, want[:M]), M
+
+
+@pytest.mark.parametrize("I,Kd", [(1, 4), (33, 64), (40, 516), (96, 1152), (160, 4100), (64, 8192), (8200, 2000)])
 @pytest.mark.parametrize("M", [1, 2, 3, 8, 9, 16])
 def test_gemm_f32_swiglu(M, I, Kd):
     """Gate/up and activation in the few-row product's epilogue: the bits of the product and the activation kernel one behind the
@@ -954,7 +971,7 @@ def test_gemm_f32_swiglu(M, I, Kd):
     out = torch.full((M, I + 3), 7.0, device=DEV)
     assert not k.gemm_f32_swiglu_supported(a[:, :Kd - 1], w[:, :Kd - 1]) and not k.gemm_f32_swiglu_supported(a.repeat(17, 1), w)
     if not k.gemm_f32_swiglu_supported(a, w):
-        assert M > (4 if Kd <= 64 else 8) and (Kd > 4096 or Kd <= 128)
+        assert M > (4 if Kd <= 64 else 8)
         with pytest.raises(ShapeError):
             k.gemm_f32_swiglu(a, w, out[:, :I])
         return

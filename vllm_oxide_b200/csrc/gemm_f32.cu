@@ -9,8 +9,8 @@
 // rounds more often: relative error against 64 bits on normal values 8.1e-7 and 1.6e-6 at K = 2,048 and 8,192, here 1.6e-7 and 1.7e-7.)
 //
 // Two kernels:
-//  * few rows (decode steps: M <= 8, M <= 16 while K is at most 4,096): bound by reading W once, 5.9 TB/s at M = 1 and 2.7 TB/s at M = 16 on 128,256 x 2,048, 3.4 and
-//    2.0 TB/s on 16,384 x 2,048 (64 x 64 tiles, which served every M before: 1.06 and 0.6 TB/s; 0.1 TB/s on 2,048 x 8,192, now 2.6). A thread has one or two weight rows and a chunk, all rows of A
+//  * few rows (decode steps: M <= 8, M <= 16 while K is at most 4,096): bound by reading W once, 6.9 TB/s at M = 1, 5.2 at 8 and 2.7 at
+//    16 on 128,256 x 2,048, 5.5, 4.5 and 2.4 TB/s on 16,384 x 2,048 back to back (64 x 64 tiles, which served every M before: 1.06 and 0.6 TB/s; 0.1 TB/s on 2,048 x 8,192, now 2.6). A thread has one or two weight rows and a chunk, all rows of A
 //    in its registers' sums; weights arrive by cp.async into a ring per warp, so that no barrier of the block stands in the stream.
 //  * tiles (everything else): bound by what two warps a scheduler can issue: the FMA units are busy 60 % of the cycles, shared memory
 //    48 %, and a warp waits for the result in front or for a register's read most of the rest. 8 x 8 outputs a thread from
@@ -62,9 +62,25 @@ __host__ __device__ constexpr int seg_chunks(int nc) { return (nc + 7) / 8; }
 constexpr int FEW_N = 64, FEW_K = 32;                 // weight rows of a block, k of a ring stage
 
 constexpr int few_rows_a_lane(int mb) { return mb <= 4 ? 1 : 2; }
-// three blocks an SM (two from three rows of A on) for the usual four chunks a block
+// three blocks an SM (two from three rows of A on) for four chunks a block
 __host__ __device__ constexpr int few_blocks(int mb) { return mb <= 2 ? 3 : 2; }
-constexpr int few_stages(int mb) { return mb == 4 ? 3 : 2; }
+constexpr int few_stages(int) { return 2; }
+// Shared memory of a block that adds up `chunks` chunks: its warps' rings, x of four chunks, the chunks' sums.
+constexpr size_t few_smem(int mb, int chunks) { return sizeof(float) * (size_t)(8 * few_stages(mb) * 32 * FEW_K + 4 * CHUNK * mb + chunks * mb * FEW_N); }
+// Chunks of a block, a multiple of four: an eighth of K at least (a cluster holds eight blocks); all of it, half of it or, with one or two
+// rows, a quarter, where 256 blocks are left and two of them find room on an SM. A block's start, its cluster's meeting and its end cost as much as
+// four chunks of weights do. Cold, back to back, us with an eighth (and three stages for three and four rows, as it was) / now, 1, 4 and 8 rows:
+// 16,384 x 2,048 26.5, 35, 38 / 23.7, 25.6, 29.5; 128,256 x 2,048 162, 233, 255 / 151, 164, 202; 28,672 x 4,096 91, 131, 142 / 82, 94, 111. Three
+// blocks to a K of 32 chunks (6,144 x 4,096) lose from three rows on: 32.5 / 39 at eight.
+inline int few_chunks(int rows, int mb, long long row_blocks, int nc) {
+    const int least = ((nc + 7) / 8 + 3) / 4 * 4;
+    if (mb > 8) return least;
+    for (int c = 1; c <= (rows <= 2 ? 4 : 2); c *= 2) {
+        const int q = (nc + c - 1) / c;
+        if (q > least && q % 4 == 0 && nc % q == 0 && row_blocks * c >= 256 && few_smem(mb, q) <= 112 * 1024) return q;
+    }
+    return least;
+}
 
 // GLU: W is [gate; up] ([2N, K]); the block's 64 weight rows are 32 of each half, of the same features, and C[m, n] =
 // silu(gate) * up. The sums and the activation are those of the product and the activation kernel behind one another, to the bit; a
@@ -205,14 +221,14 @@ gemm_f32_few_kernel(const float* __restrict__ A, long long lda, const float* __r
 
 template <int MB, bool GLU>
 int launch_few(const float* A, long long lda, const float* W, long long ldw, float* C, long long ldc, int M, int N, int K,
-               const float* bias, int nc, int q, int c, int early, cudaStream_t stream) {
-    constexpr int RN = few_rows_a_lane(MB), NS = few_stages(MB);
-    size_t smem = sizeof(float) * (size_t)(8 * NS * 32 * FEW_K + 4 * CHUNK * MB + min(q, nc) * MB * FEW_N);
+               const float* bias, int early, cudaStream_t stream) {
+    constexpr int RN = few_rows_a_lane(MB), NS = few_stages(MB), FEATS = GLU ? FEW_N / 2 : FEW_N;
+    const int nc = (K + CHUNK - 1) / CHUNK, q = few_chunks(M, MB, (N + FEATS - 1) / FEATS, nc), c = (nc + q - 1) / q;
+    size_t smem = few_smem(MB, min(q, nc));
     if (smem > 200 * 1024) return VOB_ERR_UNSUPPORTED;
     auto kernel = gemm_f32_few_kernel<MB, RN, NS, GLU>;
     cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return (int)e;
-    constexpr int FEATS = GLU ? FEW_N / 2 : FEW_N;
     long long blocks = (long long)((N + FEATS - 1) / FEATS) * c;
     if (blocks > 0x7fffffffLL) return VOB_ERR_UNSUPPORTED;
     cudaLaunchConfig_t cfg = {};
@@ -406,21 +422,22 @@ bool few_rows(int M, int K) {
 template <bool GLU>
 int few(const float* A, long long lda, const float* W, long long ldw, float* C, long long ldc, int M, int N, int K, const float* bias,
         int early, cudaStream_t stream) {
-    int nc = (K + CHUNK - 1) / CHUNK, q = ((nc + 7) / 8 + 3) / 4 * 4, c = (nc + q - 1) / q;
-    return M == 1   ? launch_few<1, GLU>(A, lda, W, ldw, C, ldc, M, N, K, bias, nc, q, c, early, stream)
-           : M == 2 ? launch_few<2, GLU>(A, lda, W, ldw, C, ldc, M, N, K, bias, nc, q, c, early, stream)
-           : M <= 4 ? launch_few<4, GLU>(A, lda, W, ldw, C, ldc, M, N, K, bias, nc, q, c, early, stream)
-           : M <= 8 ? launch_few<8, GLU>(A, lda, W, ldw, C, ldc, M, N, K, bias, nc, q, c, early, stream)
-                    : launch_few<16, GLU>(A, lda, W, ldw, C, ldc, M, N, K, bias, nc, q, c, early, stream);
+    if constexpr (!GLU)
+        if (M > 8) return launch_few<16, GLU>(A, lda, W, ldw, C, ldc, M, N, K, bias, early, stream);
+    return M == 1   ? launch_few<1, GLU>(A, lda, W, ldw, C, ldc, M, N, K, bias, early, stream)
+           : M == 2 ? launch_few<2, GLU>(A, lda, W, ldw, C, ldc, M, N, K, bias, early, stream)
+           : M <= 4 ? launch_few<4, GLU>(A, lda, W, ldw, C, ldc, M, N, K, bias, early, stream)
+                    : launch_few<8, GLU>(A, lda, W, ldw, C, ldc, M, N, K, bias, early, stream);
 }
 
 }  // namespace
 
 // Whether vob_gemm_f32_swiglu takes a product of these sizes (then it is also the faster way).
 VOB_EXPORT int vob_gemm_f32_swiglu_supported(int M, int I, int K) {
-    if (M <= 0 || I <= 0 || K <= 0 || K % 4 != 0 || M > 16 || !few_rows(M, K)) return 0;
-    int nc = (K + CHUNK - 1) / CHUNK, q = ((nc + 7) / 8 + 3) / 4 * 4, mb = M <= 2 ? M : M <= 4 ? 4 : M <= 8 ? 8 : 16;
-    return sizeof(float) * (size_t)(8 * few_stages(mb) * 32 * FEW_K + 4 * CHUNK * mb + (q < nc ? q : nc) * mb * FEW_N) <= 200 * 1024;
+    if (M <= 0 || I <= 0 || K <= 0 || K % 4 != 0 || M > 8 || !few_rows(M, K)) return 0;      // 12 rows: 1 % slower in a whole step
+    int nc = (K + CHUNK - 1) / CHUNK, mb = M <= 2 ? M : M <= 4 ? 4 : 8;
+    int q = few_chunks(M, mb, (I + FEW_N / 2 - 1) / (FEW_N / 2), nc);
+    return few_smem(mb, q < nc ? q : nc) <= 200 * 1024;
 }
 
 // C[M, I] = silu(A Wg^T) * (A Wu^T), W = [Wg; Wu] of shape [2I, K], few rows; the bits of vob_gemm_f32 and vob_swiglu one behind the other.
