@@ -941,9 +941,9 @@ def test_gemm_fused_residual_and_folded_norm(T, N, Kd, splits):
     assert rel(out, want_delta) <= max(2e-6, 2.0 ** -22 * math.sqrt(Kd)) * 4
 
 
-@pytest.mark.parametrize("N,Kd", [(16390, 2000), (16384, 1024), (8200, 4096), (4100, 8192), (32777, 1536)])
+@pytest.mark.parametrize("N,Kd", [(16390, 2000), (16384, 1024), (8200, 4096), (4100, 8192), (500, 8200), (32777, 1536)])
 def test_gemm_f32_few_rows_chunks_of_a_block(N, Kd):
-    """A block of the few-row kernel that has all, half or a quarter of K's chunks; every count of rows
+    """A block of the few-row kernel that has all, half or a quarter of K's chunks, and rows taken eight at a time: every count of rows
     gives the bits that the same rows have in a product of 40, which the tiles compute."""
     g = torch.Generator().manual_seed(N + Kd)
     a = torch.randn(40, Kd, generator=g).to(DEV)
@@ -952,7 +952,7 @@ def test_gemm_f32_few_rows_chunks_of_a_block(N, Kd):
     want = torch.empty(40, N, device=DEV)
     k.gemm_f32(a, w, want)
     assert rel(want[:2], (a[:2].double() @ w.double().t()).cpu()) <= 2.0 ** -22 * math.sqrt(Kd)
-    for M in (1, 2, 3, 4, 5, 8, 16):
+    for M in (1, 2, 3, 4, 5, 8, 9, 16, 17, 24, 25):
         out = torch.full((M, N), 7.0, device=DEV)
         k.gemm_f32(a[:M], w, out)
         assert torch.equal(out, want[:M]), M

@@ -9,7 +9,7 @@
 // rounds more often: relative error against 64 bits on normal values 8.1e-7 and 1.6e-6 at K = 2,048 and 8,192, here 1.6e-7 and 1.7e-7.)
 //
 // Two kernels:
-//  * few rows (decode steps: M <= 8, M <= 16 while K is at most 4,096): bound by reading W once, 6.9 TB/s at M = 1, 5.2 at 8 and 2.7 at
+//  * few rows (decode steps: M <= 8, M <= 16 while K is at most 4,096, by eights beyond): bound by reading W once, 6.9 TB/s at M = 1, 5.2 at 8 and 2.7 at
 //    16 on 128,256 x 2,048, 5.5, 4.5 and 2.4 TB/s on 16,384 x 2,048 back to back (64 x 64 tiles, which served every M before: 1.06 and 0.6 TB/s; 0.1 TB/s on 2,048 x 8,192, now 2.6). A thread has one or two weight rows and a chunk, all rows of A
 //    in its registers' sums; weights arrive by cp.async into a ring per warp, so that no barrier of the block stands in the stream.
 //  * tiles (everything else): bound by what two warps a scheduler can issue: the FMA units are busy 60 % of the cycles, shared memory
@@ -460,12 +460,24 @@ VOB_EXPORT int vob_gemm_f32(const float* A, long long lda, const float* W, long 
     int vec = K % 4 == 0 && lda % 4 == 0 && ldw % 4 == 0 && ((uintptr_t)A & 15) == 0 && ((uintptr_t)W & 15) == 0;
     // 16 rows: what a lane's registers hold. Cold, 9 to 16 rows, us here / in tiles (32 rows at least): 2,048 x 512 16 / 23, 2,048 x 2,048
     // 19 / 21, 4,096 x 4,096 41 / 55, 16,384 x 2,048 68 / 94, 128,256 x 2,048 391 / 644; where K has more than 32 chunks a block of 16
-    // rows has its SM to itself, and the tiles win: 2,048 x 8,192 66 / 57, 4,096 x 14,336 209 / 170. Up to 8 rows the tiles never do: there
+    // rows has its SM to itself, and the tiles win: 2,048 x 8,192 66 / 57, 4,096 x 14,336 209 / 170 (see below). Up to 8 rows the tiles never do: there
     // 29 / 57 and 83 / 169 at 8 rows, 25 / 57 and 70 / 170 at one. A single chunk is too short for what a block of 5 rows and more sets
     // up (back to back, 16 rows: 64 x 64 7.3 / 2.9, 2,048 x 64 7.7 / 3.1, 128 x 128 7.5 / 4.7; 8 rows 4.4 / 2.9, 4.6 / 3.1, 4.5 / 4.7).
     if (vec && few_rows(M, K)) {
         int e = few<false>(A, lda, W, ldw, C, ldc, M, N, K, bias, early, stream);
         if (e != VOB_ERR_UNSUPPORTED) return e;       // a K whose sums find no room in shared memory: tiles
+    }
+    // More than 32 chunks, where a block of 16 rows would have its SM to itself: eight rows at a time, which find most of the weights in L2
+    // from the second eight on. Cold, us in eights / in tiles: 2,048 x 8,192 at 9, 16, 24 rows 32, 36, 53 / 87, 87, 85; 1,024 x 6,144 26, 31, 47 /
+    // 52, 52, 52 (58 at 25 rows); 4,096 x 14,336 at 9, 16, 17 rows 109, 133, 175 / 163; 16,384 x 4,608 131, 163, 211 / 213. Larger matrices
+    // come from memory every time: 8,192 x 28,672 at 16 rows 776 / 629. A decode step of 12 requests at 1B sizes 3,590 -> 2,660 us.
+    const double w_bytes = 4.0 * N * K;
+    if (vec && M > 8 && nc > 32 && (M <= 16 ? w_bytes <= 320e6 : M <= 24 && w_bytes <= 70e6)) {
+        for (int m = 0; m < M; m += 8) {
+            int e = few<false>(A + (size_t)m * lda, lda, W, ldw, C + (size_t)m * ldc, ldc, min(8, M - m), N, K, bias, early, stream);
+            if (e) return e;
+        }
+        return 0;
     }
     // Tiles of 128, 64 or 32 rows, a block or eight to a tile: the one whose waves of blocks cost least. A wave's cost is its
     // rows times its resident blocks; smaller tiles read more from shared memory per FMA (measured at 2,048 x 2,048 and
