@@ -958,6 +958,25 @@ def test_gemm_f32_few_rows_chunks_of_a_block(N, Kd):
         assert torch.equal(out, want[:M]), M
 
 
+@pytest.mark.parametrize("N,Kd", [(2100, 1152), (9000, 200), (2050, 1155), (9000, 203), (16384, 1028), (70, 2052), (740, 200), (740, 203)])
+def test_gemm_f32_tiles_of_every_height(N, Kd):
+    """Tiles of 80, 96 and 112 rows beside those of 32, 64 and 128, K shared over a cluster and not, operands that come by 16 and by 4
+    bytes: whatever the launcher takes, a row has the bits it has in the few-row kernel or in another tile."""
+    g = torch.Generator().manual_seed(N + Kd)
+    a = torch.randn(640, Kd, generator=g).to(DEV)
+    w = torch.randn(N, Kd, generator=g).to(DEV)
+    k = K()
+    want = torch.empty(640, N, device=DEV)
+    for r in range(0, 640, 8):
+        k.gemm_f32(a[r:r + 8], w, want[r:r + 8])
+    assert rel(want[:64], (a[:64].double() @ w.double().t()).cpu()) <= 2.0 ** -22 * math.sqrt(Kd)
+    for M in (65, 70, 80, 81, 90, 96, 97, 100, 112, 113, 150, 160, 200, 224, 260, 288, 300, 400, 517, 640):
+        out = torch.full((M + 1, N), 7.0, device=DEV)
+        k.gemm_f32(a[:M], w, out[:M])
+        assert torch.equal(out[:M], want[:M]), M
+        assert float((out[M:] - 7.0).abs().max()) == 0.0
+
+
 @pytest.mark.parametrize("I,Kd", [(1, 4), (33, 64), (40, 516), (96, 1152), (160, 4100), (64, 8192), (8200, 2000)])
 @pytest.mark.parametrize("M", [1, 2, 3, 8, 9, 16])
 def test_gemm_f32_swiglu(M, I, Kd):

@@ -248,13 +248,13 @@ int launch_few(const float* A, long long lda, const float* W, long long ldw, flo
 }
 
 // ------------------------------------------------------------------------------------------------ tiles
-// A block of 128 threads computes 16 * TR rows by 64 columns, a thread TR x 8 of them (rows tm + 16 i, columns tn + 8 j). K
+// A block of 128 threads computes 16 * TR rows by 64 columns (TR 2, 4 to 8), a thread TR x 8 of them (rows tm + 16 i, columns tn + 8 j). K
 // comes in slabs of 16 through a ring of three stages, [row][k] as it lies in memory, rows 20 floats apart: the 16-byte reads
 // of different rows that a warp makes at once fall into different banks. The sums of the chunks so far wait in shared
 // memory: the segment's, and (CL == 1) the finished segments'. Or a cluster of CL = 8 blocks shares K, a segment each, and
 // adds the segments' sums: eight times the blocks, for few tiles or a last wave that would be nearly empty.
 constexpr int TN = 64, TK = 16, TLD = TK + 4, TSTAGES = 3, GRID_Y = 32768;
-__host__ __device__ constexpr int tile_blocks(int tr) { return tr == 8 ? 2 : tr == 4 ? 3 : 4; }   // resident on an SM
+__host__ __device__ constexpr int tile_blocks(int tr) { return tr >= 5 ? 2 : tr == 4 ? 3 : 4; }   // resident on an SM
 
 template <int TR, bool VEC, int CL>
 __global__ void __launch_bounds__(128, tile_blocks(TR))
@@ -279,9 +279,10 @@ gemm_f32_tile_kernel(const float* __restrict__ A, long long lda, const float* __
             put_at = put_at + 1 == TSTAGES ? 0 : put_at + 1;
             int k = kb + s * TK + lk;
 #pragma unroll
-            for (int i = 0; i < (TM + TN) / 32; ++i) {
+            for (int i = 0; i < (TM + TN + 31) / 32; ++i) {
                 int r = i * 32 + (tid >> 2);
-                bool isA = i < TM / 32;
+                if ((TM + TN) % 32 != 0 && r >= TM + TN) break;
+                bool isA = TM % 32 == 0 ? i < TM / 32 : r < TM;
                 int g = isA ? m0 + r : n0 + r - TM;
                 const float* p = isA ? A + (size_t)g * lda : W + (size_t)g * ldw;
                 bool row = g < (isA ? M : N);
@@ -479,23 +480,30 @@ VOB_EXPORT int vob_gemm_f32(const float* A, long long lda, const float* W, long 
         }
         return 0;
     }
-    // Tiles of 128, 64 or 32 rows, a block or eight to a tile: the one whose waves of blocks cost least. A wave's cost is its
+    // Tiles of 128, 112, 96, 80, 64 or 32 rows, a block or eight to a tile: the one whose waves of blocks cost least. A wave's cost is its
     // rows times its resident blocks; smaller tiles read more from shared memory per FMA (measured at 2,048 x 2,048 and
-    // 16,384 x 2,048: 1.15 and 1.5 times the time per row), a shared K is added up over the cluster (dearer where operands come by 4
+    // 16,384 x 2,048: 1.15 and 1.5 times the time per row at 64 and 32 rows; the factors in between are set so that no size measured is
+    // slower than with 128, 64 and 32 alone). What 80, 96 and 112 save is rows that are not there: 16,384 x 2,048 at 70, 90, 100, 130, 400, 700
+    // rows 242, 245, 247, 378, 940, 1,407 us -> 175, 206, 227, 335, 827, 1,273; 2,048 x 8,192 124, 124, 125, 203, 492, 713 -> 87, 103, 115, 174, 414,
+    // 661; 64 rows, 180, 260 and 300, 1,000 to 2,048 as before. A shared K is added up over the cluster (dearer where operands come by 4
     // bytes: 8,192 x 2,050 at 300 rows 579 us shared, 429 not). A grid that finds an SM of its own for every block beside the
     // neighbouring kernel's costs half: 512 x 2,048 at 48 rows 13.7 us in 64 blocks of 64 rows, 21.6 in 128 of 32; 4,096 x 130 10.5 and 17.0.
     int best_tr = 8, best_c = 1;
     double best = 1e300;
-    for (int tr = 2; tr <= 8; tr *= 2)
-        for (int c = 1; c <= 8; c += 7) {
-            if (c > 1 && nc < 8) continue;
+    static const struct { int tr; double per_row; } tiles[] = {{2, 1.5}, {4, 1.15}, {5, 1.15}, {6, 1.2}, {7, 1.08}, {8, 1.0}};
+    for (const auto& t : tiles)
+        for (int tr = t.tr, c = 1; c <= 8; c += 7) {
+            if ((c > 1 && nc < 8) || (tr > 4 && tr < 8 && M <= 64)) continue;
             double slots = 148.0 * tile_blocks(tr), blocks = (double)((M + 16 * tr - 1) / (16 * tr)) * ((N + TN - 1) / TN) * c;
             double waves = (double)(long long)((blocks + slots - 1) / slots);
             if (tr < 8 && blocks <= 74) waves = 0.5;
-            double cost = waves * tile_blocks(tr) * tr * (tr == 8 ? 1.0 : tr == 4 ? 1.15 : 1.5) / c * (c == 1 ? 1.0 : vec ? 1.1 : 1.4);
+            double cost = waves * tile_blocks(tr) * tr * t.per_row / c * (c == 1 ? 1.0 : vec ? 1.1 : 1.4);
             if (cost < best) { best = cost; best_tr = tr; best_c = c; }
         }
     if (best_tr == 8) return launch_tile<8>(A, lda, W, ldw, C, ldc, M, N, K, bias, nc, best_c, vec, stream);
+    if (best_tr == 7) return launch_tile<7>(A, lda, W, ldw, C, ldc, M, N, K, bias, nc, best_c, vec, stream);
+    if (best_tr == 6) return launch_tile<6>(A, lda, W, ldw, C, ldc, M, N, K, bias, nc, best_c, vec, stream);
+    if (best_tr == 5) return launch_tile<5>(A, lda, W, ldw, C, ldc, M, N, K, bias, nc, best_c, vec, stream);
     if (best_tr == 4) return launch_tile<4>(A, lda, W, ldw, C, ldc, M, N, K, bias, nc, best_c, vec, stream);
     return launch_tile<2>(A, lda, W, ldw, C, ldc, M, N, K, bias, nc, best_c, vec, stream);
 }
