@@ -913,7 +913,11 @@ VOB_EXPORT int vob_gemm_sm100_pick_splits(int T, int N, int K, int num_sms) {
     int tiles = ((N + BM - 1) / BM) * ((T + bt - 1) / bt);
     int total_kb = (K + BK - 1) / BK;
     if (T > 64 || tiles * 2 > num_sms) return 1;
-    int want = num_sms / tiles;
+    // 1.6 blocks an SM where the tiles allow it (two find room): what an SM gets of the bandwidth follows the bytes it has in flight. With one
+    // at most, the 8B sizes' QKV ran in 144 blocks and O and down in 128. A decode step, us, one / 1.3 / 1.6 an SM: 8B, 4 requests 3,170 /
+    // 2,918 / 2,885; 3B, 4 requests 1,655 / 1,608 / 1,599; 1B, 1, 8 and 24 requests 662, 728, 880 / 658, 723, 868 / 658, 724, 868. Fewer blocks
+    // lose: QKV of the 1B sizes with 3 instead of 6 to a tile 662 -> 692, down with 4 instead of 8 712.
+    int want = num_sms * 16 / 10 / tiles;
     if (want > 8) want = 8;                                           // the portable cluster size
     int max_splits = total_kb / 4 > 0 ? total_kb / 4 : 1;             // at least 4 k-blocks (256 of K) per split
     int s = want < max_splits ? want : max_splits;
