@@ -919,7 +919,8 @@ VOB_EXPORT int vob_gemm_sm100_pick_splits(int T, int N, int K, int num_sms) {
     // 1.6 blocks an SM where the tiles allow it (two find room): what an SM gets of the bandwidth follows the bytes it has in flight. With one
     // at most, the 8B sizes' QKV ran in 144 blocks and O and down in 128. A decode step, us, one / 1.3 / 1.6 an SM: 8B, 4 requests 3,170 /
     // 2,918 / 2,885; 3B, 4 requests 1,655 / 1,608 / 1,599; 1B, 1, 8 and 24 requests 662, 728, 880 / 658, 723, 868 / 658, 724, 868. Fewer blocks
-    // lose: QKV of the 1B sizes with 3 instead of 6 to a tile 662 -> 692, down with 4 instead of 8 712.
+    // lose: QKV of the 1B sizes with 3 instead of 6 to a tile 662 -> 692, down with 4 instead of 8 712. So do two an SM, which leave the next
+    // kernel no room to start beside this one: 8B 3,203, 3B 1,707.
     int want = num_sms * 16 / 10 / tiles;
     if (want > 8) want = 8;                                           // the portable cluster size
     int max_splits = total_kb / 4 > 0 ? total_kb / 4 : 1;             // at least 4 k-blocks (256 of K) per split
