@@ -958,6 +958,23 @@ def test_gemm_f32_few_rows_chunks_of_a_block(N, Kd):
         assert torch.equal(out, want[:M]), M
 
 
+@pytest.mark.parametrize("N,Kd", [(70, 53252), (70, 61440), (70, 61444), (33, 65536), (1024, 65536)])
+def test_gemm_f32_few_rows_of_a_k_without_room(N, Kd):
+    """A K whose chunks' sums find no room in a block of the few-row kernel goes to the tiles, rows taken eight at a time too: the
+    bits of a product of 40 rows, up to the longest K that fits and beyond it."""
+    g = torch.Generator().manual_seed(N + Kd)
+    a = torch.randn(40, Kd, generator=g).to(DEV)
+    w = torch.randn(N, Kd, generator=g).to(DEV)
+    k = K()
+    want = torch.empty(40, N, device=DEV)
+    k.gemm_f32(a, w, want)
+    assert rel(want[:2], (a[:2].double() @ w.double().t()).cpu()) <= 2.0 ** -22 * math.sqrt(Kd)
+    for M in (1, 4, 8, 9, 12, 16, 17, 24):
+        out = torch.full((M, N), 7.0, device=DEV)
+        k.gemm_f32(a[:M], w, out)
+        assert torch.equal(out, want[:M]), M
+
+
 @pytest.mark.parametrize("N,Kd", [(2100, 1152), (9000, 200), (2050, 1155), (9000, 203), (16384, 1028), (70, 2052), (740, 200), (740, 203)])
 def test_gemm_f32_tiles_of_every_height(N, Kd):
     """Tiles of 80, 96 and 112 rows beside those of 32, 64 and 128, K shared over a cluster and not, operands that come by 16 and by 4

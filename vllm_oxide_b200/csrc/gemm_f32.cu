@@ -81,6 +81,13 @@ inline int few_chunks(int rows, int mb, long long row_blocks, int nc) {
     }
     return least;
 }
+// Whether a block finds room for its chunks' sums: it does up to K = 61,440 at 5 to 8 rows, 131,072 at 3 and 4, 548,864 at one.
+constexpr size_t FEW_SMEM_MOST = 200 * 1024;
+constexpr int few_registers(int rows) { return rows <= 2 ? rows : rows <= 4 ? 4 : rows <= 8 ? 8 : 16; }      // MB of `rows` rows
+inline bool few_fits(int rows, long long row_blocks, int nc) {
+    const int mb = few_registers(rows), q = few_chunks(rows, mb, row_blocks, nc);
+    return few_smem(mb, q < nc ? q : nc) <= FEW_SMEM_MOST;
+}
 
 // GLU: W is [gate; up] ([2N, K]); the block's 64 weight rows are 32 of each half, of the same features, and C[m, n] =
 // silu(gate) * up. The sums and the activation are those of the product and the activation kernel behind one another, to the bit; a
@@ -225,7 +232,7 @@ int launch_few(const float* A, long long lda, const float* W, long long ldw, flo
     constexpr int RN = few_rows_a_lane(MB), NS = few_stages(MB), FEATS = GLU ? FEW_N / 2 : FEW_N;
     const int nc = (K + CHUNK - 1) / CHUNK, q = few_chunks(M, MB, (N + FEATS - 1) / FEATS, nc), c = (nc + q - 1) / q;
     size_t smem = few_smem(MB, min(q, nc));
-    if (smem > 200 * 1024) return VOB_ERR_UNSUPPORTED;
+    if (smem > FEW_SMEM_MOST) return VOB_ERR_UNSUPPORTED;
     auto kernel = gemm_f32_few_kernel<MB, RN, NS, GLU>;
     cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return (int)e;
@@ -436,9 +443,7 @@ int few(const float* A, long long lda, const float* W, long long ldw, float* C, 
 // Whether vob_gemm_f32_swiglu takes a product of these sizes (then it is also the faster way).
 VOB_EXPORT int vob_gemm_f32_swiglu_supported(int M, int I, int K) {
     if (M <= 0 || I <= 0 || K <= 0 || K % 4 != 0 || M > 8 || !few_rows(M, K)) return 0;      // 12 rows: 1 % slower in a whole step
-    int nc = (K + CHUNK - 1) / CHUNK, mb = M <= 2 ? M : M <= 4 ? 4 : 8;
-    int q = few_chunks(M, mb, (I + FEW_N / 2 - 1) / (FEW_N / 2), nc);
-    return few_smem(mb, q < nc ? q : nc) <= 200 * 1024;
+    return few_fits(M, (I + FEW_N / 2 - 1) / (FEW_N / 2), (K + CHUNK - 1) / CHUNK);
 }
 
 // C[M, I] = silu(A Wg^T) * (A Wu^T), W = [Wg; Wu] of shape [2I, K], few rows; the bits of vob_gemm_f32 and vob_swiglu one behind the other.
@@ -473,7 +478,7 @@ VOB_EXPORT int vob_gemm_f32(const float* A, long long lda, const float* W, long 
     // 52, 52, 52 (58 at 25 rows); 4,096 x 14,336 at 9, 16, 17 rows 109, 133, 175 / 163; 16,384 x 4,608 131, 163, 211 / 213. Larger matrices
     // come from memory every time: 8,192 x 28,672 at 16 rows 776 / 629. A decode step of 12 requests at 1B sizes 3,590 -> 2,660 us.
     const double w_bytes = 4.0 * N * K;
-    if (vec && M > 8 && nc > 32 && (M <= 16 ? w_bytes <= 320e6 : M <= 24 && w_bytes <= 70e6)) {
+    if (vec && M > 8 && nc > 32 && (M <= 16 ? w_bytes <= 320e6 : M <= 24 && w_bytes <= 70e6) && few_fits(8, (N + FEW_N - 1) / FEW_N, nc)) {
         for (int m = 0; m < M; m += 8) {
             int e = few<false>(A + (size_t)m * lda, lda, W, ldw, C + (size_t)m * ldc, ldc, min(8, M - m), N, K, bias, early, stream);
             if (e) return e;
