@@ -958,6 +958,26 @@ def test_gemm_f32_few_rows_chunks_of_a_block(N, Kd):
         assert torch.equal(out, want[:M]), M
 
 
+def test_gemm_f32_few_rows_stages():
+    """Three and four rows have a ring of three stages where the grid fills at most two waves (two cost up to a quarter of the time),
+    and two where it has more or where a block adds up more than an eighth of K; all give the bits of the tiles."""
+    from vllm_oxide_b200 import kernels
+    plan = kernels._fn("gemm_f32", "vob_gemm_f32_few_plan", [kernels._I] * 4)
+    for M in (3, 4):
+        for N, Kd, stages in ((3072, 1024, 3), (1024, 8960, 3), (896, 14336, 3), (500, 516, 3), (49152, 1280, 2), (16384, 2048, 2)):
+            assert plan(M, N, Kd, 64) % 8 == stages, (M, N, Kd)
+    assert {plan(M, 3072, 1024, 64) % 8 for M in (1, 2, 5, 8, 9, 16)} == {2}
+    g = torch.Generator().manual_seed(3)
+    for N, Kd in ((3072, 1024), (897, 14336), (500, 516), (9000, 1280)):
+        a, w = torch.randn(40, Kd, generator=g).to(DEV), torch.randn(N, Kd, generator=g).to(DEV)
+        want = torch.empty(40, N, device=DEV)
+        kernels.gemm_f32(a, w, want)
+        for M in (3, 4):
+            out = torch.full((M, N), 7.0, device=DEV)
+            kernels.gemm_f32(a[:M], w, out)
+            assert torch.equal(out, want[:M]), (M, N, Kd)
+
+
 @pytest.mark.parametrize("N,Kd", [(70, 53252), (70, 61440), (70, 61444), (33, 65536), (1024, 65536)])
 def test_gemm_f32_few_rows_of_a_k_without_room(N, Kd):
     """A K whose chunks' sums find no room in a block of the few-row kernel goes to the tiles, rows taken eight at a time too: the

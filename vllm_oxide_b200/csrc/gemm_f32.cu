@@ -64,29 +64,38 @@ constexpr int FEW_N = 64, FEW_K = 32;                 // weight rows of a block,
 constexpr int few_rows_a_lane(int mb) { return mb <= 4 ? 1 : 2; }
 // three blocks an SM (two from three rows of A on) for four chunks a block
 __host__ __device__ constexpr int few_blocks(int mb) { return mb <= 2 ? 3 : 2; }
-constexpr int few_stages(int) { return 2; }
 // Shared memory of a block that adds up `chunks` chunks: its warps' rings, x of four chunks, the chunks' sums.
-constexpr size_t few_smem(int mb, int chunks) { return sizeof(float) * (size_t)(8 * few_stages(mb) * 32 * FEW_K + 4 * CHUNK * mb + chunks * mb * FEW_N); }
-// Chunks of a block, a multiple of four: an eighth of K at least (a cluster holds eight blocks); all of it, half of it or, with one or two
-// rows, a quarter, where 256 blocks are left and two of them find room on an SM. A block's start, its cluster's meeting and its end cost as much as
-// four chunks of weights do. Cold, back to back, us with an eighth (and three stages for three and four rows, as it was) / now, 1, 4 and 8 rows:
-// 16,384 x 2,048 26.5, 35, 38 / 23.7, 25.6, 29.5; 128,256 x 2,048 162, 233, 255 / 151, 164, 202; 28,672 x 4,096 91, 131, 142 / 82, 94, 111. Three
-// blocks to a K of 32 chunks (6,144 x 4,096) lose from three rows on: 32.5 / 39 at eight.
-inline int few_chunks(int rows, int mb, long long row_blocks, int nc) {
-    const int least = ((nc + 7) / 8 + 3) / 4 * 4;
-    if (mb > 8) return least;
-    for (int c = 1; c <= (rows <= 2 ? 4 : 2); c *= 2) {
-        const int q = (nc + c - 1) / c;
-        if (q > least && q % 4 == 0 && nc % q == 0 && row_blocks * c >= 256 && few_smem(mb, q) <= 112 * 1024) return q;
-    }
-    return least;
+constexpr size_t few_smem(int mb, int chunks, int stages) {
+    return sizeof(float) * (size_t)(8 * stages * 32 * FEW_K + 4 * CHUNK * mb + chunks * mb * FEW_N);
 }
-// Whether a block finds room for its chunks' sums: it does up to K = 61,440 at 5 to 8 rows, 131,072 at 3 and 4, 548,864 at one.
 constexpr size_t FEW_SMEM_MOST = 200 * 1024;
 constexpr int few_registers(int rows) { return rows <= 2 ? rows : rows <= 4 ? 4 : rows <= 8 ? 8 : 16; }      // MB of `rows` rows
+
+// Chunks of a block, a multiple of four: an eighth of K at least (a cluster holds eight blocks); all of it, half of it or, with one or two
+// rows, a quarter, where 256 blocks are left and two of them find room on an SM. A block's start, its cluster's meeting and its end cost as much as
+// four chunks of weights do. Cold, back to back, us with an eighth / now, 1, 4 and 8 rows: 16,384 x 2,048 26.5, 35, 38 / 23.7, 25.6, 29.5;
+// 128,256 x 2,048 162, 233, 255 / 151, 164, 202; 28,672 x 4,096 91, 131, 142 / 82, 94, 111. Three blocks to a K of 32 chunks (6,144 x 4,096)
+// lose from three rows on: 32.5 / 39 at eight.
+//
+// Stages of a warp's ring: two, and three for three and four rows whose blocks did not get longer and fill at most two waves: there a warp's
+// latency is not hidden by others. Three / two, us, 4 rows: 3,072 x 1,024 5.5 / 6.2, 1,024 x 8,960 16.1 / 19.6, 896 x 14,336 22 / 27; many
+// waves 49,152 x 1,280 67.3 / 65.1. One and two rows have three blocks an SM, five and more a lane's two rows: two stages there.
+struct FewPlan { int chunks, stages; };
+inline FewPlan few_plan(int rows, long long row_blocks, int nc) {
+    const int least = ((nc + 7) / 8 + 3) / 4 * 4, mb = few_registers(rows);
+    if (mb > 8) return {least, 2};
+    for (int c = 1; c <= (rows <= 2 ? 4 : 2); c *= 2) {
+        const int q = (nc + c - 1) / c;
+        if (q > least && q % 4 == 0 && nc % q == 0 && row_blocks * c >= 256 && few_smem(mb, q, 2) <= 112 * 1024) return {q, 2};
+    }
+    const long long blocks = row_blocks * ((nc + least - 1) / least);
+    const bool deep = mb == 4 && blocks <= 2 * 148 * few_blocks(mb) && few_smem(mb, least < nc ? least : nc, 3) <= FEW_SMEM_MOST;
+    return {least, deep ? 3 : 2};
+}
+// Whether a block finds room for its chunks' sums: it does up to K = 61,440 at 5 to 8 rows, 131,072 at 3 and 4, 548,864 at one.
 inline bool few_fits(int rows, long long row_blocks, int nc) {
-    const int mb = few_registers(rows), q = few_chunks(rows, mb, row_blocks, nc);
-    return few_smem(mb, q < nc ? q : nc) <= FEW_SMEM_MOST;
+    const FewPlan p = few_plan(rows, row_blocks, nc);
+    return few_smem(few_registers(rows), p.chunks < nc ? p.chunks : nc, p.stages) <= FEW_SMEM_MOST;
 }
 
 // GLU: W is [gate; up] ([2N, K]); the block's 64 weight rows are 32 of each half, of the same features, and C[m, n] =
@@ -226,12 +235,12 @@ gemm_f32_few_kernel(const float* __restrict__ A, long long lda, const float* __r
     if (c > 1) { cluster_arrive(); cluster_wait(); }  // peers have read this block's sums
 }
 
-template <int MB, bool GLU>
+template <int MB, int NS, bool GLU>
 int launch_few(const float* A, long long lda, const float* W, long long ldw, float* C, long long ldc, int M, int N, int K,
-               const float* bias, int early, cudaStream_t stream) {
-    constexpr int RN = few_rows_a_lane(MB), NS = few_stages(MB), FEATS = GLU ? FEW_N / 2 : FEW_N;
-    const int nc = (K + CHUNK - 1) / CHUNK, q = few_chunks(M, MB, (N + FEATS - 1) / FEATS, nc), c = (nc + q - 1) / q;
-    size_t smem = few_smem(MB, min(q, nc));
+               const float* bias, int q, int early, cudaStream_t stream) {
+    constexpr int RN = few_rows_a_lane(MB), FEATS = GLU ? FEW_N / 2 : FEW_N;
+    const int nc = (K + CHUNK - 1) / CHUNK, c = (nc + q - 1) / q;
+    size_t smem = few_smem(MB, min(q, nc), NS);
     if (smem > FEW_SMEM_MOST) return VOB_ERR_UNSUPPORTED;
     auto kernel = gemm_f32_few_kernel<MB, RN, NS, GLU>;
     cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
@@ -430,12 +439,16 @@ bool few_rows(int M, int K) {
 template <bool GLU>
 int few(const float* A, long long lda, const float* W, long long ldw, float* C, long long ldc, int M, int N, int K, const float* bias,
         int early, cudaStream_t stream) {
+    constexpr int FEATS = GLU ? FEW_N / 2 : FEW_N;
+    const FewPlan p = few_plan(M, (N + FEATS - 1) / FEATS, (K + CHUNK - 1) / CHUNK);
+    const int q = p.chunks;
     if constexpr (!GLU)
-        if (M > 8) return launch_few<16, GLU>(A, lda, W, ldw, C, ldc, M, N, K, bias, early, stream);
-    return M == 1   ? launch_few<1, GLU>(A, lda, W, ldw, C, ldc, M, N, K, bias, early, stream)
-           : M == 2 ? launch_few<2, GLU>(A, lda, W, ldw, C, ldc, M, N, K, bias, early, stream)
-           : M <= 4 ? launch_few<4, GLU>(A, lda, W, ldw, C, ldc, M, N, K, bias, early, stream)
-                    : launch_few<8, GLU>(A, lda, W, ldw, C, ldc, M, N, K, bias, early, stream);
+        if (M > 8) return launch_few<16, 2, GLU>(A, lda, W, ldw, C, ldc, M, N, K, bias, q, early, stream);
+    return M == 1          ? launch_few<1, 2, GLU>(A, lda, W, ldw, C, ldc, M, N, K, bias, q, early, stream)
+           : M == 2        ? launch_few<2, 2, GLU>(A, lda, W, ldw, C, ldc, M, N, K, bias, q, early, stream)
+           : M > 4         ? launch_few<8, 2, GLU>(A, lda, W, ldw, C, ldc, M, N, K, bias, q, early, stream)
+           : p.stages == 3 ? launch_few<4, 3, GLU>(A, lda, W, ldw, C, ldc, M, N, K, bias, q, early, stream)
+                           : launch_few<4, 2, GLU>(A, lda, W, ldw, C, ldc, M, N, K, bias, q, early, stream);
 }
 
 }  // namespace
@@ -453,6 +466,13 @@ VOB_EXPORT int vob_gemm_f32_swiglu(const float* A, long long lda, const float* W
     if (K <= 0 || lda < K || ldw < K || ldc < I) return VOB_ERR_BAD_ARG;
     if (!vob_gemm_f32_swiglu_supported(M, I, K) || lda % 4 || ldw % 4 || ((uintptr_t)A & 15) || ((uintptr_t)W & 15)) return VOB_ERR_UNSUPPORTED;
     return few<true>(A, lda, W, ldw, C, ldc, M, I, K, nullptr, early, stream);
+}
+
+// For tests: 8 * chunks of a block + stages of a ring of the few-row kernel (`features`: 64 a block, 32 with the activation in the epilogue).
+VOB_EXPORT int vob_gemm_f32_few_plan(int rows, int N, int K, int features) {
+    if (rows < 1 || rows > 16 || N < 1 || K < 1 || (features != FEW_N && features != FEW_N / 2)) return 0;
+    const FewPlan p = few_plan(rows, (N + features - 1) / features, (K + CHUNK - 1) / CHUNK);
+    return 8 * p.chunks + p.stages;
 }
 
 // `bias` (N entries, may be null) is added to every row after the sum over k. `early`: W holds weights, which no kernel writes, and
