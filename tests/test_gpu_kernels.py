@@ -978,6 +978,35 @@ def test_gemm_f32_few_rows_stages():
             assert torch.equal(out, want[:M]), (M, N, Kd)
 
 
+def test_gemm_f32_few_rows_waves():
+    """A block of the few-row kernel takes more than an eighth of K only where its waves of blocks are at least 0.7 full (sizes just above one
+    wave lost up to a fifth); wherever it is cut, a row has the bits it has in the tiles."""
+    from vllm_oxide_b200 import kernels
+    plan = kernels._fn("gemm_f32", "vob_gemm_f32_few_plan", [kernels._I] * 4)
+    longer = 0
+    for N in list(range(64, 34000, 1088)) + [6144, 11008, 16384, 22016, 28672, 128256]:
+        for Kd in (516, 2048, 2560, 4096, 8192, 14336):
+            for M in range(1, 9):
+                nc = -(-Kd // 128)
+                q, mb = plan(M, N, Kd, 64) // 8, M if M <= 2 else 4 if M <= 4 else 8
+                if q == ((nc + 7) // 8 + 3) // 4 * 4:
+                    continue
+                smem = 4 * (8 * 2 * 32 * 32 + 4 * 128 * mb + q * mb * 64)
+                waves = -(-N // 64) * -(-nc // q) / (148 * min(3 if mb <= 2 else 2, 227 * 1024 // (smem + 1024)))
+                assert waves <= 1 or waves >= 0.7 * math.ceil(waves), (N, Kd, M, q)
+                longer += 1
+    assert longer > 100 and plan(2, 6144, 8192, 64) // 8 == 8 and plan(1, 16384, 2048, 64) // 8 == 16
+    g = torch.Generator().manual_seed(4)
+    for N, Kd in ((6144, 4096), (11008, 2048), (22016, 1280)):
+        a, w = torch.randn(40, Kd, generator=g).to(DEV), torch.randn(N, Kd, generator=g).to(DEV)
+        want = torch.empty(40, N, device=DEV)
+        kernels.gemm_f32(a, w, want)
+        for M in (1, 2, 4, 8):
+            out = torch.full((M, N), 7.0, device=DEV)
+            kernels.gemm_f32(a[:M], w, out)
+            assert torch.equal(out, want[:M]), (M, N, Kd)
+
+
 @pytest.mark.parametrize("N,Kd", [(70, 53252), (70, 61440), (70, 61444), (33, 65536), (1024, 65536)])
 def test_gemm_f32_few_rows_of_a_k_without_room(N, Kd):
     """A K whose chunks' sums find no room in a block of the few-row kernel goes to the tiles, rows taken eight at a time too: the

@@ -18,6 +18,7 @@
 // Both multiply and add pairs of k in one instruction (fma.rn.f32x2, each half rounded as fmaf rounds it): single FMAs
 // reach half the rate on this GPU (a tile kernel of 8 x 8 outputs a thread: 37 TFLOP/s with fmaf).
 #include "common.cuh"
+#include <cmath>
 #include <cooperative_groups.h>
 VOB_PDL_SWITCH(gemm_f32)
 
@@ -75,18 +76,26 @@ constexpr int few_registers(int rows) { return rows <= 2 ? rows : rows <= 4 ? 4 
 // rows, a quarter, where 256 blocks are left and two of them find room on an SM. A block's start, its cluster's meeting and its end cost as much as
 // four chunks of weights do. Cold, back to back, us with an eighth / now, 1, 4 and 8 rows: 16,384 x 2,048 26.5, 35, 38 / 23.7, 25.6, 29.5;
 // 128,256 x 2,048 162, 233, 255 / 151, 164, 202; 28,672 x 4,096 91, 131, 142 / 82, 94, 111. Three blocks to a K of 32 chunks (6,144 x 4,096)
-// lose from three rows on: 32.5 / 39 at eight.
+// lose from three rows on: 32.5 / 39 at eight. A last wave that is nearly empty takes back more than that: where the longer blocks would fill less
+// than 0.7 of their waves K stays in eighths, or in the next smaller part (two rows, us, eighths / longer: 6,144 x 8,192, 1.3 waves, 39.3 / 46.5;
+// 11,008 x 8,192, 1.2 waves of halves, 72.4 / 80.6; 22,016 x 2,560, 1.2 waves, 44.1 / 47.8; at 0.7 to 0.8 equal within 2 %).
 //
 // Stages of a warp's ring: two, and three for three and four rows whose blocks did not get longer and fill at most two waves: there a warp's
 // latency is not hidden by others. Three / two, us, 4 rows: 3,072 x 1,024 5.5 / 6.2, 1,024 x 8,960 16.1 / 19.6, 896 x 14,336 22 / 27; many
 // waves 49,152 x 1,280 67.3 / 65.1. One and two rows have three blocks an SM, five and more a lane's two rows: two stages there.
 struct FewPlan { int chunks, stages; };
+inline double few_waves(int mb, int chunks, long long blocks) {        // on 148 SMs
+    const int room = (int)(227 * 1024 / (few_smem(mb, chunks, 2) + 1024));
+    return (double)blocks / (148.0 * (room < few_blocks(mb) ? room : few_blocks(mb)));
+}
 inline FewPlan few_plan(int rows, long long row_blocks, int nc) {
     const int least = ((nc + 7) / 8 + 3) / 4 * 4, mb = few_registers(rows);
     if (mb > 8) return {least, 2};
     for (int c = 1; c <= (rows <= 2 ? 4 : 2); c *= 2) {
         const int q = (nc + c - 1) / c;
-        if (q > least && q % 4 == 0 && nc % q == 0 && row_blocks * c >= 256 && few_smem(mb, q, 2) <= 112 * 1024) return {q, 2};
+        if (q <= least || q % 4 != 0 || nc % q != 0 || row_blocks * c < 256 || few_smem(mb, q, 2) > 112 * 1024) continue;
+        const double waves = few_waves(mb, q, row_blocks * c);
+        if (waves <= 1.0 || waves >= 0.7 * std::ceil(waves)) return {q, 2};
     }
     const long long blocks = row_blocks * ((nc + least - 1) / least);
     const bool deep = mb == 4 && blocks <= 2 * 148 * few_blocks(mb) && few_smem(mb, least < nc ? least : nc, 3) <= FEW_SMEM_MOST;
