@@ -1007,6 +1007,24 @@ def test_gemm_f32_few_rows_waves():
             assert torch.equal(out, want[:M]), (M, N, Kd)
 
 
+@pytest.mark.parametrize("N,Kd", [(500, 4612), (500, 5120), (1024, 4100), (2048, 5000), (3200, 4100), (3204, 4100), (3072, 16512), (3076, 16388)])
+def test_gemm_f32_rows_by_eights(N, Kd):
+    """On both sides of the lines between rows taken eight at a time and the tiles: the bits of a product of 40 rows."""
+    from vllm_oxide_b200 import kernels
+    pieces = kernels._fn("gemm_f32", "vob_gemm_f32_launches", [kernels._I] * 3)
+    narrow = N < 1024 and Kd < 4993 or N > 3072 and Kd > 16384
+    g = torch.Generator().manual_seed(N + Kd)
+    a, w = torch.randn(40, Kd, generator=g).to(DEV), torch.randn(N, Kd, generator=g).to(DEV)
+    want = torch.empty(40, N, device=DEV)
+    kernels.gemm_f32(a, w, want)
+    for M in (8, 9, 16, 17, 24, 25):
+        by_eights = 8 < M <= 16 and not narrow or 16 < M <= 24 and 1536 <= N <= 3200 and 33e6 < 4 * N * Kd <= 70e6
+        assert pieces(M, N, Kd) == (-(-M // 8) if by_eights else 1), M
+        out = torch.full((M, N), 7.0, device=DEV)
+        kernels.gemm_f32(a[:M], w, out)
+        assert torch.equal(out, want[:M]), M
+
+
 @pytest.mark.parametrize("N,Kd", [(70, 53252), (70, 61440), (70, 61444), (33, 65536), (1024, 65536)])
 def test_gemm_f32_few_rows_of_a_k_without_room(N, Kd):
     """A K whose chunks' sums find no room in a block of the few-row kernel goes to the tiles, rows taken eight at a time too: the

@@ -445,6 +445,21 @@ bool few_rows(int M, int K) {
     return M <= (K <= 64 ? 4 : 8) || (M <= 16 && q == 4 && nc > 1);
 }
 
+// More than 32 chunks and 9 to 24 rows: whether eight rows at a time are faster than the tiles. (A block of 16 rows would have its SM to itself
+// there.) Cold, back to back, us in eights / in tiles of 32 rows with K shared, at 9, 16, 17 and 24 rows: 2,048 x 8,192 33, 36, 50, 53 / 86 to 87;
+// 8,192 x 8,192, whose weights come from memory every time, 116, 146, 189, 218 / 184; 500 x 5,120 19, 23, 30, 33 / 23. Three eights gain only
+// where the tiles are at their worst, with 24 to 50 clusters of eight blocks, and where L2 keeps the weights: 1,024 x 6,144 at 17 and 24 rows 42, 46 /
+// 46 (39 with the weights in L2), 3,072 x 6,144 70, 85 / 71. Under 40 chunks the last block of a K has little to do, and a narrow N goes to
+// the tiles (500 x 4,612 at 16 rows 24.6 / 23.0); beyond 128 a block of eight rows has its SM to itself (3,584 x 18,944 at 16 rows 245 / 218,
+// 2,560 x 18,944 0.86 of the tiles' time). A decode step of 12 requests at 1B sizes 3,590 -> 2,660 us.
+bool by_eights(int M, int N, int K) {
+    const int nc = (K + CHUNK - 1) / CHUNK;
+    const double w_bytes = 4.0 * N * K;
+    if (M <= 8 || M > 24 || nc <= 32 || !few_fits(8, (N + FEW_N - 1) / FEW_N, nc)) return false;
+    if (M <= 16) return w_bytes <= 320e6 && (nc >= 40 || N >= 1024) && (nc <= 128 || N <= 3072);
+    return N >= 1536 && N <= 3200 && w_bytes > 33e6 && w_bytes <= 70e6;
+}
+
 template <bool GLU>
 int few(const float* A, long long lda, const float* W, long long ldw, float* C, long long ldc, int M, int N, int K, const float* bias,
         int early, cudaStream_t stream) {
@@ -484,6 +499,9 @@ VOB_EXPORT int vob_gemm_f32_few_plan(int rows, int N, int K, int features) {
     return 8 * p.chunks + p.stages;
 }
 
+// Kernels that a product of these sizes takes (operands that come by 16 bytes).
+VOB_EXPORT int vob_gemm_f32_launches(int M, int N, int K) { return M > 0 && N > 0 && K > 0 && K % 4 == 0 && by_eights(M, N, K) ? (M + 7) / 8 : 1; }
+
 // `bias` (N entries, may be null) is added to every row after the sum over k. `early`: W holds weights, which no kernel writes, and
 // may be read while the kernels in front still run.
 VOB_EXPORT int vob_gemm_f32(const float* A, long long lda, const float* W, long long ldw, float* C,
@@ -494,20 +512,14 @@ VOB_EXPORT int vob_gemm_f32(const float* A, long long lda, const float* W, long 
     int nc = (K + CHUNK - 1) / CHUNK;
     int vec = K % 4 == 0 && lda % 4 == 0 && ldw % 4 == 0 && ((uintptr_t)A & 15) == 0 && ((uintptr_t)W & 15) == 0;
     // 16 rows: what a lane's registers hold. Cold, 9 to 16 rows, us here / in tiles (32 rows at least): 2,048 x 512 16 / 23, 2,048 x 2,048
-    // 19 / 21, 4,096 x 4,096 41 / 55, 16,384 x 2,048 68 / 94, 128,256 x 2,048 391 / 644; where K has more than 32 chunks a block of 16
-    // rows has its SM to itself, and the tiles win: 2,048 x 8,192 66 / 57, 4,096 x 14,336 209 / 170 (see below). Up to 8 rows the tiles never do: there
-    // 29 / 57 and 83 / 169 at 8 rows, 25 / 57 and 70 / 170 at one. A single chunk is too short for what a block of 5 rows and more sets
+    // 19 / 21, 4,096 x 4,096 41 / 55, 16,384 x 2,048 68 / 94, 128,256 x 2,048 391 / 644; where K has more than 32 chunks see
+    // `by_eights`. Up to 8 rows the tiles never win: 2,048 x 8,192 in 32 rows of a tile 86, here 18 at eight rows. A single chunk is too short for what a block of 5 rows and more sets
     // up (back to back, 16 rows: 64 x 64 7.3 / 2.9, 2,048 x 64 7.7 / 3.1, 128 x 128 7.5 / 4.7; 8 rows 4.4 / 2.9, 4.6 / 3.1, 4.5 / 4.7).
     if (vec && few_rows(M, K)) {
         int e = few<false>(A, lda, W, ldw, C, ldc, M, N, K, bias, early, stream);
         if (e != VOB_ERR_UNSUPPORTED) return e;       // a K whose sums find no room in shared memory: tiles
     }
-    // More than 32 chunks, where a block of 16 rows would have its SM to itself: eight rows at a time, which find most of the weights in L2
-    // from the second eight on. Cold, us in eights / in tiles: 2,048 x 8,192 at 9, 16, 24 rows 32, 36, 53 / 87, 87, 85; 1,024 x 6,144 26, 31, 47 /
-    // 52, 52, 52 (58 at 25 rows); 4,096 x 14,336 at 9, 16, 17 rows 109, 133, 175 / 163; 16,384 x 4,608 131, 163, 211 / 213. Larger matrices
-    // come from memory every time: 8,192 x 28,672 at 16 rows 776 / 629. A decode step of 12 requests at 1B sizes 3,590 -> 2,660 us.
-    const double w_bytes = 4.0 * N * K;
-    if (vec && M > 8 && nc > 32 && (M <= 16 ? w_bytes <= 320e6 : M <= 24 && w_bytes <= 70e6) && few_fits(8, (N + FEW_N - 1) / FEW_N, nc)) {
+    if (vec && by_eights(M, N, K)) {
         for (int m = 0; m < M; m += 8) {
             int e = few<false>(A + (size_t)m * lda, lda, W, ldw, C + (size_t)m * ldc, ldc, min(8, M - m), N, K, bias, early, stream);
             if (e) return e;
