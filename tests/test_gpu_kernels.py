@@ -1009,7 +1009,8 @@ def test_gemm_f32_few_rows_waves():
 
 @pytest.mark.parametrize("N,Kd", [(500, 4612), (500, 5120), (1024, 4100), (2048, 5000), (3200, 4100), (3204, 4100), (3072, 16512), (3076, 16388)])
 def test_gemm_f32_rows_by_eights(N, Kd):
-    """On both sides of the lines between rows taken eight at a time and the tiles: the bits of a product of 40 rows."""
+    """On both sides of the lines between rows taken eight at a time and the tiles: the bits of a product of 40 rows, and as many launches
+    counted as there are."""
     from vllm_oxide_b200 import kernels
     pieces = kernels._fn("gemm_f32", "vob_gemm_f32_launches", [kernels._I] * 3)
     narrow = N < 1024 and Kd < 4993 or N > 3072 and Kd > 16384
@@ -1021,7 +1022,9 @@ def test_gemm_f32_rows_by_eights(N, Kd):
         by_eights = 8 < M <= 16 and not narrow or 16 < M <= 24 and 1536 <= N <= 3200 and 33e6 < 4 * N * Kd <= 70e6
         assert pieces(M, N, Kd) == (-(-M // 8) if by_eights else 1), M
         out = torch.full((M, N), 7.0, device=DEV)
+        before = kernels.launch_count()
         kernels.gemm_f32(a[:M], w, out)
+        assert kernels.launch_count() - before == pieces(M, N, Kd), M
         assert torch.equal(out, want[:M]), M
 
 

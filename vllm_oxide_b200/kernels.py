@@ -548,7 +548,10 @@ def gemm_f32(a: torch.Tensor, w: torch.Tensor, out: torch.Tensor, bias: Optional
     if bias is not None and (bias.dtype != torch.float32 or bias.shape != (N,) or not bias.is_contiguous()):
         raise ShapeError(op, f"bias must be contiguous float32 [{N}], got {bias.dtype} {list(bias.shape)}")
     f = _fn("gemm_f32", "vob_gemm_f32", [_P, _L, _P, _L, _P, _L, _I, _I, _I, _P, _I, _P])
-    _check(f(_ptr(a), a.stride(0), _ptr(w), w.stride(0), _ptr(out), out.stride(0), M, N, K, _ptr(bias), int(fixed_w), _stream()), op)
+    launches = 1
+    if 8 < M <= 24 and K > 4096 and not any(t.stride(0) % 4 or t.data_ptr() % 16 for t in (a, w)):
+        launches = _fn("gemm_f32", "vob_gemm_f32_launches", [_I, _I, _I])(M, N, K)         # rows may be taken eight at a time
+    _check(f(_ptr(a), a.stride(0), _ptr(w), w.stride(0), _ptr(out), out.stride(0), M, N, K, _ptr(bias), int(fixed_w), _stream()), op, launches)
 
 
 def gemm_f32_swiglu_supported(a: torch.Tensor, w_gate_up: torch.Tensor) -> bool:
