@@ -1117,6 +1117,23 @@ def test_gemm_sm100_pair(T, N, Kd, odt):
         assert torch.equal(sub, out[T - 2:])
 
 
+@pytest.mark.parametrize("odt", [torch.bfloat16, torch.float32], ids=["bf16out", "f32out"])
+@pytest.mark.parametrize("T,N,Kd,bn", [(513, 16392, 520, 192), (1000, 16384, 456, 256)])
+def test_gemm_sm100_pair_wide_token_tiles(T, N, Kd, bn, odt):
+    """The plain store with tiles of 192 and 256 tokens, several to a pair of SMs, and a ring that wraps."""
+    from vllm_oxide_b200 import kernels
+    assert kernels._fn("gemm_sm100_pair", "vob_gemm_sm100_pair_tokens", [kernels._I] * 4)(T, N, 0, 74) == bn
+    g = torch.Generator().manual_seed(T + N)
+    a = torch.randn(T, Kd, generator=g).to(torch.bfloat16).to(DEV)
+    w = torch.randn(N, Kd, generator=g).to(torch.bfloat16).to(DEV)
+    out = torch.full((T + 1, N), 7.0, dtype=odt, device=DEV)
+    kernels.gemm_sm100_pair(a, w, out[:T])
+    torch.cuda.synchronize()
+    kernels.gemm_sm100_check()
+    assert rel(out[:T], (a.double() @ w.double().t()).cpu()) <= (2.0 ** -8 if odt == torch.bfloat16 else max(2e-6, 2.0 ** -22 * math.sqrt(Kd)))
+    assert float((out[T:].float() - 7.0).abs().max()) == 0.0
+
+
 def test_gemm_sm100_pair_narrow_output_rows():
     """An output whose rows are not 16-byte aligned takes the element-wise store path."""
     g = torch.Generator().manual_seed(3)
@@ -1147,9 +1164,25 @@ def test_gemm_pair_swiglu(T, I, Kd):
     assert torch.equal(out, out2)
 
 
-@pytest.mark.parametrize("T,I,Kd,early", [(33, 8192, 64, True), (64, 128, 832, True), (100, 64, 704, False), (300, 8192, 72, True), (517, 4224, 128, False),
-                                          (600, 8192, 64, True), (1201, 640, 200, True)])
-def test_gemm_pair_swiglu_token_tiles(T, I, Kd, early):
+# tokens, features, K, weights asked for early, tokens of a tile on 74 pairs of SMs
+PAIR_TOKEN_TILES = [(33, 8192, 64, True, 64), (64, 128, 832, True, 32), (100, 64, 704, False, 32), (300, 8192, 72, True, 160), (517, 4224, 128, False, 160),
+                    (600, 8192, 64, True, 224), (1201, 640, 200, True, 96), (120, 9472, 712, True, 128), (350, 5632, 584, True, 128), (517, 8192, 520, True, 192),
+                    (600, 8192, 520, False, 224), (1000, 8192, 456, True, 256), (700, 14336, 456, False, 256)]
+
+
+def test_gemm_pair_token_tiles_are_all_tested():
+    from vllm_oxide_b200 import kernels
+    pick = kernels._fn("gemm_sm100_pair", "vob_gemm_sm100_pair_tokens", [kernels._I] * 4)
+    assert [pick(T, I, 1, 74) for T, I, *_ in PAIR_TOKEN_TILES] == [bn for *_, bn in PAIR_TOKEN_TILES]
+    assert {bn for *_, bn in PAIR_TOKEN_TILES} == {pick(T, I, 1, 74) for T in range(1, 2049, 3) for I in (64, 640, 1024, 2816, 4224, 5632, 8192, 9472, 14336)}
+    # several tiles a pair and more K blocks than the ring has stages (ten, or what 192 KB hold)
+    for bn in (128, 192, 224, 256):
+        assert any(b == bn and -(-T // b) * -(-I // 128) > 74 and -(-Kd // 64) > min(10, 196608 // (16384 + 64 * b))
+                   for T, I, Kd, _, b in PAIR_TOKEN_TILES), bn
+
+
+@pytest.mark.parametrize("T,I,Kd,early,bn", PAIR_TOKEN_TILES)
+def test_gemm_pair_swiglu_token_tiles(T, I, Kd, early, bn):
     """Token tiles of every width the launcher picks (32 to 256), more K blocks than a ring of ten stages holds, several tiles a
     pair of SMs; weights asked for before the kernels in front are done or behind them: the same bits."""
     g = torch.Generator().manual_seed(T * 3 + I)

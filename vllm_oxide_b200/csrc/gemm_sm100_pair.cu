@@ -442,6 +442,12 @@ VOB_EXPORT int vob_gemm_sm100_pair(const void* X, long long ldx, const void* W, 
                                : launch<__nv_bfloat16, PAIR_STORE>(mw, X, ldx, C, ldc, T, N, K, 0, err_flag, stream);
 }
 
+// For tests: tokens of a tile for T tokens and N output features (`swiglu`: gate and up of N features) on `pairs` pairs of SMs.
+VOB_EXPORT int vob_gemm_sm100_pair_tokens(int T, int N, int swiglu, int pairs) {
+    const int feats = swiglu ? BMH : 2 * BMH;
+    return T < 1 || N < 1 || pairs < 1 ? 0 : pick_tokens(T, (N + feats - 1) / feats, pairs);
+}
+
 // C[T, I] (bfloat16) = silu(X Wg^T) * (X Wu^T), W = [Wg; Wu] of shape [2I, K].
 VOB_EXPORT int vob_gemm_sm100_pair_swiglu(const void* X, long long ldx, const void* W, long long ldw, void* C, long long ldc,
                                           int T, int I, int K, int early, int* err_flag, cudaStream_t stream) {
