@@ -941,6 +941,37 @@ def test_gemm_fused_residual_and_folded_norm(T, N, Kd, splits):
     assert rel(out, want_delta) <= max(2e-6, 2.0 ** -22 * math.sqrt(Kd)) * 4
 
 
+@pytest.mark.parametrize("N,Kd,splits", [(640, 320, 5), (392, 1344, 6), (4096, 4096, 7), (512, 832, 7), (4096, 14336, 7)])
+@pytest.mark.parametrize("T", [1, 8, 16, 24, 32])
+def test_few_row_product_on_clusters_of_five_to_seven(T, N, Kd, splits):
+    """K shared by five, six and seven blocks, the last with less of it than the others: the residual epilogue and the plain one. Seven is what
+    4,096 features get."""
+    from vllm_oxide_b200.kernels import EPI_RESID
+    k = K()
+    if N == 4096:
+        assert k._pick_splits(T, N, Kd, torch.device("cuda", 0)) == splits
+    g = torch.Generator().manual_seed(T * 3 + N + Kd)
+    a = torch.randn(T, Kd, generator=g).to(torch.bfloat16).to(DEV)
+    w = (torch.randn(N, Kd, generator=g) / math.sqrt(Kd)).to(torch.bfloat16).to(DEV)
+    want = a.double() @ w.double().t()
+    tol = max(2e-6, 2.0 ** -22 * math.sqrt(Kd))
+    out = torch.full((T, N), 7.0, device=DEV)
+    k.gemm_sm100(a, w, out, splits)
+    assert rel(out, want.cpu()) <= tol
+    resid0, next_w = torch.randn(T, N, generator=g).to(DEV), (1.0 + 0.3 * torch.randn(N, generator=g)).to(DEV)
+    resid = resid0.clone()
+    xn_out = torch.full((T, N), 7.0, dtype=torch.bfloat16, device=DEV)
+    ssq_out = torch.full((-(-N // 128), 64), 7.0, device=DEV)
+    k.gemm_fused(a, w, None, EPI_RESID, N, resid=(resid, next_w, xn_out, ssq_out), splits=splits)
+    torch.cuda.synchronize()
+    k.gemm_sm100_check()
+    want_resid = resid0.double() + want
+    assert rel(resid, want_resid.cpu()) <= tol
+    assert rel(xn_out, (want_resid * next_w.double()).cpu()) <= 2 ** -8
+    for i in range(-(-N // 128)):
+        assert rel(ssq_out[i, :T], (resid.double()[:, i * 128:(i + 1) * 128] ** 2).sum(1).cpu()) <= 1e-5
+
+
 @pytest.mark.parametrize("N,Kd", [(16390, 2000), (16384, 1024), (8200, 4096), (4100, 8192), (500, 8200), (32777, 1536)])
 def test_gemm_f32_few_rows_chunks_of_a_block(N, Kd):
     """A block of the few-row kernel that has all, half or a quarter of K's chunks, and rows taken eight at a time: every count of rows
