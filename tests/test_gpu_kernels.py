@@ -1059,6 +1059,43 @@ def test_gemm_f32_rows_by_eights(N, Kd):
         assert torch.equal(out, want[:M]), M
 
 
+@pytest.mark.parametrize("N,Kd,M,tr,c", [
+    (65, 516, 17, 2, 1), (65, 1028, 17, 2, 8), (1541, 516, 65, 4, 1), (65, 1028, 177, 4, 8), (8201, 516, 65, 5, 1), (65, 1028, 300, 5, 8),
+    (4101, 516, 350, 6, 1), (65, 1028, 350, 6, 8), (3101, 516, 640, 7, 1), (501, 1028, 97, 7, 8), (8201, 516, 225, 8, 1), (501, 1028, 113, 8, 8),
+    (65, 130, 17, 2, 1), (65, 1030, 17, 2, 8), (1541, 130, 65, 4, 1), (65, 1030, 130, 4, 8), (1541, 130, 130, 5, 1), (65, 1030, 300, 5, 8),
+    (8201, 130, 81, 6, 1), (65, 1030, 350, 6, 8), (3101, 130, 640, 7, 1), (65, 1030, 640, 7, 8), (12301, 130, 350, 8, 1), (501, 1030, 113, 8, 8)])
+def test_gemm_f32_tile_choice(N, Kd, M, tr, c):
+    """Every tile height with and without a shared K, operands that come by 16 and by 4 bytes: the choice that the rule makes at these sizes, and the
+    bits that the few-row kernel or, where operands come by 4 bytes, tiles of 32 rows give."""
+    from vllm_oxide_b200 import kernels
+    choice = kernels._fn("gemm_f32", "vob_gemm_f32_tile", [kernels._I] * 4)
+    assert divmod(choice(M, N, Kd, int(Kd % 4 == 0)), 16) == (tr, c)
+    g = torch.Generator().manual_seed(N + Kd + M)
+    a, w = torch.randn(M, Kd, generator=g).to(DEV), torch.randn(N, Kd, generator=g).to(DEV)
+    want = torch.empty(M, N, device=DEV)
+    for r in range(0, M, 8):
+        kernels.gemm_f32(a[r:r + 8], w, want[r:r + 8])
+    assert rel(want, (a.double() @ w.double().t()).cpu()) <= 2.0 ** -22 * math.sqrt(Kd)
+    out = torch.full((M + 1, N), 7.0, device=DEV)
+    kernels.gemm_f32(a, w, out[:M])
+    assert torch.equal(out[:M], want)
+    assert float((out[M:] - 7.0).abs().max()) == 0.0
+
+
+def test_gemm_f32_tiles_of_an_idle_chip():
+    """Where every tile has an SM to itself the smallest tiles are the fastest, whatever rows of them are not there (higher ones, chosen by their
+    waves alone, took half as long again)."""
+    from vllm_oxide_b200 import kernels
+    choice = kernels._fn("gemm_f32", "vob_gemm_f32_tile", [kernels._I] * 4)
+    for M in (17, 33, 65, 72, 81, 97, 130, 160, 260, 400, 700, 1000, 2048):
+        for N in (1, 64, 200, 500, 1000, 2048):
+            tiles = -(-M // 32) * -(-N // 64)
+            if tiles <= 48:
+                assert all(choice(M, N, Kd, v) // 16 == 2 for Kd in (128, 516, 892) for v in (0, 1)), (M, N)
+            if tiles <= 8:
+                assert all(choice(M, N, Kd, 1) == 2 * 16 + 8 for Kd in (1024, 2048, 8192)), (M, N)
+
+
 @pytest.mark.parametrize("N,Kd", [(70, 53252), (70, 61440), (70, 61444), (33, 65536), (1024, 65536)])
 def test_gemm_f32_few_rows_of_a_k_without_room(N, Kd):
     """A K whose chunks' sums find no room in a block of the few-row kernel goes to the tiles, rows taken eight at a time too: the

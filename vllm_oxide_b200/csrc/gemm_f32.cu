@@ -439,6 +439,48 @@ int launch_tile(const float* A, long long lda, const float* W, long long ldw, fl
     return e != cudaSuccess ? (int)e : vob_launch_status();
 }
 
+// Tiles of 128, 112, 96, 80, 64 or 32 rows, a block or eight to a tile: the choice whose estimated time is least. The table holds us per chunk of K.
+// One block to a tile: for grids of at most 48 and 74 blocks, which find an SM each beside their neighbours', for 1, 2, 3 and 4 blocks on the fullest of
+// 148 SMs, and per block beyond. Eight to a tile, a segment of K each: for at most 4, 6, 8, 10, 12, 15, 23, 32, 42, 48 and 64 clusters, and per 16
+// clusters beyond. `by4`: how much longer both take where operands come by 4 bytes. What is added is a block's start and the cluster's sums. In
+// the long run a row costs alike at 64 rows and more (0.93 to 1.03 us a chunk, 16 rows and SM), 1.36 at 32: rows that are not there, waves and
+// idle SMs decide.
+// The numbers are fitted to 3,125 sizes (N 64 to 32,000, K 96 to 14,336, 17 to 4,096 rows), where every height with and without a shared K was timed
+// twice: back to back, and with another kernel in between, which places small grids otherwise. Over both the choice takes 1.015 and 1.034 of the
+// best one's time on average; 128, 64 and 32 rows by rows and waves took 1.10 and 1.13, all six by rows and waves 1.09 and 1.10. Against those three
+// heights 24 and 15 sizes lose more than 2 %, all but a few of small grids. us, those three / now: 64 x 516 at 160 rows 17.5 / 17.5, 3,072 x 516 at 81
+// 32.4 / 32.4, 16,384 x 2,048 at 72, 300, 450 and 2,048 rows 242, 563, 941, 3,262 / 170, 563, 799, 3,262; 2,048 x 8,192 at 97 and 450 126, 494 /
+// 115, 494; 8,192 x 4,096 at 300 610 / 610; 2,048 x 2,050 at 260 159 / 140.
+struct TilePick { int tr, c; };
+TilePick pick_tile(int M, int N, int K, bool vec) {
+    static const struct { int tr; float one[7], shared[12], by4[2]; } times[] = {
+        {2, {3.57f, 4.51f, 7.15f, 7.67f, 10.0f, 11.2f, 2.73f}, {4.66f, 3.76f, 4.65f, 5.16f, 6.28f, 6.25f, 9.21f, 11.2f, 9.7f, 12.3f, 11.9f, 2.38f}, {1.52f, 1.4f}},
+        {4, {5.24f, 5.91f, 10.3f, 11.5f, 12.8f, 16.8f, 3.87f}, {5.39f, 5.16f, 5.68f, 9.14f, 8.9f, 9.39f, 12.6f, 12.2f, 10.6f, 12.3f, 18.3f, 3.69f}, {1.4f, 1.28f}},
+        {5, {8.48f, 7.85f, 8.05f, 10.3f, 15.4f, 19.5f, 5.13f}, {6.0f, 7.22f, 7.23f, 7.99f, 7.81f, 7.01f, 9.7f, 10.1f, 15.8f, 18.5f, 22.1f, 4.87f}, {1.27f, 1.24f}},
+        {6, {8.49f, 9.84f, 10.1f, 11.5f, 17.7f, 22.0f, 5.65f}, {7.05f, 9.26f, 7.99f, 8.95f, 9.27f, 10.5f, 13.4f, 12.3f, 18.8f, 22.8f, 26.3f, 5.67f}, {1.27f, 1.13f}},
+        {7, {8.07f, 9.7f, 11.2f, 13.6f, 20.7f, 26.2f, 6.75f}, {7.22f, 9.68f, 9.29f, 9.78f, 10.4f, 11.0f, 15.7f, 14.5f, 21.2f, 27.5f, 29.1f, 6.15f}, {1.32f, 1.13f}},
+        {8, {8.64f, 10.5f, 13.4f, 14.9f, 23.5f, 29.7f, 7.44f}, {8.76f, 9.88f, 9.67f, 12.6f, 11.4f, 13.1f, 15.5f, 16.3f, 23.5f, 28.6f, 31.4f, 6.72f}, {1.32f, 1.14f}}};
+    static const int clusters[] = {4, 6, 8, 10, 12, 15, 23, 32, 42, 48, 64};
+    const int nc = (K + CHUNK - 1) / CHUNK;
+    TilePick best = {8, 1};
+    double least = 1e300;
+    for (const auto& t : times) {
+        if (t.tr > 4 && t.tr < 8 && M <= 64) continue;
+        const long long tiles = ((long long)M + 16 * t.tr - 1) / (16 * t.tr) * ((N + TN - 1) / TN);
+        const long long per_sm = (tiles + 147) / 148;
+        const double chunk = tiles <= 48 ? t.one[0] : tiles <= 74 ? t.one[1] : per_sm <= 4 ? t.one[per_sm + 1] : t.one[6] * (double)per_sm;
+        const double one = chunk * (K / (double)CHUNK) * (vec ? 1.0 : t.by4[0]) + 1.5 + 0.13 * t.tr * (double)per_sm;
+        if (one < least) { least = one; best = {t.tr, 1}; }
+        if (nc < 8) continue;
+        int i = 0;
+        while (i < 11 && tiles > clusters[i]) ++i;
+        const double segment = i < 11 ? t.shared[i] : t.shared[11] * ((double)tiles / 16.0 + 0.7);
+        const double shared = segment * seg_chunks(nc) * (vec ? 1.0 : t.by4[1]) + 2.0 + 0.1 * t.tr * ((double)tiles / 16.0);
+        if (shared < least) { least = shared; best = {t.tr, 8}; }
+    }
+    return best;
+}
+
 // Whether the kernel for few rows is the faster one (see vob_gemm_f32).
 bool few_rows(int M, int K) {
     int nc = (K + CHUNK - 1) / CHUNK, q = ((nc + 7) / 8 + 3) / 4 * 4;
@@ -499,6 +541,13 @@ VOB_EXPORT int vob_gemm_f32_few_plan(int rows, int N, int K, int features) {
     return 8 * p.chunks + p.stages;
 }
 
+// For tests: 16 * a tile's rows / 16 + blocks that share its K.
+VOB_EXPORT int vob_gemm_f32_tile(int M, int N, int K, int vec) {
+    if (M < 1 || N < 1 || K < 1) return 0;
+    const TilePick t = pick_tile(M, N, K, vec != 0);
+    return 16 * t.tr + t.c;
+}
+
 // Kernels that a product of these sizes takes (operands that come by 16 bytes).
 VOB_EXPORT int vob_gemm_f32_launches(int M, int N, int K) { return M > 0 && N > 0 && K > 0 && K % 4 == 0 && by_eights(M, N, K) ? (M + 7) / 8 : 1; }
 
@@ -526,30 +575,13 @@ VOB_EXPORT int vob_gemm_f32(const float* A, long long lda, const float* W, long 
         }
         return 0;
     }
-    // Tiles of 128, 112, 96, 80, 64 or 32 rows, a block or eight to a tile: the one whose waves of blocks cost least. A wave's cost is its
-    // rows times its resident blocks; smaller tiles read more from shared memory per FMA (measured at 2,048 x 2,048 and
-    // 16,384 x 2,048: 1.15 and 1.5 times the time per row at 64 and 32 rows; the factors in between are set so that no size measured is
-    // slower than with 128, 64 and 32 alone). What 80, 96 and 112 save is rows that are not there: 16,384 x 2,048 at 70, 90, 100, 130, 400, 700
-    // rows 242, 245, 247, 378, 940, 1,407 us -> 175, 206, 227, 335, 827, 1,273; 2,048 x 8,192 124, 124, 125, 203, 492, 713 -> 87, 103, 115, 174, 414,
-    // 661; 64 rows, 180, 260 and 300, 1,000 to 2,048 as before. A shared K is added up over the cluster (dearer where operands come by 4
-    // bytes: 8,192 x 2,050 at 300 rows 579 us shared, 429 not). A grid that finds an SM of its own for every block beside the
-    // neighbouring kernel's costs half: 512 x 2,048 at 48 rows 13.7 us in 64 blocks of 64 rows, 21.6 in 128 of 32; 4,096 x 130 10.5 and 17.0.
-    int best_tr = 8, best_c = 1;
-    double best = 1e300;
-    static const struct { int tr; double per_row; } tiles[] = {{2, 1.5}, {4, 1.15}, {5, 1.15}, {6, 1.2}, {7, 1.08}, {8, 1.0}};
-    for (const auto& t : tiles)
-        for (int tr = t.tr, c = 1; c <= 8; c += 7) {
-            if ((c > 1 && nc < 8) || (tr > 4 && tr < 8 && M <= 64)) continue;
-            double slots = 148.0 * tile_blocks(tr), blocks = (double)((M + 16 * tr - 1) / (16 * tr)) * ((N + TN - 1) / TN) * c;
-            double waves = (double)(long long)((blocks + slots - 1) / slots);
-            if (tr < 8 && blocks <= 74) waves = 0.5;
-            double cost = waves * tile_blocks(tr) * tr * t.per_row / c * (c == 1 ? 1.0 : vec ? 1.1 : 1.4);
-            if (cost < best) { best = cost; best_tr = tr; best_c = c; }
-        }
-    if (best_tr == 8) return launch_tile<8>(A, lda, W, ldw, C, ldc, M, N, K, bias, nc, best_c, vec, stream);
-    if (best_tr == 7) return launch_tile<7>(A, lda, W, ldw, C, ldc, M, N, K, bias, nc, best_c, vec, stream);
-    if (best_tr == 6) return launch_tile<6>(A, lda, W, ldw, C, ldc, M, N, K, bias, nc, best_c, vec, stream);
-    if (best_tr == 5) return launch_tile<5>(A, lda, W, ldw, C, ldc, M, N, K, bias, nc, best_c, vec, stream);
-    if (best_tr == 4) return launch_tile<4>(A, lda, W, ldw, C, ldc, M, N, K, bias, nc, best_c, vec, stream);
-    return launch_tile<2>(A, lda, W, ldw, C, ldc, M, N, K, bias, nc, best_c, vec, stream);
+    const TilePick t = pick_tile(M, N, K, vec);
+    switch (t.tr) {
+        case 2: return launch_tile<2>(A, lda, W, ldw, C, ldc, M, N, K, bias, nc, t.c, vec, stream);
+        case 4: return launch_tile<4>(A, lda, W, ldw, C, ldc, M, N, K, bias, nc, t.c, vec, stream);
+        case 5: return launch_tile<5>(A, lda, W, ldw, C, ldc, M, N, K, bias, nc, t.c, vec, stream);
+        case 6: return launch_tile<6>(A, lda, W, ldw, C, ldc, M, N, K, bias, nc, t.c, vec, stream);
+        case 7: return launch_tile<7>(A, lda, W, ldw, C, ldc, M, N, K, bias, nc, t.c, vec, stream);
+        default: return launch_tile<8>(A, lda, W, ldw, C, ldc, M, N, K, bias, nc, t.c, vec, stream);
+    }
 }
