@@ -76,17 +76,20 @@ constexpr int few_registers(int rows) { return rows <= 2 ? rows : rows <= 4 ? 4 
 // rows, a quarter, where 256 blocks are left and two of them find room on an SM. A block's start, its cluster's meeting and its end cost as much as
 // four chunks of weights do. Cold, back to back, us with an eighth / now, 1, 4 and 8 rows: 16,384 x 2,048 26.5, 35, 38 / 23.7, 25.6, 29.5;
 // 128,256 x 2,048 162, 233, 255 / 151, 164, 202; 28,672 x 4,096 91, 131, 142 / 82, 94, 111. Three blocks to a K of 32 chunks (6,144 x 4,096)
-// lose from three rows on: 32.5 / 39 at eight. A last wave that is nearly empty takes back more than that: where the longer blocks would fill less
-// than 0.7 of their waves K stays in eighths, or in the next smaller part (two rows, us, eighths / longer: 6,144 x 8,192, 1.3 waves, 39.3 / 46.5;
-// 11,008 x 8,192, 1.2 waves of halves, 72.4 / 80.6; 22,016 x 2,560, 1.2 waves, 44.1 / 47.8; at 0.7 to 0.8 equal within 2 %).
+// lose from three rows on: 32.5 / 39 at eight. With one and two rows a last wave that is nearly empty takes back more than that: where the
+// longer blocks would fill less than 0.7 of their waves K stays in eighths, or in the next smaller part (two rows, us, eighths / longer:
+// 6,144 x 8,192, 1.3 waves, 39.3 / 46.5; 11,008 x 8,192, 1.2 waves of halves, 72.4 / 80.6; 22,016 x 2,560, 1.2 waves, 44.1 / 47.8; just above
+// one wave, as at 0.7 to 0.8, they gain or are equal). From three rows on they gain there, too (11,008 x 4,096, 1.2 waves, at 4 and 8 rows 53, 60 / 44, 51).
 //
-// Stages of a warp's ring: two, and three for three and four rows whose blocks did not get longer and fill at most two waves: there a warp's
-// latency is not hidden by others. Three / two, us, 4 rows: 3,072 x 1,024 5.5 / 6.2, 1,024 x 8,960 16.1 / 19.6, 896 x 14,336 22 / 27; many
-// waves 49,152 x 1,280 67.3 / 65.1. One and two rows have three blocks an SM, five and more a lane's two rows: two stages there.
+// Stages of a warp's ring: two, and three for three and four rows whose blocks did not get longer, where that leaves two blocks an SM and at most two
+// waves, or one block an SM and at most 120 blocks (clusters of eight one to an SM do not find the last places): there a warp's latency is
+// not hidden by others. Three / two, us, 4 rows: 3,072 x 1,024 5.5 / 6.2, 1,024 x 8,960 16.1 / 19.6, 896 x 14,336 22 / 27; beyond, 49,152 x 1,280
+// 67.3 / 65.1, 1,024 x 11,008 32.9 / 20.8, 4,100 x 14,336 109 / 60. One and two rows have three blocks an SM, five and more a lane's two rows:
+// two stages there.
 struct FewPlan { int chunks, stages; };
-inline double few_waves(int mb, int chunks, long long blocks) {        // on 148 SMs
-    const int room = (int)(227 * 1024 / (few_smem(mb, chunks, 2) + 1024));
-    return (double)blocks / (148.0 * (room < few_blocks(mb) ? room : few_blocks(mb)));
+inline int few_resident(int mb, int chunks, int stages) {
+    const int room = (int)(227 * 1024 / (few_smem(mb, chunks, stages) + 1024));
+    return room < few_blocks(mb) ? room : few_blocks(mb);
 }
 inline FewPlan few_plan(int rows, long long row_blocks, int nc) {
     const int least = ((nc + 7) / 8 + 3) / 4 * 4, mb = few_registers(rows);
@@ -94,11 +97,13 @@ inline FewPlan few_plan(int rows, long long row_blocks, int nc) {
     for (int c = 1; c <= (rows <= 2 ? 4 : 2); c *= 2) {
         const int q = (nc + c - 1) / c;
         if (q <= least || q % 4 != 0 || nc % q != 0 || row_blocks * c < 256 || few_smem(mb, q, 2) > 112 * 1024) continue;
-        const double waves = few_waves(mb, q, row_blocks * c);
-        if (waves <= 1.0 || waves >= 0.7 * std::ceil(waves)) return {q, 2};
+        const double waves = (double)(row_blocks * c) / (148.0 * few_resident(mb, q, 2));
+        if (rows > 2 || waves <= 1.05 || waves >= 0.7 * std::ceil(waves)) return {q, 2};
     }
+    if (mb != 4) return {least, 2};
+    const int chunks = least < nc ? least : nc;
     const long long blocks = row_blocks * ((nc + least - 1) / least);
-    const bool deep = mb == 4 && blocks <= 2 * 148 * few_blocks(mb) && few_smem(mb, least < nc ? least : nc, 3) <= FEW_SMEM_MOST;
+    const bool deep = few_smem(mb, chunks, 3) <= FEW_SMEM_MOST && blocks <= (few_resident(mb, chunks, 3) >= 2 ? 2 * 2 * 148 : 120);
     return {least, deep ? 3 : 2};
 }
 // Whether a block finds room for its chunks' sums: it does up to K = 61,440 at 5 to 8 rows, 131,072 at 3 and 4, 548,864 at one.
