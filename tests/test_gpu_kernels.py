@@ -1040,13 +1040,13 @@ def test_gemm_f32_few_rows_waves():
             assert torch.equal(out, want[:M]), (M, N, Kd)
 
 
-@pytest.mark.parametrize("N,Kd", [(500, 4612), (500, 5120), (1024, 4100), (2048, 5000), (3200, 4100), (3204, 4100), (3072, 16512), (3076, 16388)])
+@pytest.mark.parametrize("N,Kd", [(500, 4612), (764, 4992), (768, 4612), (500, 5120), (1024, 4100), (2048, 5000), (3200, 4100), (3204, 4100), (3072, 16512), (3076, 16388)])
 def test_gemm_f32_rows_by_eights(N, Kd):
     """On both sides of the lines between rows taken eight at a time and the tiles: the bits of a product of 40 rows, and as many launches
     counted as there are."""
     from vllm_oxide_b200 import kernels
     pieces = kernels._fn("gemm_f32", "vob_gemm_f32_launches", [kernels._I] * 3)
-    narrow = N < 1024 and Kd < 4993 or N > 3072 and Kd > 16384
+    narrow = N < 768 and Kd < 4993 or N > 3072 and Kd > 16384
     g = torch.Generator().manual_seed(N + Kd)
     a, w = torch.randn(40, Kd, generator=g).to(DEV), torch.randn(N, Kd, generator=g).to(DEV)
     want = torch.empty(40, N, device=DEV)

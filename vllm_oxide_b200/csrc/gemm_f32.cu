@@ -497,13 +497,13 @@ bool few_rows(int M, int K) {
 // 8,192 x 8,192, whose weights come from memory every time, 116, 146, 189, 218 / 184; 500 x 5,120 19, 23, 30, 33 / 23. Three eights gain only
 // where the tiles are at their worst, with 24 to 50 clusters of eight blocks, and where L2 keeps the weights: 1,024 x 6,144 at 17 and 24 rows 42, 46 /
 // 46 (39 with the weights in L2), 3,072 x 6,144 70, 85 / 71. Under 40 chunks the last block of a K has little to do, and a narrow N goes to
-// the tiles (500 x 4,612 at 16 rows 24.6 / 23.0); beyond 128 a block of eight rows has its SM to itself (3,584 x 18,944 at 16 rows 245 / 218,
+// the tiles (500 x 4,612 at 16 rows 24.6 / 23.0, 896 x 4,864 24.6 / 29.2); beyond 128 a block of eight rows has its SM to itself (3,584 x 18,944 at 16 rows 245 / 218,
 // 2,560 x 18,944 0.86 of the tiles' time). A decode step of 12 requests at 1B sizes 3,590 -> 2,660 us.
 bool by_eights(int M, int N, int K) {
     const int nc = (K + CHUNK - 1) / CHUNK;
     const double w_bytes = 4.0 * N * K;
     if (M <= 8 || M > 24 || nc <= 32 || !few_fits(8, (N + FEW_N - 1) / FEW_N, nc)) return false;
-    if (M <= 16) return w_bytes <= 320e6 && (nc >= 40 || N >= 1024) && (nc <= 128 || N <= 3072);
+    if (M <= 16) return w_bytes <= 320e6 && (nc >= 40 || N >= 768) && (nc <= 128 || N <= 3072);
     return N >= 1536 && N <= 3200 && w_bytes > 33e6 && w_bytes <= 70e6;
 }
 
