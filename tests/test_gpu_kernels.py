@@ -1063,9 +1063,9 @@ def test_gemm_f32_rows_by_eights(N, Kd):
 
 @pytest.mark.parametrize("N,Kd,M,tr,c", [
     (65, 516, 17, 2, 1), (65, 1028, 17, 2, 8), (1541, 516, 65, 4, 1), (65, 1028, 177, 4, 8), (8201, 516, 65, 5, 1), (65, 1028, 300, 5, 8),
-    (4101, 516, 350, 6, 1), (65, 1028, 350, 6, 8), (3101, 516, 640, 7, 1), (501, 1028, 97, 7, 8), (8201, 516, 225, 8, 1), (501, 1028, 113, 8, 8),
-    (65, 130, 17, 2, 1), (65, 1030, 17, 2, 8), (1541, 130, 65, 4, 1), (65, 1030, 130, 4, 8), (1541, 130, 130, 5, 1), (65, 1030, 300, 5, 8),
-    (8201, 130, 81, 6, 1), (65, 1030, 350, 6, 8), (3101, 130, 640, 7, 1), (65, 1030, 640, 7, 8), (12301, 130, 350, 8, 1), (501, 1030, 113, 8, 8)])
+    (4101, 516, 350, 6, 1), (501, 1028, 81, 6, 8), (3101, 516, 640, 7, 1), (501, 1028, 97, 7, 8), (8201, 516, 225, 8, 1), (501, 1028, 113, 8, 8),
+    (65, 130, 17, 2, 1), (65, 1030, 17, 2, 8), (1541, 130, 65, 4, 1), (65, 1030, 130, 4, 8), (4101, 130, 65, 5, 1), (65, 1030, 300, 5, 8),
+    (8201, 130, 81, 6, 1), (201, 1030, 177, 6, 8), (3101, 130, 640, 7, 1), (501, 1030, 97, 7, 8), (12301, 130, 350, 8, 1), (501, 1030, 113, 8, 8)])
 def test_gemm_f32_tile_choice(N, Kd, M, tr, c):
     """Every tile height with and without a shared K, operands that come by 16 and by 4 bytes: the choice that the rule makes at these sizes, and the
     bits that the few-row kernel or, where operands come by 4 bytes, tiles of 32 rows give."""

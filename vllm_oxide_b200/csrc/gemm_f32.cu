@@ -448,23 +448,23 @@ int launch_tile(const float* A, long long lda, const float* W, long long ldw, fl
 // One block to a tile: for grids of at most 48 and 74 blocks, which find an SM each beside their neighbours', for 1, 2, 3 and 4 blocks on the fullest of
 // 148 SMs, and per block beyond. Eight to a tile, a segment of K each: for at most 4, 6, 8, 10, 12, 15, 23, 32, 42, 48 and 64 clusters, and per 16
 // clusters beyond. `by4`: how much longer both take where operands come by 4 bytes. What is added is a block's start and the cluster's sums. In
-// the long run a row costs alike at 64 rows and more (0.93 to 1.03 us a chunk, 16 rows and SM), 1.36 at 32: rows that are not there, waves and
+// the long run a row costs alike at 64 rows and more (0.93 to 1.01 us a chunk, 16 rows and SM), 1.37 at 32: rows that are not there, waves and
 // idle SMs decide.
 // The numbers are fitted to 3,125 sizes (N 64 to 32,000, K 96 to 14,336, 17 to 4,096 rows), where every height with and without a shared K was timed
-// twice: back to back, and with another kernel in between, which places small grids otherwise. Over both the choice takes 1.015 and 1.034 of the
+// twice: back to back, and with another kernel in between, which places small grids otherwise. Over both the choice takes 1.014 and 1.033 of the
 // best one's time on average; 128, 64 and 32 rows by rows and waves took 1.10 and 1.13, all six by rows and waves 1.09 and 1.10. Against those three
-// heights 24 and 15 sizes lose more than 2 %, all but a few of small grids. us, those three / now: 64 x 516 at 160 rows 17.5 / 17.5, 3,072 x 516 at 81
+// heights 20 and 18 sizes lose more than 2 %, all but a few of small grids. us, those three / now: 64 x 516 at 160 rows 17.5 / 17.5, 3,072 x 516 at 81
 // 32.4 / 32.4, 16,384 x 2,048 at 72, 300, 450 and 2,048 rows 242, 563, 941, 3,262 / 170, 563, 799, 3,262; 2,048 x 8,192 at 97 and 450 126, 494 /
 // 115, 494; 8,192 x 4,096 at 300 610 / 610; 2,048 x 2,050 at 260 159 / 140.
 struct TilePick { int tr, c; };
 TilePick pick_tile(int M, int N, int K, bool vec) {
     static const struct { int tr; float one[7], shared[12], by4[2]; } times[] = {
-        {2, {3.57f, 4.51f, 7.15f, 7.67f, 10.0f, 11.2f, 2.73f}, {4.66f, 3.76f, 4.65f, 5.16f, 6.28f, 6.25f, 9.21f, 11.2f, 9.7f, 12.3f, 11.9f, 2.38f}, {1.52f, 1.4f}},
-        {4, {5.24f, 5.91f, 10.3f, 11.5f, 12.8f, 16.8f, 3.87f}, {5.39f, 5.16f, 5.68f, 9.14f, 8.9f, 9.39f, 12.6f, 12.2f, 10.6f, 12.3f, 18.3f, 3.69f}, {1.4f, 1.28f}},
-        {5, {8.48f, 7.85f, 8.05f, 10.3f, 15.4f, 19.5f, 5.13f}, {6.0f, 7.22f, 7.23f, 7.99f, 7.81f, 7.01f, 9.7f, 10.1f, 15.8f, 18.5f, 22.1f, 4.87f}, {1.27f, 1.24f}},
-        {6, {8.49f, 9.84f, 10.1f, 11.5f, 17.7f, 22.0f, 5.65f}, {7.05f, 9.26f, 7.99f, 8.95f, 9.27f, 10.5f, 13.4f, 12.3f, 18.8f, 22.8f, 26.3f, 5.67f}, {1.27f, 1.13f}},
-        {7, {8.07f, 9.7f, 11.2f, 13.6f, 20.7f, 26.2f, 6.75f}, {7.22f, 9.68f, 9.29f, 9.78f, 10.4f, 11.0f, 15.7f, 14.5f, 21.2f, 27.5f, 29.1f, 6.15f}, {1.32f, 1.13f}},
-        {8, {8.64f, 10.5f, 13.4f, 14.9f, 23.5f, 29.7f, 7.44f}, {8.76f, 9.88f, 9.67f, 12.6f, 11.4f, 13.1f, 15.5f, 16.3f, 23.5f, 28.6f, 31.4f, 6.72f}, {1.32f, 1.14f}}};
+        {2, {3.27f, 4.51f, 7.15f, 7.67f, 10.0f, 10.5f, 2.73f}, {4.66f, 4.08f, 4.91f, 5.17f, 5.54f, 6.25f, 9.21f, 11.4f, 9.7f, 12.3f, 12.2f, 2.38f}, {1.44f, 1.4f}},
+        {4, {5.23f, 5.53f, 10.3f, 10.6f, 12.2f, 15.8f, 3.87f}, {5.4f, 5.16f, 5.68f, 9.46f, 7.72f, 9.58f, 12.6f, 12.2f, 10.3f, 12.6f, 16.9f, 3.69f}, {1.41f, 1.3f}},
+        {5, {7.91f, 7.85f, 7.85f, 10.1f, 15.1f, 19.5f, 5.07f}, {6.0f, 7.22f, 7.23f, 7.29f, 7.77f, 7.01f, 8.95f, 8.63f, 15.8f, 17.2f, 20.4f, 4.78f}, {1.27f, 1.25f}},
+        {6, {8.39f, 9.84f, 10.1f, 11.9f, 16.5f, 21.5f, 5.65f}, {7.05f, 9.26f, 8.11f, 8.95f, 9.24f, 11.1f, 12.9f, 12.5f, 17.5f, 20.9f, 25.4f, 5.67f}, {1.27f, 1.13f}},
+        {7, {8.07f, 9.7f, 11.4f, 13.6f, 20.7f, 26.4f, 6.7f}, {7.22f, 9.38f, 8.67f, 9.78f, 11.2f, 11.0f, 15.7f, 15.5f, 20.0f, 25.3f, 27.8f, 6.24f}, {1.32f, 1.15f}},
+        {8, {8.64f, 10.5f, 14.9f, 14.9f, 23.5f, 29.7f, 7.44f}, {8.76f, 9.88f, 8.78f, 12.6f, 11.8f, 13.1f, 15.9f, 16.3f, 23.3f, 27.9f, 30.2f, 6.76f}, {1.33f, 1.14f}}};
     static const int clusters[] = {4, 6, 8, 10, 12, 15, 23, 32, 42, 48, 64};
     const int nc = (K + CHUNK - 1) / CHUNK;
     TilePick best = {8, 1};
