@@ -9,12 +9,13 @@
 // rounds more often: relative error against 64 bits on normal values 8.1e-7 and 1.6e-6 at K = 2,048 and 8,192, here 1.6e-7 and 1.7e-7.)
 //
 // Two kernels:
-//  * few rows (decode steps: M <= 8, M <= 16 while K is at most 4,096, by eights beyond): bound by reading W once, 6.9 TB/s at M = 1, 5.2 at 8 and 2.7 at
-//    16 on 128,256 x 2,048, 5.5, 4.5 and 2.4 TB/s on 16,384 x 2,048 back to back (64 x 64 tiles, which served every M before: 1.06 and 0.6 TB/s; 0.1 TB/s on 2,048 x 8,192, now 2.6). A thread has one or two weight rows and a chunk, all rows of A
+//  * few rows (decode steps: M <= 8, M <= 16 while K is at most 4,096, eight at a time where `by_eights` says): bound by reading W once, 6.9 TB/s at
+//    M = 1, 5.2 at 8 and 2.7 at 16 on 128,256 x 2,048, 5.5, 4.5 and 2.4 TB/s on 16,384 x 2,048 back to back (64 x 64 tiles, which served every M
+//    before: 1.06 and 0.6 TB/s; 0.1 TB/s on 2,048 x 8,192, now 3.6 at eight rows). A thread has one or two weight rows and a chunk, all rows of A
 //    in its registers' sums; weights arrive by cp.async into a ring per warp, so that no barrier of the block stands in the stream.
 //  * tiles (everything else): bound by what two warps a scheduler can issue: the FMA units are busy 60 % of the cycles, shared memory
 //    48 %, and a warp waits for the result in front or for a register's read most of the rest. 8 x 8 outputs a thread from
-//    shared memory: 40 to 42 TFLOP/s on 16,384 x 2,048 at M = 1,250 and 2,048 (33 and 34 before), 31 TFLOP/s on 2,048 x 8,192 at M = 128 (6).
+//    shared memory: 40 to 42 TFLOP/s on 16,384 x 2,048 at M = 1,250 and 2,048 (33 and 34 before), 33 TFLOP/s on 2,048 x 8,192 at M = 128 (6).
 // Both multiply and add pairs of k in one instruction (fma.rn.f32x2, each half rounded as fmaf rounds it): single FMAs
 // reach half the rate on this GPU (a tile kernel of 8 x 8 outputs a thread: 37 TFLOP/s with fmaf).
 #include "common.cuh"

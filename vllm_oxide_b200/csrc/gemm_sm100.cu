@@ -23,22 +23,19 @@
 // order (a fixed order: the result does not depend on timing) and writes C. Nothing goes through
 // global memory and nothing needs resetting between launches.
 //
-// Tiles of 16 tokens (decode steps of up to 16 requests) do the products another way. Measured on
-// this GPU: a tcgen05.mma costs the tensor pipe some 160 clocks however few tokens it has (its A
-// operand, 128 weight rows x 32 bytes, is fetched from shared memory at about 32 bytes a clock), so a
-// stage of 64 k took 0.33 us of products whatever the token count, and the product phase of a block
-// whose weights had all been prefetched was as long as its whole epilogue. For these tiles the four
-// epilogue warps therefore do the products themselves: 32 weight rows each, fragments by ldmatrix
+// Tiles of 16 tokens (decode steps of up to 16 requests) do the products another way: the four
+// epilogue warps do them themselves, 32 weight rows each, fragments by ldmatrix
 // straight from the TMA ring's swizzled tiles, mma.sync.m16n8k16 with float32 accumulators in
 // registers (one 8-token half only when the step has at most 8 tokens); no tensor memory, no issuing
 // threads, and the per-token scale's round trip to L2 hides behind the product loop. The rest of
 // the kernel (TMA ring, cluster split of K, epilogues) is the same. A decode step at batch 1 / 8 / 16
-// went from 0.750 / 0.858 / 1.002 to 0.733 / 0.848 / 0.966 ms. (Two or four accumulator sets to
+// went from 0.750 / 0.858 / 1.002 to 0.733 / 0.848 / 0.966 ms, against tcgen05.mma issued by `lane == 0`. (Two or four accumulator sets to
 // shorten the chain of dependent products cost registers, a second block no longer fitted the SM,
 // and the step took 0.88 / 1.04 ms: dropped.)
-// (With elected issuers a 128 x 16 x 16 product takes 42 clocks, and tcgen05 for these tiles, or eight multiplying warps instead of four, give the
-// same step within 1 %: 662 us at batch 1 this way, 666 and 668 those. With the weights in L2 gate/up takes 10.0 us, from memory
-// 12.3, whichever multiplies: the bytes in flight set the pace.)
+// With elected issuers tcgen05 for these tiles, or eight multiplying warps instead of four, give the same step within 1 %: 662 us at
+// batch 1 this way, 666 and 668 those; the multiply phase is not what bounds them. With the weights in L2 / from memory the
+// 1B sizes' products take, us: QKV 4.6 / 4.7, O 4.0 / 4.2, gate/up 10.0 / 12.3, down 6.8 / 8.8. Bytes in flight cost the two long ones a
+// quarter; QKV and O cost what their own chain takes between the wait and the exit.
 //
 // Every wait on an mbarrier is bounded (two seconds): on expiry the block raises the error flag,
 // stops issuing work, frees its tensor memory and returns; the host turns the flag into an
@@ -248,12 +245,11 @@ gemm_sm100_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_consta
             }
         }
     } else if (!MS && (warp == 1 || warp >= 6)) {
-        // ISSUERS issuing threads. One thread gets a small tcgen05.mma through about every 42 clocks
-        // (and a commit more per stage), and an instruction of 128 x 16 x 16 consumes only 4 KB of weights: a
-        // single issuer just about keeps pace with HBM, and its chain is what a block with few
-        // k-blocks waits for. Each thread takes its share of every stage's K steps into an
-        // accumulator of its own; the epilogue adds them in a fixed order. (Measured on a decode
-        // step of 8 rows: two issuers +2.5 %, four +2.7 %.)
+        // ISSUERS issuing threads, each with its share of every stage's K steps and an accumulator of its
+        // own; the epilogue adds them in a fixed order. One would do: an elected thread gets a product of 128 x 16 x 16 through every
+        // 42 clocks and one of 128 x 64 x 16 every 51, 4 KB of weights each, three to four times HBM's rate over 148 SMs. (Two were
+        // +2.5 % on a decode step of 8 rows, four +2.7 %, while `lane == 0` issued and tiles of 16 tokens came this way, too.) A step
+        // of 24 and 32 rows, 1B sizes, us, two / one: 859 to 872 and 930 / 862 to 865 and 923 to 936.
         if (elect_one()) {
             constexpr uint32_t idesc = umma_idesc(BT);
             constexpr int KSTEPS = BK / UMMA_K / ISSUERS;
@@ -915,12 +911,18 @@ VOB_EXPORT int vob_gemm_sm100_pick_splits(int T, int N, int K, int num_sms) {
     int bt = pick_bt(T);
     int tiles = ((N + BM - 1) / BM) * ((T + bt - 1) / bt);
     int total_kb = (K + BK - 1) / BK;
+    // From 75 tiles on K is not shared. Cold, back to back, us at 1, 8 and 32 rows, one / two / three blocks to a tile: 9,600 x 2,048 (75 tiles) 9.5, 9.7, 11.4 /
+    // 9.2, 10.3, 12.6 / 8.6, 9.1, 10.8; 11,264 x 4,096 (88) 18.8, 19.3, 21.2 / 16.6, 18.5, 21.3 / 16.7, 17.3, 18.9; 12,288 x 2,048 (96) 10.4, 10.6, 12.3 / 10.8, 11.3, 14.0;
+    // 14,336 x 4,096 (112) 21.8, 22.3, 24.1 / 20.3, 21.2, 23.3. So two are no better at K = 2,048, and some at 4,096; three would gain 3 to 11 % up
+    // to 88 tiles and lose beyond.
     if (T > 64 || tiles * 2 > num_sms) return 1;
-    // 1.6 blocks an SM where the tiles allow it (two find room): what an SM gets of the bandwidth follows the bytes it has in flight. With one
+    // 1.6 blocks an SM where the tiles allow it (two find room; eight blocks to a tile at most, so O and down of the 1B sizes keep their 128
+    // blocks): what an SM gets of the bandwidth follows the bytes it has in flight. With one
     // at most, the 8B sizes' QKV ran in 144 blocks and O and down in 128. A decode step, us, one / 1.3 / 1.6 an SM: 8B, 4 requests 3,170 /
     // 2,918 / 2,885; 3B, 4 requests 1,655 / 1,608 / 1,599; 1B, 1, 8 and 24 requests 662, 728, 880 / 658, 723, 868 / 658, 724, 868. Fewer blocks
     // lose: QKV of the 1B sizes with 3 instead of 6 to a tile 662 -> 692, down with 4 instead of 8 712. So do two an SM, which leave the next
-    // kernel no room to start beside this one: 8B 3,203, 3B 1,707.
+    // kernel no room to start beside this one: 8B 3,203, 3B 1,707. Shorter partial sums: the float32 result's error against 64 bits is smaller
+    // at all of 63 sizes and rows measured, 0.66 of what it was on average (4,096 x 14,336 at 8 rows 3.8e-6 -> 2.1e-6).
     int want = num_sms * 16 / 10 / tiles;
     if (want > 8) want = 8;                                           // the portable cluster size
     int max_splits = total_kb / 4 > 0 ? total_kb / 4 : 1;             // at least 4 k-blocks (256 of K) per split
