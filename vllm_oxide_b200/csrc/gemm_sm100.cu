@@ -57,8 +57,8 @@ constexpr int NTHREADS_FEW = 192 + 32 * (ISSUERS - 1);
 // kind::f16 instruction descriptor of this file's products: M = 128 weight rows, N = n tokens, both K-major.
 __host__ __device__ constexpr uint32_t umma_idesc(int n) { return umma_idesc_bf16(BM, n, false); }
 
-// For tiles of 16 tokens the products are done by mma.sync from the TMA ring (see the kernel's header
-// comment below): 8 x 8 matrices of 16-bit elements from shared memory, four at a time, and the
+// For tiles of 16 tokens the products are done by mma.sync from the TMA ring (why: see the file's
+// header): 8 x 8 matrices of 16-bit elements from shared memory, four at a time, and the
 // 16 x 8 x 16 product with float32 accumulators in registers.
 __device__ __forceinline__ void ldmatrix_x4(uint32_t (&r)[4], uint32_t addr) {
     asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0, %1, %2, %3}, [%4];" : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(addr));
@@ -67,11 +67,6 @@ __device__ __forceinline__ void mma_16816(float (&c)[4], const uint32_t (&a)[4],
     asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, {%0, %1, %2, %3};"
                  : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3]) : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
 }
-#ifdef VOB_FEW16_TCGEN05
-constexpr bool FEW16_MMA_SYNC = false;
-#else
-constexpr bool FEW16_MMA_SYNC = true;
-#endif
 
 template <typename OutT> __device__ __forceinline__ void store_out(OutT* p, float v);
 template <> __device__ __forceinline__ void store_out<float>(float* p, float v) { *p = v; }
@@ -170,7 +165,7 @@ gemm_sm100_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_consta
     constexpr int A_BYTES = BM * BK * 2;
     // Tiles of 16 tokens: the four epilogue warps do the products themselves with mma.sync, reading the
     // ring's tiles with ldmatrix; no tensor memory, no issuing threads (see the note above the kernel).
-    constexpr bool MS = BT == 16 && FEW16_MMA_SYNC;
+    constexpr bool MS = BT == 16;
     constexpr int PRE = BT >= 64 ? 12 : (BT >= 32 ? 8 : 4);   // tokens per block whose rotation is worked out ahead
     pdl_launch_dependents();
     extern __shared__ unsigned char smem_raw[];
