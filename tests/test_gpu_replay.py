@@ -377,3 +377,41 @@ def test_trace_run_program(tmp_path):
                 assert max_rel_diff(torch.from_numpy(data[r].copy()), ref[base + w]) <= TOL[torch.float32]
                 r += 1
             pos[e["id"]] = base + len(e["tokens"])
+
+
+def test_mixed_steps_repeat_to_the_bit():
+    """Prompts of very different lengths in portions beside decoded tokens, at the layer sizes of a 3B model (head size 128, the two-SM gate/up product, K
+    shared over five and eight blocks): pass after pass the same logits and tokens. With issuing threads chosen by elect.sync
+    one pass in twelve of such a call gave other logits."""
+    import torch
+    from vllm_oxide_b200 import config as C
+    from vllm_oxide_b200.engine import LLM, ModelRunner
+    from vllm_oxide_b200.sampling import SamplingParams
+    h, ff, heads, kv, hd, layers, vocab = 3072, 8192, 24, 8, 128, 8, 2048
+    g = torch.Generator(device="cuda").manual_seed(5)
+
+    def mat(rows, cols, std=0.02):
+        return (torch.randn(rows, cols, generator=g, device="cuda") * std).to(torch.bfloat16)
+    w = {"model.embed_tokens.weight": mat(vocab, h, 1.0), "model.norm.weight": torch.ones(h, device="cuda", dtype=torch.bfloat16)}
+    for i in range(layers):
+        p = f"model.layers.{i}."
+        for name, rows, cols in (("self_attn.q_proj", heads * hd, h), ("self_attn.k_proj", kv * hd, h), ("self_attn.v_proj", kv * hd, h),
+                                 ("self_attn.o_proj", h, heads * hd), ("mlp.gate_proj", ff, h), ("mlp.up_proj", ff, h), ("mlp.down_proj", h, ff)):
+            w[p + name + ".weight"] = mat(rows, cols)
+        for name in ("input_layernorm", "post_attention_layernorm"):
+            w[p + name + ".weight"] = torch.ones(h, device="cuda", dtype=torch.bfloat16)
+    cfg = C.LlamaConfig(hidden_size=h, intermediate_size=ff, num_hidden_layers=layers, num_attention_heads=heads, num_key_value_heads=kv, head_dim=hd,
+                        vocab_size=vocab, max_position_embeddings=8192, rms_norm_eps=1e-5, rope_theta=500000.0,
+                        rope_scaling=C.RopeScaling(32.0, 1.0, 4.0, 8192), tie_word_embeddings=True, bos_token_id=1, eos_token_ids=(2,))
+    llm = LLM(ModelRunner(cfg, w, C.EngineConfig(max_batch_tokens=2048, max_seqs=12, max_model_len=3200, block_size=16, num_pages=1400, dtype="bfloat16")))
+    lengths = [130, 2255, 300, 1700, 173, 3000, 530, 400, 1276, 960, 225, 700]
+    pg = torch.Generator().manual_seed(6)
+    prompts = [torch.randint(3, vocab, (n,), generator=pg).tolist() for n in lengths]
+    params = [SamplingParams(max_new_tokens=24, temperature=0.0, stop_token_ids=(), capture_logits=(23,)) for _ in lengths]
+    first = None
+    for n in range(60):
+        outs = llm.generate(prompts, params)
+        got = ([o.token_ids for o in outs], torch.stack([o.logits[23] for o in outs]))
+        if first is None:
+            first = got
+        assert got[0] == first[0] and torch.equal(got[1], first[1]), n

@@ -24,7 +24,7 @@
 //
 // What bounds it: the rows' own phases, one after the other (64 exponentials a row at 16 a clock and SM are 0.27 us of
 // the 0.42 us that a tile takes), and behind them the issue of a tile's products (4 + 4 of 32 clocks of tensor-core
-// work, some 34 each from one elected thread, and two commits); two blocks per SM overlap. Tried and
+// work, some 48 each from one thread, and two commits); two blocks per SM overlap. Tried and
 // measured slower: two threads per row (16 softmax warps per SM), exponentials shared with the
 // FMA pipe by a cubic, separate issuing threads for the two products.
 //
@@ -212,7 +212,7 @@ attn_prefill_sm100_kernel(const __grid_constant__ CUtensorMap map_q, const __gri
         }
     } else if (warp == 1) {
         // ------------------------------------------------------------------ MMA issuer
-        if (elect_one()) {
+        if (lane == 0) {
             constexpr uint32_t idesc_qk = umma_idesc_bf16(BM, BN, false);
             constexpr uint32_t idesc_pv = umma_idesc_bf16(BM, 64, true);          // one 64-wide half of O at a time
             constexpr uint32_t idesc_pv_wide = umma_idesc_bf16(BM, HD, true);

@@ -32,8 +32,8 @@
 // went from 0.750 / 0.858 / 1.002 to 0.733 / 0.848 / 0.966 ms, against tcgen05.mma issued by `lane == 0`. (Two or four accumulator sets to
 // shorten the chain of dependent products cost registers, a second block no longer fitted the SM,
 // and the step took 0.88 / 1.04 ms: dropped.)
-// With elected issuers tcgen05 for these tiles, or eight multiplying warps instead of four, give the same step within 1 %: 662 us at
-// batch 1 this way, 666 and 668 those; the multiply phase is not what bounds them. With the weights in L2 / from memory the
+// Measured with faster (elected) issuers, tcgen05 for these tiles, or eight multiplying warps instead of four, gave the same step within 1 %:
+// 662 us at batch 1 this way, 666 and 668 those; the multiply phase is not what bounds them. With the weights in L2 / from memory the
 // 1B sizes' products take, us: QKV 4.6 / 4.7, O 4.0 / 4.2, gate/up 10.0 / 12.3, down 6.8 / 8.8. Bytes in flight cost the two long ones a
 // quarter; QKV and O cost what their own chain takes between the wait and the exit.
 //
@@ -205,7 +205,7 @@ gemm_sm100_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_consta
     const uint32_t tmem_base = MS ? 0u : *tmem_holder;
 
     if (warp == 0) {
-        if (elect_one()) {
+        if (lane == 0) {
             // Weights are written by no kernel (unless the caller says so), so their loads start at once and overlap whatever
             // still runs before this kernel; the activations are loaded only after the wait.
             if (qa.late_w) pdl_wait();
@@ -241,11 +241,11 @@ gemm_sm100_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_consta
         }
     } else if (!MS && (warp == 1 || warp >= 6)) {
         // ISSUERS issuing threads, each with its share of every stage's K steps and an accumulator of its
-        // own; the epilogue adds them in a fixed order. One would do: an elected thread gets a product of 128 x 16 x 16 through every
-        // 42 clocks and one of 128 x 64 x 16 every 51, 4 KB of weights each, three to four times HBM's rate over 148 SMs. (Two were
-        // +2.5 % on a decode step of 8 rows, four +2.7 %, while `lane == 0` issued and tiles of 16 tokens came this way, too.) A step
-        // of 24 and 32 rows, 1B sizes, us, two / one: 859 to 872 and 930 / 862 to 865 and 923 to 936.
-        if (elect_one()) {
+        // own; the epilogue adds them in a fixed order. A thread gets a product of 128 x 16 x 16 through every
+        // 49 clocks and one of 128 x 64 x 16 every 51, 4 KB of weights each, three times HBM's rate over 148 SMs, so it is not the rate that asks
+        // for two. (Two were +2.5 % on a decode step of 8 rows, four +2.7 %, while tiles of 16 tokens came this way, too. With elected
+        // issuers a step of 24 and 32 rows, 1B sizes, took 859 to 872 and 930 us with two, 862 to 865 and 923 to 936 with one.)
+        if (lane == 0) {
             constexpr uint32_t idesc = umma_idesc(BT);
             constexpr int KSTEPS = BK / UMMA_K / ISSUERS;
             const int w = warp >= 6 ? warp - 5 : 0;
@@ -696,7 +696,7 @@ gemm_sm100_persistent_kernel(const __grid_constant__ CUtensorMap map_w, const __
     pdl_wait(13);
 
     if (warp == 0) {
-        if (elect_one()) {
+        if (lane == 0) {
             uint32_t it = 0;
             bool ok = true;
             for (int tile = blockIdx.x; tile < num_tiles && ok; tile += gridDim.x) {
@@ -713,7 +713,7 @@ gemm_sm100_persistent_kernel(const __grid_constant__ CUtensorMap map_w, const __
             }
         }
     } else if (warp == 1) {
-        if (elect_one()) {
+        if (lane == 0) {
             constexpr uint32_t idesc = umma_idesc(BT);
             uint32_t it = 0, local = 0;
             bool ok = true;

@@ -129,7 +129,7 @@ gemm_sm100_pair_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_c
     if (warp != 0) pdl_wait(15);
 
     if (warp == 0) {
-        if (elect_one()) {
+        if (lane == 0) {
             auto load_w = [&](int m_tile, int kb, int s) {
                 unsigned char* a = tiles + s * stage_bytes;
                 if (rank == 0) mbar_expect_tx(full_bar + s, 2 * stage_bytes);        // both blocks' bytes
@@ -164,7 +164,7 @@ gemm_sm100_pair_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_c
             }
         }
     } else if (warp == 1) {
-        if (rank == 0 && elect_one()) {
+        if (rank == 0 && lane == 0) {
             const uint32_t idesc = umma_idesc_bf16(2 * BMH, bn, false);
             uint32_t local = 0, ph = 0;
             int s = 0;

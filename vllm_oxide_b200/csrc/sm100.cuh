@@ -35,16 +35,10 @@ __device__ __forceinline__ bool mbar_try_wait(uint64_t* bar, uint32_t parity) {
                  : "=r"(ok) : "r"(smem_u32(bar)), "r"(parity) : "memory");
     return ok != 0;
 }
-// True in one lane of a converged warp. The compiler knows that a branch on it holds one thread, which it does not know of
-// `lane == 0`, where a tcgen05 instruction's uniform operands are prepared for every set of active lanes: clocks per product of 128 x N x 16
-// from one thread, lane == 0 / here: A from tensor memory, N = 64 48 / 34; A from shared memory, N = 16 49 / 42, N = 64 51 / 51,
-// N = 128 and 256 67 and 131 (the tensor pipe's rate) either way. Prompt attention at head size 128, 8,192 and 2,048 tokens: 523.5 and
-// 45.3 us before, 496.9 and 43.3 now; head size 64: 371.5 and 34.0, 367.8 and 33.2; a decode step of 32 rows (1B sizes) 962 -> 932 us.
-__device__ __forceinline__ bool elect_one() {
-    uint32_t p;
-    asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(p));
-    return p != 0;
-}
+// The threads that issue tcgen05 and TMA instructions are chosen by `lane == 0`, not by elect.sync. With elect.sync the compiler knows that one thread is
+// left and issues faster (clocks per product of 128 x N x 16, elected / lane == 0: A from tensor memory, N = 64 34 / 48; A from shared memory,
+// N = 16 42 / 49, N = 64 51 / 51; prompt attention at head size 128, 8,192 tokens, 497 / 524 us), but with it one pass in twelve of a 3B serving call
+// (12 prompts of 130 to 3,000 tokens, 24 tokens each) gave other logits than the passes before and after. With lane == 0 none does.
 __device__ __forceinline__ unsigned long long global_ns() {
     unsigned long long t;
     asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
